@@ -1,0 +1,298 @@
+"""The workloads whose speed this repository tracks, through the entry points its users call.
+
+Sizes are those of the Qwen2-0.5B / 1.5B / 7B layers that the benchmark and the tests use, plus odd ones
+in between.  Six kinds of work:
+
+  sq / fp8 / awq   one quantized linear layer (the modules of `llmqrt_b200.linear`), 1 to 4096 tokens
+  attn_decode      one decode step over a ragged KV cache (`flash_attn_with_kvcache`, appending the new token)
+  attn_prefill     prompt attention (`flash_attn_func`)
+  decode / prefill a whole int8 model (`Qwen2Decoder`)
+  block            a whole model assembled from the drop-in modules (`LlamaLikeModel` with AWQ layers)
+"""
+from __future__ import annotations
+
+import math
+
+import torch
+
+from llmqrt_b200 import attention
+from llmqrt_b200.fused_utils import FusedGateUpMLP, fuse_linears
+from llmqrt_b200.linear import (FP8DynamicLinear, FP8StaticLinear, SqW8A8BBF16OBF16PerChannel,
+                                SqW8A8BBF16OBF16PerTensor, WQLinear_GEMM)
+from llmqrt_b200.nonlinear import LlamaLikeBlock, LlamaLikeModel, RMSNorm
+from llmqrt_b200.qwen2 import Qwen2Config, Qwen2Decoder
+
+# layers, hidden, intermediate, query heads, KV heads, head dimension
+MODELS = {
+    "qwen2-0.5b": (24, 896, 4864, 14, 2, 64),
+    "qwen2-1.5b": (28, 1536, 8960, 12, 2, 128),
+    "qwen2-7b": (28, 3584, 18944, 28, 4, 128),
+}
+VOCAB = 152064
+DTYPES = {"fp16": torch.float16, "bf16": torch.bfloat16}
+
+
+def listed():
+    return [
+        # the smallest call: one int8 projection for a handful of sequences
+        {"name": "sq_m16", "kind": "sq", "per_channel": True, "M": 16, "N": 4864, "K": 896, "dtype": "fp16"},
+        # per-tensor scales (the layer the reference's method registry serves), a short prompt of odd length
+        {"name": "sq_tensor_m333", "kind": "sq", "per_channel": False, "M": 333, "N": 3584, "K": 3584, "dtype": "fp16"},
+        # fp8 decode of a batch: dynamic per-token scales
+        {"name": "fp8_token_m64", "kind": "fp8", "mode": "token", "M": 64, "N": 4864, "K": 896},
+        # fp8 prefill: dynamic per-tensor scale
+        {"name": "fp8_tensor_m4096", "kind": "fp8", "mode": "tensor", "M": 4096, "N": 4864, "K": 896},
+        # 4-bit weights: a single sequence, a mid-sized odd batch (speculative or chunked decode), a prompt
+        {"name": "awq_m1", "kind": "awq", "M": 1, "N": 17920, "K": 1536, "G": 128},
+        {"name": "awq_m100", "kind": "awq", "M": 100, "N": 1536, "K": 8960, "G": 128},
+        {"name": "awq_m2048", "kind": "awq", "M": 2048, "N": 17920, "K": 1536, "G": 128},
+        # 32 sequences of 512 to 8192 cached tokens
+        {"name": "attn_decode_b32", "kind": "attn_decode", "B": 32, "lo": 512, "hi": 8192, "Hq": 28, "Hkv": 4, "d": 128,
+         "dtype": "fp16"},
+        # four prompts of 2048 tokens
+        {"name": "attn_prefill_4x2048", "kind": "attn_prefill", "B": 4, "S": 2048, "Hq": 28, "Hkv": 4, "d": 128,
+         "dtype": "fp16", "causal": True},
+        # the headline: one greedy step of 64 sequences
+        {"name": "decode_7b_b64", "kind": "decode", "model": "qwen2-7b", "B": 64, "ctx": 1024},
+        # the prompts of four sequences through the whole model
+        {"name": "prefill_7b_4x2048", "kind": "prefill", "model": "qwen2-7b", "B": 4, "S": 2048},
+        # interactive use of a 4-bit model: one sequence, one token
+        {"name": "block_awq_b1", "kind": "block", "model": "qwen2-1.5b", "B": 1, "ctx": 700},
+    ]
+
+
+def _log_int(rng, lo, hi):
+    return max(lo, min(hi, int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))))
+
+
+def _linear_shape(rng, n_mult, k_mult):
+    """(N, K): a projection of one of the models, or sizes of no model in particular."""
+    if rng.random() < 0.5:
+        _, h, i, hq, hkv, d = MODELS[rng.choice(sorted(MODELS))]
+        return rng.choice([(hq * d + 2 * hkv * d, h), (h, hq * d), (2 * i, h), (i, h), (h, i)])
+    return _log_int(rng, 128, 16384) // n_mult * n_mult, _log_int(rng, 256, 12288) // k_mult * k_mult
+
+
+def draw(rng):
+    kind = rng.choice(["sq", "fp8", "awq", "attn_decode", "attn_prefill", "decode", "prefill", "block"])
+    if kind == "sq":
+        N, K = _linear_shape(rng, 8, 16)
+        return {"kind": kind, "per_channel": rng.random() < 0.6, "M": _log_int(rng, 1, 4096), "N": N, "K": K,
+                "dtype": rng.choice(["fp16", "bf16"])}
+    if kind == "fp8":
+        N, K = _linear_shape(rng, 8, 16)
+        return {"kind": kind, "mode": rng.choice(["token", "token", "tensor", "static"]), "M": _log_int(rng, 1, 4096),
+                "N": N, "K": K}
+    if kind == "awq":
+        N, K = _linear_shape(rng, 8, 128)
+        return {"kind": kind, "M": _log_int(rng, 1, 4096), "N": N, "K": K, "G": rng.choice([128, 128, 64, 32])}
+    model = rng.choice(sorted(MODELS))
+    _, _, _, hq, hkv, d = MODELS[model]
+    if kind == "attn_decode":
+        hi = _log_int(rng, 64, 8192)
+        return {"kind": kind, "B": _log_int(rng, 1, 64), "lo": max(1, int(hi * rng.uniform(0.05, 1.0))), "hi": hi, "Hq": hq,
+                "Hkv": hkv, "d": d, "dtype": rng.choice(["fp16", "bf16"])}
+    if kind == "attn_prefill":
+        S = _log_int(rng, 16, 4096)
+        return {"kind": kind, "B": _log_int(rng, 1, max(1, min(16, 8192 // S))), "S": S, "Hq": hq, "Hkv": hkv, "d": d,
+                "dtype": rng.choice(["fp16", "bf16"]), "causal": rng.random() < 0.85}
+    if kind == "decode":
+        return {"kind": kind, "model": model, "B": _log_int(rng, 1, 64), "ctx": _log_int(rng, 16, 1500)}
+    if kind == "prefill":
+        S = _log_int(rng, 16, 2048)
+        return {"kind": kind, "model": model, "B": _log_int(rng, 1, max(1, min(16, 8192 // S))), "S": S}
+    return {"kind": kind, "model": rng.choice(["qwen2-0.5b", "qwen2-1.5b"]), "B": _log_int(rng, 1, 8),
+            "ctx": _log_int(rng, 8, 1500)}
+
+
+# ---------------------------------------------------------------------------------------------
+# preparation: weights, inputs and caches from the seed alone
+# ---------------------------------------------------------------------------------------------
+def _gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def _activations(g, M, K, dtype):
+    """N(0, 1) with one channel in a hundred twenty times larger (the outliers SmoothQuant is about)."""
+    x = torch.randn(M, K, generator=g, device="cuda")
+    return torch.where(torch.rand(K, generator=g, device="cuda") < 0.01, x * 20, x).to(dtype)
+
+
+def _dense(g, N, K):
+    lin = torch.nn.Linear(K, N, bias=True, device="meta").to_empty(device="cuda")
+    lin.weight.data.normal_(0, 0.02, generator=g)
+    lin.bias.data.normal_(0, 0.1, generator=g)
+    return lin
+
+
+def _awq_layer(g, N, K, G, bias=True):
+    layer = WQLinear_GEMM(4, G, K, N, bias, "cuda")
+    layer.qweight.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+    layer.qzeros.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+    layer.scales.uniform_(0.001, 0.02, generator=g)
+    if bias:
+        layer.bias.normal_(0, 0.1, generator=g)
+    return layer
+
+
+def _awq_model(g, model, B, ctx):
+    layers, h, i, hq, hkv, d = MODELS[model]
+    blocks = []
+    for _ in range(layers):
+        qkv = fuse_linears([_awq_layer(g, n * d, h, 128) for n in (hq, hkv, hkv)])
+        o = _awq_layer(g, h, hq * d, 128, bias=False)
+        mlp = FusedGateUpMLP(_awq_layer(g, i, h, 128, bias=False), _awq_layer(g, i, h, 128, bias=False),
+                             _awq_layer(g, h, i, 128, bias=False))
+        for layer in (qkv, o, mlp.gate_up, mlp.down_proj):
+            layer.packed()
+        norms = [RMSNorm(torch.ones(h, dtype=torch.float16, device="cuda")) for _ in range(2)]
+        block = LlamaLikeBlock(h, hq, hkv, qkv, None, None, None, o, mlp, *norms, dev="cuda", max_seq_len=ctx + 8,
+                               rope_theta=1e6)
+        a = block.attn
+        if B > 1:
+            a.cache.increase_batch_size(B)
+            a.cache_batch_size = B
+        a.cache.k.normal_(generator=g)
+        a.cache.v.normal_(generator=g)
+        blocks.append(block)
+    embed = torch.nn.Embedding(VOCAB, h, device="cuda", dtype=torch.float16)
+    embed.weight.data.normal_(0, 1, generator=g)
+    return LlamaLikeModel(VOCAB, blocks, embed, RMSNorm(torch.ones(h, dtype=torch.float16, device="cuda")))
+
+
+def prepare(case, seed):
+    g, kind, s = _gen(seed), case["kind"], {"kind": case["kind"]}
+    if kind in ("sq", "fp8", "awq"):
+        M, N, K = case["M"], case["N"], case["K"]
+        if kind == "sq":
+            cls = SqW8A8BBF16OBF16PerChannel if case["per_channel"] else SqW8A8BBF16OBF16PerTensor
+            dt = DTYPES[case["dtype"]]
+            s["layer"] = cls.from_linear(_dense(g, N, K), 8, 0, init_only=False, dtype=dt)
+        elif kind == "fp8":
+            dt = torch.bfloat16
+            if case["mode"] == "static":
+                s["layer"] = FP8StaticLinear.from_linear(_dense(g, N, K), init_only=False, dtype=dt)
+                s["layer"].input_scale.data.fill_(80.0 / 448)
+                s["layer"].output_scale.data.fill_(1.0)
+            else:
+                s["layer"] = FP8DynamicLinear.from_linear(_dense(g, N, K), init_only=False, dtype=dt,
+                                                          per_tensor=case["mode"] == "tensor")
+        else:
+            dt = torch.float16
+            s["layer"] = _awq_layer(g, N, K, case["G"])
+            s["layer"].packed()
+        s["x"] = _activations(g, M, K, dt)
+    elif kind == "attn_decode":
+        B, Hq, Hkv, d, dt = case["B"], case["Hq"], case["Hkv"], case["d"], DTYPES[case["dtype"]]
+        cpu = torch.Generator().manual_seed(seed)
+        s["lens"] = torch.randint(case["lo"], case["hi"] + 1, (B,), generator=cpu, dtype=torch.int32).cuda()
+        s["k_cache"], s["v_cache"] = (torch.randn(B, case["hi"] + 8, Hkv, d, generator=g, device="cuda", dtype=dt)
+                                      for _ in range(2))
+        s["q"], s["k"], s["v"] = (torch.randn(B, 1, h, d, generator=g, device="cuda", dtype=dt) for h in (Hq, Hkv, Hkv))
+    elif kind == "attn_prefill":
+        B, S, Hq, Hkv, d, dt = (case[n] for n in ("B", "S", "Hq", "Hkv", "d", "dtype"))
+        s["q"], s["k"], s["v"] = (torch.randn(B, S, h, d, generator=g, device="cuda", dtype=DTYPES[dt])
+                                  for h in (Hq, Hkv, Hkv))
+        s["causal"] = case["causal"]
+    elif kind == "block":
+        s["model"], s["ctx"] = _awq_model(g, case["model"], case["B"], case["ctx"]), case["ctx"]
+        s["tokens"] = torch.randint(0, VOCAB, (case["B"], 1), generator=g, device="cuda")
+    else:
+        layers, h, i, hq, hkv, d = MODELS[case["model"]]
+        cfg = Qwen2Config(num_layers=layers, hidden=h, intermediate=i, num_heads=hq, num_kv_heads=hkv, head_dim=d,
+                          vocab=VOCAB)
+        B = case["B"]
+        m = s["model"] = Qwen2Decoder(cfg, "cuda", B, case["ctx" if kind == "decode" else "S"] + 8, seed=seed)
+        # Large embeddings and residual projections scaled by 1 / sqrt(2 layers): each layer then changes the residual
+        # stream by a few percent, as the middle layers of a trained model do.  (With every weight N(0, 0.02) a
+        # rounding difference in one layer grows to 20 % of the logits, and nothing could be compared.)
+        m.embed.mul_(400.0)
+        for layer in m.layers:
+            layer.so.mul_((2 * layers) ** -0.5)
+            layer.sd.mul_((2 * layers) ** -0.5)
+        if kind == "decode":
+            for layer in m.layers:
+                layer.k_cache.normal_(generator=g)
+                layer.v_cache.normal_(generator=g)
+            s["ctx"] = case["ctx"]
+            s["tokens"] = torch.randint(0, VOCAB, (B,), generator=g, device="cuda")
+            m.reset_position(s["ctx"])
+            m.decode_step(s["tokens"])                       # captures the step's graph, once per model
+        else:
+            s["tokens"] = torch.randint(0, VOCAB, (B, case["S"]), generator=g, device="cuda")
+    return s
+
+
+# ---------------------------------------------------------------------------------------------
+# one pass
+# ---------------------------------------------------------------------------------------------
+def run(s):
+    kind = s["kind"]
+    if kind in ("sq", "fp8", "awq"):
+        return s["layer"](s["x"])
+    if kind == "attn_decode":
+        out = attention.flash_attn_with_kvcache(q=s["q"], k_cache=s["k_cache"], v_cache=s["v_cache"], k=s["k"], v=s["v"],
+                                                cache_seqlens=s["lens"], causal=True)
+        return out, s["k_cache"], s["v_cache"]
+    if kind == "attn_prefill":
+        return attention.flash_attn_func(s["q"], s["k"], s["v"], causal=s["causal"])
+    m = s["model"]
+    if kind == "block":
+        for block in m.blocks:                               # every pass decodes the same position
+            block.attn.start_pos = s["ctx"]
+        out = m(s["tokens"])
+        return out, [b.attn.cache.k for b in m.blocks], [b.attn.cache.v for b in m.blocks]
+    if kind == "decode":
+        m.reset_position(s["ctx"])
+        m.decode_step(s["tokens"])
+    else:
+        m.prefill(s["tokens"])
+    # (the sampled ids are the arg-max of these rows)
+    return m.last_logits, [layer.k_cache for layer in m.layers], [layer.v_cache for layer in m.layers]
+
+
+# ---------------------------------------------------------------------------------------------
+# what a pass cannot do without, and how far two correct implementations may differ
+# ---------------------------------------------------------------------------------------------
+def work(case):
+    kind = case["kind"]
+    if kind in ("sq", "fp8", "awq"):
+        M, N, K = case["M"], case["N"], case["K"]
+        weight = N * K if kind != "awq" else N * K // 2 + K // case["G"] * N * 5 // 2
+        return {"bytes": 2 * M * K + weight + 2 * N + 2 * M * N + (4 * N if kind != "awq" else 0), "flops": 2 * M * N * K}
+    if kind == "attn_decode":
+        B, Hq, Hkv, d = case["B"], case["Hq"], case["Hkv"], case["d"]
+        ctx = B * ((case["lo"] + case["hi"]) // 2 + 1)
+        return {"bytes": ctx * Hkv * d * 4 + 4 * B * (Hq + 2 * Hkv) * d, "flops": 4 * ctx * Hq * d}
+    if kind == "attn_prefill":
+        B, S, Hq, Hkv, d = case["B"], case["S"], case["Hq"], case["Hkv"], case["d"]
+        return {"bytes": 4 * B * S * (Hq + Hkv) * d, "flops": 4 * B * Hq * S * S * d // (2 if case["causal"] else 1)}
+    layers, h, i, hq, hkv, d = MODELS[case["model"]]
+    B = case["B"]
+    params = h * (hq + 2 * hkv) * d + hq * d * h + 3 * h * i
+    if kind == "prefill":
+        M, ctx = B * case["S"], case["S"] / 2
+    else:
+        M, ctx = B, case["ctx"] + 1
+    kv_rows = B * (case["S"] if kind == "prefill" else ctx)
+    bytes_ = layers * (params * (0.5195 if kind == "block" else 1) + kv_rows * hkv * d * 4)
+    flops = layers * (2 * M * params + 4 * M * ctx * hq * d)
+    if kind != "block":
+        bytes_ += VOCAB * h * 2 + B * VOCAB * 2
+        flops += 2 * B * VOCAB * h
+    return {"bytes": int(bytes_), "flops": int(flops)}
+
+
+def tolerance(case):
+    kind = case["kind"]
+    if kind == "sq":                                         # exact integers, one rounding to 16 bits
+        return {"rel": 1e-3 if case["dtype"] == "fp16" or not case["per_channel"] else 4e-3}
+    if kind == "fp8":
+        return {"rel": 4e-3}
+    if kind == "awq":
+        return {"rel": 1e-3}
+    if kind in ("attn_decode", "attn_prefill"):
+        return {"rel": 2e-3 if case["dtype"] == "fp16" else 1e-2}
+    # a whole model passes a rounding difference on through int8 re-quantization in every layer: with another
+    # attention kernel put in, the logits moved by 1 % and the caches' rows of the last layers as much
+    return {"rel": 0.03}
