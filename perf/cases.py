@@ -293,6 +293,110 @@ def tolerance(case):
         return {"rel": 1e-3}
     if kind in ("attn_decode", "attn_prefill"):
         return {"rel": 2e-3 if case["dtype"] == "fp16" else 1e-2}
-    # a whole model passes a rounding difference on through int8 re-quantization in every layer: with another
-    # attention kernel put in, the logits moved by 1 % and the caches' rows of the last layers as much
-    return {"rel": 0.03}
+    # A whole model passes a rounding difference on.  The int8 models re-quantize in every layer: with another
+    # attention kernel put in, the logits moved by 1 %.  The 4-bit model's random weights amplify each layer's 16-bit
+    # rounding: its output is 2 % off what 64 bits give.
+    return {"rel": 0.08 if kind == "block" else 0.04}
+
+
+# ---------------------------------------------------------------------------------------------
+# the same pass in 64 bits, by plain torch
+# ---------------------------------------------------------------------------------------------
+def _scale16(amax, qmax, floor):
+    """The dynamic quantizers' scale: rounded to the activations' own 16 bits after the clamp and the division."""
+    return amax.clamp(min=floor).div(qmax)
+
+
+def _awq_weight(layer):
+    """[K, N] in 64 bits; nibble i of a word holds column 8j + (0, 2, 4, 6, 1, 3, 5, 7)[i]."""
+    def unpack(words):
+        out = torch.empty(*words.shape, 8, dtype=torch.int8, device=words.device)
+        for i, col in enumerate((0, 2, 4, 6, 1, 3, 5, 7)):
+            out[..., col] = ((words >> (4 * i)) & 15).to(torch.int8)
+        return out.reshape(words.shape[0], -1)
+    q, z = unpack(layer.qweight), unpack(layer.qzeros)
+    G = q.shape[0] // z.shape[0]
+    return (q - z.repeat_interleave(G, 0)).double() * layer.scales.double().repeat_interleave(G, 0)
+
+
+def _awq_linear(layer, x):
+    y = x @ _awq_weight(layer)
+    return y if layer.bias is None else y + layer.bias.double()
+
+
+def _attend(q, k, v, causal):
+    """One sequence: q [S, Hq, d], k and v [T, Hkv, d]."""
+    S, Hq, d = q.shape
+    rep = Hq // k.shape[1]
+    out = torch.empty(S, Hq, d, dtype=torch.float64, device=q.device)
+    for h in range(Hq):
+        s = q[:, h].double() @ k[:, h // rep].double().t() * d ** -0.5
+        if causal and S > 1:
+            s.masked_fill_(torch.ones_like(s, dtype=torch.bool).triu_(1), -math.inf)
+        out[:, h] = s.softmax(-1) @ v[:, h // rep].double()
+    return out
+
+
+def _exact_block(s, case):
+    layers, h, i, hq, hkv, d = MODELS[case["model"]]
+    B, ctx = case["B"], case["ctx"]
+
+    def norm(x):
+        return x * (x.square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+
+    ang = ctx * 1e6 ** (-torch.arange(0, d, 2, dtype=torch.float64, device="cuda") / d)
+
+    def rotate(x):                                           # half-split pairs
+        a, b = x.chunk(2, -1)
+        return torch.cat([a * ang.cos() - b * ang.sin(), a * ang.sin() + b * ang.cos()], -1)
+
+    x, keys, values = s["model"].embedding.weight[s["tokens"]].double(), [], []
+    for block in s["model"].blocks:
+        qkv = _awq_linear(block.attn.qkv_proj, norm(x)).view(B, hq + 2 * hkv, d)
+        q, k, v = qkv.split([hq, hkv, hkv], 1)
+        kc, vc = block.attn.cache.k.double(), block.attn.cache.v.double()
+        for pos in (ctx, ctx + 1):                           # the new token is written, and attended to, twice
+            kc[:, pos], vc[:, pos] = rotate(k), v
+        q = rotate(q)
+        o = torch.stack([_attend(q[b:b + 1], kc[b, :ctx + 2], vc[b, :ctx + 2], False)[0] for b in range(B)])
+        x = x + _awq_linear(block.attn.o_proj, o.view(B, 1, hq * d))
+        gate, up = _awq_linear(block.mlp.gate_up, norm(x)).chunk(2, -1)
+        x = x + _awq_linear(block.mlp.down_proj, torch.nn.functional.silu(gate) * up)
+        keys.append(kc)
+        values.append(vc)
+    return norm(x), keys, values
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind in ("decode", "prefill"):
+        return None                                          # int8 re-quantization in every layer: no such value
+    s = prepare(case, seed)
+    if kind == "block":
+        return _exact_block(s, case)
+    if kind == "attn_prefill":
+        return torch.stack([_attend(q, k, v, s["causal"]) for q, k, v in zip(s["q"], s["k"], s["v"])])
+    if kind == "attn_decode":
+        out = torch.empty(s["q"].shape, dtype=torch.float64, device="cuda")
+        for b, n in enumerate(s["lens"].tolist()):
+            s["k_cache"][b, n], s["v_cache"][b, n] = s["k"][b, 0], s["v"][b, 0]
+            out[b] = _attend(s["q"][b], s["k_cache"][b, :n + 1], s["v_cache"][b, :n + 1], False)
+        return out, s["k_cache"], s["v_cache"]
+    layer, x = s["layer"], s["x"]
+    if kind == "awq":
+        return _awq_linear(layer, x.double())
+    per_row = case.get("per_channel") or case.get("mode") == "token"
+    amax = x.abs().amax(1, keepdim=True) if per_row else x.abs().amax()
+    if kind == "sq":
+        scale = _scale16(amax, 127, 1e-5)
+        xq = (x / scale).round().clamp(-128, 127)
+        scales = (scale.double() * layer.weight_scale.double() if per_row
+                  else (scale * layer.weight_scale.item()).double())       # one scale: rounded to 16 bits as well
+        w, bias = layer.qweight, layer.bias.double() if per_row else layer.bias.half().double()
+    else:
+        static = case["mode"] == "static"
+        scale = layer.input_scale if static else _scale16(amax, 448, 1e-12)
+        xq = (x / scale).clamp(-448, 448).to(torch.float8_e4m3fn)
+        scales = scale.double() * layer.weight_scale.double().reshape(1, -1)
+        w, bias = layer.weight.to(torch.float8_e4m3fn), layer.bias.double()
+    return xq.double() @ w.double().t() * scales + bias
