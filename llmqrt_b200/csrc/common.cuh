@@ -122,6 +122,69 @@ template <> __device__ __forceinline__ float from_f32<float>(float v) { return v
 // 16-bit tensor does to its fp32 intermediate).
 template <typename T> __device__ __forceinline__ float round_to(float v) { return to_f32<T>(from_f32<T>(v)); }
 
+template <typename T> struct Pair16;
+template <> struct Pair16<__half> {
+  using type = __half2;
+  static __device__ __forceinline__ __half2 pack(float a, float b) { return __floats2half2_rn(a, b); }
+  static __device__ __forceinline__ float2 unpack(__half2 v) { return __half22float2(v); }
+};
+template <> struct Pair16<__nv_bfloat16> {
+  using type = __nv_bfloat162;
+  static __device__ __forceinline__ __nv_bfloat162 pack(float a, float b) { return __floats2bfloat162_rn(a, b); }
+  static __device__ __forceinline__ float2 unpack(__nv_bfloat162 v) { return __bfloat1622float2(v); }
+};
+// Two packed 16-bit values <-> two floats, one conversion instruction for the pair.
+template <typename T> __device__ __forceinline__ uint32_t pack_pair(float a, float b) {
+  const typename Pair16<T>::type v = Pair16<T>::pack(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <typename T> __device__ __forceinline__ float2 unpack_pair(uint32_t w) {
+  return Pair16<T>::unpack(*reinterpret_cast<const typename Pair16<T>::type*>(&w));
+}
+
+// Division of a row's 16-bit values by the row's 16-bit scale, as the reference's tensor / tensor (a true
+// fp32 division).  With r = 1 / s correctly rounded, fma(fma(x r, s, -x), -r, x r) is the correctly rounded
+// quotient (Markstein 1990; the scale's short mantissa is never the excepted all-ones one), and in this form
+// a negative zero keeps its sign: three multiply-adds per element instead of the general division's
+// reciprocal, iterations and range checks.
+// An infinite scale (an infinite element in the row) is carried as {0, 0}: x r is then 0, and NaN for the
+// infinite element, as the division gives.
+struct RowScale {
+  float s, r;
+};
+__device__ __forceinline__ RowScale row_scale(float s) {
+  return s <= 3.0e38f ? RowScale{s, __fdiv_rn(1.0f, s)} : RowScale{0.f, 0.f};
+}
+__device__ __forceinline__ float div_row_scale(float x, RowScale c) {
+  const float q0 = __fmul_rn(x, c.r);
+  return __fmaf_rn(__fmaf_rn(q0, c.s, -x), -c.r, q0);
+}
+// Four 32-bit integers clamped to int8 and packed, first one in the low byte.
+__device__ __forceinline__ uint32_t pack_sat_s8(int a, int b, int c, int d) {
+  uint32_t hi, w;
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(d), "r"(c), "r"(0));
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(b), "r"(a), "r"(hi));
+  return w;
+}
+// clamp(round_half_even(T(x / s)), -128, 127) of eight packed 16-bit values; NaN converts to 0.
+template <typename T>
+__device__ __forceinline__ uint2 quantize8_int8(const uint4& v, RowScale c) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  int o[8];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 x = unpack_pair<T>(w[p]);
+    const float2 d = unpack_pair<T>(pack_pair<T>(div_row_scale(x.x, c), div_row_scale(x.y, c)));
+    o[2 * p] = __float2int_rn(d.x);
+    o[2 * p + 1] = __float2int_rn(d.y);
+  }
+  return make_uint2(pack_sat_s8(o[0], o[1], o[2], o[3]), pack_sat_s8(o[4], o[5], o[6], o[7]));
+}
+// The int8 quantizers' scale of a row: T(T(max(absmax, 1e-5)) * (1 / 127)).
+template <typename T> __device__ __forceinline__ float int8_scale(float amax) {
+  return round_to<T>(__fmul_rn(round_to<T>(fmaxf(amax, 1e-5f)), 1.0f / 127.0f));
+}
+
 // Loads a 16-bit float of runtime dtype (LLMQRT_F16 / LLMQRT_BF16 / LLMQRT_F32) as fp32.
 __device__ __forceinline__ float load_as_f32(const void* p, int64_t i, int dtype) {
   if (dtype == LLMQRT_F16) return __half2float(reinterpret_cast<const __half*>(p)[i]);

@@ -193,23 +193,43 @@ silu_mul_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ y, in
   if (cl > 1) cg::this_cluster().sync();
 }
 
-// Block-wide reduction for a block of any whole number of warps (up to 32).
+// Block-wide reduction with one barrier: every warp leaves its value, every thread combines them in warp
+// order.  For ONE call per kernel and operation (nothing protects the scratch against a second call).
 template <bool IS_MAX>
-__device__ __forceinline__ float block_reduce_any(float v) {
+__device__ __forceinline__ float block_reduce_once(float v) {
   __shared__ float red[32];
-  __shared__ float result;
-  const int nwarps = blockDim.x >> 5;
   v = IS_MAX ? warp_max(v) : warp_sum(v);
-  __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    float w = (int)threadIdx.x < nwarps ? red[threadIdx.x] : 0.f;
-    w = IS_MAX ? warp_max(w) : warp_sum(w);
-    if (threadIdx.x == 0) result = w;
+  float r = red[0];
+  const int nwarps = blockDim.x >> 5;
+  for (int w = 1; w < nwarps; ++w) r = IS_MAX ? fmaxf(r, red[w]) : r + red[w];
+  return r;
+}
+
+// silu in T: the quotient gate / (1 + e^-gate) as the approximate reciprocal (1 ulp of fp32) times gate,
+// then the rounding to 16 bits that dwarfs both.
+template <typename T>
+__device__ __forceinline__ float silu_f32(float g) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-g)));
+  return g * r;
+}
+
+// Eight packed results of silu(gate) * up (in T); the running absolute maximum goes up with them.
+template <typename T>
+__device__ __forceinline__ uint4 silu_mul8(const uint4& g, const uint4& up, float& amax) {
+  const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {up.x, up.y, up.z, up.w};
+  uint32_t h[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 gv = unpack_pair<T>(gw[p]), uv = unpack_pair<T>(uw[p]);
+    const float2 act = unpack_pair<T>(pack_pair<T>(silu_f32<T>(gv.x), silu_f32<T>(gv.y)));       // silu in T
+    h[p] = pack_pair<T>(act.x * uv.x, act.y * uv.y);                                              // * up, in T
+    const float2 hv = unpack_pair<T>(h[p]);
+    amax = fmaxf(amax, fmaxf(fabsf(hv.x), fabsf(hv.y)));
   }
-  __syncthreads();
-  return result;
+  return make_uint4(h[0], h[1], h[2], h[3]);
 }
 
 // SiLU(gate) * up with the row split over the CTAs of a cluster (possibly of one) and U units of eight
@@ -224,36 +244,27 @@ silu_mul_regs_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ 
   pdl_wait_then_trigger();
   const int cl = gridDim.x, rank = blockIdx.x;
   const int64_t m = blockIdx.y, c0 = (int64_t)rank * slice;
-  float f[U][8];
   float amax = 0.f;
   const T* gr = gate_up + m * ld + c0;
-  T g[U][8], up[U][8];
+  uint4 h[U], up[U];
 #pragma unroll
   for (int k = 0; k < U; ++k) {                        // all loads first: U independent pairs in flight
     const int64_t u = threadIdx.x + (int64_t)k * blockDim.x;
     if (u * 8 < slice) {
-      load_unit<T, true>(gr, u, g[k]);
-      load_unit<T, true>(gr + I, u, up[k]);
+      h[k] = *reinterpret_cast<const uint4*>(gr + u * 8);
+      up[k] = *reinterpret_cast<const uint4*>(gr + I + u * 8);
     }
   }
 #pragma unroll
   for (int k = 0; k < U; ++k) {
     const int64_t u = threadIdx.x + (int64_t)k * blockDim.x;
     if (u * 8 < slice) {
-      T h[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float gv = to_f32<T>(g[k][j]);
-        const float act = round_to<T>(gv / (1.0f + expf(-gv)));             // silu in T
-        f[k][j] = round_to<T>(act * to_f32<T>(up[k][j]));                   // * up, in T
-        h[j] = from_f32<T>(f[k][j]);
-        amax = fmaxf(amax, fabsf(f[k][j]));
-      }
-      if (y) store_unit<T, true>(y + m * I + c0, u, h);
+      h[k] = silu_mul8<T>(h[k], up[k], amax);
+      if (y) *reinterpret_cast<uint4*>(y + m * I + c0 + u * 8) = h[k];
     }
   }
   if (q) {
-    amax = block_reduce_any<true>(amax);
+    amax = block_reduce_once<true>(amax);
     if (cl > 1) {
       // every CTA stores its maximum into its slot in EVERY CTA of the cluster, then ONE cluster barrier
       // (release / acquire) and each CTA reads its own copy: nobody reads remote memory afterwards, so
@@ -268,25 +279,84 @@ silu_mul_regs_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ 
       amax = 0.f;
       for (int c = 0; c < cl; ++c) amax = fmaxf(amax, slot_amax[c]);
     }
-    float s = round_to<T>(fmaxf(amax, 1e-5f));
-    s = round_to<T>(__fmul_rn(s, 1.0f / 127.0f));
+    const float s = int8_scale<T>(amax);
     if (rank == 0 && threadIdx.x == 0) scale_f32[m] = s;
+    const RowScale rs = row_scale(s);
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       const int64_t u = threadIdx.x + (int64_t)k * blockDim.x;
-      if (u * 8 < slice) {
-        __align__(8) int8_t o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float v = rintf(round_to<T>(__fdiv_rn(f[k][j], s)));
-          v = v != v ? v : fminf(fmaxf(v, -128.f), 127.f);
-          o[j] = (int8_t)(int)v;
-        }
-        *reinterpret_cast<uint2*>(q + m * I + c0 + u * 8) = *reinterpret_cast<const uint2*>(o);
-      }
+      if (u * 8 < slice) *reinterpret_cast<uint2*>(q + m * I + c0 + u * 8) = quantize8_int8<T>(h[k], rs);
     }
   }
 }
+
+// SiLU(gate) * up for prefill-sized M: one block per row, U units of eight elements per thread, the packed
+// results kept in registers from the loads to the quantized store.
+// HBM-bound (8192 rows of 2 x 18944: 932 MB, 140 us at 6.65 TB/s) only if the arithmetic is short: the
+// staged form below spends over 60 instructions and five special-function operations on an element and
+// took 385 us; here it is about 30 and three (e^x, reciprocal, float -> int), and all of a thread's loads are
+// in flight at once.
+template <typename T, int U>
+__global__ void __launch_bounds__(512, U <= 5 ? 2 : 1)
+silu_mul_rows_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ y, int8_t* __restrict__ q,
+                     float* __restrict__ scale_f32, int64_t I) {
+  pdl_wait_then_trigger();
+  const int64_t m = blockIdx.x;
+  const int units = (int)(I / 8);
+  const T* gr = gate_up + m * ld;
+  uint4 g[U], up[U];
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u < units) {
+      g[k] = ldg_cg_16B(gr + (int64_t)u * 8);
+      up[k] = ldg_cg_16B(gr + I + (int64_t)u * 8);
+    }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u >= units) continue;
+    g[k] = silu_mul8<T>(g[k], up[k], amax);
+    if (y) *reinterpret_cast<uint4*>(y + m * I + (int64_t)u * 8) = g[k];
+  }
+  if (!q) return;
+  const float s = int8_scale<T>(block_reduce_once<true>(amax));
+  if (threadIdx.x == 0) scale_f32[m] = s;
+  const RowScale rs = row_scale(s);
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u < units) *reinterpret_cast<uint2*>(q + m * I + (int64_t)u * 8) = quantize8_int8<T>(g[k], rs);
+  }
+}
+
+template <typename T>
+int launch_silu_rows(const void* gate_up, int64_t ld, void* y, int8_t* q, float* scale_f32, int64_t M, int64_t I,
+                     cudaStream_t st) {
+  const int units = (int)(I / 8), U = (units + 511) / 512;
+  const unsigned threads = (unsigned)(((units + U - 1) / U + 31) / 32 * 32);
+  auto go = [&](auto kern) {
+    return launch_chained(kern, dim3((unsigned)M), dim3(threads), 0, st, 1, reinterpret_cast<const T*>(gate_up), ld,
+                          reinterpret_cast<T*>(y), q, scale_f32, I);
+  };
+  int rc;
+  switch (U) {
+    case 1: rc = go(silu_mul_rows_kernel<T, 1>); break;
+    case 2: rc = go(silu_mul_rows_kernel<T, 2>); break;
+    case 3: rc = go(silu_mul_rows_kernel<T, 3>); break;
+    case 4: rc = go(silu_mul_rows_kernel<T, 4>); break;
+    case 5: rc = go(silu_mul_rows_kernel<T, 5>); break;
+    default: rc = go(silu_mul_rows_kernel<T, 8>); break;
+  }
+  if (rc) return rc;
+  return check_launch("silu_mul");
+}
+
+// Rows from which one block per row is the faster split of SiLU (two blocks to an SM): 300 rows of 4864 / 8960 /
+// 18944 elements take 13.7 / 12.3 / 18.4 us against 16.1 / 16.4 / 24.6 us in clusters; fewer leave SMs idle.
+constexpr int64_t kSiluRowsMinM = 296;
 
 // RMSNorm of one row held in registers, eight elements per thread (rows of up to 8192 elements, one
 // block per row): `h` are the row's values already rounded to T (x, or x + residual), `on` says
@@ -296,41 +366,106 @@ __device__ __forceinline__ void rmsnorm_regs_finish(bool on, float (&f)[8], int6
                                                     const T* __restrict__ weight, float eps, T* __restrict__ y,
                                                     int8_t* __restrict__ q, float* __restrict__ scale_f32) {
   const int64_t off = m * H;
-  T e[8], w[8];
+  T w[8];
   float ss = 0.f;
   if (on) {
     load_unit<T, true>(weight, u, w);
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
   }
-  ss = block_reduce_any<false>(ss);
+  ss = block_reduce_once<false>(ss);
   const float inv = rsqrtf(ss / (float)H + eps);
   float amax = 0.f;
+  uint4 packed = make_uint4(0u, 0u, 0u, 0u);
   if (on) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float n = round_to<T>(f[j] * inv);                            // (x32 * inv).to(T)
       f[j] = round_to<T>(to_f32<T>(w[j]) * n);                            // weight * that, in T
-      e[j] = from_f32<T>(f[j]);
       amax = fmaxf(amax, fabsf(f[j]));
     }
-    if (y) store_unit<T, true>(y + off, u, e);
+    packed = make_uint4(pack_pair<T>(f[0], f[1]), pack_pair<T>(f[2], f[3]), pack_pair<T>(f[4], f[5]),
+                        pack_pair<T>(f[6], f[7]));
+    if (y) *reinterpret_cast<uint4*>(y + off + u * 8) = packed;
   }
   if (q) {
-    amax = block_reduce_any<true>(amax);
-    float s = round_to<T>(fmaxf(amax, 1e-5f));
-    s = round_to<T>(__fmul_rn(s, 1.0f / 127.0f));
+    const float s = int8_scale<T>(block_reduce_once<true>(amax));
     if (threadIdx.x == 0) scale_f32[m] = s;
-    if (on) {
-      __align__(8) int8_t o[8];
+    if (on) *reinterpret_cast<uint2*>(q + off + u * 8) = quantize8_int8<T>(packed, row_scale(s));
+  }
+}
+
+// The same for many rows: one block of at most 128 threads per row, U units of eight elements per thread.
+// HBM-bound (8192 rows of 3584 with residual and int8 output: 205 MB, 31 us at 6.65 TB/s).  With one unit per
+// thread a row's two reductions each stall a whole 448-thread block, four blocks to an SM: 74 us.  Four
+// units per thread put fifteen rows on an SM and make the reductions a quarter as wide: 43 us.
+template <typename T, int U>
+__global__ void __launch_bounds__(128)
+rmsnorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ residual, T* __restrict__ x_out,
+                    const T* __restrict__ weight, float eps, T* __restrict__ y, int8_t* __restrict__ q,
+                    float* __restrict__ scale_f32, int64_t H) {
+  pdl_wait_then_trigger();
+  const int64_t m = blockIdx.x, off = m * H;
+  const int units = (int)(H / 8);
+  uint4 e[U], r[U];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float v = rintf(round_to<T>(__fdiv_rn(f[j], s)));
-        v = v != v ? v : fminf(fmaxf(v, -128.f), 127.f);
-        o[j] = (int8_t)(int)v;
-      }
-      *reinterpret_cast<uint2*>(q + off + u * 8) = *reinterpret_cast<const uint2*>(o);
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u < units) {
+      e[k] = ldg_cg_16B(x + off + u * 8);
+      if (residual) r[k] = ldg_cg_16B(residual + off + u * 8);
     }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u >= units) continue;
+    uint32_t w[4] = {e[k].x, e[k].y, e[k].z, e[k].w};
+    const uint32_t rw[4] = {r[k].x, r[k].y, r[k].z, r[k].w};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      float2 v = unpack_pair<T>(w[p]);
+      if (residual) {
+        const float2 rv = unpack_pair<T>(rw[p]);
+        w[p] = pack_pair<T>(v.x + rv.x, v.y + rv.y);                      // h = x + r in T
+        v = unpack_pair<T>(w[p]);
+      }
+      ss += v.x * v.x;
+      ss += v.y * v.y;
+    }
+    e[k] = make_uint4(w[0], w[1], w[2], w[3]);
+    if (x_out) *reinterpret_cast<uint4*>(x_out + off + u * 8) = e[k];
+  }
+  ss = block_reduce_once<false>(ss);
+  const float inv = rsqrtf(ss / (float)H + eps);
+  float amax = 0.f;
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u >= units) continue;
+    const uint4 wt = *reinterpret_cast<const uint4*>(weight + u * 8);
+    const uint32_t ww[4] = {wt.x, wt.y, wt.z, wt.w};
+    uint32_t w[4] = {e[k].x, e[k].y, e[k].z, e[k].w};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const float2 v = unpack_pair<T>(w[p]), wv = unpack_pair<T>(ww[p]);
+      const float2 n = unpack_pair<T>(pack_pair<T>(v.x * inv, v.y * inv));     // (x32 * inv).to(T)
+      w[p] = pack_pair<T>(wv.x * n.x, wv.y * n.y);                             // weight * that, in T
+      const float2 o = unpack_pair<T>(w[p]);
+      amax = fmaxf(amax, fmaxf(fabsf(o.x), fabsf(o.y)));
+    }
+    e[k] = make_uint4(w[0], w[1], w[2], w[3]);
+    if (y) *reinterpret_cast<uint4*>(y + off + u * 8) = e[k];
+  }
+  if (!q) return;
+  const float s = int8_scale<T>(block_reduce_once<true>(amax));
+  if (threadIdx.x == 0) scale_f32[m] = s;
+  const RowScale rs = row_scale(s);
+#pragma unroll
+  for (int k = 0; k < U; ++k) {
+    const int u = threadIdx.x + k * blockDim.x;
+    if (u < units) *reinterpret_cast<uint2*>(q + off + u * 8) = quantize8_int8<T>(e[k], rs);
   }
 }
 
@@ -627,6 +762,23 @@ int llmqrt_rmsnorm(const void* x, const void* residual, void* x_out, const void*
   const bool vec = H % 8 == 0 && aligned16(x) && aligned16(residual) && aligned16(x_out) && aligned16(weight) &&
                    aligned16(y) && (reinterpret_cast<uintptr_t>(q) & 7) == 0;
   if (vec && H <= 8192 && M <= 0x7fffffffll) {
+    if (M >= 2 * sm_count()) {                         // rows enough to fill the chip with small blocks
+      const int units = (int)(H / 8), U = units <= 128 ? 1 : units <= 256 ? 2 : units <= 512 ? 4 : 8;
+      const unsigned threads = (unsigned)(((units + U - 1) / U + 31) / 32 * 32);
+      auto go = [&](auto kern, auto tag) {
+        using T = decltype(tag);
+        return launch_chained(kern, dim3((unsigned)M), dim3(threads), 0, st, 1, reinterpret_cast<const T*>(x),
+                              reinterpret_cast<const T*>(residual), reinterpret_cast<T*>(x_out),
+                              reinterpret_cast<const T*>(weight), eps, reinterpret_cast<T*>(y), q, scale_f32, H);
+      };
+      auto pick = [&](auto tag) {
+        using T = decltype(tag);
+        return U == 1 ? go(rmsnorm_rows_kernel<T, 1>, tag) : U == 2 ? go(rmsnorm_rows_kernel<T, 2>, tag)
+               : U == 4 ? go(rmsnorm_rows_kernel<T, 4>, tag) : go(rmsnorm_rows_kernel<T, 8>, tag);
+      };
+      if (int rc = dtype == LLMQRT_F16 ? pick(__half()) : pick(__nv_bfloat16())) return rc;
+      return check_launch("rmsnorm");
+    }
     // the row fits the registers of one block: one block per row, rows on gridDim.x
     const unsigned threads = (unsigned)(((H / 8) + 31) / 32 * 32);
     int rc;
@@ -710,6 +862,10 @@ int llmqrt_silu_mul(const void* gate_up, int64_t ld, void* y, int8_t* q, float* 
   cudaStream_t st = (cudaStream_t)stream;
   const bool vec = I % 8 == 0 && ld % 8 == 0 && aligned16(gate_up) && aligned16(y) &&
                    (reinterpret_cast<uintptr_t>(q) & 7) == 0;
+  // Enough rows to fill the chip twice over with one block each, and rows that fit a block's registers.
+  if (vec && M >= kSiluRowsMinM && M <= 0x7fffffffll && I <= 8 * 8 * 512)
+    return dtype == LLMQRT_F16 ? launch_silu_rows<__half>(gate_up, ld, y, q, scale_f32, M, I, st)
+                               : launch_silu_rows<__nv_bfloat16>(gate_up, ld, y, q, scale_f32, M, I, st);
   // Register-resident variant: the smallest cluster whose slices fit one block (8 elements per
   // thread), widened while that still leaves every SM at most a few blocks and slices of >= 128 threads.
   // (Timed alone, fewer and larger blocks win -- 64 rows of 18944: two CTAs with two units per thread

@@ -34,3 +34,49 @@ def test_rope_vectorised_equals_general(B, S, Hq, Hkv, d, dt):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
     assert torch.equal(got[0][2][:, pos0:pos0 + S].flatten(2), x[..., (Hq + Hkv) * d:])
     assert not got[0][1][:, :pos0].any() and not got[0][1][:, pos0 + S:].any()
+
+
+@pytest.mark.parametrize("I", [8, 24, 4096, 4104, 8960, 12296, 18944, 24584, 32768, 32776])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_silu_one_block_per_row(I, dt):
+    """300 rows: one block each, one to eight units per thread (the last size is beyond that form)."""
+    from llmqrt_b200 import glue
+    from oracle import quant as oq
+    gu = torch.randn(300, 2 * I, generator=_g(2), device="cuda") * 4
+    gu[7, : I // 2] = -120.0                                 # e^-gate overflows: silu is 0
+    gu[9, 0] = float("inf")                                  # infinite scale: 0, and 0 for inf / inf
+    gu = gu.to(dt)
+    y, q, s = glue.silu_mul(gu, quantize=True)
+    g32, u32 = gu[:, :I].double(), gu[:, I:].float()
+    act = (g32 * torch.sigmoid(g32)).to(dt)
+    want = (act.float() * u32).to(dt)
+    # the first rounding may fall the other way (one unit: a relative 2 eps at most), and then the second as well
+    eps = 2.0 ** (-10 if dt == torch.float16 else -7)
+    tiny = 2.0 ** -22 if dt == torch.float16 else 1e-30
+    ok = (y.float() - want.float()).abs() <= 2.02 * eps * want.float().abs() + tiny * (1 + u32.abs())
+    assert bool((ok | ~torch.isfinite(want)).all())
+    rows = [r for r in range(300) if r != 9]
+    qr, sr = oq.quantize_int8(y[rows].cpu(), per_token=True)
+    assert torch.equal(q[rows].cpu(), qr) and torch.equal(s[rows].cpu(), sr.float().reshape(-1))
+    assert torch.isinf(s[9]) and not q[9].any()
+
+
+@pytest.mark.parametrize("H", [8, 1016, 1024, 1032, 3584, 4104, 8192])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_rmsnorm_small_blocks(H, dt):
+    """300 rows: one small block each, one to eight units per thread."""
+    from llmqrt_b200 import glue
+    from oracle import quant as oq
+    x, r = (torch.randn(300, H, generator=_g(5 + i), device="cuda").to(dt) for i in range(2))
+    w = (1 + 0.1 * torch.randn(H, generator=_g(7), device="cuda")).to(dt)
+    y, h, q, s = glue.rmsnorm(x, w, 1e-6, residual=r, quantize=True)
+    want_h = (x.float() + r.float()).to(dt)
+    assert torch.equal(h, want_h)
+    n = (want_h.double() * (want_h.double().square().mean(-1, keepdim=True) + 1e-6).rsqrt()).float().to(dt)
+    want = (n.float() * w.float()).to(dt)
+    eps = 2.0 ** (-10 if dt == torch.float16 else -7)        # one unit in the last place of the first rounding, passed on
+    assert bool(((y.float() - want.float()).abs() <= 2.02 * eps * want.float().abs()).all())
+    qr, sr = oq.quantize_int8(y.cpu(), True)
+    assert torch.equal(q.cpu(), qr) and torch.equal(s.cpu(), sr.float().reshape(-1))
+    y2, _, _, _ = glue.rmsnorm(want_h, w, 1e-6)
+    assert torch.equal(y2, y)
