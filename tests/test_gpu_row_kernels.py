@@ -61,6 +61,41 @@ def test_silu_one_block_per_row(I, dt):
     assert torch.isinf(s[9]) and not q[9].any()
 
 
+@pytest.mark.parametrize("M,K", [(1, 8), (3, 1032), (3, 18944), (2, 65536), (2, 65544), (300, 1016), (300, 1024), (300, 2056),
+                                 (300, 4104), (296, 8200), (1200, 896)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_quantizers_match_oracle_bits(M, K, dt):
+    """Every unit count per thread and both row splits, a zero row and an infinite one; flat per-tensor passes."""
+    from llmqrt_b200 import ops
+    from oracle import quant as oq
+    x = torch.randn(M, K, generator=_g(3), device="cuda")
+    x = (x * torch.exp(4 * torch.randn(M, 1, generator=_g(4), device="cuda"))).clamp(-60000, 60000).to(dt)
+    if M > 2:
+        x[1] = 0
+    c = x.cpu()
+    q, _, s = ops.quantize_int8(x, True)
+    qr, sr = oq.quantize_int8(c, True)
+    assert torch.equal(q.cpu(), qr) and torch.equal(s.cpu(), sr.float().reshape(-1))
+    q, s = ops.quantize_fp8(x, True)
+    qr, sr = oq.quantize_fp8(c, True)
+    nan = qr.float().isnan()
+    assert torch.equal(q.cpu().float().isnan(), nan) and torch.equal(s.cpu().reshape(-1), sr.float().reshape(-1))
+    assert torch.equal(q.cpu().view(torch.uint8)[~nan], qr.view(torch.uint8)[~nan])
+    q, _, s = ops.quantize_int8(x, False)
+    qr, sr = oq.quantize_int8(c, False)
+    assert torch.equal(q.cpu(), qr) and float(s) == float(sr)
+    q, s = ops.quantize_fp8(x, False)
+    qr, sr = oq.quantize_fp8(c, False)
+    assert torch.equal(q.cpu().view(torch.uint8), qr.view(torch.uint8)) and float(s) == float(sr)
+    scale = torch.tensor([0.37], device="cuda")
+    q = ops.quantize_fp8_static(x, scale)
+    assert torch.equal(q.cpu().view(torch.uint8), oq.quantize_fp8_static(c, scale.cpu()).view(torch.uint8))
+    if M > 2:
+        x[2, 0] = float("inf")
+        q, _, s = ops.quantize_int8(x[2:3], True)
+        assert torch.isinf(s).all() and not q.any()
+
+
 @pytest.mark.parametrize("H", [8, 1016, 1024, 1032, 3584, 4104, 8192])
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
 def test_rmsnorm_small_blocks(H, dt):
