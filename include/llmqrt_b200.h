@@ -84,6 +84,13 @@ int llmqrt_quantize_fp8(const void* x, int x_dtype, int64_t M, int64_t K, int64_
 int llmqrt_quantize_fp8_static(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const float* scale,
                                uint8_t* q, llmqrt_stream_t stream);
 
+/* Per-tensor FP8 quantization that also leaves the factor of the GEMM behind it on the device:
+ * alpha[0] = scale * weight_scale[0], the scale being static_scale[0] or, with static_scale NULL, that of
+ * llmqrt_quantize_fp8. */
+int llmqrt_quantize_fp8_alpha(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx,
+                              const float* static_scale, const float* weight_scale, uint8_t* q, float* alpha,
+                              void* workspace, llmqrt_stream_t stream);
+
 /* ------------------------------------------------------------------------------------------
  * W8A8 GEMMs.   acc[m, n] = sum_k a[m, k] * w[n, k]
  * Requirements: K % 16 == 0, lda % 16 == 0, ldw % 16 == 0, 16-byte aligned a and w.

@@ -39,6 +39,7 @@ _PROTOS = {
     "llmqrt_quantize_int8": (c_int, [P, I32, I64, I64, I64, I32, P, P, P, F, P, P]),
     "llmqrt_quantize_fp8": (c_int, [P, I32, I64, I64, I64, I32, P, P, F, P, P]),
     "llmqrt_quantize_fp8_static": (c_int, [P, I32, I64, I64, I64, P, P, P]),
+    "llmqrt_quantize_fp8_alpha": (c_int, [P, I32, I64, I64, I64, P, P, P, P, P, P]),
     "llmqrt_w8a8_int8_linear_per_tensor": (c_int, [P, I64, P, I64, P, F, P, F, P, I64, I64, I64, I64, P, P, I32]),
     "llmqrt_w8a8_int8_linear_per_channel": (c_int, [P, I64, P, I64, P, I32, P, P, P, I32, I64, I64, I64, I64, P, P, I32]),
     "llmqrt_w8a8_int8_linear_per_channel_noalloc": (c_int, [P, I64, P, I64, P, I32, P, P, P, I32, I64, I64, I64, I64, P]),
@@ -87,7 +88,7 @@ def _bind(lib: ctypes.CDLL) -> list[str]:
     return missing
 
 
-ABI_VERSION = 5          # llmqrt_abi_version() of the sources these prototypes describe
+ABI_VERSION = 6          # llmqrt_abi_version() of the sources these prototypes describe
 
 _missing = _bind(_lib)
 if not _missing and _lib.llmqrt_abi_version() != ABI_VERSION:
@@ -104,6 +105,22 @@ if _missing:
         _missing = ["llmqrt_abi_version == %d" % ABI_VERSION]
     if _missing:
         raise ImportError(f"{LIB_PATH} lacks symbols {_missing}; rebuild with `python llmqrt_b200/build.py --force`")
+
+
+def _load_fast():
+    """The native host path (csrc/fastpath.cpp), built beside the library it calls."""
+    import importlib.machinery
+    import importlib.util
+    from . import build as _build
+    if not os.path.exists(_build.FAST):
+        _build.build()
+    loader = importlib.machinery.ExtensionFileLoader("_fast", _build.FAST)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fast", loader))
+    loader.exec_module(module)
+    return module
+
+
+fast = _load_fast()
 
 
 def last_error() -> str:
@@ -169,6 +186,8 @@ def workspace(device: torch.device) -> torch.Tensor:
                 _workspaces[key] = ws
     return ws
 
+
+fast.set_workspace_maker(lambda index: workspace(torch.device("cuda", index)))
 
 # Byte offset, inside a workspace, of the word a kernel sets to 1 when one of its bounded waits ran out.
 STATUS_OFFSET = 64 * 1024 - 64 * 4 + 4

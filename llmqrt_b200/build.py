@@ -6,6 +6,7 @@
 
 Every .cu under llmqrt_b200/csrc is compiled with nvcc to an object file and the objects are
 linked into llmqrt_b200/lib/libllmqrt_b200.so.  nvcc cross-compiles, so no GPU is needed.
+csrc/fastpath.cpp becomes the Python extension llmqrt_b200/lib/_fast.so (g++, ATen), which calls that library.
 """
 from __future__ import annotations
 
@@ -22,6 +23,8 @@ CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libllmqrt_b200.so")
+FAST_SRC = os.path.join(CSRC, "fastpath.cpp")
+FAST = os.path.join(LIBDIR, "_fast.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 NVCC_FLAGS = [
@@ -81,7 +84,27 @@ def build(force: bool = False, verbose: bool = False) -> str:
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n" + p.stdout + p.stderr)
+    if force or _stale(FAST, [FAST_SRC, LIB, os.path.join(INCLUDE, "llmqrt_b200.h")]):
+        _build_fast()
     return LIB
+
+
+def _build_fast() -> None:
+    import sysconfig
+
+    import torch
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    tmp = FAST + ".tmp%d" % os.getpid()
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(tdir, "include"),
+           "-I" + os.path.join(tdir, "include", "torch", "csrc", "api", "include"), "-I" + os.path.join(cuda, "include"),
+           "-I" + INCLUDE, FAST_SRC, "-o", tmp, "-L" + LIBDIR, "-lllmqrt_b200", "-L" + os.path.join(tdir, "lib"), "-lc10",
+           "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("building the host path failed:\n" + p.stdout + p.stderr)
+    os.replace(tmp, FAST)
 
 
 if __name__ == "__main__":

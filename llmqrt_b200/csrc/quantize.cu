@@ -214,12 +214,14 @@ template <typename T, bool FP8>
 __global__ void __launch_bounds__(kThreads)
 quantize_flat_kernel(const T* __restrict__ x, int64_t units, uint8_t* __restrict__ q, const float* __restrict__ parts,
                      int num_parts, const float* __restrict__ static_scale, T* __restrict__ scale_x,
-                     float* __restrict__ scale_f32, float scale_mul) {
+                     float* __restrict__ scale_f32, float scale_mul, const float* __restrict__ mul_dev) {
   pdl_wait_then_trigger();
+  if (mul_dev) scale_mul = *mul_dev;
   const int64_t step = (int64_t)gridDim.x * kThreads;
   int64_t u = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (static_scale) {
     const float s = *static_scale;
+    if (scale_f32 && u == 0) scale_f32[0] = __fmul_rn(s, scale_mul);
     for (; u < units; u += step) {
       const uint4 v = ldg_cg_16B(x + u * 8);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -280,8 +282,10 @@ template <typename T, bool FP8>
 __global__ void __launch_bounds__(kThreads)
 quantize_per_tensor_kernel(const T* __restrict__ x, int64_t K, int64_t ldx, uint8_t* __restrict__ q,
                            const unsigned* __restrict__ amax_bits, const float* __restrict__ static_scale,
-                           T* __restrict__ scale_x, float* __restrict__ scale_f32, float scale_mul, bool vec_ok) {
+                           T* __restrict__ scale_x, float* __restrict__ scale_f32, float scale_mul,
+                           const float* __restrict__ mul_dev, bool vec_ok) {
   const int64_t m = blockIdx.x;
+  if (mul_dev) scale_mul = *mul_dev;
   float s = static_scale ? *static_scale : scale_from_absmax<T, FP8>(__uint_as_float(*amax_bits));
   if (m == 0 && threadIdx.x == 0) {
     if (scale_x) scale_x[0] = from_f32<T>(s);
@@ -302,7 +306,8 @@ quantize_per_tensor_kernel(const T* __restrict__ x, int64_t K, int64_t ldx, uint
 
 template <typename T, bool FP8>
 int launch(const void* x, int64_t M, int64_t K, int64_t ldx, int per_token, uint8_t* q, void* scale_x,
-           float* scale_f32, float scale_mul, const float* static_scale, void* workspace, cudaStream_t st) {
+           float* scale_f32, float scale_mul, const float* static_scale, const float* mul_dev, void* workspace,
+           cudaStream_t st) {
   const T* xp = reinterpret_cast<const T*>(x);
   const bool vec_ok = (K % 8 == 0) && (ldx % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
                       ((reinterpret_cast<uintptr_t>(q) & 7) == 0);
@@ -316,13 +321,13 @@ int launch(const void* x, int64_t M, int64_t K, int64_t ldx, int per_token, uint
   if (static_scale && flat) {
     if (int rc = launch_chained(quantize_flat_kernel<T, FP8>, dim3((unsigned)flat_blocks), dim3(kThreads), 0, st, 1, xp,
                                 flat_units, q, static_cast<const float*>(nullptr), 0, static_scale,
-                                static_cast<T*>(nullptr), static_cast<float*>(nullptr), 1.f))
+                                static_cast<T*>(nullptr), scale_f32, scale_mul, mul_dev))
       return rc;
     return check_launch("quantize_static");
   }
   if (static_scale) {
     quantize_per_tensor_kernel<T, FP8><<<(unsigned)M, kThreads, 0, st>>>(xp, K, ldx, q, nullptr, static_scale,
-                                                                        nullptr, nullptr, 1.f, vec_ok);
+                                                                        nullptr, scale_f32, scale_mul, mul_dev, vec_ok);
     return check_launch("quantize_static");
   }
   if (per_token && vec_ok && K <= 8 * 8 * 1024)        // the row fits a block's registers
@@ -342,7 +347,8 @@ int launch(const void* x, int64_t M, int64_t K, int64_t ldx, int per_token, uint
     if (int rc = check_launch("absmax")) return rc;
     if (int rc = launch_chained(quantize_flat_kernel<T, FP8>, dim3((unsigned)flat_blocks), dim3(kThreads), 0, st, 1, xp,
                                 flat_units, q, static_cast<const float*>(parts), (int)flat_blocks,
-                                static_cast<const float*>(nullptr), reinterpret_cast<T*>(scale_x), scale_f32, scale_mul))
+                                static_cast<const float*>(nullptr), reinterpret_cast<T*>(scale_x), scale_f32, scale_mul,
+                                mul_dev))
       return rc;
     return check_launch("quantize_per_tensor");
   }
@@ -351,23 +357,24 @@ int launch(const void* x, int64_t M, int64_t K, int64_t ldx, int per_token, uint
   absmax_kernel<T><<<(unsigned)M, kThreads, 0, st>>>(xp, K, ldx, amax_bits, vec_ok);
   if (int rc = check_launch("absmax")) return rc;
   quantize_per_tensor_kernel<T, FP8><<<(unsigned)M, kThreads, 0, st>>>(
-      xp, K, ldx, q, amax_bits, nullptr, reinterpret_cast<T*>(scale_x), scale_f32, scale_mul, vec_ok);
+      xp, K, ldx, q, amax_bits, nullptr, reinterpret_cast<T*>(scale_x), scale_f32, scale_mul, mul_dev, vec_ok);
   return check_launch("quantize_per_tensor");
 }
 
 template <bool FP8>
 int dispatch(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, int per_token, uint8_t* q, void* scale_x,
-             float* scale_f32, float scale_mul, const float* static_scale, void* workspace, cudaStream_t st) {
+             float* scale_f32, float scale_mul, const float* static_scale, void* workspace, cudaStream_t st,
+             const float* mul_dev = nullptr) {
   LLMQRT_REQUIRE(M >= 0 && K >= 0 && ldx >= K, "quantize: bad shape M=%lld K=%lld ldx=%lld", (long long)M,
                  (long long)K, (long long)ldx);
   LLMQRT_REQUIRE(M < (1ll << 31), "quantize: M too large");
   if (M == 0 || K == 0) return LLMQRT_OK;
   LLMQRT_REQUIRE(x && q, "quantize: null pointer");
   if (x_dtype == LLMQRT_F16)
-    return launch<__half, FP8>(x, M, K, ldx, per_token, q, scale_x, scale_f32, scale_mul, static_scale, workspace, st);
+    return launch<__half, FP8>(x, M, K, ldx, per_token, q, scale_x, scale_f32, scale_mul, static_scale, mul_dev, workspace, st);
   if (x_dtype == LLMQRT_BF16)
     return launch<__nv_bfloat16, FP8>(x, M, K, ldx, per_token, q, scale_x, scale_f32, scale_mul, static_scale,
-                                      workspace, st);
+                                      mul_dev, workspace, st);
   return set_error(LLMQRT_ERR_INVALID, "quantize: x must be fp16 or bf16");
 }
 
@@ -393,6 +400,14 @@ int llmqrt_quantize_fp8_static(const void* x, int x_dtype, int64_t M, int64_t K,
   if (!scale) return llmqrt::set_error(LLMQRT_ERR_INVALID, "quantize_fp8_static: null scale");
   return llmqrt::dispatch<true>(x, x_dtype, M, K, ldx, 1, q, nullptr, nullptr, 1.f, scale, nullptr,
                                 (cudaStream_t)stream);
+}
+
+int llmqrt_quantize_fp8_alpha(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const float* static_scale,
+                              const float* weight_scale, uint8_t* q, float* alpha, void* workspace,
+                              llmqrt_stream_t stream) {
+  if (!weight_scale || !alpha) return llmqrt::set_error(LLMQRT_ERR_INVALID, "quantize_fp8_alpha: null pointer");
+  return llmqrt::dispatch<true>(x, x_dtype, M, K, ldx, 0, q, nullptr, alpha, 1.f, static_scale, workspace,
+                                (cudaStream_t)stream, weight_scale);
 }
 
 }  // extern "C"

@@ -11,6 +11,7 @@ from __future__ import annotations
 import torch
 
 from .. import ops
+from .._lib import fast
 from .linear_base import LinearBase, tensor_key
 
 AWQ_PACK_ORDER = [0, 2, 4, 6, 1, 3, 5, 7]
@@ -81,18 +82,15 @@ class WQLinear_GEMM(LinearBase):
             self._packed_key = key
         return self._packed
 
-    @torch.no_grad()
     def forward(self, x):
         assert x.device == self.qweight.device, "when awq linear fwd, input and qweight must be same device!"
-        out_shape = x.shape[:-1] + (self.out_features,)
-        if x.shape[0] == 0 or x.numel() == 0:
-            return torch.zeros(out_shape, dtype=x.dtype, device=x.device)
+        if x.numel() == 0:
+            return torch.zeros(x.shape[:-1] + (self.out_features,), dtype=x.dtype, device=x.device)
         input_dtype = x.dtype
-        x16 = x if input_dtype == torch.float16 else x.to(torch.float16)
-        out = ops.awq_gemm(x16.reshape(-1, self.in_features), self.packed(), self.bias)
-        if input_dtype != torch.float16:
-            out = out.to(input_dtype)
-        return out.reshape(out_shape)
+        p = self.packed()
+        if input_dtype == torch.float16:
+            return fast.awq_linear(x, p.wq_t, p.sz_t, self.bias, p.K, p.N, p.G)
+        return fast.awq_linear(x.detach().to(torch.float16), p.wq_t, p.sz_t, self.bias, p.K, p.N, p.G).to(input_dtype)
 
     def extra_repr(self) -> str:
         return "in_features={}, out_features={}, bias={}, w_bit={}, group_size={}".format(

@@ -1,5 +1,7 @@
 import torch
 
+from .._lib import fast
+
 
 class LinearBase(torch.nn.Module):
     """Common base of the quantized linear layers (ref: runtime/nn_models/modules/linear/linear_base.py)."""
@@ -10,4 +12,4 @@ class LinearBase(torch.nn.Module):
 
 def tensor_key(*tensors):
     """Identity + in-place-version key of tensors, used to invalidate caches derived from buffers."""
-    return tuple((t.data_ptr(), t._version, tuple(t.shape), t.dtype, t.device) for t in tensors if t is not None)
+    return fast.tensor_key(*tensors)

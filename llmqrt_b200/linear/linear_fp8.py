@@ -12,6 +12,7 @@ from typing import Tuple
 import torch
 
 from .. import ops
+from .._lib import fast
 from .linear_base import LinearBase, tensor_key
 
 dtype_to_str = {torch.bfloat16: "bfloat16", torch.float16: "float16"}
@@ -60,7 +61,8 @@ class _FP8Base(LinearBase):
         return self._qw
 
     def _bias_for(self, dt):
-        return None if self.bias is None else self.bias.data.to(dt)
+        bias = self.bias
+        return bias if bias is None or bias.dtype == dt else bias.data.to(dt)
 
 
 class FP8DynamicLinear(_FP8Base):
@@ -90,27 +92,18 @@ class FP8DynamicLinear(_FP8Base):
             layer.bias.data.copy_(module.bias.data.to(dtype))
         return layer
 
-    @torch.no_grad()
     def forward(self, x):
         assert x.device == self.weight.device, "when fp8 linear fwd, input and qweight must be same device!"
-        x_shape = x.shape
-        if x.shape[0] == 0 or x.numel() == 0:
+        if x.numel() == 0:
             return torch.zeros(x.shape[:-1] + (self.out_features,), dtype=x.dtype, device=x.device)
-        x2 = x.reshape(-1, x_shape[-1])
         qw = self._fp8_weight()
         if self.per_tensor:
-            qx, x_scale = ops.quantize_fp8(x2, per_token=False)
-            alpha = self.weight_scale.data.reshape(1) * x_scale                 # stays on the device
-            out = ops.fp8_linear_tensorwise(qx, qw, self._bias_for(self.dtype), alpha, 1.0, self.dtype,
-                                            static_weight=True)
-        else:
-            qx, x_scale = ops.quantize_fp8(x2, per_token=True)
-            bias = self.bias.data if self.bias is not None else None
-            if bias is not None and bias.dtype not in (torch.bfloat16, torch.float32):
-                bias = bias.float()
-            out = ops.fp8_linear_rowwise(qx, qw, bias, x_scale, self.weight_scale.data.reshape(1, -1),
-                                         static_weight=True)
-        return out.to(x.dtype).view(*x_shape[:-1], -1)
+            out = fast.fp8_per_tensor(x, qw, self._bias_for(self.dtype), self.weight_scale, None, self.dtype)
+            return out if out.dtype == x.dtype else out.to(x.dtype)
+        bias = self.bias
+        if bias is not None and bias.dtype not in (torch.bfloat16, torch.float32):
+            bias = bias.data.float()
+        return fast.fp8_per_token(x, qw, bias, self.weight_scale)
 
 
 class FP8StaticLinear(_FP8Base):
@@ -146,15 +139,10 @@ class FP8StaticLinear(_FP8Base):
     def forward(self, x):
         assert x.device == self.weight.device, "when fp8 linear fwd, input and qweight must be same device!"
         assert self.per_tensor, "[error!!] static activation quant only support per tensor!"
-        x_shape = x.shape
-        if x.shape[0] == 0 or x.numel() == 0:
+        if x.numel() == 0:
             return torch.zeros(x.shape[:-1] + (self.out_features,), dtype=x.dtype, device=x.device)
-        x2 = x.reshape(-1, x_shape[-1])
-        qx = ops.quantize_fp8_static(x2, self.input_scale.data)
-        alpha = self.weight_scale.data.reshape(1) * self.input_scale.data.reshape(1)
-        out = ops.fp8_linear_tensorwise(qx, self._fp8_weight(), self._bias_for(self.dtype), alpha, 1.0, self.dtype,
-                                        static_weight=True)
-        out = out.view(*x_shape[:-1], -1)
+        out = fast.fp8_per_tensor(x, self._fp8_weight(), self._bias_for(self.dtype), self.weight_scale, self.input_scale,
+                                  self.dtype)
         if self.quantize_output:
             qout = ops.quantize_fp8_static(out, self.output_scale.data).view(out.shape)
             out = qout.to(out.dtype) * self.output_scale.data

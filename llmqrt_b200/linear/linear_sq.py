@@ -10,6 +10,7 @@ from __future__ import annotations
 import torch
 
 from .. import ops
+from .._lib import fast
 from .linear_base import LinearBase, tensor_key
 
 
@@ -71,16 +72,10 @@ class SqW8A8BBF16OBF16PerTensor(LinearBase):
             self._bias_key = key
         return self._bias_f16
 
-    @torch.no_grad()
     def forward(self, x):
-        assert x.device == self.qweight.device, "when sq linear fwd, input and qweight must be same device!"
-        x_shape = x.shape
-        x2 = x.reshape(-1, x_shape[-1])
-        if x2.shape[0] == 0:
-            return torch.zeros(*x_shape[:-1], self.out_features, dtype=x.dtype, device=x.device)
-        qx, _, alpha = ops.quantize_int8(x2, per_token=False, scale_mul=self._weight_scale_value())
-        y = ops.int8_linear_per_tensor(qx, self.qweight, self._bias_as_f16(x.device), alpha, 1.0, static_weight=True)
-        return y.to(x.dtype).view(*x_shape[:-1], -1)
+        qweight = self.qweight
+        assert x.device == qweight.device, "when sq linear fwd, input and qweight must be same device!"
+        return fast.sq_per_tensor(x, qweight, self._bias_as_f16(x.device), self._weight_scale_value())
 
     @classmethod
     def from_linear(cls, module: torch.nn.Linear, w_bit, group_size, init_only=True, dtype=torch.float16,
@@ -124,17 +119,10 @@ class SqW8A8BBF16OBF16PerChannel(LinearBase):
             self.bias = None
         self.register_buffer("weight_scale", torch.ones(out_features, dtype=torch.float32, device=dev))
 
-    @torch.no_grad()
     def forward(self, x):
-        assert x.device == self.qweight.device, "when sq linear fwd, input and qweight must be same device!"
-        x_shape = x.shape
-        x2 = x.reshape(-1, x_shape[-1])
-        if x2.shape[0] == 0:
-            return torch.zeros(*x_shape[:-1], self.out_features, dtype=x.dtype, device=x.device)
-        qx, _, a_scale = ops.quantize_int8(x2, per_token=True)
-        y = ops.int8_linear_per_channel(qx, self.qweight, self.bias, a_scale, self.weight_scale, x.dtype,
-                                        static_weight=True)
-        return y.view(*x_shape[:-1], -1)
+        qweight = self.qweight
+        assert x.device == qweight.device, "when sq linear fwd, input and qweight must be same device!"
+        return fast.sq_per_channel(x, qweight, self.bias, self.weight_scale)
 
     def forward_quantized(self, qx: torch.Tensor, a_scale: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
         """GEMM + epilogue on activations a fused producer kernel has already quantized."""

@@ -212,13 +212,4 @@ def awq_gemm(x: torch.Tensor, packed: AwqPacked, bias=None) -> torch.Tensor:
     """C[M, N] fp16 = x[M, K] fp16 @ dequant(W) (+ bias): one fused kernel below 1024 tokens (a weight-streaming
     mma.sync kernel up to 64, the tcgen05 GEMM with in-kernel dequantization above); from 1024 tokens on the
     weights are expanded panel-wise into the workspace and multiplied by the two-CTA fp16 kernel."""
-    dev = L.require_cuda(x, packed.wq_t, bias)
-    x2 = _rows(x)
-    M, K = x2.shape
-    if K != packed.K:
-        raise RuntimeError(f"awq_gemm: x has K={K}, layer has K={packed.K}")
-    out = torch.empty((M, packed.N), dtype=torch.float16, device=dev)
-    with torch.cuda.device(dev):
-        L.call("llmqrt_awq_gemm", L.ptr(x2), x2.stride(0), L.ptr(packed.wq_t), L.ptr(packed.sz_t), L.ptr(bias),
-               L.ptr(out), packed.N, M, packed.N, K, packed.G, L.ptr(L.workspace(dev)), L.stream(dev))
-    return out
+    return L.fast.awq_linear(_rows(x), packed.wq_t, packed.sz_t, bias, packed.K, packed.N, packed.G)
