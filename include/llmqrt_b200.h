@@ -253,6 +253,17 @@ int llmqrt_attn_decode_append(const void* q, int64_t q_batch_stride, const void*
                               float* out_scale, int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d,
                               int64_t max_seqlen, float softcap, void* workspace, llmqrt_stream_t stream);
 
+/* One decode step without rotary embedding: the newest token's key and value (k_new / v_new, or NULL: already in
+ * the cache) go into row len - 1 of the caches and q attends to rows [0, min(len, max_seqlen)), where sequence
+ * b's len is (seqlens ? seqlens[b] : 0) + len_add.  The row is written wherever it lies inside the caches'
+ * cache_rows rows, also beyond max_seqlen.
+ * ref: runtime/nn_models/modules/nonlinear/attn.py:275-303. */
+int llmqrt_attn_decode_step(const void* q, int64_t q_batch_stride, const void* k_new, const void* v_new,
+                            int64_t kv_batch_stride, void* k_cache, void* v_cache, int64_t cache_batch_stride,
+                            int64_t cache_row_stride, int64_t cache_rows, const int32_t* seqlens, int32_t len_add, void* out,
+                            int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d, int64_t max_seqlen, float softcap,
+                            void* workspace, llmqrt_stream_t stream);
+
 /* Prefill attention over the new tokens: q [B, S, Hq, d], k / v [B, S, Hkv, d], out [B, S, Hq, d],
  * token stride given in elements (heads and d contiguous), causal mask optional.
  * ref: flash_attn_func call site, runtime/nn_models/modules/nonlinear/attn.py:283-298. */

@@ -55,6 +55,8 @@ _PROTOS = {
     "llmqrt_attn_decode": (c_int, [P, I64, P, P, I64, I64, P, P, P, P, I32, I64, I64, I64, I64, I64, F, P, P]),
     "llmqrt_attn_decode_append": (c_int, [P, I64, P, P, I64, P, P, I64, P, P, I64, I64, P, P, P, P, I32, I64, I64,
                                           I64, I64, I64, F, P, P]),
+    "llmqrt_attn_decode_step": (c_int, [P, I64, P, P, I64, P, P, I64, I64, I64, P, c_int32, P, I32, I64, I64, I64, I64,
+                                        I64, F, P, P]),
     "llmqrt_attn_prefill":(c_int, [P, I64, P, P, I64, P, I64, I32, I64, I64, I64, I64, I64, I32, F, P]),
     "llmqrt_rmsnorm": (c_int, [P, P, P, P, F, P, P, P, I32, I64, I64, P]),
     "llmqrt_rope_kv_write": (c_int, [P, I64, P, P, I64, P, P, I64, I64, c_int32, P, P, P, I64, I32, I64, I64, I64,
@@ -88,7 +90,7 @@ def _bind(lib: ctypes.CDLL) -> list[str]:
     return missing
 
 
-ABI_VERSION = 6          # llmqrt_abi_version() of the sources these prototypes describe
+ABI_VERSION = 7          # llmqrt_abi_version() of the sources these prototypes describe
 
 _missing = _bind(_lib)
 if not _missing and _lib.llmqrt_abi_version() != ABI_VERSION:

@@ -85,22 +85,22 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
     dev = L.require_cuda(q, k_cache, v_cache, k, v)
     if cache_seqlens is None:
         raise RuntimeError("flash_attn_with_kvcache: cache_seqlens is required")
-    if isinstance(cache_seqlens, int):
-        cache_seqlens = torch.full((B,), cache_seqlens, dtype=torch.int32, device=dev)
-    seqlens = cache_seqlens
+    if k is not None and v is None:
+        raise RuntimeError("flash_attn_with_kvcache: k and v must be given together")
     cap = k_cache.shape[1]
     bound = min(cap, max_seqlen_k) if max_seqlen_k is not None else cap
-    if k is not None:
-        if v is None:
-            raise RuntimeError("flash_attn_with_kvcache: k and v must be given together")
-        seqlens = cache_seqlens + k.shape[1]
-        if rotary:
-            Hkv = k_cache.shape[2]
-            out = attn_decode(q.reshape(B, Hq, d), k_cache, v_cache, seqlens, bound, softcap,
-                              k_new=k.to(k_cache.dtype).reshape(B, Hkv, d).contiguous(),
-                              v_new=v.to(v_cache.dtype).reshape(B, Hkv, d).contiguous(),
-                              cos=rotary_cos.float().contiguous(), sin=rotary_sin.float().contiguous())
-            return out.reshape(B, 1, Hq, d)
-        kv_append(k_cache, v_cache, k.to(k_cache.dtype), v.to(v_cache.dtype), cache_seqlens=cache_seqlens)
-    out = attn_decode(q.reshape(B, Hq, d), k_cache, v_cache, seqlens, bound, softcap)
-    return out.reshape(B, 1, Hq, d)
+    if rotary:
+        Hkv = k_cache.shape[2]
+        if isinstance(cache_seqlens, int):
+            cache_seqlens = torch.full((B,), cache_seqlens, dtype=torch.int32, device=dev)
+        out = attn_decode(q.reshape(B, Hq, d), k_cache, v_cache, cache_seqlens + 1, bound, softcap,
+                          k_new=k.to(k_cache.dtype).reshape(B, Hkv, d).contiguous(),
+                          v_new=v.to(v_cache.dtype).reshape(B, Hkv, d).contiguous(),
+                          cos=rotary_cos.float().contiguous(), sin=rotary_sin.float().contiguous())
+        return out.reshape(B, 1, Hq, d)
+    lens, add = (None, cache_seqlens) if isinstance(cache_seqlens, int) else (cache_seqlens, 0)
+    if k is not None and k.shape[1] != 1:                  # several tokens: written by a kernel of their own
+        kv_append(k_cache, v_cache, k.to(k_cache.dtype), v.to(v_cache.dtype), cache_seqlens=lens, start_pos=add)
+        return L.fast.attn_decode_step(q, k_cache, v_cache, None, None, lens, add + k.shape[1], bound, softcap)
+    return L.fast.attn_decode_step(q, k_cache, v_cache, k, v if k is not None else None, lens,
+                                   add + (1 if k is not None else 0), bound, softcap)

@@ -25,6 +25,7 @@ namespace {
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kClusterMergeMaxLen = 4096;   // longest sequence whose splits a cluster merges (512 keys per block)
 constexpr int kRing = 3;            // cp.async stages per warp (2 measured slower: too few bytes in flight)
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src) {
@@ -46,7 +47,7 @@ template <bool BF16> __device__ __forceinline__ uint32_t pack2(float a, float b)
   }
 }
 
-// Merges the split partials of sequence b (all heads) into `out` and, with out_q, quantizes the merged
+// Merges the split partials of units [u_begin, u_end) of eight outputs of sequence b (all of them with out_q) into `out` and, with out_q, quantizes the merged
 // token row to int8 with a per-token scale -- the arithmetic of the stand-alone per-token quantizer
 // applied to the 16-bit result.  Called by every thread of a block; `row_s` (shared, Hq * D 16-bit
 // words, needed only with out_q) and `red` (shared, 32 floats) are scratch.
@@ -54,12 +55,11 @@ template <bool BF16, int D>
 __device__ __forceinline__ void merge_sequence(int b, int n_splits, uint16_t* __restrict__ out, int Hq, int max_splits,
                                                const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                int8_t* __restrict__ out_q, float* __restrict__ out_scale,
-                                               uint16_t* row_s, float* red) {
+                                               uint16_t* row_s, float* red, int u_begin, int u_end) {
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
-  const int units = Hq * D / 8;
   uint16_t* orow = out + (int64_t)b * Hq * D;
   float amax = 0.f;
-  for (int u = threadIdx.x; u < units; u += blockDim.x) {
+  for (int u = u_begin + (int)threadIdx.x; u < u_end; u += blockDim.x) {
     __align__(16) T e[8];
     if (n_splits <= 1) {
       *reinterpret_cast<uint4*>(e) = __ldcg(reinterpret_cast<const uint4*>(orow + u * 8));
@@ -105,7 +105,7 @@ __device__ __forceinline__ void merge_sequence(int b, int n_splits, uint16_t* __
   float s = round_to<T>(fmaxf(amax, 1e-5f));
   s = round_to<T>(__fmul_rn(s, 1.0f / 127.0f));
   if (threadIdx.x == 0) out_scale[b] = s;
-  for (int u = threadIdx.x; u < units; u += blockDim.x) {
+  for (int u = threadIdx.x; u < u_end; u += blockDim.x) {
     __align__(16) T e[8];
     *reinterpret_cast<uint4*>(e) = *reinterpret_cast<const uint4*>(row_s + u * 8);
     __align__(8) int8_t o8[8];
@@ -130,6 +130,10 @@ struct DecodeAppend {
   const float* cos_tab;              // null: no rotation
   const float* sin_tab;
   int table_rows;
+  int len_add;                       // length of sequence b: (seqlens ? seqlens[b] : 0) + len_add
+  int merge_in_cluster;              // (host) the splits of a short sequence may be merged by a cluster
+  int cache_rows;                    // > 0: the new row is written wherever it lies inside a cache of that many rows,
+                                     // also beyond the bound of this call; 0: only within the bound
 };
 
 template <bool BF16> __device__ __forceinline__ float bits_to_f32(uint16_t h) {
@@ -148,7 +152,7 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
                    const int32_t* __restrict__ seqlens, uint16_t* __restrict__ out, int Hq, int Hkv, int chunk,
                    int max_splits, int max_len, float scale, float softcap, float* __restrict__ part_o,
                    float* __restrict__ part_ml, DecodeAppend ap, int8_t* __restrict__ out_q,
-                   float* __restrict__ out_scale, int q_cluster) {
+                   float* __restrict__ out_scale, int q_cluster, int merge_cluster) {
   constexpr int NJ = D / 32;          // 16-byte K chunks per lane (quad covers 64 B per step)
   constexpr int NH = D / 64;          // 16-byte V chunks per lane (8 lanes cover 128 B per step)
   pdl_wait();
@@ -158,10 +162,20 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
   // A length beyond the bound the grid and the partial slots were sized for (the host's max_seqlen,
   // at most the cache capacity) is clamped: the sequence is attended over its first max_len rows and
   // nothing is appended, so neither the cache nor a neighbour's partial slots are touched.
-  const int L_raw = seqlens[b];
+  const int L_raw = (seqlens ? seqlens[b] : 0) + ap.len_add;
   const int L = min(L_raw, max_len);
   const int key_begin = split * chunk;
-  if (key_begin >= L && !(L == 0 && split == 0)) return;
+  if (ap.cache_rows > 0 && split == 0 && L_raw > max_len && L_raw <= ap.cache_rows) {
+    // the new row lies beyond what this call attends to: no block covers it, the first one writes it
+    const int64_t src = (int64_t)b * ap.kv_batch_stride + (int64_t)hkv * D;
+    const int64_t dst = (int64_t)b * cache_batch_stride + (int64_t)(L_raw - 1) * cache_row_stride + (int64_t)hkv * D;
+    for (int i = threadIdx.x; i < D; i += kThreads) {
+      const_cast<uint16_t*>(k_cache)[dst + i] = ap.k_new[src + i];
+      const_cast<uint16_t*>(v_cache)[dst + i] = ap.v_new[src + i];
+    }
+  }
+  // (a block without keys leaves -- unless its cluster merges the splits and counts on it)
+  if (key_begin >= L && !(L == 0 && split == 0) && !(merge_cluster > 1 && L >= 0)) return;
   const int key_end = min(L, key_begin + chunk);
   const int n_splits = L == 0 ? 1 : (L + chunk - 1) / chunk;
 
@@ -387,6 +401,8 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
   // resident blocks over the next carve-out step and cost L1)
   uint16_t* row_bits = reinterpret_cast<uint16_t*>(ring_all + kWarps * 8 * D * 4);
   float* red_amax = reinterpret_cast<float*>(ring_all + kWarps * 8 * D * 4 + 8 * D * 2);
+  float* cl_o = red_amax + 8;                          // [rep][D] and [rep][2], see the cluster's merge
+  float* cl_ml = cl_o + 8 * D;
   float amax = 0.f;
   for (int i = tid; i < rep * D; i += kThreads) {
     const int hd = i / D, dd = i - hd * D;
@@ -403,7 +419,13 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
       }
     }
     const int hq = hkv * rep + hd;
-    if (n_splits == 1) {
+    if (merge_cluster > 1) {                           // this block's share of the heads, for the cluster's merge below
+      cl_o[i] = osum;
+      if (dd == 0) {
+        cl_ml[2 * hd] = M;
+        cl_ml[2 * hd + 1] = lsum;
+      }
+    } else if (n_splits == 1) {
       const float r = lsum > 0.f ? osum / lsum : 0.f;
       uint16_t bits;
       if constexpr (BF16) { __nv_bfloat16 hv = __float2bfloat16_rn(r); bits = *reinterpret_cast<uint16_t*>(&hv); }
@@ -421,6 +443,44 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
         part_ml[slot * 2 + 1] = lsum;
       }
     }
+  }
+  if (merge_cluster > 1) {
+    // Few, short sequences: the blocks of one (sequence, KV head) are a cluster, and every one of them merges its
+    // share of the outputs from the partials in its peers' shared memory -- no partials in global memory and no
+    // second kernel.  (28 layers of 12 / 2 heads, one sequence of 700 tokens: the merge kernel alone took 4.6 us a
+    // layer beside 4.5 us of attention.)
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    const uint32_t lo = (uint32_t)__cvta_generic_to_shared(cl_o), lml = (uint32_t)__cvta_generic_to_shared(cl_ml);
+    for (int i = split * kThreads + tid; i < rep * D; i += merge_cluster * kThreads) {
+      const int hd = i / D, dd = i - hd * D;
+      float M = -INFINITY, lsum = 0.f, osum = 0.f;
+      float pm[8], pl[8], po[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        pm[r] = -INFINITY;
+        pl[r] = po[r] = 0.f;
+        if (r < merge_cluster) {
+          uint32_t ro, rml;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ro) : "r"(lo + 4u * (uint32_t)i), "r"((uint32_t)r));
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rml) : "r"(lml + 8u * (uint32_t)hd), "r"((uint32_t)r));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(po[r]) : "r"(ro) : "memory");
+          asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(pm[r]), "=f"(pl[r]) : "r"(rml) : "memory");
+        }
+        M = fmaxf(M, pm[r]);
+      }
+      if (M > -INFINITY) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {                  // split order: the same sum on every run
+          const float f = exp2f(pm[r] - M);
+          lsum += pl[r] * f;
+          osum += po[r] * f;
+        }
+      }
+      out[((int64_t)b * Hq + hkv * rep + hd) * D + dd] = f32_to_bits<BF16>(lsum > 0.f ? osum / lsum : 0.f);
+    }
+    // nobody leaves while a peer may still read its partial
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    return;
   }
   if (out_q) {                                       // block-uniform; the arithmetic of the stand-alone per-token quantizer
     amax = warp_max(amax);
@@ -458,13 +518,13 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
   }
 }
 
-// Merge of the splits, one block per sequence.  Dynamic shared memory: Hq * D 16-bit words when out_q
-// is given.  (Letting the last block of a sequence do this inside the main kernel, counted off with
-// an atomic per block, was measured slower: the round trip of the atomic holds every block's shared
+// Merge of the splits.  With out_q one block per sequence, which then holds the whole token row (dynamic shared
+// memory: Hq * D 16-bit words).  (Letting the last block of a sequence do this inside the main kernel, counted off
+// with an atomic per block, was measured slower: the round trip of the atomic holds every block's shared
 // memory for about a microsecond and the last merges form a serial tail.)
 template <bool BF16, int D>
 __global__ void __launch_bounds__(1024)
-attn_decode_combine_kernel(const int32_t* __restrict__ seqlens, uint16_t* __restrict__ out, int Hq, int chunk,
+attn_decode_combine_kernel(const int32_t* __restrict__ seqlens, int len_add, uint16_t* __restrict__ out, int Hq, int chunk,
                            int max_splits, int max_len, const float* __restrict__ part_o,
                            const float* __restrict__ part_ml,
                            int8_t* __restrict__ out_q, float* __restrict__ out_scale) {
@@ -472,11 +532,15 @@ attn_decode_combine_kernel(const int32_t* __restrict__ seqlens, uint16_t* __rest
   __shared__ float red[32];
   pdl_wait_then_trigger();
   const int b = blockIdx.x;
-  const int L = min(seqlens[b], max_len);          // same clamp as the main kernel
+  const int L = min((seqlens ? seqlens[b] : 0) + len_add, max_len);          // same clamp as the main kernel
   const int n_splits = (L + chunk - 1) / chunk;
   if (n_splits <= 1 && !out_q) return;             // the main kernel already wrote the result
+  // without out_q the row's units of eight outputs are dealt out to the blocks of gridDim.y as well: the partials
+  // of a long sequence (28 heads x 128 x 9 splits: 129 KB) are too much for one SM to fetch (32 ragged sequences of up to 8192 tokens: 5 us of a step's 68)
+  const int units = Hq * D / 8, per = (units + (int)gridDim.y - 1) / (int)gridDim.y;
   merge_sequence<BF16, D>(b, n_splits, out, Hq, max_splits, part_o, part_ml, out_q, out_scale,
-                          reinterpret_cast<uint16_t*>(row_raw), red);
+                          reinterpret_cast<uint16_t*>(row_raw), red, (int)blockIdx.y * per,
+                          min(units, ((int)blockIdx.y + 1) * per));
 }
 
 __global__ void kv_append_kernel(uint4* __restrict__ k_cache, uint4* __restrict__ v_cache, int64_t batch_stride16,
@@ -531,20 +595,33 @@ int launch_decode(const void* q, int64_t qbs, const void* kc, const void* vc, in
   }();
   if (forced_chunk) chunk = forced_chunk;
   int max_splits = (int)ceil_div(max_seqlen > 0 ? max_seqlen : 1, chunk);
+  // Few short sequences: as many as eight splits per (sequence, KV head), merged by the cluster that they form,
+  // where all of the clusters are resident at once and a block's share stays short.  One sequence of 700 tokens,
+  // 12 / 2 heads of 128: 6.0 us in one kernel, against 4.5 + 4.6 us in 64-key splits with the merge kernel.
+  int merge_cluster = 1;
+  if (max_splits > 1 && ap.merge_in_cluster && !out_q && !forced_chunk && max_seqlen <= kClusterMergeMaxLen) {
+    const int splits = max_splits < 8 ? max_splits : 8;
+    if ((int64_t)B * Hkv * splits <= 2 * (int64_t)sm_count() - 16) {
+      chunk = (int)ceil_div(ceil_div(max_seqlen, splits), 16 * kWarps) * 16 * kWarps;
+      max_splits = (int)ceil_div(max_seqlen, chunk);
+      merge_cluster = max_splits;
+    }
+  }
   while (max_splits > 1 && (size_t)B * Hq * max_splits * (D + 2) * 4 > LLMQRT_WS_PARTIAL_BYTES) {
     chunk *= 2;
     max_splits = (int)ceil_div(max_seqlen, chunk);
   }
   float* part_o = nullptr;
   float* part_ml = nullptr;
-  if (max_splits > 1) {
+  if (max_splits > 1 && merge_cluster == 1) {
     if (!workspace) return set_error(LLMQRT_ERR_WORKSPACE, "attn_decode: split-KV needs the workspace");
     part_o = reinterpret_cast<float*>(ws_partials(workspace));
     part_ml = part_o + (size_t)B * Hq * max_splits * D;
   }
   const float scale = 1.0f / sqrtf((float)D);
   constexpr int smem = kWarps * kRing * 2 * 16 * D * 2;           // per-warp rings; also holds the 16 KiB merge tile
-  static_assert(smem >= kWarps * 8 * D * 4 + 8 * D * 2 + kWarps * 4 + 4, "ring too small for the merge tile and the quantization scratch");
+  static_assert(smem >= kWarps * 8 * D * 4 + 8 * D * 2 + 8 * 4 + 8 * D * 4 + 64, "ring too small for the merge tile and the scratch behind it");
+  static_assert(kWarps + 1 <= 8, "scratch layout");
   auto kern = attn_decode_kernel<BF16, D>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
   // No splits: the attention blocks of a sequence produce the whole token row and quantize it
@@ -553,21 +630,23 @@ int launch_decode(const void* q, int64_t qbs, const void* kc, const void* vc, in
   // exchange the row maximum through distributed shared memory.
   const bool quant_in_kernel = out_q != nullptr && Hkv <= 8 && max_splits == 1 && Hq / Hkv <= 8 && quant_fused_enabled();
   const int q_cluster = quant_in_kernel ? Hkv : 1;
-  const bool need_merge = max_splits > 1 || (out_q != nullptr && !quant_in_kernel);
-  if (int rc = launch_chained(kern, dim3(max_splits, Hkv, B), dim3(kThreads), smem, st, dim3(1, (unsigned)q_cluster, 1),
+  const bool need_merge = (max_splits > 1 && merge_cluster == 1) || (out_q != nullptr && !quant_in_kernel);
+  if (int rc = launch_chained(kern, dim3(max_splits, Hkv, B), dim3(kThreads), smem, st,
+                              dim3((unsigned)merge_cluster, (unsigned)q_cluster, 1),
                               reinterpret_cast<const uint16_t*>(q), qbs, reinterpret_cast<const uint16_t*>(kc),
                               reinterpret_cast<const uint16_t*>(vc), bs, rs, seqlens, reinterpret_cast<uint16_t*>(out),
                               Hq, Hkv, chunk, max_splits, max_seqlen, scale, softcap, part_o, part_ml, ap,
                               quant_in_kernel ? out_q : (int8_t*)nullptr, quant_in_kernel ? out_scale : (float*)nullptr,
-                              q_cluster))
+                              q_cluster, merge_cluster))
     return rc;
   if (int rc = check_launch("attn_decode")) return rc;
   if (need_merge) {
     const int units = Hq * D / 8;
-    const int threads = units >= 1024 ? 1024 : (units + 31) / 32 * 32;
+    const int cap = out_q ? 1024 : 128;
+    const int threads = units >= cap ? cap : (units + 31) / 32 * 32;
     const size_t row_smem = out_q ? (size_t)Hq * D * 2 : 0;
-    if (int rc = launch_chained(attn_decode_combine_kernel<BF16, D>, dim3(B), dim3(threads), row_smem, st, 1, seqlens,
-                                reinterpret_cast<uint16_t*>(out), Hq, chunk, max_splits, max_seqlen,
+    if (int rc = launch_chained(attn_decode_combine_kernel<BF16, D>, dim3(B, out_q ? 1u : (unsigned)ceil_div(units, cap)),
+                                dim3(threads), row_smem, st, 1, seqlens, ap.len_add, reinterpret_cast<uint16_t*>(out), Hq, chunk, max_splits, max_seqlen,
                                 static_cast<const float*>(part_o), static_cast<const float*>(part_ml), out_q,
                                 out_scale))
       return rc;
@@ -615,7 +694,7 @@ static int attn_decode_entry(const void* q, int64_t q_batch_stride, const void* 
   LLMQRT_REQUIRE(q_batch_stride >= Hq * d && q_batch_stride % 8 == 0, "attn_decode: q_batch_stride must be a multiple of 8 and at least Hq * d");
   LLMQRT_REQUIRE(!out_q || (out_scale && Hq * d <= 8192), "attn_decode: quantized output needs out_scale and Hq * d <= 8192");
   if (B == 0) return LLMQRT_OK;
-  LLMQRT_REQUIRE(q && k_cache && v_cache && seqlens && out, "attn_decode: null pointer");
+  LLMQRT_REQUIRE(q && k_cache && v_cache && (seqlens || ap.len_add > 0) && out, "attn_decode: null pointer");
   LLMQRT_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) |
                    reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(out_q) & 7) == 0, "attn_decode: pointers must be 16-byte aligned (out_q: 8)");
@@ -634,7 +713,7 @@ int llmqrt_attn_decode(const void* q, int64_t q_batch_stride, const void* k_cach
                        int64_t cache_batch_stride, int64_t cache_row_stride, const int32_t* seqlens, void* out,
                        int8_t* out_q, float* out_scale, int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d,
                        int64_t max_seqlen, float softcap, void* workspace, llmqrt_stream_t stream) {
-  const DecodeAppend none = {nullptr, nullptr, 0, nullptr, nullptr, 0};
+  const DecodeAppend none = {nullptr, nullptr, 0, nullptr, nullptr, 0, 0, 0, 0};
   return attn_decode_entry(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, cache_row_stride, seqlens, out,
                            out_q, out_scale, dtype, B, Hq, Hkv, d, max_seqlen, softcap, workspace, stream, none);
 }
@@ -654,9 +733,25 @@ int llmqrt_attn_decode_append(const void* q, int64_t q_batch_stride, const void*
                                 ((reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table)) & 7) == 0),
                  "attn_decode_append: rotary tables must be 8-byte aligned fp32 [table_rows, d/2]");
   const DecodeAppend ap = {static_cast<const uint16_t*>(k_new), static_cast<const uint16_t*>(v_new),
-                           (long long)kv_batch_stride, cos_table, sin_table, (int)table_rows};
+                           (long long)kv_batch_stride, cos_table, sin_table, (int)table_rows, 0, 0, 0};
   return attn_decode_entry(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, cache_row_stride, seqlens, out,
                            out_q, out_scale, dtype, B, Hq, Hkv, d, max_seqlen, softcap, workspace, stream, ap);
+}
+
+int llmqrt_attn_decode_step(const void* q, int64_t q_batch_stride, const void* k_new, const void* v_new,
+                            int64_t kv_batch_stride, void* k_cache, void* v_cache, int64_t cache_batch_stride,
+                            int64_t cache_row_stride, int64_t cache_rows, const int32_t* seqlens, int32_t len_add, void* out,
+                            int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d, int64_t max_seqlen, float softcap,
+                            void* workspace, llmqrt_stream_t stream) {
+  LLMQRT_REQUIRE((k_new == nullptr) == (v_new == nullptr), "attn_decode_step: k_new and v_new go together");
+  LLMQRT_REQUIRE(len_add >= 0 && cache_rows >= 0 && cache_rows <= 0x7fffffffll && max_seqlen <= cache_rows, "attn_decode_step: bad lengths");
+  LLMQRT_REQUIRE(!k_new || (kv_batch_stride >= Hkv * d && kv_batch_stride % 8 == 0 &&
+                            ((reinterpret_cast<uintptr_t>(k_new) | reinterpret_cast<uintptr_t>(v_new)) & 15) == 0),
+                 "attn_decode_step: k_new / v_new must be 16-byte aligned with a batch stride that is a multiple of 8");
+  const DecodeAppend ap = {static_cast<const uint16_t*>(k_new), static_cast<const uint16_t*>(v_new),
+                           (long long)kv_batch_stride, nullptr, nullptr, 0, (int)len_add, 1, k_new ? (int)cache_rows : 0};
+  return attn_decode_entry(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, cache_row_stride, seqlens, out,
+                           nullptr, nullptr, dtype, B, Hq, Hkv, d, max_seqlen, softcap, workspace, stream, ap);
 }
 
 }  // extern "C"

@@ -496,6 +496,52 @@ FAST_FN(attn_decode) {
   FAST_END
 }
 
+// (q [B, 1, Hq, d], k_cache, v_cache, k, v (one new token [B, 1, Hkv, d], or None), cache_seqlens or None, length added
+// to those, max_seqlen, softcap) -> out [B, 1, Hq, d]
+FAST_FN(attn_decode_step) {
+  FAST_BEGIN(9)
+  const Tensor q4 = tensor_arg(a[0], "q"), kc = tensor_arg(a[1], "k_cache"), vc = tensor_arg(a[2], "v_cache");
+  const Tensor k4 = tensor_arg(a[3], "k"), v4 = tensor_arg(a[4], "v"), lens = tensor_arg(a[5], "cache_seqlens");
+  const int64_t len_add = int_arg(a[6]), max_seqlen = int_arg(a[7]);
+  const float softcap = (float)float_arg(a[8]);
+  GilRelease gil;
+  Call c(same_device({&q4, &kc, &vc, &k4, &v4, &lens}));
+  TORCH_CHECK(q4.dim() == 4 && kc.dim() == 4 && vc.dim() == 4, "attn_decode: q must be [B, 1, Hq, d] and the caches [B, S, Hkv, d]");
+  const int64_t B = q4.size(0), Hq = q4.size(2), d = q4.size(3), Hkv = kc.size(2);
+  TORCH_CHECK(kc.stride(3) == 1 && kc.stride(2) == d && vc.strides() == kc.strides(),
+              "attn_decode: caches must be [B, S, Hkv, d] with heads and d contiguous");
+  TORCH_CHECK_TYPE(kc.scalar_type() == q4.scalar_type() && vc.scalar_type() == q4.scalar_type(),
+                   "attn_decode: q and the caches must share one dtype");
+  TORCH_CHECK_TYPE(!lens.defined() || lens.scalar_type() == at::kInt, "attn_decode: seqlens must be int32");
+  auto usable = [&](const Tensor& t, int64_t H) {
+    return t.stride(3) == 1 && t.stride(2) == d && (B <= 1 || (t.stride(0) >= H * d && t.stride(0) % 8 == 0)) &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  const Tensor q = B == 0 || usable(q4, Hq) ? q4 : q4.contiguous();
+  Tensor k, v;
+  if (k4.defined()) {
+    TORCH_CHECK(k4.dim() == 4 && v4.defined() && v4.sizes() == k4.sizes() && k4.size(0) == B && k4.size(1) == 1 &&
+                k4.size(2) == Hkv && k4.size(3) == d, "attn_decode: k and v must be [B, 1, Hkv, d]");
+    k = k4.to(kc.scalar_type());
+    v = v4.to(vc.scalar_type());
+    if (B > 0 && !(usable(k, Hkv) && usable(v, Hkv) && (B == 1 || k.stride(0) == v.stride(0)))) {
+      k = k.contiguous();
+      v = v.contiguous();
+      // (contiguous storage may still start off a 16-byte boundary)
+      if (!usable(k, Hkv)) k = k.clone();
+      if (!usable(v, Hkv)) v = v.clone();
+    }
+  }
+  Tensor out = empty(q4, q4.sizes(), q4.scalar_type());
+  check(llmqrt_attn_decode_step(ptr(q), B > 1 ? q.stride(0) : Hq * d, ptr(k), ptr(v), k.defined() && B > 1 ? k.stride(0) : Hkv * d,
+                                mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), kc.size(1),
+                                static_cast<const int32_t*>(ptr(lens)), (int32_t)len_add, mptr(out),
+                                dtype_code(q4.scalar_type()), B, Hq, Hkv, d, max_seqlen, softcap, c.workspace(), c.stream));
+  gil.done();
+  return wrap(out);
+  FAST_END
+}
+
 // (tensor or None, ...) -> identity and in-place version of the tensors, as one tuple of integers.
 FAST_FN(tensor_key) {
   HANDLE_TH_ERRORS
@@ -528,7 +574,7 @@ FAST_FN(set_workspace_maker) {
 #define FAST_DEF(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST_DEF(sq_per_channel), FAST_DEF(sq_per_tensor), FAST_DEF(fp8_per_token), FAST_DEF(fp8_per_tensor),
                          FAST_DEF(awq_linear), FAST_DEF(rmsnorm), FAST_DEF(silu_mul), FAST_DEF(rope_kv_write),
-                         FAST_DEF(attn_prefill), FAST_DEF(kv_append), FAST_DEF(attn_decode), FAST_DEF(tensor_key),
+                         FAST_DEF(attn_prefill), FAST_DEF(kv_append), FAST_DEF(attn_decode), FAST_DEF(attn_decode_step), FAST_DEF(tensor_key),
                          FAST_DEF(set_workspace_maker), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast", "Native host path of llmqrt_b200.", -1, methods,
                       nullptr, nullptr, nullptr, nullptr};

@@ -93,7 +93,9 @@ class QuantAttentionFused(nn.Module):
             xk = self.k_norm(xk)
 
         self.cache.to(xq)
-        xq, xk, xv = xq.contiguous(), xk.contiguous(), xv.contiguous()
+        if seqlen > 1 or not all(t.stride(3) == 1 and t.stride(2) == d for t in (xq, xk, xv)) or \
+                xk.stride(1) != xv.stride(1) or any(t.stride(0) != t.stride(1) for t in (xq, xk, xv)):
+            xq, xk, xv = xq.contiguous(), xk.contiguous(), xv.contiguous()    # (one token: rotated where the projection left it)
         # rotary embedding of q and k, and cache[:, start_pos : start_pos + seqlen] = (k, v), one kernel
         glue.rope_kv_write(xq, xk, xv, self.rope.cos, self.rope.sin, pos0=self.start_pos,
                            k_cache=self.cache.k[:bsz], v_cache=self.cache.v[:bsz])
@@ -102,14 +104,12 @@ class QuantAttentionFused(nn.Module):
         else:
             cap = self.cache.k.shape[1]
             if self.REFERENCE_DOUBLE_APPEND and self.start_pos + 1 < cap:
-                seqlens = torch.full((bsz,), self.start_pos + 1, dtype=torch.int32, device=xq.device)
                 output = attention.flash_attn_with_kvcache(
-                    q=xq, k=xk, k_cache=self.cache.k, v=xv, v_cache=self.cache.v, cache_seqlens=seqlens,
+                    q=xq, k=xk, k_cache=self.cache.k, v=xv, v_cache=self.cache.v, cache_seqlens=self.start_pos + 1,
                     causal=True, softcap=self.attn_logit_softcapping, max_seqlen_k=self.start_pos + 2)
             else:
-                seqlens = torch.full((bsz,), self.start_pos + 1, dtype=torch.int32, device=xq.device)
                 output = attention.flash_attn_with_kvcache(
-                    q=xq, k_cache=self.cache.k, v_cache=self.cache.v, cache_seqlens=seqlens, causal=True,
+                    q=xq, k_cache=self.cache.k, v_cache=self.cache.v, cache_seqlens=self.start_pos + 1, causal=True,
                     softcap=self.attn_logit_softcapping, max_seqlen_k=self.start_pos + 1)
         attention_weight = output.reshape(bsz, seqlen, -1)
         attn_output = self.o_proj(attention_weight)

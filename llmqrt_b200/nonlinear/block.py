@@ -8,6 +8,7 @@ import torch
 import torch.nn as nn
 
 from .attn import QuantAttentionFused
+from .norm import RMSNorm
 
 
 class LlamaLikeBlock(nn.Module):
@@ -29,8 +30,13 @@ class LlamaLikeBlock(nn.Module):
 
     def forward(self, hidden_states):
         attn_output, _, _ = self.attn.forward(hidden_states=self.norm_1(hidden_states))
-        h = hidden_states.to(attn_output.device) + attn_output
-        return h + self.mlp.forward(self.norm_2(h))
+        hidden_states = hidden_states.to(attn_output.device)
+        if type(self.norm_2) is RMSNorm:
+            h, y = self.norm_2.add(hidden_states, attn_output)
+        else:
+            h = hidden_states + attn_output
+            y = self.norm_2(h)
+        return h + self.mlp.forward(y)
 
 
 class LlamaLikeModel(nn.Module):
