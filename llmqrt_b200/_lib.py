@@ -113,10 +113,11 @@ def _load_fast():
     """The native host path (csrc/fastpath.cpp), built beside the library it calls."""
     import importlib.machinery
     import importlib.util
-    from . import build as _build
-    if not os.path.exists(_build.FAST):
+    path = os.path.join(_PKG, "lib", "_fast.so")
+    if not os.path.exists(path):
+        from . import build as _build
         _build.build()
-    loader = importlib.machinery.ExtensionFileLoader("_fast", _build.FAST)
+    loader = importlib.machinery.ExtensionFileLoader("_fast", path)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fast", loader))
     loader.exec_module(module)
     return module

@@ -207,12 +207,13 @@ __device__ __forceinline__ float block_reduce_once(float v) {
   return r;
 }
 
-// silu in T: the quotient gate / (1 + e^-gate) as the approximate reciprocal (1 ulp of fp32) times gate,
-// then the rounding to 16 bits that dwarfs both.
+// silu in T: the special-function unit's exponential and reciprocal (each within 2 ulp of fp32), then the rounding
+// to 16 bits that dwarfs both.
 template <typename T>
 __device__ __forceinline__ float silu_f32(float g) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + expf(-g)));
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
   return g * r;
 }
 
