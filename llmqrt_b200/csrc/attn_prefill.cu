@@ -39,6 +39,7 @@
 #include "tc_primitives.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace llmqrt {
 namespace {
@@ -287,27 +288,36 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     // The whole warp runs the loop; only the tcgen05 instructions themselves are issued by one elected lane.
     if (n_max > 0) {
       bool ok = tc::mbar_wait_warp(tc::smem_u32(&bar_q), 0u, abort);
+      // The instructions of a product are issued back to back by one elected lane, their descriptors a constant
+      // apart from a base made once: with an election and two descriptors per instruction the warp, which shares
+      // its scheduler with two softmax warps, could not issue as fast as the tensor pipe multiplies.
       // S_w = Q_w K^T: both operands K-major; D / 16 instructions of K = 16
       auto issue_s = [&](int w, int st) {
-        const uint32_t qa = tc::smem_u32(sQ + w * kTile), ka = tc::smem_u32(sK + st * kTile);
+        const uint64_t da = tc::smem_desc_k_major_sw128(tc::smem_u32(sQ + w * kTile));
+        const uint64_t db = tc::smem_desc_k_major_sw128(tc::smem_u32(sK + st * kTile));
         const uint32_t d_tmem = tmem_base + kColS + (uint32_t)(w * 128);
+        if (tc::elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint32_t off = (uint32_t)((ks / 4) * kSubBytes + (ks % 4) * 32);
-          const uint64_t da = tc::smem_desc_k_major_sw128(qa + off), db = tc::smem_desc_k_major_sw128(ka + off);
-          if (tc::elect_one()) tc::mma_ss<tc::MMA_F16>(d_tmem, da, db, prm.idesc_s, ks > 0 ? 1u : 0u);
+          for (int ks = 0; ks < D / 16; ++ks) {
+            constexpr uint64_t kSubUnits = kSubBytes >> 4;       // (descriptor addresses count 16 bytes)
+            const uint64_t off = (uint64_t)(ks / 4) * kSubUnits + (uint64_t)(ks % 4) * 2;
+            tc::mma_ss<tc::MMA_F16>(d_tmem, da + off, db + off, prm.idesc_s, ks > 0 ? 1u : 0u);
+          }
+          tc::mma_commit(tc::smem_u32(&bar_s_full[w]));
         }
-        if (tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_s_full[w]));
+        __syncwarp();
       };
       // O_w = P_w V: P from tensor memory (8 packed columns per 16 keys), V MN-major (16 key rows per step)
-      auto issue_pv = [&](int w, int st, int j, int t_begin, int t_end) {
-        const uint32_t va = tc::smem_u32(sV + st * kTile);
+      auto issue_pv = [&](int w, int st, int j, auto t_begin, auto t_end) {
+        const uint64_t db = smem_desc_mn_major_sw128(tc::smem_u32(sV + st * kTile), kSubBytes, 1024);
         const uint32_t d_tmem = tmem_base + kColO + (uint32_t)(w * 128), a_tmem = tmem_base + kColS + (uint32_t)(w * 128);
+        if (tc::elect_one()) {
 #pragma unroll
-        for (int t = t_begin; t < t_end; ++t) {
-          const uint64_t db = smem_desc_mn_major_sw128(va + (uint32_t)(t * 16 * 128), kSubBytes, 1024);
-          if (tc::elect_one()) mma_ts_f16(d_tmem, a_tmem + (uint32_t)(t * 8), db, prm.idesc_pv, (j > 0 || t > 0) ? 1u : 0u);
+          for (int t = t_begin; t < t_end; ++t)
+            mma_ts_f16(d_tmem, a_tmem + (uint32_t)(t * 8), db + (uint64_t)(t * (16 * 128 >> 4)), prm.idesc_pv,
+                       (j > 0 || t > 0) ? 1u : 0u);
         }
+        __syncwarp();
       };
       // the last query tile that reads key tile t (the second one sees at least as many tiles as the
       // first, unless it lies beyond the sequence altogether)
@@ -327,10 +337,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           if (!tc::mbar_wait_warp(tc::smem_u32(&bar_p_ready[w]), (uint32_t)j & 1u, abort)) { ok = false; break; }
           if (!tc::mbar_wait_warp(tc::smem_u32(&bar_v_full[vs]), vph, abort)) { ok = false; break; }
           tc::fence_after_sync();
-          issue_pv(w, vs, j, 0, kPvFirst);
+          issue_pv(w, vs, j, std::integral_constant<int, 0>(), std::integral_constant<int, kPvFirst>());
           if (!tc::mbar_wait_warp(tc::smem_u32(&bar_p_rest[w]), (uint32_t)j & 1u, abort)) { ok = false; break; }
           tc::fence_after_sync();
-          issue_pv(w, vs, j, kPvFirst, kRows / 16);
+          issue_pv(w, vs, j, std::integral_constant<int, kPvFirst>(), std::integral_constant<int, kRows / 16>());
           if (j == n_tiles[w] - 1 && tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_o_full[w]));     // last tile: O complete
           if (w == last_user(j) && tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_v_empty[vs]));      // V_j free once these retire
           if (j + 1 < n_tiles[w]) {
