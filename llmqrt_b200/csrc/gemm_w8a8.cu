@@ -35,7 +35,7 @@ int run(int kind, const void* a, int64_t lda, const void* w, int64_t ldw, int64_
   const bool stream = path == 1 || (path == 0 && M <= kStreamMaxM);
   if (stream)
     return w8a8_gemm_stream(kind, reinterpret_cast<const uint8_t*>(a), lda, reinterpret_cast<const uint8_t*>(w), ldw,
-                            M, N, K, epi, workspace, st);
+                            M, N, K, epi, workspace, st, (flags & LLMQRT_GEMM_STATIC_WEIGHT) != 0);
   return gemm_tc(kind, a, lda, w, ldw, M, N, K, epi, workspace, st, (flags & LLMQRT_GEMM_STATIC_WEIGHT) != 0);
 }
 

@@ -15,7 +15,7 @@ enum GemmKind : int {
 
 // Register-operand streaming kernel (gemm_stream.cu): any M, tuned for M <= 16.
 int w8a8_gemm_stream(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N,
-                     int64_t K, const Epilogue& epi, void* workspace, cudaStream_t st);
+                     int64_t K, const Epilogue& epi, void* workspace, cudaStream_t st, bool static_w);
 
 // TMA + tcgen05/TMEM kernel (gemm_tc.cu): any M; lda/ldw in elements.  static_w: W is a stored weight
 // that nothing queued on the stream writes, so its first tiles may be requested before the

@@ -1,0 +1,28 @@
+"""The int8 / fp8 GEMM of at most 16 tokens at the edges of its blocks and chunks."""
+import pytest
+import torch
+
+from tests.util import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(1, 16), (15, 48), (16, 64), (17, 80), (40, 1040), (4864, 896), (3584, 18944), (24000, 272)])
+def test_few_tokens(M, N, K):
+    """Ragged K (a chunk of 64 bytes cut short), N off the 16-row block, every number of warps: exact for int8."""
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    want = a.double() @ w.double().t()
+    assert torch.equal(ops.int8_gemm_s32(a, w).double(), want)
+    s, ws = torch.rand(M, generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
+    bias = torch.randn(N, generator=g, device="cuda").half()
+    y = ops.int8_linear_per_channel(a, w, bias, s, ws, torch.bfloat16, True)
+    ref = (want.float() * ws * s[:, None] + bias.float()).bfloat16()
+    assert torch.equal(y, ref)
+    x8 = torch.randn(M, K, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    w8 = torch.randn(N, K, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    y = ops.fp8_linear_rowwise(x8, w8, None, s.view(M, 1), ws.view(1, N))
+    assert rel_fro(y, (x8.double() @ w8.double().t()) * s[:, None] * ws) < 2 ** -8      # bf16 result
