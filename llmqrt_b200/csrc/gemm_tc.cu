@@ -1235,6 +1235,29 @@ cudaLaunchConfig_t make_config(int grid, int cluster, cudaStream_t st, cudaLaunc
   return cfg;
 }
 
+// Estimated microseconds of the two schedules for more than 128 tokens, fitted to times measured over N = 896 .. 37888,
+// K = 896 .. 18944 and M = 160 .. 1024 (within 10 %): both are bound by what one SM can fetch from L2 (about
+// 105 GB/s), 32 KiB per K block of 128 bytes and CTA -- for a 128 x 128 tile in panels, for half of a 256 x 256
+// tile in pairs.  panel_us also picks the cluster size of the split (1 .. 8) where `splits` asks for it; `active`
+// says how many clusters of a size fit the device (without it: one CTA per SM).
+double pair_us(int64_t tiles, int k_blocks) {
+  return 2.2 + (double)ceil_div(tiles, sm_count() / 2) * (0.297 * k_blocks + 3.5);
+}
+double panel_us(int64_t tiles, int k_blocks, int* splits, int (*active)(int) = nullptr) {
+  double best = 5.2 + (double)ceil_div(tiles, sm_count()) * (0.306 * k_blocks + 1.7);
+  if (splits) *splits = 1;
+  for (int s = 2; s <= 8 && k_blocks >= 2 * s && tiles < sm_count(); ++s) {
+    const int n = active ? active(s) : sm_count() / s;
+    if (n <= 0) continue;
+    const double t = 5.2 + (double)ceil_div(tiles, n) * (0.306 * k_blocks / s + 5.2);
+    if (t < best) {
+      best = t;
+      if (splits) *splits = s;
+    }
+  }
+  return best;
+}
+
 // How many clusters of `cluster` CTAs of this kernel can be resident at once (cached per device).
 template <int KIND, int BN, bool AWQ = false, bool PUSH = false>
 int max_active_clusters(int cluster) {
@@ -1272,7 +1295,8 @@ int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& 
     // reduce-scatter and epilogue).
     const float fixed = 8.f;
     float best = (float)ceil_div(tiles, sms) * ((float)prm.k_blocks + fixed);
-    for (int s = 2; s <= 8; ++s) {                     // (any size: 36 tiles fit as clusters of three, not of four)
+    if (prm.tiles_q > 1 && !AWQ) panel_us(tiles, prm.k_blocks, &splits, max_active_clusters<KIND, BN, AWQ, PUSH>);
+    else for (int s = 2; s <= 8; ++s) {                     // (any size: 36 tiles fit as clusters of three, not of four)
       if (prm.k_blocks < 2 * s || BN / 8 < s) continue;
       const int active = max_active_clusters<KIND, BN, AWQ, PUSH>(s);
       if (active <= 0) continue;
@@ -1389,16 +1413,27 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   LLMQRT_REQUIRE((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0,
                  "tcgen05 gemm: operands must be 16-byte aligned");
 
-  // A mid-sized M with a narrow N has only a handful of 128 x 256 tiles, and that schedule has no
-  // split-K: most SMs would idle (M = 256, N = 1536, K = 8960: 12 tiles).  Such problems run through
-  // the small-M schedule instead -- weights as the 128-lane operand, tokens in panels of 128 as the
-  // column operand, cluster split-K -- as ONE launch whose grid covers every (weight tile, token
-  // panel) pair; neighbouring clusters share a weight tile, so the panels after the first read it
-  // from L2.
+  // More than 128 tokens: the two-CTA kernel wherever its vector stores may be used (16-byte aligned output rows),
+  // unless the small-M schedule -- weights as the 128-lane operand, tokens in panels of 128 as the column operand,
+  // cluster split-K -- is estimated to be faster, as it is where few 256 x 256 tiles meet a long reduction
+  // (M = 160, N = 896, K = 4864: 11.7 us in panels, 16.4 us in pairs; M = 160, N = K = 3584: 15.1 against 14.0).
+  // The 128 x 256 tiles of a lone CTA feed 48 KiB per K block through one SM's share of L2 (28 us at
+  // M = 160 .. 640, N = K = 3584): they are left to the outputs that neither can serve.
+  const int es = (epi.mode == EPI_RAW || epi.out_dtype == LLMQRT_F32) ? 4 : 2;
+  const bool out_ok = (reinterpret_cast<uintptr_t>(epi.out) & 15) == 0 && (epi.ldo * es) % 16 == 0;
+  const int k_blocks = (int)ceil_div(K * elt, kRowBytes);
+  const bool pair_ok = !awq && !push && M > 128 && N > 128 && out_ok && pair_enabled();
   bool panels = false;
   if (M > 128 && M <= 1024) {
-    const int64_t tiles = ceil_div(M, (int64_t)kBM) * ceil_div(N, (int64_t)(N <= 128 ? 128 : 256));
-    panels = tiles * 4 <= sm_count();
+    const int64_t panel_tiles = ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM);
+    if (pair_ok) {
+      panels = panel_us(panel_tiles, k_blocks, nullptr) < pair_us(ceil_div(M, (int64_t)256) * ceil_div(N, (int64_t)256), k_blocks);
+    } else if (awq) {
+      const int64_t tiles = ceil_div(M, (int64_t)kBM) * ceil_div(N, (int64_t)(N <= 128 ? 128 : 256));
+      panels = tiles * 4 <= sm_count();
+    } else {
+      panels = true;
+    }
   }
 
   TcParams prm{};
@@ -1408,7 +1443,8 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   prm.early_w = static_w ? 1 : 0;
   prm.swap = (M <= 128 || panels) ? 1 : 0;
   int bn;
-  if (prm.swap) bn = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
+  // (4-bit weights: 64 columns also for few tokens, so that the reduction may be split in eight instead of four)
+  if (prm.swap) bn = M <= 32 && !awq ? 32 : (M <= 64 ? 64 : 128);
   else bn = N <= 128 ? 128 : 256;
   if (awq && !prm.swap) {
     // AWQ with many tokens: the weights stay the 128-lane operand and the tokens come in tiles of 256.
@@ -1442,24 +1478,17 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   else if (kind == KIND_F16) { mk = tc::MMA_F16; }
   else if (kind == KIND_BF16) { mk = tc::MMA_F16; fmt_act = fmt_w = 1; }
 
-  // Prefill-sized problems whose 256-row pair tiles waste no more rows than 128-row tiles would: the
-  // two-CTA kernel.  Its vector stores need a 16-byte aligned output with a 16-byte multiple row pitch.
-  {
-    const int es = (epi.mode == EPI_RAW || epi.out_dtype == LLMQRT_F32) ? 4 : 2;
-    const bool out_ok = (reinterpret_cast<uintptr_t>(epi.out) & 15) == 0 && (epi.ldo * es) % 16 == 0;
-    const bool rows_ok = M >= 2048 || ceil_div(M, (int64_t)256) * 256 == ceil_div(M, (int64_t)128) * 128;
-    if (!awq && !prm.swap && bn == 256 && M >= 512 && rows_ok && out_ok && pair_enabled()) {
-      prm.tiles_p = (int)ceil_div(M, (int64_t)(2 * kBM));
-      prm.tiles_q = (int)ceil_div(N, (int64_t)kPairBN);
-      prm.idesc = tc::instr_desc(c_fmt, fmt_act, fmt_w, 2 * kBM, kPairBN);
-      prm.store32 = ((reinterpret_cast<uintptr_t>(epi.out) & 31) == 0 && (epi.ldo * es) % 32 == 0) ? 1 : 0;
-      CUtensorMap tm_a, tm_w;
-      if (int rc = make_operand_map(&tm_a, A, elt, M, K, lda, kBM)) return rc;
-      if (int rc = make_operand_map(&tm_w, W, elt, N, K, ldw, kPairHalfB)) return rc;
-      if (mk == tc::MMA_I8) return launch_pair<tc::MMA_I8>(tm_a, tm_w, prm, st);
-      if (mk == tc::MMA_F8) return launch_pair<tc::MMA_F8>(tm_a, tm_w, prm, st);
-      return launch_pair<tc::MMA_F16>(tm_a, tm_w, prm, st);
-    }
+  if (pair_ok && !panels) {
+    prm.tiles_p = (int)ceil_div(M, (int64_t)(2 * kBM));
+    prm.tiles_q = (int)ceil_div(N, (int64_t)kPairBN);
+    prm.idesc = tc::instr_desc(c_fmt, fmt_act, fmt_w, 2 * kBM, kPairBN);
+    prm.store32 = ((reinterpret_cast<uintptr_t>(epi.out) & 31) == 0 && (epi.ldo * es) % 32 == 0) ? 1 : 0;
+    CUtensorMap tm_a, tm_w;
+    if (int rc = make_operand_map(&tm_a, A, elt, M, K, lda, kBM)) return rc;
+    if (int rc = make_operand_map(&tm_w, W, elt, N, K, ldw, kPairHalfB)) return rc;
+    if (mk == tc::MMA_I8) return launch_pair<tc::MMA_I8>(tm_a, tm_w, prm, st);
+    if (mk == tc::MMA_F8) return launch_pair<tc::MMA_F8>(tm_a, tm_w, prm, st);
+    return launch_pair<tc::MMA_F16>(tm_a, tm_w, prm, st);
   }
   prm.idesc = tc::instr_desc(c_fmt, prm.swap ? fmt_w : fmt_act, prm.swap ? fmt_act : fmt_w, kBM, (uint32_t)bn);
 

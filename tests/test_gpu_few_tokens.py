@@ -26,3 +26,19 @@ def test_few_tokens(M, N, K):
     w8 = torch.randn(N, K, generator=g, device="cuda").to(torch.float8_e4m3fn)
     y = ops.fp8_linear_rowwise(x8, w8, None, s.view(M, 1), ws.view(1, N))
     assert rel_fro(y, (x8.double() @ w8.double().t()) * s[:, None] * ws) < 2 ** -8      # bf16 result
+
+
+@pytest.mark.parametrize("M", [129, 160, 255, 257, 333, 512, 640, 1025, 1100])
+@pytest.mark.parametrize("N,K", [(40, 1040), (136, 64), (896, 4864), (1000, 1536), (1001, 512), (1536, 8960), (4864, 896)])
+def test_chunk_schedules(M, N, K):
+    """Two-CTA tiles, token panels with and without a split, and output rows (N = 1001) no vector store can write:
+    whichever the size selects, the int32 sums are exact."""
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    want = a.double() @ w.double().t()
+    assert torch.equal(ops.int8_gemm_s32(a, w).double(), want)
+    s, ws = torch.rand(M, generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
+    y = ops.int8_linear_per_channel(a, w, None, s, ws, torch.float16, True)
+    assert torch.equal(y, (want.float() * ws * s[:, None]).half())

@@ -1,0 +1,30 @@
+"""Prompt attention at the edges of its 64-key halves and 128-row tiles, with maxima that keep moving."""
+import pytest
+import torch
+
+from tests.util import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("S", [1, 63, 64, 65, 127, 128, 129, 192, 193, 255, 256, 257, 320, 385, 641])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("dt,d,growth", [(torch.float16, 128, 0), (torch.bfloat16, 64, 0), (torch.float16, 64, 40), (torch.float16, 128, 40),
+                                         (torch.bfloat16, 128, -40)])
+def test_prefill_halves(S, causal, dt, d, growth):
+    """growth: the score rises (falls) by that many powers of e over every 64 keys, so a row's reference maximum moves
+    in every half and the accumulator is rescaled while a product may be on its way (or never again)."""
+    from llmqrt_b200.attention import flash_attn_func
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(2, S, h, d, generator=g, device="cuda") for h in (4, 2, 2))
+    if growth:
+        q[..., 0] = 8.0
+        k[..., 0] = growth * d ** 0.5 / 8 * torch.arange(S, device="cuda")[None, :, None] / 64
+    q, k, v = (t.to(dt) for t in (q, k, v))
+    out = flash_attn_func(q, k, v, causal=causal)
+    s = torch.einsum("bshd,bthd->bhst", q.double(), k.double().repeat_interleave(2, 2)) * d ** -0.5
+    if causal:
+        s.masked_fill_(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.einsum("bhst,bthd->bshd", s.softmax(-1), v.double().repeat_interleave(2, 2))
+    # P and the result are rounded to 16 bits: 2^-11 (fp16) or 2^-8 (bf16) each at most
+    assert rel_fro(out, want) < (1e-3 if dt == torch.float16 else 8e-3)
