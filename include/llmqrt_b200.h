@@ -188,6 +188,13 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
                     void* out, int64_t ldo, int64_t M, int64_t N, int64_t K, int64_t group_size, void* workspace,
                     llmqrt_stream_t stream);
 
+/* The same for at most 16 tokens with the next step of a decoder block done on the sums, rounded to fp16 in between:
+ * residual given: out[m, n] = residual[m, n] + y[m, n];  residual NULL: the layer's rows are N / 2 gate rows and
+ * N / 2 up rows, out[m, n] = silu(y[m, n]) * y[m, N / 2 + n] (N a multiple of 16). */
+int llmqrt_awq_gemm_tail(const void* x, int64_t ldx, const uint32_t* wq_t, const uint32_t* sz_t, const void* bias,
+                         const void* residual, int64_t ldr, void* out, int64_t ldo, int64_t M, int64_t N, int64_t K,
+                         int64_t group_size, llmqrt_stream_t stream);
+
 /* Dequantize the repacked layer to W^T fp16 [N, K] (K contiguous), the operand layout of the
  * tcgen05 fp16 GEMM used for large M. */
 int llmqrt_awq_dequantize_t(const uint32_t* wq_t, const uint32_t* sz_t, int64_t K, int64_t N, int64_t group_size,
@@ -253,16 +260,18 @@ int llmqrt_attn_decode_append(const void* q, int64_t q_batch_stride, const void*
                               float* out_scale, int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d,
                               int64_t max_seqlen, float softcap, void* workspace, llmqrt_stream_t stream);
 
-/* One decode step without rotary embedding: the newest token's key and value (k_new / v_new, or NULL: already in
- * the cache) go into row len - 1 of the caches and q attends to rows [0, min(len, max_seqlen)), where sequence
- * b's len is (seqlens ? seqlens[b] : 0) + len_add.  The row is written wherever it lies inside the caches'
- * cache_rows rows, also beyond max_seqlen.
+/* One decode step: the newest token's key and value (k_new / v_new, or NULL: already in the cache) go into row
+ * len - 1 of the caches and q attends to rows [0, min(len, max_seqlen)), where sequence b's len is
+ * (seqlens ? seqlens[b] : 0) + len_add.  The row is written wherever it lies inside the caches' cache_rows rows,
+ * also beyond max_seqlen.  With cos / sin tables q and the new key are rotated first, at angle row len - 1 - twice;
+ * twice = 1 writes the new row to len - 2 as well (the reference appends a token it has already written).
  * ref: runtime/nn_models/modules/nonlinear/attn.py:275-303. */
 int llmqrt_attn_decode_step(const void* q, int64_t q_batch_stride, const void* k_new, const void* v_new,
-                            int64_t kv_batch_stride, void* k_cache, void* v_cache, int64_t cache_batch_stride,
-                            int64_t cache_row_stride, int64_t cache_rows, const int32_t* seqlens, int32_t len_add, void* out,
-                            int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d, int64_t max_seqlen, float softcap,
-                            void* workspace, llmqrt_stream_t stream);
+                            int64_t kv_batch_stride, const float* cos_table, const float* sin_table, int64_t table_rows,
+                            int twice, void* k_cache, void* v_cache, int64_t cache_batch_stride, int64_t cache_row_stride,
+                            int64_t cache_rows, const int32_t* seqlens, int32_t len_add, void* out, int dtype, int64_t B,
+                            int64_t Hq, int64_t Hkv, int64_t d, int64_t max_seqlen, float softcap, void* workspace,
+                            llmqrt_stream_t stream);
 
 /* Prefill attention over the new tokens: q [B, S, Hq, d], k / v [B, S, Hkv, d], out [B, S, Hq, d],
  * token stride given in elements (heads and d contiguous), causal mask optional.

@@ -49,14 +49,15 @@ _PROTOS = {
     "llmqrt_awq_dequantize": (c_int, [P, P, P, I64, I64, I64, P, P]),
     "llmqrt_awq_repack": (c_int, [P, P, P, I64, I64, I64, P, P, P]),
     "llmqrt_awq_gemm": (c_int, [P, I64, P, P, P, P, I64, I64, I64, I64, I64, P, P]),
+    "llmqrt_awq_gemm_tail": (c_int, [P, I64, P, P, P, P, I64, P, I64, I64, I64, I64, I64, P]),
     "llmqrt_awq_dequantize_t": (c_int, [P, P, I64, I64, I64, P, P]),
     "llmqrt_gemm_16bit": (c_int, [P, I64, P, I64, P, P, I64, I32, I64, I64, I64, P, P]),
     "llmqrt_kv_append": (c_int, [P, P, I64, I64, P, P, P, c_int32, I32, I64, I64, I64, I64, I64, P]),
     "llmqrt_attn_decode": (c_int, [P, I64, P, P, I64, I64, P, P, P, P, I32, I64, I64, I64, I64, I64, F, P, P]),
     "llmqrt_attn_decode_append": (c_int, [P, I64, P, P, I64, P, P, I64, P, P, I64, I64, P, P, P, P, I32, I64, I64,
                                           I64, I64, I64, F, P, P]),
-    "llmqrt_attn_decode_step": (c_int, [P, I64, P, P, I64, P, P, I64, I64, I64, P, c_int32, P, I32, I64, I64, I64, I64,
-                                        I64, F, P, P]),
+    "llmqrt_attn_decode_step": (c_int, [P, I64, P, P, I64, P, P, I64, I32, P, P, I64, I64, I64, P, c_int32, P, I32,
+                                        I64, I64, I64, I64, I64, F, P, P]),
     "llmqrt_attn_prefill":(c_int, [P, I64, P, P, I64, P, I64, I32, I64, I64, I64, I64, I64, I32, F, P]),
     "llmqrt_rmsnorm": (c_int, [P, P, P, P, F, P, P, P, I32, I64, I64, P]),
     "llmqrt_rope_kv_write": (c_int, [P, I64, P, P, I64, P, P, I64, I64, c_int32, P, P, P, I64, I32, I64, I64, I64,
@@ -90,7 +91,7 @@ def _bind(lib: ctypes.CDLL) -> list[str]:
     return missing
 
 
-ABI_VERSION = 7          # llmqrt_abi_version() of the sources these prototypes describe
+ABI_VERSION = 8          # llmqrt_abi_version() of the sources these prototypes describe
 
 _missing = _bind(_lib)
 if not _missing and _lib.llmqrt_abi_version() != ABI_VERSION:

@@ -101,6 +101,16 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
     lens, add = (None, cache_seqlens) if isinstance(cache_seqlens, int) else (cache_seqlens, 0)
     if k is not None and k.shape[1] != 1:                  # several tokens: written by a kernel of their own
         kv_append(k_cache, v_cache, k.to(k_cache.dtype), v.to(v_cache.dtype), cache_seqlens=lens, start_pos=add)
-        return L.fast.attn_decode_step(q, k_cache, v_cache, None, None, lens, add + k.shape[1], bound, softcap)
+        return L.fast.attn_decode_step(q, k_cache, v_cache, None, None, lens, add + k.shape[1], bound, softcap,
+                                       None, None, False)
     return L.fast.attn_decode_step(q, k_cache, v_cache, k, v if k is not None else None, lens,
-                                   add + (1 if k is not None else 0), bound, softcap)
+                                   add + (1 if k is not None else 0), bound, softcap, None, None, False)
+
+
+def decode_rotary_step(q, k, v, k_cache, v_cache, cos, sin, pos: int, twice: bool = False, softcap: float = 0.0):
+    """One kernel for a decode step whose sequences all stand at row `pos`: q and k [B, 1, H, d] are rotated at angle
+    row `pos` (neither tensor changes), k and v are written to cache row pos -- with `twice` to row pos + 1 as well --
+    and q attends to everything up to the last row written."""
+    _check_common(q, None)
+    n = pos + (2 if twice else 1)
+    return L.fast.attn_decode_step(q, k_cache, v_cache, k, v, None, n, n, softcap, cos, sin, twice)

@@ -130,6 +130,7 @@ struct DecodeAppend {
   const float* cos_tab;              // null: no rotation
   const float* sin_tab;
   int table_rows;
+  int twice;                         // 1: the new row is also written one row earlier, and its angle is that row's
   int len_add;                       // length of sequence b: (seqlens ? seqlens[b] : 0) + len_add
   int merge_in_cluster;              // (host) the splits of a short sequence may be merged by a cluster
   int cache_rows;                    // > 0: the new row is written wherever it lies inside a cache of that many rows,
@@ -194,12 +195,12 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
   }
 
   // ---- newest token: rotate q in registers; the block that covers its cache row writes K and V ----
-  const int pos = L - 1;
-  const bool rotate = ap.cos_tab != nullptr && pos >= 0 && pos < ap.table_rows;
+  const int pos = L - 1, angle = pos - ap.twice;
+  const bool rotate = ap.cos_tab != nullptr && angle >= 0 && angle < ap.table_rows;
   if (rotate) {
     // chunk 4j+t pairs with chunk 4(j + NJ/2)+t: element i with i + D/2, both held by this thread
-    const float* cr = ap.cos_tab + (int64_t)pos * (D / 2);
-    const float* sr = ap.sin_tab + (int64_t)pos * (D / 2);
+    const float* cr = ap.cos_tab + (int64_t)angle * (D / 2);
+    const float* sr = ap.sin_tab + (int64_t)angle * (D / 2);
 #pragma unroll
     for (int j = 0; j < NJ / 2; ++j) {
       const int i0 = 8 * (4 * j + t);
@@ -219,26 +220,29 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
   }
   // (block-uniform condition; like the stand-alone rotary kernel, a position outside the table
   // leaves the cache untouched)
-  if (ap.k_new != nullptr && L_raw <= max_len && pos >= key_begin && pos < key_end &&
+  if (ap.k_new != nullptr && L_raw <= max_len && pos >= key_begin && pos - ap.twice < key_end &&
       (ap.cos_tab == nullptr || rotate)) {
     const int64_t src = (int64_t)b * ap.kv_batch_stride + (int64_t)hkv * D;
-    const int64_t dst = (int64_t)b * cache_batch_stride + (int64_t)pos * cache_row_stride + (int64_t)hkv * D;
     uint16_t* kc = const_cast<uint16_t*>(k_cache);
     uint16_t* vc = const_cast<uint16_t*>(v_cache);
-    if (tid < D / 2) {
-      const float a = bits_to_f32<BF16>(ap.k_new[src + tid]), bb = bits_to_f32<BF16>(ap.k_new[src + tid + D / 2]);
-      float c = 1.f, sn = 0.f;
-      if (rotate) {
-        c = ap.cos_tab[(int64_t)pos * (D / 2) + tid];
-        sn = ap.sin_tab[(int64_t)pos * (D / 2) + tid];
+    for (int row = max(pos - ap.twice, key_begin); row <= pos && row < key_end; ++row) {
+      if (row < 0) continue;
+      const int64_t dst = (int64_t)b * cache_batch_stride + (int64_t)row * cache_row_stride + (int64_t)hkv * D;
+      if (tid < D / 2) {
+        const float a = bits_to_f32<BF16>(ap.k_new[src + tid]), bb = bits_to_f32<BF16>(ap.k_new[src + tid + D / 2]);
+        float c = 1.f, sn = 0.f;
+        if (rotate) {
+          c = ap.cos_tab[(int64_t)angle * (D / 2) + tid];
+          sn = ap.sin_tab[(int64_t)angle * (D / 2) + tid];
+        }
+        kc[dst + tid] = rotate ? f32_to_bits<BF16>(a * c - bb * sn) : ap.k_new[src + tid];
+        kc[dst + tid + D / 2] = rotate ? f32_to_bits<BF16>(a * sn + bb * c) : ap.k_new[src + tid + D / 2];
+      } else if (tid < D / 2 + D / 8) {
+        const int i = (tid - D / 2) * 8;
+        *reinterpret_cast<uint4*>(vc + dst + i) = *reinterpret_cast<const uint4*>(ap.v_new + src + i);
       }
-      kc[dst + tid] = rotate ? f32_to_bits<BF16>(a * c - bb * sn) : ap.k_new[src + tid];
-      kc[dst + tid + D / 2] = rotate ? f32_to_bits<BF16>(a * sn + bb * c) : ap.k_new[src + tid + D / 2];
-    } else if (tid < D / 2 + D / 8) {
-      const int i = (tid - D / 2) * 8;
-      *reinterpret_cast<uint4*>(vc + dst + i) = *reinterpret_cast<const uint4*>(ap.v_new + src + i);
     }
-    __syncthreads();                               // the row is in place before any warp of the block fetches it
+    __syncthreads();                               // the rows are in place before any warp of the block fetches them
   }
 
   float o[NH][8][4];
@@ -713,7 +717,7 @@ int llmqrt_attn_decode(const void* q, int64_t q_batch_stride, const void* k_cach
                        int64_t cache_batch_stride, int64_t cache_row_stride, const int32_t* seqlens, void* out,
                        int8_t* out_q, float* out_scale, int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d,
                        int64_t max_seqlen, float softcap, void* workspace, llmqrt_stream_t stream) {
-  const DecodeAppend none = {nullptr, nullptr, 0, nullptr, nullptr, 0, 0, 0, 0};
+  const DecodeAppend none = {nullptr, nullptr, 0, nullptr, nullptr, 0, 0, 0, 0, 0};
   return attn_decode_entry(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, cache_row_stride, seqlens, out,
                            out_q, out_scale, dtype, B, Hq, Hkv, d, max_seqlen, softcap, workspace, stream, none);
 }
@@ -733,23 +737,31 @@ int llmqrt_attn_decode_append(const void* q, int64_t q_batch_stride, const void*
                                 ((reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table)) & 7) == 0),
                  "attn_decode_append: rotary tables must be 8-byte aligned fp32 [table_rows, d/2]");
   const DecodeAppend ap = {static_cast<const uint16_t*>(k_new), static_cast<const uint16_t*>(v_new),
-                           (long long)kv_batch_stride, cos_table, sin_table, (int)table_rows, 0, 0, 0};
+                           (long long)kv_batch_stride, cos_table, sin_table, (int)table_rows, 0, 0, 0, 0};
   return attn_decode_entry(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, cache_row_stride, seqlens, out,
                            out_q, out_scale, dtype, B, Hq, Hkv, d, max_seqlen, softcap, workspace, stream, ap);
 }
 
 int llmqrt_attn_decode_step(const void* q, int64_t q_batch_stride, const void* k_new, const void* v_new,
-                            int64_t kv_batch_stride, void* k_cache, void* v_cache, int64_t cache_batch_stride,
-                            int64_t cache_row_stride, int64_t cache_rows, const int32_t* seqlens, int32_t len_add, void* out,
-                            int dtype, int64_t B, int64_t Hq, int64_t Hkv, int64_t d, int64_t max_seqlen, float softcap,
-                            void* workspace, llmqrt_stream_t stream) {
+                            int64_t kv_batch_stride, const float* cos_table, const float* sin_table, int64_t table_rows,
+                            int twice, void* k_cache, void* v_cache, int64_t cache_batch_stride, int64_t cache_row_stride,
+                            int64_t cache_rows, const int32_t* seqlens, int32_t len_add, void* out, int dtype, int64_t B,
+                            int64_t Hq, int64_t Hkv, int64_t d, int64_t max_seqlen, float softcap, void* workspace,
+                            llmqrt_stream_t stream) {
   LLMQRT_REQUIRE((k_new == nullptr) == (v_new == nullptr), "attn_decode_step: k_new and v_new go together");
+  LLMQRT_REQUIRE((cos_table == nullptr) == (sin_table == nullptr), "attn_decode_step: cos and sin tables go together");
   LLMQRT_REQUIRE(len_add >= 0 && cache_rows >= 0 && cache_rows <= 0x7fffffffll && max_seqlen <= cache_rows, "attn_decode_step: bad lengths");
+  LLMQRT_REQUIRE((twice == 0 || twice == 1) && (!(twice || cos_table) || (k_new && !seqlens && len_add <= max_seqlen)),
+                 "attn_decode_step: rotation and the doubled row need k_new and one length within max_seqlen");
   LLMQRT_REQUIRE(!k_new || (kv_batch_stride >= Hkv * d && kv_batch_stride % 8 == 0 &&
                             ((reinterpret_cast<uintptr_t>(k_new) | reinterpret_cast<uintptr_t>(v_new)) & 15) == 0),
                  "attn_decode_step: k_new / v_new must be 16-byte aligned with a batch stride that is a multiple of 8");
+  LLMQRT_REQUIRE(!cos_table || (table_rows > 0 && table_rows <= 0x7fffffffll &&
+                                ((reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table)) & 7) == 0),
+                 "attn_decode_step: rotary tables must be 8-byte aligned fp32 [table_rows, d/2]");
   const DecodeAppend ap = {static_cast<const uint16_t*>(k_new), static_cast<const uint16_t*>(v_new),
-                           (long long)kv_batch_stride, nullptr, nullptr, 0, (int)len_add, 1, k_new ? (int)cache_rows : 0};
+                           (long long)kv_batch_stride, cos_table, sin_table, (int)table_rows, twice, (int)len_add, 1,
+                           k_new ? (int)cache_rows : 0};
   return attn_decode_entry(q, q_batch_stride, k_cache, v_cache, cache_batch_stride, cache_row_stride, seqlens, out,
                            nullptr, nullptr, dtype, B, Hq, Hkv, d, max_seqlen, softcap, workspace, stream, ap);
 }

@@ -12,11 +12,9 @@
 // Dequantization is then  (h + (-(1024+zero))) * scale  = exactly fp16((v - zero) * scale): the
 // subtraction is exact and the product is rounded once, like the reference's kernels.
 //
-// The decode-sized GEMM (M <= 64) is computed transposed (weights are the 16-row MMA operand, tokens the
-// 8-column one), each warp owns 32 weight rows so that one activation fragment feeds two weight
-// fragments, and the reduction dimension is split across blocks with a deterministic last-arriver
-// fix-up.  Above 64 tokens the same entry point runs the TMA + tcgen05 GEMM kernel with the weight
-// operand dequantized tile by tile into shared memory by extra warps of that kernel (gemm_tc.cu).
+// The GEMM has three forms: a weight-streaming kernel of warp-level MMAs for few tokens (below), the TMA + tcgen05
+// GEMM with the weight operand dequantized tile by tile into shared memory by extra warps (gemm_tc.cu) up to 128
+// tokens, and above that the expansion of the weights, panel by panel, ahead of the dense tcgen05 GEMM.
 #include "gemm_w8a8.cuh"
 
 namespace llmqrt {
@@ -86,210 +84,175 @@ __device__ __forceinline__ void dequant_word(uint32_t w, __half2 negz, __half2 s
   }
 }
 
+// A thread expands kDequantWords words a block's width apart: loads of 128 and stores of 512 contiguous bytes
+// per warp, several of each in flight, 32-bit index arithmetic.  With one word per thread and
+// 64-bit divisions the expansion of 17920 x 1536 (14 MB read, 55 MB written) took 21.5 us; so it takes 13.8.
+constexpr int kDequantWords = 4;
 __global__ void __launch_bounds__(256)
-awq_dequantize_t_kernel(const uint32_t* __restrict__ wq_t, const uint32_t* __restrict__ sz_t, int64_t KW, int64_t N,
-                        int64_t G, __half* __restrict__ out) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= N * KW) return;
-  const int64_t n = idx / KW, j = idx - n * KW;
-  const uint32_t szv = sz_t[n * (KW * 8 / G) + (8 * j) / G];
-  const __half2 sz = *reinterpret_cast<const __half2*>(&szv);
-  uint32_t o[4];
-  dequant_word(wq_t[idx], __half2half2(__high2half(sz)), __half2half2(__low2half(sz)), o);
-  *reinterpret_cast<uint4*>(out + idx * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+awq_dequantize_t_kernel(const uint32_t* __restrict__ wq_t, const uint32_t* __restrict__ sz_t, uint32_t KW, uint32_t total,
+                        uint32_t words_per_group, uint32_t KG, __half* __restrict__ out) {
+  pdl_wait_then_trigger();
+  const uint32_t i0 = blockIdx.x * (256u * kDequantWords) + threadIdx.x;
+  uint32_t w[kDequantWords], szv[kDequantWords];
+#pragma unroll
+  for (int k = 0; k < kDequantWords; ++k) {
+    const uint32_t idx = i0 + 256u * k;
+    if (idx < total) {
+      const uint32_t n = idx / KW, j = idx - n * KW;
+      w[k] = __ldg(wq_t + idx);
+      szv[k] = __ldg(sz_t + (size_t)n * KG + j / words_per_group);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kDequantWords; ++k) {
+    const uint32_t idx = i0 + 256u * k;
+    if (idx < total) {
+      const __half2 sz = *reinterpret_cast<const __half2*>(&szv[k]);
+      uint32_t o[4];
+      dequant_word(w[k], __half2half2(__high2half(sz)), __half2half2(__low2half(sz)), o);
+      *reinterpret_cast<uint4*>(out + (size_t)idx * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
 }
 
-// ---- streaming dequant-GEMM -------------------------------------------------------------------------
-constexpr int kThreads = 128;          // 4 warps
-constexpr int kRowsPerWarp = 32;
-constexpr int kRowsPerBlock = 128;
+int launch_dequantize_t(const uint32_t* wq_t, const uint32_t* sz_t, int64_t K, int64_t N, int64_t G, __half* out, cudaStream_t st) {
+  const int64_t max_rows = ((1ll << 31) - 256 * kDequantWords) / (K / 8);     // (indices of a launch fit 32 bits)
+  LLMQRT_REQUIRE(max_rows > 0, "awq_dequantize_t: K too large");
+  for (int64_t n0 = 0; n0 < N; n0 += max_rows) {
+    const int64_t total = (N - n0 < max_rows ? N - n0 : max_rows) * (K / 8);
+    if (int rc = launch_chained(awq_dequantize_t_kernel, dim3((unsigned)ceil_div(total, 256 * kDequantWords)), dim3(256), 0, st, 1,
+                                wq_t + n0 * (K / 8), sz_t + n0 * (K / G), (uint32_t)(K / 8), (uint32_t)total,
+                                (uint32_t)(G / 8), (uint32_t)(K / G), out + n0 * K))
+      return rc;
+    if (int rc = check_launch("awq_dequantize_t")) return rc;
+  }
+  return LLMQRT_OK;
+}
+
+// ---- dequant-GEMM of few tokens ---------------------------------------------------------------------
+// Computed transposed: weights are the 16-row MMA operand, tokens the 8-column one.  One block owns 16 weight rows
+// over the WHOLE reduction dimension: its warps take the 128-value chunks of K in turn and their sums meet in shared
+// memory, so there are no partials in global memory, no arrival counter and no last block that adds the slices up.
+// Activations (a few rows) come straight from L2, no staging and no barrier before the first weights; the weights of
+// kRowsAhead chunks of a warp are in flight together, and 64 registers a thread keep two 512-thread blocks on an SM.
+// Latency-bound: a 17920 x 1536 layer (14 MB) at one token is 2 us of HBM time.  Weights from HBM, against 128-row
+// blocks with the slices of K in separate blocks: 17920 x 1536 at one token 8.0 us (11.1), 1536 x 8960 7.5 (12.1),
+// 2048 x 1536 2.6 (6.0), 3584 x 18944 20.0 (22.5); 16 tokens 16.4 (14.7), 12.4 (19.4), 3.8 (10.6), 33.7 us (35.3).
 constexpr int kChunkK = 128;           // k-values per warp step: 4 lanes x 32 per weight row
-
-// Activation slice in shared memory: row stride = kps*2 + 16 bytes and 16-byte chunk c stored at
-// c ^ (((c >> 3) & 1) << 1), which makes the eight lanes of every 128-bit load phase hit 32 distinct banks.
-__host__ __device__ inline int xs_stride_bytes(int kps) { return kps * 2 + 16; }
-__device__ __forceinline__ int xs_chunk(int c) { return c ^ (((c >> 3) & 1) << 1); }
-
-template <int MB>
-__global__ void __launch_bounds__(kThreads)
-awq_gemm_stream_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* __restrict__ wq_t,
-                       const uint32_t* __restrict__ sz_t, int M, int N, int K, int G, int kps, int num_splits,
-                       float* __restrict__ partials, int* __restrict__ counters, Epilogue epi) {
-  extern __shared__ __align__(16) uint8_t xs[];
-  __shared__ int s_ticket;
+constexpr int kRowsAhead = 2;
+//
+// What follows the GEMM in a decoder block may be done on its sums (each step rounded to fp16 as the separate kernels
+// round it): TAIL_RESIDUAL adds a row of the residual stream, TAIL_SILU makes the 16 rows of a block eight gate and
+// the eight up rows half a layer apart and stores silu(gate) * up.
+enum RowsTail { TAIL_NONE, TAIL_RESIDUAL, TAIL_SILU };
+template <int MB, int TAIL>
+__global__ void __launch_bounds__(512, MB <= 2 ? 2 : 1)
+awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* __restrict__ wq_t,
+                     const uint32_t* __restrict__ sz_t, int M, int N, int K, int G, int chunks, Epilogue epi,
+                     const __half* __restrict__ residual, int64_t ldr) {
+  extern __shared__ __align__(16) float red[];         // [warp][token][16 rows]
+  pdl_wait_then_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int k_begin = blockIdx.y * kps;
-  const int k_len = min(kps, K - k_begin);        // multiple of 32
-  const int stride = xs_stride_bytes(kps);
+  const int warps = blockDim.x >> 5, n0 = blockIdx.x * (TAIL == TAIL_SILU ? 8 : 16);
   const int KW = K / 8, KG = K / G;
-
-  {
-    const int chunks = kps / 8;                   // 16-byte chunks (8 halves) per row
-    for (int i = tid; i < MB * 8 * chunks; i += kThreads) {
-      const int r = i / chunks, c = i - r * chunks;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < M && c * 8 < k_len) v = *reinterpret_cast<const uint4*>(X + (int64_t)r * ldx + k_begin + c * 8);
-      *reinterpret_cast<uint4*>(xs + r * stride + xs_chunk(c) * 16) = v;
-    }
-  }
-  __syncthreads();
-
-  const int n0 = blockIdx.x * kRowsPerBlock + warp * kRowsPerWarp;
-  float acc[2][MB][4];
+  const int second = TAIL == TAIL_SILU ? N / 2 : 8;    // (N / 2 is a multiple of eight: whole blocks)
+  const int rows[2] = {min(n0 + g, N - 1), min(n0 + g + second, N - 1)};
+  float acc[MB][4];
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+  for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
-    for (int i = 0; i < MB; ++i)
+    for (int j = 0; j < 4; ++j) acc[mb][j] = 0.f;
+  for (int c0 = warp; c0 < chunks; c0 += warps * kRowsAhead) {
+    uint4 w[kRowsAhead][2];
+    uint32_t sz[kRowsAhead][2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[h][i][j] = 0.f;
-
-  if (n0 < N) {
-    // rows handled by this lane: n0 + 16h + g and n0 + 16h + g + 8
-    int rows[4];
+    for (int i = 0; i < kRowsAhead; ++i) {
+      const int kk = (c0 + i * warps) * kChunkK + 32 * t;      // this lane's 32 values of the chunk: one group
+      const bool valid = kk < K;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) rows[r] = min(n0 + 16 * (r >> 1) + g + 8 * (r & 1), N - 1);
-    const int my_len = k_len - 32 * t;
-
-    // The weights of step kc + 1 are requested before step kc is consumed (two register sets), so a
-    // block's steps overlap their load latency instead of paying it one after the other.
-    uint4 wnext[4];
-    uint32_t sznext[4];
-    auto fetch = [&](int kc) {
-      const bool valid = kc < my_len;
-      const int kk = k_begin + kc + 32 * t;       // first k of this lane's 32 values
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < 2; ++r) {
+        w[i][r] = make_uint4(0u, 0u, 0u, 0u);
+        sz[i][r] = 0u;                                         // scale 0: contributes nothing
         if (valid) {
-          wnext[r] = ldg_stream_16B(wq_t + (int64_t)rows[r] * KW + kk / 8);
-          sznext[r] = __ldg(sz_t + (int64_t)rows[r] * KG + kk / G);
-        } else {
-          wnext[r] = make_uint4(0, 0, 0, 0);
-          sznext[r] = 0;                            // scale 0: contributes nothing
-        }
-      }
-    };
-    fetch(0);
-    for (int kc = 0; kc < k_len; kc += kChunkK) {
-      uint4 wv[4];
-      uint32_t szv[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        wv[r] = wnext[r];
-        szv[r] = sznext[r];
-      }
-      if (kc + kChunkK < k_len) fetch(kc + kChunkK);
-      const uint32_t* wp[4] = {&wv[0].x, &wv[1].x, &wv[2].x, &wv[3].x};
-#pragma unroll
-      for (int wi = 0; wi < 4; ++wi) {
-        uint32_t a[4][4];                           // [row][pair]
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const __half2 sz = *reinterpret_cast<const __half2*>(&szv[r]);
-          dequant_word(wp[r][wi], __half2half2(__high2half(sz)), __half2half2(__low2half(sz)), a[r]);
-        }
-        const int c = (kc + 32 * t) / 8 + wi;       // 16-byte chunk of the activation row
-#pragma unroll
-        for (int mb = 0; mb < MB; ++mb) {
-          const uint4 x = *reinterpret_cast<const uint4*>(xs + (mb * 8 + g) * stride + xs_chunk(c) * 16);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            mma_16816<false>(acc[h][mb], a[2 * h][0], a[2 * h + 1][0], a[2 * h][1], a[2 * h + 1][1], x.x, x.y);
-            mma_16816<false>(acc[h][mb], a[2 * h][2], a[2 * h + 1][2], a[2 * h][3], a[2 * h + 1][3], x.z, x.w);
-          }
+          w[i][r] = ldg_stream_16B(wq_t + (int64_t)rows[r] * KW + kk / 8);
+          sz[i][r] = __ldg(sz_t + (int64_t)rows[r] * KG + kk / G);
         }
       }
     }
-  }
-
-  const float alpha = 1.f;
-  auto for_each_acc = [&](auto&& fn) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int i = 0; i < kRowsAhead; ++i) {
+      if (c0 + i * warps >= chunks) break;
+      const int kk = (c0 + i * warps) * kChunkK + 32 * t;
+      uint4 x[MB][4];                                          // tokens mb * 8 + g
 #pragma unroll
       for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = n0 + 16 * h + g + (j >> 1) * 8, m = mb * 8 + 2 * t + (j & 1);
-          if (n < N && m < M) fn(acc[h][mb][j], m, n);
+        for (int wi = 0; wi < 4; ++wi) {
+          x[mb][wi] = make_uint4(0u, 0u, 0u, 0u);
+          if (kk < K && mb * 8 + g < M)
+            x[mb][wi] = *reinterpret_cast<const uint4*>(X + (int64_t)(mb * 8 + g) * ldx + kk + 8 * wi);
         }
-  };
-
-  if (num_splits == 1) {
-    if (n0 < N) for_each_acc([&](float v, int m, int n) { epilogue_store<float>(epi, v, m, n, alpha); });
-    return;
-  }
-  if (n0 < N) {
-    float* mine = partials + (int64_t)blockIdx.y * M * N;
-    for_each_acc([&](float v, int m, int n) { mine[(int64_t)m * N + n] = v; });
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_ticket = atomicAdd(&counters[blockIdx.x], 1);
-  __syncthreads();
-  if (s_ticket != num_splits - 1) return;
-  __threadfence();
-  // N is a multiple of 8: four columns per thread, slices four at a time (independent loads, so the
-  // fix-up costs a few L2 round trips instead of one per slice and element)
-  const int nb0 = blockIdx.x * kRowsPerBlock;
-  constexpr int kVecs = kRowsPerBlock / 4;
-  if (M < 4) {                                     // too few rows to keep every thread busy with vectors
-    for (int i = tid; i < M * kRowsPerBlock; i += kThreads) {
-      const int m = i / kRowsPerBlock, n = nb0 + (i % kRowsPerBlock);
-      if (n >= N) continue;
-      float sum = 0.f;
-#pragma unroll 4
-      for (int s = 0; s < num_splits; ++s) sum += __ldcg(partials + ((int64_t)s * M + m) * N + n);
-      epilogue_store<float>(epi, sum, m, n, alpha);
-    }
-    if (tid == 0) counters[blockIdx.x] = 0;
-    return;
-  }
-  for (int i = tid; i < M * kVecs; i += kThreads) {
-    const int m = i / kVecs, n = nb0 + (i % kVecs) * 4;
-    if (n >= N) continue;
-    float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int s = 0; s < num_splits; ++s) {
-      const float4 p = __ldcg(reinterpret_cast<const float4*>(partials + ((int64_t)s * M + m) * N + n));
-      sum[0] += p.x; sum[1] += p.y; sum[2] += p.z; sum[3] += p.w;
-    }
+      const uint32_t wr[2][4] = {{w[i][0].x, w[i][0].y, w[i][0].z, w[i][0].w}, {w[i][1].x, w[i][1].y, w[i][1].z, w[i][1].w}};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) epilogue_store<float>(epi, sum[j], m, n + j, alpha);
+      for (int wi = 0; wi < 4; ++wi) {
+        uint32_t a[2][4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const __half2 s2 = *reinterpret_cast<const __half2*>(&sz[i][r]);
+          dequant_word(wr[r][wi], __half2half2(__high2half(s2)), __half2half2(__low2half(s2)), a[r]);
+        }
+#pragma unroll
+        for (int mb = 0; mb < MB; ++mb) {
+          mma_16816<false>(acc[mb], a[0][0], a[1][0], a[0][1], a[1][1], x[mb][wi].x, x[mb][wi].y);
+          mma_16816<false>(acc[mb], a[0][2], a[1][2], a[0][3], a[1][3], x[mb][wi].z, x[mb][wi].w);
+        }
+      }
+    }
   }
-  if (tid == 0) counters[blockIdx.x] = 0;
+  float* mine = red + warp * MB * 128;
+#pragma unroll
+  for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mine[(mb * 8 + 2 * t + (j & 1)) * 16 + g + 8 * (j >> 1)] = acc[mb][j];
+  __syncthreads();
+  auto total = [&](int i) {
+    float sum = 0.f;
+    for (int v = 0; v < warps; ++v) sum += red[v * MB * 128 + i];           // (warp order: the same sum on every run)
+    return sum;
+  };
+  if constexpr (TAIL == TAIL_SILU) {
+    for (int i = tid; i < M * 8; i += blockDim.x) {
+      const int m = i >> 3, r = i & 7, n = n0 + r;
+      const float gate = round_to<__half>(epilogue_value(epi, total(m * 16 + r), m, n, 1.f));
+      const float up = round_to<__half>(epilogue_value(epi, total(m * 16 + 8 + r), m, n + second, 1.f));
+      reinterpret_cast<__half*>(epi.out)[m * epi.ldo + n] = from_f32<__half>(round_to<__half>(silu_f32(gate)) * up);
+    }
+  } else {
+    for (int i = tid; i < M * 16; i += blockDim.x) {
+      const int m = i >> 4, n = n0 + (i & 15);
+      if (n >= N) continue;
+      if constexpr (TAIL == TAIL_RESIDUAL) {
+        const float v = round_to<__half>(epilogue_value(epi, total(i), m, n, 1.f));
+        reinterpret_cast<__half*>(epi.out)[m * epi.ldo + n] = from_f32<__half>(to_f32<__half>(residual[m * ldr + n]) + v);
+      } else {
+        epilogue_store<float>(epi, total(i), m, n, 1.f);
+      }
+    }
+  }
 }
 
-template <int MB>
-int launch_gemm(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32_t* sz_t, int M, int N, int K, int G,
-                const Epilogue& epi, void* workspace, cudaStream_t st) {
-  const int n_blocks = (int)ceil_div(N, kRowsPerBlock);
-  const int max_kps_smem = ((96 * 1024) / (MB * 8) - 16) / 2 / kChunkK * kChunkK;
-  // enough blocks to cover every SM about four times, but at most 16 slices: the block that arrives
-  // last adds them all, and that serial tail outweighs finer slices
-  int want_splits = (int)ceil_div(4 * sm_count(), n_blocks);
-  if (want_splits > 16) want_splits = 16;
-  int kps = (int)ceil_div(ceil_div(K, want_splits), kChunkK) * kChunkK;
-  if (kps < 256) kps = 256;
-  if (kps > max_kps_smem) kps = max_kps_smem;
-  if (kps > (int)ceil_div(K, kChunkK) * kChunkK) kps = (int)ceil_div(K, kChunkK) * kChunkK;
-  int splits = (int)ceil_div(K, kps);
-  while (splits > 1 && (size_t)splits * M * N * 4 > LLMQRT_WS_PARTIAL_BYTES) {
-    kps += kChunkK;
-    if (kps > max_kps_smem) return set_error(LLMQRT_ERR_WORKSPACE, "awq gemm: partial sums do not fit the workspace");
-    splits = (int)ceil_div(K, kps);
-  }
-  if (splits > 1) {
-    if (!workspace) return set_error(LLMQRT_ERR_WORKSPACE, "awq gemm: split-K needs the workspace");
-    if (n_blocks > LLMQRT_WS_NUM_COUNTERS) return set_error(LLMQRT_ERR_INVALID, "awq gemm: N too large");
-  }
-  const size_t smem = (size_t)MB * 8 * xs_stride_bytes(kps);
-  auto kern = awq_gemm_stream_kernel<MB>;
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem)) return rc;
-  kern<<<dim3(n_blocks, splits), kThreads, smem, st>>>(
-      X, ldx, wq_t, sz_t, M, N, K, G, kps, splits,
-      workspace ? reinterpret_cast<float*>(ws_partials(workspace)) : nullptr,
-      workspace ? ws_counters(workspace) : nullptr, epi);
-  return check_launch("awq_gemm_stream");
+template <int MB, int TAIL = TAIL_NONE>
+int launch_rows(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32_t* sz_t, int M, int N, int K, int G,
+                const Epilogue& epi, cudaStream_t st, const __half* residual, int64_t ldr) {
+  const int blocks = (int)ceil_div(N, 16), chunks = (int)ceil_div(K, kChunkK);
+  // warps per block: about 40 per SM in all, at least four, at most one per chunk
+  int warps = (int)ceil_div(40 * sm_count(), blocks);
+  warps = warps < 4 ? 4 : warps > 16 ? 16 : warps;
+  if (warps > chunks) warps = chunks;
+  if (int rc = launch_chained(awq_gemm_rows_kernel<MB, TAIL>, dim3((unsigned)blocks), dim3((unsigned)(32 * warps)), (size_t)warps * MB * 512, st, 1,
+                              X, ldx, wq_t, sz_t, M, N, K, G, chunks, epi, residual, ldr))
+    return rc;
+  return check_launch("awq_gemm_rows");
 }
 
 int check_layer(int64_t K, int64_t N, int64_t G) {
@@ -337,9 +300,7 @@ int llmqrt_awq_dequantize_t(const uint32_t* wq_t, const uint32_t* sz_t, int64_t 
   if (int rc = check_layer(K, N, group_size)) return rc;
   LLMQRT_REQUIRE(K % 8 == 0 && group_size % 8 == 0, "awq_dequantize_t: K and group size must be multiples of 8");
   LLMQRT_REQUIRE(wq_t && sz_t && out, "awq_dequantize_t: null pointer");
-  awq_dequantize_t_kernel<<<(unsigned)ceil_div(N * (K / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      wq_t, sz_t, K / 8, N, group_size, reinterpret_cast<__half*>(out));
-  return check_launch("awq_dequantize_t");
+  return launch_dequantize_t(wq_t, sz_t, K, N, group_size, reinterpret_cast<__half*>(out), (cudaStream_t)stream);
 }
 
 int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint32_t* sz_t, const void* bias,
@@ -357,20 +318,21 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   e.ldo = ldo;
   const __half* xp = reinterpret_cast<const __half*>(x);
   cudaStream_t st = (cudaStream_t)stream;
-  if (M >= 1024 && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0) {
-    // A thousand tokens and more: the GEMM is compute-bound, the two-CTA fp16 kernel runs about twice
-    // as fast as the kernel that dequantizes into its own shared memory (whose dequantizing warps and
-    // tensor core share the SM's shared-memory bandwidth), and writing the fp16 weights out once and
-    // reading them back costs a tenth of the GEMM.  The weights are expanded panel by panel into the
-    // workspace (same rounding: fp16((v - z) * s)) and each panel is multiplied by the dense kernel.
+  // More than 128 tokens: the weights are expanded panel by panel into the workspace (same rounding:
+  // fp16((v - z) * s)) and each panel is multiplied by the dense kernel, whose tensor core is not held up by the
+  // dequantizing warps' traffic in the same shared memory.  256 / 512 tokens: 17920 x 1536 25 / 34 us (fused 31 / 51),
+  // 4608 x 3584 28 / 29 (30 / 49), 3584 x 18944 88 / 127 (101 / 197).  A layer of more than one panel travels to HBM
+  // and back as fp16, which only pays from about 640 tokens on: 37888 x 3584 at 256 / 512 / 768 tokens 132 / 174 / 219
+  // us against 93 / 166 / 238.  (Panels of 64 MB, which would stay in L2, are worse: 113 us for 3584 x 18944 at 256.)
+  const bool one_panel = N * K * 2 <= (int64_t)LLMQRT_WS_PARTIAL_BYTES;
+  if (M > 128 && (one_panel || M >= 640) && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0) {
     const int64_t cap_rows = (int64_t)(LLMQRT_WS_PARTIAL_BYTES / (size_t)(K * 2)) / 256 * 256;
     if (cap_rows >= 256) {
       __half* deq = reinterpret_cast<__half*>(ws_partials(workspace));
       for (int64_t n0 = 0; n0 < N; n0 += cap_rows) {
         const int64_t nc = (N - n0 < cap_rows) ? (N - n0) : cap_rows;
-        awq_dequantize_t_kernel<<<(unsigned)ceil_div(nc * (K / 8), 256), 256, 0, st>>>(
-            wq_t + n0 * (K / 8), sz_t + n0 * (K / group_size), K / 8, nc, group_size, deq);
-        if (int rc = check_launch("awq_dequantize_t")) return rc;
+        if (int rc = launch_dequantize_t(wq_t + n0 * (K / 8), sz_t + n0 * (K / group_size), K, nc, group_size, deq, st))
+          return rc;
         Epilogue ep = e;
         ep.out = reinterpret_cast<__half*>(out) + n0;
         ep.bias = bias ? reinterpret_cast<const __half*>(bias) + n0 : nullptr;
@@ -379,25 +341,42 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
       return LLMQRT_OK;
     }
   }
-  if (M > 64) {
-    // 64 < M < 1024: ONE kernel.  The tcgen05 GEMM runs with four extra warps that turn the
-    // packed 4-bit tiles into fp16 operand tiles in shared memory (same rounding: fp16((v - z) * s)),
-    // so the dequantized weights never exist in global memory.
-    e.out = out;
-    const AwqOperand op = {wq_t, sz_t, group_size};
-    return gemm_tc(KIND_F16, x, ldx, nullptr, 0, M, N, K, e, workspace, st, false, &op);
+  if (M <= 0) return LLMQRT_OK;
+  e.out = out;
+  // At most 16 tokens, and up to 32 where the layer is narrow enough for the activations, which every block of 16
+  // rows fetches, not to outweigh the weights: 32 tokens 1536 x 8960 15.0 us (tcgen05 17.3), 4608 x 3584 15.4
+  // (19.3), 3584 x 18944 52 (50), 17920 x 1536 25.8 (19.2).
+  if (M <= 16 || (M <= 32 && N <= 64 * (int64_t)sm_count())) {
+    auto go = M <= 8 ? launch_rows<1> : M <= 16 ? launch_rows<2> : launch_rows<4>;
+    return go(xp, ldx, wq_t, sz_t, (int)M, (int)N, (int)K, (int)group_size, e, st, nullptr, 0);
   }
-  for (int64_t m0 = 0; m0 < M; m0 += 32) {       // token panels of 32: larger M re-streams the weights per panel
-    const int mc = (int)((M - m0 < 32) ? (M - m0) : 32);
-    e.out = reinterpret_cast<__half*>(out) + m0 * ldo;
-    const __half* xr = xp + m0 * ldx;
-    int rc;
-    if (mc <= 8) rc = launch_gemm<1>(xr, ldx, wq_t, sz_t, mc, (int)N, (int)K, (int)group_size, e, workspace, st);
-    else if (mc <= 16) rc = launch_gemm<2>(xr, ldx, wq_t, sz_t, mc, (int)N, (int)K, (int)group_size, e, workspace, st);
-    else rc = launch_gemm<4>(xr, ldx, wq_t, sz_t, mc, (int)N, (int)K, (int)group_size, e, workspace, st);
-    if (rc) return rc;
-  }
-  return LLMQRT_OK;
+  // ONE kernel: the tcgen05 GEMM runs with extra warps that turn the packed 4-bit tiles into fp16 operand tiles in
+  // shared memory (same rounding), so the dequantized weights never exist in global memory.
+  const AwqOperand op = {wq_t, sz_t, group_size};
+  return gemm_tc(KIND_F16, x, ldx, nullptr, 0, M, N, K, e, workspace, st, false, &op);
+}
+
+int llmqrt_awq_gemm_tail(const void* x, int64_t ldx, const uint32_t* wq_t, const uint32_t* sz_t, const void* bias,
+                         const void* residual, int64_t ldr, void* out, int64_t ldo, int64_t M, int64_t N, int64_t K,
+                         int64_t group_size, llmqrt_stream_t stream) {
+  if (int rc = check_layer(K, N, group_size)) return rc;
+  const bool silu = residual == nullptr;
+  const int64_t cols = silu ? N / 2 : N;
+  LLMQRT_REQUIRE(x && wq_t && sz_t && out, "awq_gemm_tail: null pointer");
+  LLMQRT_REQUIRE(M > 0 && M <= 16, "awq_gemm_tail: M = %lld is outside [1, 16]", (long long)M);
+  LLMQRT_REQUIRE(K % 32 == 0 && group_size % 32 == 0 && (!silu || N % 16 == 0), "awq_gemm_tail: K and group size must be "
+                 "multiples of 32, N of 16");
+  LLMQRT_REQUIRE(ldx >= K && ldx % 8 == 0 && ldo >= cols && (silu || ldr >= cols), "awq_gemm_tail: bad leading dimension");
+  LLMQRT_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(wq_t) & 15) == 0,
+                 "awq_gemm_tail: operands must be 16-byte aligned");
+  Epilogue e{};
+  e.mode = EPI_TENSOR; e.out_dtype = LLMQRT_F16; e.bias_dtype = LLMQRT_F16; e.alpha = 1.f; e.beta = 1.f; e.bias = bias;
+  e.ldo = ldo; e.out = out;
+  const __half* r = reinterpret_cast<const __half*>(residual);
+  auto go = M <= 8 ? (silu ? launch_rows<1, TAIL_SILU> : launch_rows<1, TAIL_RESIDUAL>)
+                   : (silu ? launch_rows<2, TAIL_SILU> : launch_rows<2, TAIL_RESIDUAL>);
+  return go(reinterpret_cast<const __half*>(x), ldx, wq_t, sz_t, (int)M, (int)N, (int)K, (int)group_size, e,
+            (cudaStream_t)stream, r, ldr);
 }
 
 }  // extern "C"

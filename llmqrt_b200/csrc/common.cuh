@@ -180,6 +180,14 @@ __device__ __forceinline__ uint2 quantize8_int8(const uint4& v, RowScale c) {
   }
   return make_uint2(pack_sat_s8(o[0], o[1], o[2], o[3]), pack_sat_s8(o[4], o[5], o[6], o[7]));
 }
+// x / (1 + e^-x), for a result that is then rounded to 16 bits: the special-function unit's exponential and
+// reciprocal (each within 2 ulp of fp32) instead of the library's, an eighth of the instructions.
+__device__ __forceinline__ float silu_f32(float x) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return x * r;
+}
 // The int8 quantizers' scale of a row: T(T(max(absmax, 1e-5)) * (1 / 127)).
 template <typename T> __device__ __forceinline__ float int8_scale(float amax) {
   return round_to<T>(__fmul_rn(round_to<T>(fmaxf(amax, 1e-5f)), 1.0f / 127.0f));

@@ -305,6 +305,32 @@ FAST_FN(awq_linear) {
   FAST_END
 }
 
+// (x fp16 of at most 16 tokens, wq_t, sz_t, bias or None, residual or None, K, N, G) -> residual + y, or without a
+// residual silu(first half of y) * second half.
+FAST_FN(awq_tail) {
+  FAST_BEGIN(8)
+  const Tensor x = tensor_arg(a[0], "x"), wq = tensor_arg(a[1], "wq_t"), sz = tensor_arg(a[2], "sz_t");
+  const Tensor bias = tensor_arg(a[3], "bias"), res = tensor_arg(a[4], "residual");
+  const int64_t K = int_arg(a[5]), N = int_arg(a[6]), G = int_arg(a[7]);
+  GilRelease gil;
+  const Tensor x2 = rows(x);
+  const int64_t M = x2.size(0), cols = res.defined() ? N : N / 2;
+  Call c(same_device({&x, &wq, &bias, &res}));
+  TORCH_CHECK(x2.size(1) == K, "awq_gemm: x has K=", x2.size(1), ", layer has K=", K);
+  Tensor r2;
+  if (res.defined()) {
+    r2 = rows(res);
+    TORCH_CHECK(res.scalar_type() == at::kHalf && r2.size(0) == M && r2.size(1) == N, "awq_gemm: residual must be fp16 [M, N]");
+  }
+  Tensor out = empty(x, out_shape(x, cols), at::kHalf);
+  check(llmqrt_awq_gemm_tail(ptr(x2), x2.stride(0), static_cast<const uint32_t*>(ptr(wq)),
+                             static_cast<const uint32_t*>(ptr(sz)), ptr(bias), ptr(r2), res.defined() ? r2.stride(0) : 0,
+                             mptr(out), cols, M, N, K, G, c.stream));
+  gil.done();
+  return wrap(out);
+  FAST_END
+}
+
 // ---- row kernels -----------------------------------------------------------------------------------
 
 // (x, weight, eps, residual or None, quantize, want_y) -> (y, h, q, scale), absent ones None.
@@ -497,15 +523,17 @@ FAST_FN(attn_decode) {
 }
 
 // (q [B, 1, Hq, d], k_cache, v_cache, k, v (one new token [B, 1, Hkv, d], or None), cache_seqlens or None, length added
-// to those, max_seqlen, softcap) -> out [B, 1, Hq, d]
+// to those, max_seqlen, softcap, cos or None, sin or None, write the row twice) -> out [B, 1, Hq, d]
 FAST_FN(attn_decode_step) {
-  FAST_BEGIN(9)
+  FAST_BEGIN(12)
   const Tensor q4 = tensor_arg(a[0], "q"), kc = tensor_arg(a[1], "k_cache"), vc = tensor_arg(a[2], "v_cache");
   const Tensor k4 = tensor_arg(a[3], "k"), v4 = tensor_arg(a[4], "v"), lens = tensor_arg(a[5], "cache_seqlens");
   const int64_t len_add = int_arg(a[6]), max_seqlen = int_arg(a[7]);
   const float softcap = (float)float_arg(a[8]);
+  const Tensor cos = tensor_arg(a[9], "cos"), sin = tensor_arg(a[10], "sin");
+  const bool twice = bool_arg(a[11]);
   GilRelease gil;
-  Call c(same_device({&q4, &kc, &vc, &k4, &v4, &lens}));
+  Call c(same_device({&q4, &kc, &vc, &k4, &v4, &lens, &cos, &sin}));
   TORCH_CHECK(q4.dim() == 4 && kc.dim() == 4 && vc.dim() == 4, "attn_decode: q must be [B, 1, Hq, d] and the caches [B, S, Hkv, d]");
   const int64_t B = q4.size(0), Hq = q4.size(2), d = q4.size(3), Hkv = kc.size(2);
   TORCH_CHECK(kc.stride(3) == 1 && kc.stride(2) == d && vc.strides() == kc.strides(),
@@ -532,9 +560,14 @@ FAST_FN(attn_decode_step) {
       if (!usable(v, Hkv)) v = v.clone();
     }
   }
+  if (cos.defined())
+    TORCH_CHECK(sin.defined() && cos.scalar_type() == at::kFloat && sin.scalar_type() == at::kFloat &&
+                cos.sizes() == sin.sizes() && cos.size(-1) == d / 2 && cos.is_contiguous() && sin.is_contiguous(),
+                "attn_decode: cos / sin must be contiguous fp32 [rows, d/2]");
   Tensor out = empty(q4, q4.sizes(), q4.scalar_type());
   check(llmqrt_attn_decode_step(ptr(q), B > 1 ? q.stride(0) : Hq * d, ptr(k), ptr(v), k.defined() && B > 1 ? k.stride(0) : Hkv * d,
-                                mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), kc.size(1),
+                                static_cast<const float*>(ptr(cos)), static_cast<const float*>(ptr(sin)),
+                                cos.defined() ? cos.size(0) : 0, twice ? 1 : 0, mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), kc.size(1),
                                 static_cast<const int32_t*>(ptr(lens)), (int32_t)len_add, mptr(out),
                                 dtype_code(q4.scalar_type()), B, Hq, Hkv, d, max_seqlen, softcap, c.workspace(), c.stream));
   gil.done();
@@ -573,7 +606,7 @@ FAST_FN(set_workspace_maker) {
 
 #define FAST_DEF(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST_DEF(sq_per_channel), FAST_DEF(sq_per_tensor), FAST_DEF(fp8_per_token), FAST_DEF(fp8_per_tensor),
-                         FAST_DEF(awq_linear), FAST_DEF(rmsnorm), FAST_DEF(silu_mul), FAST_DEF(rope_kv_write),
+                         FAST_DEF(awq_linear), FAST_DEF(awq_tail), FAST_DEF(rmsnorm), FAST_DEF(silu_mul), FAST_DEF(rope_kv_write),
                          FAST_DEF(attn_prefill), FAST_DEF(kv_append), FAST_DEF(attn_decode), FAST_DEF(attn_decode_step), FAST_DEF(tensor_key),
                          FAST_DEF(set_workspace_maker), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast", "Native host path of llmqrt_b200.", -1, methods,

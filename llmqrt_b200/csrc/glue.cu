@@ -207,16 +207,6 @@ __device__ __forceinline__ float block_reduce_once(float v) {
   return r;
 }
 
-// silu in T: the special-function unit's exponential and reciprocal (each within 2 ulp of fp32), then the rounding
-// to 16 bits that dwarfs both.
-template <typename T>
-__device__ __forceinline__ float silu_f32(float g) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return g * r;
-}
-
 // Eight packed results of silu(gate) * up (in T); the running absolute maximum goes up with them.
 template <typename T>
 __device__ __forceinline__ uint4 silu_mul8(const uint4& g, const uint4& up, float& amax) {
@@ -225,7 +215,7 @@ __device__ __forceinline__ uint4 silu_mul8(const uint4& g, const uint4& up, floa
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     const float2 gv = unpack_pair<T>(gw[p]), uv = unpack_pair<T>(uw[p]);
-    const float2 act = unpack_pair<T>(pack_pair<T>(silu_f32<T>(gv.x), silu_f32<T>(gv.y)));       // silu in T
+    const float2 act = unpack_pair<T>(pack_pair<T>(silu_f32(gv.x), silu_f32(gv.y)));       // silu in T
     h[p] = pack_pair<T>(act.x * uv.x, act.y * uv.y);                                              // * up, in T
     const float2 hv = unpack_pair<T>(h[p]);
     amax = fmaxf(amax, fmaxf(fabsf(hv.x), fabsf(hv.y)));

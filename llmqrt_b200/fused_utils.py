@@ -105,12 +105,27 @@ class FusedGateUpMLP(torch.nn.Module):
         self.gate_proj, self.up_proj = (None, None) if self.gate_up is not None else (gate_proj, up_proj)
         self.down_proj = down_proj
 
-    @torch.no_grad()
-    def forward(self, x):
+    def _hidden(self, x):
         from . import glue
+        if isinstance(self.gate_up, WQLinear_GEMM) and self.gate_up.takes_tail(x, 16):
+            return self.gate_up.silu_halves(x)
         if self.gate_up is not None:
             gu = self.gate_up(x)
         else:
             gu = torch.cat([self.gate_proj(x), self.up_proj(x)], dim=-1)
-        h, _, _ = glue.silu_mul(gu)
-        return self.down_proj(h)
+        return glue.silu_mul(gu)[0]
+
+    @torch.no_grad()
+    def forward(self, x):
+        return self.down_proj(self._hidden(x))
+
+    def add_to(self, residual, x):
+        """residual + forward(x)."""
+        if torch.is_grad_enabled() and residual.requires_grad:
+            return residual + self.forward(x)
+        with torch.no_grad():
+            h, down = self._hidden(x), self.down_proj
+            if isinstance(down, WQLinear_GEMM) and down.takes_tail(h) and residual.dtype == torch.float16 \
+                    and residual.device == h.device and residual.shape == (*h.shape[:-1], down.out_features):
+                return down.add_to(residual, h)
+            return residual + down(h)

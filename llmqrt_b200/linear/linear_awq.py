@@ -92,6 +92,23 @@ class WQLinear_GEMM(LinearBase):
             return fast.awq_linear(x, p.wq_t, p.sz_t, self.bias, p.K, p.N, p.G)
         return fast.awq_linear(x.detach().to(torch.float16), p.wq_t, p.sz_t, self.bias, p.K, p.N, p.G).to(input_dtype)
 
+    def takes_tail(self, x, multiple=8) -> bool:
+        """Whether `silu_halves` / `add_to` apply: a few fp16 tokens, and no hook that would see the plain output."""
+        return (x.dtype == torch.float16 and x.is_cuda and 0 < x.numel() <= 16 * self.in_features
+                and x.shape[-1] == self.in_features and self.in_features % 32 == 0 and self.group_size % 32 == 0
+                and self.out_features % multiple == 0 and x.device == self.qweight.device
+                and not (self._forward_hooks or self._forward_pre_hooks) and type(self) is WQLinear_GEMM)
+
+    def silu_halves(self, x):
+        """silu(y[..., :N/2]) * y[..., N/2:] of y = self(x), one kernel (see takes_tail, multiple 16)."""
+        p = self.packed()
+        return fast.awq_tail(x, p.wq_t, p.sz_t, self.bias, None, p.K, p.N, p.G)
+
+    def add_to(self, residual, x):
+        """residual + self(x), one kernel (see takes_tail)."""
+        p = self.packed()
+        return fast.awq_tail(x, p.wq_t, p.sz_t, self.bias, residual, p.K, p.N, p.G)
+
     def extra_repr(self) -> str:
         return "in_features={}, out_features={}, bias={}, w_bit={}, group_size={}".format(
             self.in_features, self.out_features, self.bias is not None, self.w_bit, self.group_size)

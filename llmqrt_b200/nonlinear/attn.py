@@ -93,24 +93,21 @@ class QuantAttentionFused(nn.Module):
             xk = self.k_norm(xk)
 
         self.cache.to(xq)
-        if seqlen > 1 or not all(t.stride(3) == 1 and t.stride(2) == d for t in (xq, xk, xv)) or \
-                xk.stride(1) != xv.stride(1) or any(t.stride(0) != t.stride(1) for t in (xq, xk, xv)):
-            xq, xk, xv = xq.contiguous(), xk.contiguous(), xv.contiguous()    # (one token: rotated where the projection left it)
-        # rotary embedding of q and k, and cache[:, start_pos : start_pos + seqlen] = (k, v), one kernel
-        glue.rope_kv_write(xq, xk, xv, self.rope.cos, self.rope.sin, pos0=self.start_pos,
-                           k_cache=self.cache.k[:bsz], v_cache=self.cache.v[:bsz])
         if seqlen > 1:
+            xq, xk, xv = xq.contiguous(), xk.contiguous(), xv.contiguous()
+            # rotary embedding of q and k, and cache[:, start_pos : start_pos + seqlen] = (k, v), one kernel
+            glue.rope_kv_write(xq, xk, xv, self.rope.cos, self.rope.sin, pos0=self.start_pos,
+                               k_cache=self.cache.k[:bsz], v_cache=self.cache.v[:bsz])
             output = attention.flash_attn_func(q=xq, k=xk, v=xv, causal=True, softcap=self.attn_logit_softcapping)
+        elif self.start_pos >= self.cache.k.shape[1]:        # a full cache: nothing to rotate by or to write to
+            output = attention.flash_attn_with_kvcache(
+                q=xq, k_cache=self.cache.k, v_cache=self.cache.v, cache_seqlens=self.start_pos + 1, causal=True,
+                softcap=self.attn_logit_softcapping, max_seqlen_k=self.start_pos + 1)
         else:
-            cap = self.cache.k.shape[1]
-            if self.REFERENCE_DOUBLE_APPEND and self.start_pos + 1 < cap:
-                output = attention.flash_attn_with_kvcache(
-                    q=xq, k=xk, k_cache=self.cache.k, v=xv, v_cache=self.cache.v, cache_seqlens=self.start_pos + 1,
-                    causal=True, softcap=self.attn_logit_softcapping, max_seqlen_k=self.start_pos + 2)
-            else:
-                output = attention.flash_attn_with_kvcache(
-                    q=xq, k_cache=self.cache.k, v_cache=self.cache.v, cache_seqlens=self.start_pos + 1, causal=True,
-                    softcap=self.attn_logit_softcapping, max_seqlen_k=self.start_pos + 1)
+            # rotation, cache write(s) and attention, one kernel
+            twice = self.REFERENCE_DOUBLE_APPEND and self.start_pos + 1 < self.cache.k.shape[1]
+            output = attention.decode_rotary_step(xq, xk, xv, self.cache.k, self.cache.v, self.rope.cos, self.rope.sin,
+                                                  self.start_pos, twice, self.attn_logit_softcapping)
         attention_weight = output.reshape(bsz, seqlen, -1)
         attn_output = self.o_proj(attention_weight)
         self.start_pos += seqlen

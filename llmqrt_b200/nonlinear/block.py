@@ -7,6 +7,7 @@ from typing import List
 import torch
 import torch.nn as nn
 
+from ..fused_utils import FusedGateUpMLP
 from .attn import QuantAttentionFused
 from .norm import RMSNorm
 
@@ -36,7 +37,7 @@ class LlamaLikeBlock(nn.Module):
         else:
             h = hidden_states + attn_output
             y = self.norm_2(h)
-        return h + self.mlp.forward(y)
+        return self.mlp.add_to(h, y) if type(self.mlp) is FusedGateUpMLP else h + self.mlp.forward(y)
 
 
 class LlamaLikeModel(nn.Module):

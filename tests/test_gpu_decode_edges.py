@@ -52,3 +52,78 @@ def test_decode_step(lens, cap, bound, Hq, Hkv, d, dt, append):
     if len(set(lens)) == 1:                                  # the same lengths as one number
         out2 = flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens[0] + append, max_seqlen_k=bound)
         assert rel_fro(out2, out.double()) < (1e-3 if dt == torch.float16 else 8e-3)
+
+
+@pytest.mark.parametrize("pos,cap", [(0, 2), (0, 1), (63, 65), (64, 65), (63, 64), (127, 200), (511, 1000), (700, 708), (4094, 4200)])
+@pytest.mark.parametrize("B,Hq,Hkv,d", [(1, 12, 2, 128), (3, 14, 2, 64)])
+@pytest.mark.parametrize("twice", [True, False])
+def test_decode_rotary_step(pos, cap, B, Hq, Hkv, d, twice):
+    """Rotation, one or two cache rows (in one split or in two) and attention, against the kernels it replaces."""
+    from llmqrt_b200 import glue
+    from llmqrt_b200.attention import decode_rotary_step, flash_attn_with_kvcache
+    if pos + 1 + twice > cap:
+        pytest.skip("the second row does not fit")
+    g = torch.Generator(device="cuda").manual_seed(pos + cap)
+    kc, vc = (torch.randn(B, cap, Hkv, d, generator=g, device="cuda").half() for _ in range(2))
+    row = torch.randn(B, 1, Hq + 2 * Hkv, d, generator=g, device="cuda").half()
+    q, k, v = row[:, :, :Hq], row[:, :, Hq:Hq + Hkv], row[:, :, Hq + Hkv:]
+    cos, sin = glue.rope_tables(d, cap, 1e6, "cuda")
+    q1, k1, kc1, vc1 = q.clone(), k.clone(), kc.clone(), vc.clone()
+    glue.rope_kv_write(q1, k1, v.clone(), cos, sin, pos0=pos, k_cache=kc1, v_cache=vc1)
+    if twice:
+        kc1[:, pos + 1], vc1[:, pos + 1] = k1[:, 0], v[:, 0]
+    want = flash_attn_with_kvcache(q1, kc1, vc1, cache_seqlens=pos + 1 + twice, max_seqlen_k=pos + 1 + twice)
+    before = row.clone()
+    out = decode_rotary_step(q, k, v, kc, vc, cos, sin, pos, twice)
+    assert torch.equal(row, before) and torch.equal(vc, vc1)
+    assert rel_fro(kc, kc1.double()) < 1e-4 and rel_fro(out, want.double()) < 1e-3      # (one rounding of the rotated values)
+
+
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
+@pytest.mark.parametrize("K,N,G", [(32, 16, 32), (1536, 17920, 128), (2080, 48, 32), (8960, 1536, 128)])
+def test_awq_tail(M, K, N, G):
+    """The residual and silu(gate) * up on the GEMM's sums round as the separate kernels do."""
+    from llmqrt_b200 import glue
+    from llmqrt_b200.linear import WQLinear_GEMM
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    layer = WQLinear_GEMM(4, G, K, N, M % 2 == 1, "cuda")
+    layer.qweight.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+    layer.qzeros.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+    layer.scales.uniform_(0.0001, 0.002, generator=g)
+    if layer.bias is not None:
+        layer.bias.normal_(0, 0.1, generator=g)
+    x, res = torch.randn(1, M, K, generator=g, device="cuda").half(), torch.randn(1, M, N, generator=g, device="cuda").half()
+    assert layer.takes_tail(x, 16)
+    y = layer(x)
+    assert torch.equal(layer.add_to(res, x), res + y)
+    assert torch.equal(layer.silu_halves(x), glue.silu_mul(y)[0])
+    assert not layer.takes_tail(torch.zeros(17, K, dtype=torch.float16, device="cuda"))
+
+
+@pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("K,N,G", [(32, 8, 32), (96, 24, 32), (128, 16, 128), (1536, 2056, 128), (2080, 40, 32),
+                                   (8960, 1536, 128), (4096, 17920, 64)])
+def test_awq_few_tokens(M, K, N, G):
+    """Ragged K (a chunk of 128 cut short), N off the 16-row block, every block width, with and without bias."""
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    qz = torch.randint(-2 ** 31, 2 ** 31 - 1, (K // G, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    sc = torch.rand(K // G, N, generator=g, device="cuda").mul_(0.02).half()
+    x = torch.randn(M, K, generator=g, device="cuda").half()
+    bias = torch.randn(N, generator=g, device="cuda").half() if N % 16 else None
+    want = x.double() @ ops.awq_dequantize(qw, sc, qz).double()
+    if bias is not None:
+        want += bias.double()
+    y = ops.awq_gemm(x, ops.AwqPacked(qw, sc, qz), bias)
+    assert rel_fro(y, want) < 5e-4                           # the fp16 rounding of the result (2^-11 at most per value)
+
+
+@pytest.mark.parametrize("K,N,G", [(32, 8, 32), (40, 24, 8), (1536, 72, 128), (8960, 264, 64)])
+def test_awq_expansion_bits(K, N, G):
+    """Word counts off the block's 1024, and a K that no 16-byte load divides."""
+    from llmqrt_b200 import ops
+    from oracle import awq as oa
+    qw, qz, sc = oa.random_layer(K, N, G, seed=K)
+    packed = ops.AwqPacked(qw.cuda(), sc.cuda(), qz.cuda())
+    assert torch.equal(ops.awq_dequantize_t(packed).cpu(), oa.dequantize(qw, qz, sc, G).t())

@@ -42,3 +42,17 @@ def test_chunk_schedules(M, N, K):
     s, ws = torch.rand(M, generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
     y = ops.int8_linear_per_channel(a, w, None, s, ws, torch.float16, True)
     assert torch.equal(y, (want.float() * ws * s[:, None]).half())
+
+
+@pytest.mark.parametrize("M", [17, 33, 129, 300, 700])
+@pytest.mark.parametrize("K,N,G", [(1536, 2056, 128), (96, 264, 32), (3584, 24576, 128), (256, 9480, 64)])
+def test_awq_schedules(M, K, N, G):
+    """Streamed, fused and expanded 4-bit GEMMs, the last also in two panels (24576 x 3584 is 176 MB in fp16)."""
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    qz = torch.randint(-2 ** 31, 2 ** 31 - 1, (K // G, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    sc = torch.rand(K // G, N, generator=g, device="cuda").mul_(0.02).half()
+    x, bias = torch.randn(M, K, generator=g, device="cuda").half(), torch.randn(N, generator=g, device="cuda").half()
+    want = x.double() @ ops.awq_dequantize(qw, sc, qz).double() + bias.double()
+    assert rel_fro(ops.awq_gemm(x, ops.AwqPacked(qw, sc, qz), bias), want) < 5e-4      # the fp16 rounding of the result
