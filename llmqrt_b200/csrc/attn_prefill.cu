@@ -332,10 +332,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       for (int j = 0; j < n_max && ok; ++j) {
         const int vs = j % kVS, ks1 = (j + 1) % kKS;
         const uint32_t vph = (uint32_t)(j / kVS) & 1u, kph1 = (uint32_t)((j + 1) / kKS) & 1u;
+        // (the tiles arrive long before P does: waiting for them first keeps the hand-over of P short)
+        if (!tc::mbar_wait_warp(tc::smem_u32(&bar_v_full[vs]), vph, abort)) { ok = false; break; }
+        if (j + 1 < n_max && !tc::mbar_wait_warp(tc::smem_u32(&bar_k_full[ks1]), kph1, abort)) { ok = false; break; }
         for (int w = 0; w < 2 && ok; ++w) {
           if (j >= n_tiles[w]) continue;
           if (!tc::mbar_wait_warp(tc::smem_u32(&bar_p_ready[w]), (uint32_t)j & 1u, abort)) { ok = false; break; }
-          if (!tc::mbar_wait_warp(tc::smem_u32(&bar_v_full[vs]), vph, abort)) { ok = false; break; }
           tc::fence_after_sync();
           issue_pv(w, vs, j, std::integral_constant<int, 0>(), std::integral_constant<int, kPvFirst>());
           if (!tc::mbar_wait_warp(tc::smem_u32(&bar_p_rest[w]), (uint32_t)j & 1u, abort)) { ok = false; break; }
@@ -344,7 +346,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           if (j == n_tiles[w] - 1 && tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_o_full[w]));     // last tile: O complete
           if (w == last_user(j) && tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_v_empty[vs]));      // V_j free once these retire
           if (j + 1 < n_tiles[w]) {
-            if (!tc::mbar_wait_warp(tc::smem_u32(&bar_k_full[ks1]), kph1, abort)) { ok = false; break; }
             issue_s(w, ks1);
             if (w == last_user(j + 1) && tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_k_empty[ks1]));   // K_{j+1} likewise
           }
