@@ -298,6 +298,92 @@ int launch_rows(const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, in
   return check_launch("w8a8_rows");
 }
 
+// ---- 17 to 32 tokens of a small layer -----------------------------------------------------------------
+// The same shape of kernel with 32 weight rows to a block, so that a fragment of the activations, which every block
+// fetches from L2, serves two row tiles.  The tcgen05 kernel has about 8 us of fixed cost at these sizes (pipeline
+// fill, split-K exchange through distributed shared memory, epilogue); here a warp's first weights are in registers
+// before the quantizer has finished and the exchange is one pass through shared memory.
+constexpr int kWideRows = 32, kWideWarps = 12, kWidePitch = kWideRows + 4;     // (pitch: conflict-free accumulator stores)
+template <int KIND>
+__global__ void __launch_bounds__(kWideWarps * 32, 1)
+w8a8_wide_kernel(const uint8_t* __restrict__ A, int64_t lda, const uint8_t* __restrict__ W, int64_t ldw, int M, int N,
+                 int K, int chunks, int static_w, Epilogue epi) {
+  using Acc = typename AccOf<KIND>::type;
+  constexpr int MB = 4;                                // tokens in eights
+  extern __shared__ __align__(16) uint8_t xs[];
+  Acc* red = reinterpret_cast<Acc*>(xs);               // [warp][token][kWidePitch]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int warps = blockDim.x >> 5, n0 = blockIdx.x * kWideRows;
+  const uint8_t* wr[4];                                // rows g, g + 8 of both tiles
+#pragma unroll
+  for (int r = 0; r < 4; ++r) wr[r] = W + (int64_t)min(n0 + g + 8 * r, N - 1) * ldw + 16 * t;
+  uint4 w[4];
+  auto fetch = [&](int c) {
+    const int k = c * kChunk;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = k + 16 * t < K ? ldg_stream_16B(wr[r] + k) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  if (static_w) fetch(warp);
+  pdl_wait_then_trigger();
+  if (!static_w) fetch(warp);
+  Acc acc[2][MB][4];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[r][mb][j] = 0;
+  for (int c = warp; c < chunks; c += warps) {
+    uint4 x[MB];
+    const int k = c * kChunk + 16 * t;
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb)
+      x[mb] = k < K && mb * 8 + g < M ? *reinterpret_cast<const uint4*>(A + (int64_t)(mb * 8 + g) * lda + k) : make_uint4(0u, 0u, 0u, 0u);
+    uint4 cur[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) cur[r] = w[r];
+    if (c + warps < chunks) fetch(c + warps);
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        mma8<KIND>(acc[r][mb], cur[2 * r].x, cur[2 * r + 1].x, cur[2 * r].y, cur[2 * r + 1].y, x[mb].x, x[mb].y);
+        mma8<KIND>(acc[r][mb], cur[2 * r].z, cur[2 * r + 1].z, cur[2 * r].w, cur[2 * r + 1].w, x[mb].z, x[mb].w);
+      }
+  }
+  Acc* mine = red + warp * (MB * 8 * kWidePitch);
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        mine[(mb * 8 + 2 * t + (j & 1)) * kWidePitch + 16 * r + g + 8 * (j >> 1)] = acc[r][mb][j];
+  __syncthreads();
+  const float alpha = epi.alpha_dev ? *epi.alpha_dev : epi.alpha;
+  for (int i = tid; i < M * kWideRows; i += blockDim.x) {
+    const int m = i / kWideRows, n = n0 + i % kWideRows;
+    if (n >= N) continue;
+    Acc sum = 0;
+    for (int v = 0; v < warps; ++v) sum += red[(v * MB * 8 + m) * kWidePitch + i % kWideRows];
+    epilogue_store<Acc>(epi, sum, m, n, alpha);
+  }
+}
+
+template <int KIND>
+int launch_wide(const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int M, int N, int K, const Epilogue& epi,
+                cudaStream_t st, bool static_w) {
+  const int blocks = (int)ceil_div(N, kWideRows), chunks = (int)ceil_div(K, kChunk);
+  const int rounds = (int)ceil_div(chunks, kWideWarps), warps = (int)ceil_div(chunks, rounds);
+  const size_t smem = (size_t)warps * 32 * kWidePitch * 4;
+  auto kern = w8a8_wide_kernel<KIND>;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kWideWarps * 32 * kWidePitch * 4)) return rc;
+  if (int rc = launch_chained(kern, dim3((unsigned)blocks), dim3((unsigned)(32 * warps)), smem, st, 1, A, lda, W, ldw, M, N, K,
+                              chunks, static_w ? 1 : 0, epi))
+    return rc;
+  return check_launch("w8a8_wide");
+}
+
 template <int KIND>
 int launch_mb(const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int M, int N, int K, const Epilogue& epi,
               void* workspace, cudaStream_t st, bool static_w) {
@@ -308,6 +394,13 @@ int launch_mb(const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int 
 }
 
 }  // namespace
+
+int w8a8_gemm_wide(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
+                   const Epilogue& epi, cudaStream_t st, bool static_w) {
+  if (kind == KIND_I8) return launch_wide<KIND_I8>(A, lda, W, ldw, (int)M, (int)N, (int)K, epi, st, static_w);
+  if (kind == KIND_F8_E4M3) return launch_wide<KIND_F8_E4M3>(A, lda, W, ldw, (int)M, (int)N, (int)K, epi, st, static_w);
+  return launch_wide<KIND_F8_E5M2>(A, lda, W, ldw, (int)M, (int)N, (int)K, epi, st, static_w);
+}
 
 int w8a8_gemm_stream(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N,
                      int64_t K, const Epilogue& epi_in, void* workspace, cudaStream_t st, bool static_w) {

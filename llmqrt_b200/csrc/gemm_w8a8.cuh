@@ -13,7 +13,10 @@ enum GemmKind : int {
   KIND_BF16 = 4       // bf16 x bf16 -> fp32   (tcgen05 back end only)
 };
 
-// Register-operand streaming kernel (gemm_stream.cu): any M, tuned for M <= 16.
+// 17 to 32 tokens of a small layer (gemm_stream.cu).
+int w8a8_gemm_wide(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
+                   const Epilogue& epi, cudaStream_t st, bool static_w);
+// Register-operand streaming kernels (gemm_stream.cu): any M, tuned for M <= 16.
 int w8a8_gemm_stream(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N,
                      int64_t K, const Epilogue& epi, void* workspace, cudaStream_t st, bool static_w);
 

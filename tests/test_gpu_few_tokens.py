@@ -1,4 +1,4 @@
-"""The int8 / fp8 GEMM of at most 16 tokens at the edges of its blocks and chunks."""
+"""The int8 / fp8 GEMM of at most 32 tokens at the edges of its blocks and chunks."""
 import pytest
 import torch
 
@@ -7,7 +7,7 @@ from tests.util import rel_fro
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 31, 32])
 @pytest.mark.parametrize("N,K", [(1, 16), (15, 48), (16, 64), (17, 80), (40, 1040), (4864, 896), (3584, 18944), (24000, 272)])
 def test_few_tokens(M, N, K):
     """Ragged K (a chunk of 64 bytes cut short), N off the 16-row block, every number of warps: exact for int8."""
