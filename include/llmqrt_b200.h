@@ -292,6 +292,11 @@ int llmqrt_attn_prefill(const void* q, int64_t q_token_stride, const void* k, co
 int llmqrt_rmsnorm(const void* x, const void* residual, void* x_out, const void* weight, float eps, void* y,
                    int8_t* q, float* scale_f32, int dtype, int64_t M, int64_t H, llmqrt_stream_t stream);
 
+/* Greedy sampling: idx[m] = base + the index of row m's maximum (the lowest one on ties; a NaN counts as the
+ * greatest), val[m] its value in x's dtype (fp16 / bf16). */
+int llmqrt_argmax_rows(const void* x, int64_t ld, int dtype, int64_t M, int64_t N, int64_t base, void* val, int64_t* idx,
+                       llmqrt_stream_t stream);
+
 /* Rotary embedding (half-split pairing) of q [B, S, Hq, d] and k [B, S, Hkv, d] in place at positions
  * pos0 + s (pos_dev, when not NULL, is a device int32 scalar overriding pos0), then, when k_cache is
  * not NULL, writes the rotated k and v [B, S, Hkv, d] into the caches at rows pos + s.

@@ -62,6 +62,7 @@ _PROTOS = {
     "llmqrt_rmsnorm": (c_int, [P, P, P, P, F, P, P, P, I32, I64, I64, P]),
     "llmqrt_rope_kv_write": (c_int, [P, I64, P, P, I64, P, P, I64, I64, c_int32, P, P, P, I64, I32, I64, I64, I64,
                                      I64, I64, P]),
+    "llmqrt_argmax_rows": (c_int, [P, I64, I32, I64, I64, I64, P, P, P]),
     "llmqrt_silu_mul": (c_int, [P, I64, P, P, P, I32, I64, I64, P]),
     "llmqrt_comm_create": (c_int, [I32, I32, I64, ctypes.POINTER(c_void_p)]),
     "llmqrt_comm_handle_bytes": (c_int, []),
@@ -91,7 +92,7 @@ def _bind(lib: ctypes.CDLL) -> list[str]:
     return missing
 
 
-ABI_VERSION = 8          # llmqrt_abi_version() of the sources these prototypes describe
+ABI_VERSION = 9          # llmqrt_abi_version() of the sources these prototypes describe
 
 _missing = _bind(_lib)
 if not _missing and _lib.llmqrt_abi_version() != ABI_VERSION:

@@ -70,3 +70,17 @@ def rope_kv_write(q, k, v, cos, sin, pos0: int = 0, pos_dev=None, k_cache=None, 
 def silu_mul(gate_up, quantize: bool = False, want_y: bool = True):
     """h = silu(gate) * up for gate_up [..., 2I] (gate first).  Returns (h or None, q or None, scale or None)."""
     return L.fast.silu_mul(gate_up, quantize, want_y)
+
+
+def argmax_rows(x, base: int = 0):
+    """(values [M] in x's dtype, base + indices [M] int64) of the row maxima of x [M, N] (fp16 / bf16, unit inner
+    stride); ties go to the lowest index, a NaN counts as the greatest value."""
+    dev = L.require_cuda(x)
+    M, N = x.shape
+    if x.stride(1) != 1:
+        x = x.contiguous()
+    val, idx = torch.empty(M, dtype=x.dtype, device=dev), torch.empty(M, dtype=torch.int64, device=dev)
+    with torch.cuda.device(dev):
+        L.call("llmqrt_argmax_rows", L.ptr(x), x.stride(0) if M > 1 else N, L.dtype_code(x.dtype), M, N, int(base), L.ptr(val),
+               L.ptr(idx), L.stream(dev))
+    return val, idx

@@ -205,8 +205,8 @@ class Qwen2Decoder:
         y, _, _, _ = glue.rmsnorm(h, self.norm_f, self.cfg.rms_eps, residual=pending, comm=self.comm)
         logits = ops.gemm_16bit(y, self.lm_head)                                            # [M, V/tp]
         self.last_logits = logits
-        val, idx = logits.max(dim=-1)
-        return greedy_select(val, idx + self.vocab0, self.tp, self.group)
+        val, idx = glue.argmax_rows(logits, self.vocab0)
+        return greedy_select(val, idx, self.tp, self.group)
 
     # ------------------------------------------------------------------------------------------
     @torch.no_grad()
@@ -251,8 +251,7 @@ class Qwen2Decoder:
         h = self.embed[tokens]
         h, pending = self._layers_forward(h, self.batch, 1, decode=True)
         nxt = self._head(h, pending)
-        self.pos_dev += 1
-        self.seqlens += 1
+        torch._foreach_add_([self.pos_dev, self.seqlens], 1)           # one kernel
         return nxt
 
     @torch.no_grad()

@@ -115,3 +115,26 @@ def test_rmsnorm_small_blocks(H, dt):
     assert torch.equal(q.cpu(), qr) and torch.equal(s.cpu(), sr.float().reshape(-1))
     y2, _, _, _ = glue.rmsnorm(want_h, w, 1e-6)
     assert torch.equal(y2, y)
+
+
+@pytest.mark.parametrize("M,N", [(1, 1), (3, 7), (2, 4096), (64, 8200), (5, 9001), (64, 152064), (300, 1024)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_argmax_rows(M, N, dt):
+    """Ties (16-bit values repeat), signed zeros, infinities and NaN; one CTA and a cluster of them; odd rows."""
+    from llmqrt_b200 import glue
+    x = torch.randn(M, N, generator=_g(11), device="cuda").to(dt)
+    if N > 4:
+        x[0] = -1.0
+        x[0, 2], x[0, N - 1] = 0.0, 0.0                      # a tie far apart
+        x[0, 1] = -0.0                                       # equal to +0: the lowest index wins
+        x[M - 1, N // 2] = float("inf")
+        if M > 1:
+            x[1] = float("-inf")
+        if M > 2:
+            x[2, 5 % N], x[2, N - 1] = float("nan"), float("nan")
+    val, idx = glue.argmax_rows(x, 100)
+    f = x.float()
+    for m in range(M):
+        nan = x[m].isnan().nonzero()
+        want = int(nan[0]) if len(nan) else int((f[m] == f[m].max()).nonzero()[0])
+        assert int(idx[m]) == 100 + want and torch.equal(val[m].view(torch.int16), x[m, want].view(torch.int16))
