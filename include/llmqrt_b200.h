@@ -158,6 +158,14 @@ int llmqrt_f8f8bf16_rowwise(const uint8_t* a, int a_format, int64_t lda, const u
                             const void* bias, int bias_dtype, const float* x_scale, const float* w_scale, void* out,
                             int64_t ldo, int64_t M, int64_t N, int64_t K, void* workspace, llmqrt_stream_t stream, int flags);
 
+/* Per-token quantization and per-token x per-channel GEMM of a few tokens in one kernel, the same bits as
+ * llmqrt_quantize_int8 / _fp8 followed by llmqrt_w8a8_int8_linear_per_channel / llmqrt_f8f8bf16_rowwise.
+ * llmqrt_w8a8_dynamic_fits says whether it takes the sizes; x (fp16 / bf16) has 16-byte aligned rows. */
+int llmqrt_w8a8_dynamic_fits(int64_t M, int64_t N, int64_t K);
+int llmqrt_w8a8_linear_dynamic(int fp8, const void* x, int x_dtype, int64_t ldx, const void* w, int64_t ldw,
+                               const void* bias, int bias_dtype, const float* w_scale, void* out, int out_dtype,
+                               int64_t ldo, int64_t M, int64_t N, int64_t K, llmqrt_stream_t stream);
+
 /* Path selection of the W8A8 GEMMs, for tests and benchmarks: 0 = automatic (default),
  * 1 = register-operand streaming kernel only, 2 = tcgen05/TMEM kernel only.  Process-wide. */
 int llmqrt_set_gemm_path(int path);

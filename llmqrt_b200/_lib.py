@@ -46,6 +46,8 @@ _PROTOS = {
     "llmqrt_w8a8_int8_gemm_s32": (c_int, [P, I64, P, I64, P, I64, I64, I64, I64, P, P, I32]),
     "llmqrt_f8f8_tensorwise": (c_int, [P, I32, I64, P, I64, P, F, P, F, P, I32, I64, I64, I64, I64, P, P, I32]),
     "llmqrt_f8f8bf16_rowwise": (c_int, [P, I32, I64, P, I64, P, I32, P, P, P, I64, I64, I64, I64, P, P, I32]),
+    "llmqrt_w8a8_dynamic_fits": (c_int, [I64, I64, I64]),
+    "llmqrt_w8a8_linear_dynamic": (c_int, [I32, P, I32, I64, P, I64, P, I32, P, P, I32, I64, I64, I64, I64, P]),
     "llmqrt_awq_dequantize": (c_int, [P, P, P, I64, I64, I64, P, P]),
     "llmqrt_awq_repack": (c_int, [P, P, P, I64, I64, I64, P, P, P]),
     "llmqrt_awq_gemm": (c_int, [P, I64, P, P, P, P, I64, I64, I64, I64, I64, P, P]),
@@ -92,7 +94,7 @@ def _bind(lib: ctypes.CDLL) -> list[str]:
     return missing
 
 
-ABI_VERSION = 9          # llmqrt_abi_version() of the sources these prototypes describe
+ABI_VERSION = 10         # llmqrt_abi_version() of the sources these prototypes describe
 
 _missing = _bind(_lib)
 if not _missing and _lib.llmqrt_abi_version() != ABI_VERSION:

@@ -180,6 +180,32 @@ __device__ __forceinline__ uint2 quantize8_int8(const uint4& v, RowScale c) {
   }
   return make_uint2(pack_sat_s8(o[0], o[1], o[2], o[3]), pack_sat_s8(o[4], o[5], o[6], o[7]));
 }
+// e4m3(clamp(T(x / s), +-448)) of eight packed 16-bit values.  exact_div: the scale may be zero (an fp8 row whose
+// absmax / 448 vanishes in T), where only the true division gives NaN and the saturated values.
+template <typename T>
+__device__ __forceinline__ uint2 quantize8_fp8(const uint4& v, float s, RowScale c, bool exact_div) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 x = unpack_pair<T>(w[p]);
+    const float2 d = exact_div ? make_float2(__fdiv_rn(x.x, s), __fdiv_rn(x.y, s))
+                               : make_float2(div_row_scale(x.x, c), div_row_scale(x.y, c));
+    // (saturating: the clamp to +-448)
+    o[p] = __nv_cvt_float2_to_fp8x2(unpack_pair<T>(pack_pair<T>(d.x, d.y)), __NV_SATFINITE, __NV_E4M3);
+  }
+  return make_uint2(o[0] | (o[1] << 16), o[2] | (o[3] << 16));
+}
+// Absolute maximum of eight packed values, joined with m.
+template <typename T> __device__ __forceinline__ float absmax8(const uint4& v, float m) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 x = unpack_pair<T>(w[p]);
+    m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
+  }
+  return m;
+}
 // x / (1 + e^-x), for a result that is then rounded to 16 bits: the special-function unit's exponential and
 // reciprocal (each within 2 ulp of fp32) instead of the library's, an eighth of the instructions.
 __device__ __forceinline__ float silu_f32(float x) {
@@ -191,6 +217,10 @@ __device__ __forceinline__ float silu_f32(float x) {
 // The int8 quantizers' scale of a row: T(T(max(absmax, 1e-5)) * (1 / 127)).
 template <typename T> __device__ __forceinline__ float int8_scale(float amax) {
   return round_to<T>(__fmul_rn(round_to<T>(fmaxf(amax, 1e-5f)), 1.0f / 127.0f));
+}
+// The fp8 quantizers': T(T(max(absmax, 1e-12)) * (1 / 448)).
+template <typename T> __device__ __forceinline__ float fp8_scale(float amax) {
+  return round_to<T>(__fmul_rn(round_to<T>(fmaxf(amax, 1e-12f)), 1.0f / 448.0f));
 }
 
 // Loads a 16-bit float of runtime dtype (LLMQRT_F16 / LLMQRT_BF16 / LLMQRT_F32) as fp32.

@@ -169,6 +169,13 @@ struct QuantScratch {
   float* scale;
 };
 
+// Sizes and rows that the GEMM quantizes itself.
+bool few_tokens(const Tensor& x2, int64_t N) {
+  return x2.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(x2.data_ptr()) % 16 == 0 && x2.size(1) % 16 == 0 &&
+         x2.stride(0) >= x2.size(1) && (x2.scalar_type() == at::kHalf || x2.scalar_type() == at::kBFloat16) &&
+         llmqrt_w8a8_dynamic_fits(x2.size(0), N, x2.size(1));
+}
+
 #define FAST_FN(name) PyObject* name(PyObject*, PyObject* const* a, Py_ssize_t n)
 #define FAST_BEGIN(count)                                                                               \
   HANDLE_TH_ERRORS                                                                                      \
@@ -195,8 +202,14 @@ FAST_FN(sq_per_channel) {
   const Tensor w_s = f32_vector(ws);
   TORCH_CHECK(w_s.numel() == N, "per-channel int8 linear: a_scale must have M elements and w_scale N elements");
   const int xd = dtype_code(x.scalar_type()), bd = bias.defined() ? dtype_code(bias.scalar_type()) : LLMQRT_F16;
-  QuantScratch s(x, M, K, M);
   Tensor out = empty(x, out_shape(x, N), x.scalar_type());
+  if (few_tokens(x2, N)) {
+    check(llmqrt_w8a8_linear_dynamic(0, ptr(x2), xd, x2.stride(0), ptr(w), w.stride(0), ptr(bias), bd,
+                                     static_cast<const float*>(ptr(w_s)), mptr(out), xd, N, M, N, K, c.stream));
+    gil.done();
+    return wrap(out);
+  }
+  QuantScratch s(x, M, K, M);
   check(llmqrt_quantize_int8(ptr(x2), xd, M, K, x2.stride(0), 1, reinterpret_cast<int8_t*>(s.q), nullptr, s.scale, 1.f,
                              c.workspace(), c.stream));
   check(llmqrt_w8a8_int8_linear_per_channel(reinterpret_cast<const int8_t*>(s.q), K, static_cast<const int8_t*>(ptr(w)),
@@ -246,10 +259,17 @@ FAST_FN(fp8_per_token) {
   const int64_t M = x2.size(0), K = x2.size(1), N = w.size(0);
   Call c(same_device({&x, &w, &bias, &ws}));
   const int xd = dtype_code(x.scalar_type()), bd = bias.defined() ? dtype_code(bias.scalar_type()) : LLMQRT_BF16;
-  QuantScratch s(x, M, K, M);
   Tensor out = empty(x, out_shape(x, N), at::kBFloat16);
-  check(llmqrt_quantize_fp8(ptr(x2), xd, M, K, x2.stride(0), 1, s.q, s.scale, 1.f, c.workspace(), c.stream));
   const Tensor w_s = f32_vector(ws);
+  if (few_tokens(x2, N)) {
+    check(llmqrt_w8a8_linear_dynamic(1, ptr(x2), xd, x2.stride(0), ptr(w), w.stride(0), ptr(bias), bd,
+                                     static_cast<const float*>(ptr(w_s)), mptr(out), LLMQRT_BF16, N, M, N, K, c.stream));
+    out = out.to(x.scalar_type());
+    gil.done();
+    return wrap(out);
+  }
+  QuantScratch s(x, M, K, M);
+  check(llmqrt_quantize_fp8(ptr(x2), xd, M, K, x2.stride(0), 1, s.q, s.scale, 1.f, c.workspace(), c.stream));
   check(llmqrt_f8f8bf16_rowwise(s.q, LLMQRT_E4M3, K, static_cast<const uint8_t*>(ptr(w)), w.stride(0), ptr(bias), bd,
                                 s.scale, static_cast<const float*>(ptr(w_s)), mptr(out), N, M, N, K, c.workspace(),
                                 c.stream, LLMQRT_GEMM_STATIC_WEIGHT));

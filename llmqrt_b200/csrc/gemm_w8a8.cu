@@ -157,4 +157,25 @@ int llmqrt_f8f8bf16_rowwise(const uint8_t* a, int a_format, int64_t lda, const u
   return run(kind, a, lda, w, ldw, M, N, K, e, workspace, (cudaStream_t)stream, flags);
 }
 
+int llmqrt_w8a8_dynamic_fits(int64_t M, int64_t N, int64_t K) { return w8a8_dynamic_fits(M, N, K) && gemm_path() == 0; }
+
+int llmqrt_w8a8_linear_dynamic(int fp8, const void* x, int x_dtype, int64_t ldx, const void* w, int64_t ldw, const void* bias,
+                               int bias_dtype, const float* w_scale, void* out, int out_dtype, int64_t ldo, int64_t M,
+                               int64_t N, int64_t K, llmqrt_stream_t stream) {
+  if (int rc = check_common(x, (ldx + 15) / 16 * 16, w, ldw, out, ldo, M, N, K)) return rc;
+  LLMQRT_REQUIRE(w8a8_dynamic_fits(M, N, K), "w8a8 dynamic linear: M = %lld, N = %lld, K = %lld are not its sizes (see "
+                 "llmqrt_w8a8_dynamic_fits)", (long long)M, (long long)N, (long long)K);
+  LLMQRT_REQUIRE(x_dtype == LLMQRT_F16 || x_dtype == LLMQRT_BF16, "w8a8 dynamic linear: x must be fp16 or bf16");
+  LLMQRT_REQUIRE(ldx >= K && ldx % 8 == 0, "w8a8 dynamic linear: rows of x must be 16-byte aligned");
+  LLMQRT_REQUIRE(w_scale, "w8a8 dynamic linear: null scale");
+  LLMQRT_REQUIRE(out_dtype == LLMQRT_F16 || out_dtype == LLMQRT_BF16, "w8a8 dynamic linear: out must be fp16/bf16");
+  LLMQRT_REQUIRE(!bias || bias_dtype == LLMQRT_F16 || bias_dtype == LLMQRT_BF16 || bias_dtype == LLMQRT_F32,
+                 "w8a8 dynamic linear: bad bias dtype");
+  Epilogue e{};
+  e.mode = fp8 ? EPI_ROW_COL : EPI_COL_ROW; e.out_dtype = out_dtype; e.bias_dtype = bias_dtype; e.bias = bias;
+  e.col_scale = w_scale; e.out = out; e.ldo = ldo;
+  return w8a8_gemm_dynamic(fp8 ? KIND_F8_E4M3 : KIND_I8, x_dtype, x, ldx, static_cast<const uint8_t*>(w), ldw, M, N, K, e,
+                           (cudaStream_t)stream);
+}
+
 }  // extern "C"

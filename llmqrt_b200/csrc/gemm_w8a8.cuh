@@ -13,6 +13,11 @@ enum GemmKind : int {
   KIND_BF16 = 4       // bf16 x bf16 -> fp32   (tcgen05 back end only)
 };
 
+// A few tokens of a small layer, quantized by the GEMM itself (gemm_stream.cu): whether the sizes suit it, and the call
+// (x fp16 / bf16 with 16-byte aligned rows; kind KIND_I8 or KIND_F8_E4M3; epi's row_scale is not read).
+bool w8a8_dynamic_fits(int64_t M, int64_t N, int64_t K);
+int w8a8_gemm_dynamic(int kind, int x_dtype, const void* x, int64_t ldx, const uint8_t* W, int64_t ldw, int64_t M, int64_t N,
+                      int64_t K, const Epilogue& epi, cudaStream_t st);
 // 17 to 32 tokens of a small layer (gemm_stream.cu).
 int w8a8_gemm_wide(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
                    const Epilogue& epi, cudaStream_t st, bool static_w);

@@ -111,36 +111,11 @@ quantize_per_token_kernel(const T* __restrict__ x, int64_t K, int64_t ldx, uint8
   quantize_row<T, FP8>(row, q + m * K, K, s, vec_ok);
 }
 
-// Eight packed 16-bit values -> eight quantized bytes.  The scale may be zero (an fp8 row whose
-// absmax / 448 vanishes in T): only the true division gives NaN and the saturated values there.
+// Eight packed 16-bit values -> eight quantized bytes (see the two it chooses from).
 template <typename T, bool FP8>
 __device__ __forceinline__ uint2 quantize8(const uint4& v, float s, RowScale c, bool exact_div) {
-  if constexpr (!FP8) {
-    return quantize8_int8<T>(v, c);
-  } else {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    uint32_t o[4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const float2 x = unpack_pair<T>(w[p]);
-      const float2 d = exact_div ? make_float2(__fdiv_rn(x.x, s), __fdiv_rn(x.y, s))
-                                 : make_float2(div_row_scale(x.x, c), div_row_scale(x.y, c));
-      // (saturating: the clamp to +-448)
-      o[p] = __nv_cvt_float2_to_fp8x2(unpack_pair<T>(pack_pair<T>(d.x, d.y)), __NV_SATFINITE, __NV_E4M3);
-    }
-    return make_uint2(o[0] | (o[1] << 16), o[2] | (o[3] << 16));
-  }
-}
-
-// Absolute maximum of eight packed values, joined with m.
-template <typename T> __device__ __forceinline__ float absmax8(const uint4& v, float m) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const float2 x = unpack_pair<T>(w[p]);
-    m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
-  }
-  return m;
+  if constexpr (!FP8) return quantize8_int8<T>(v, c);
+  else return quantize8_fp8<T>(v, s, c, exact_div);
 }
 
 // Maximum over the block with one barrier (one call per kernel).

@@ -56,3 +56,30 @@ def test_awq_schedules(M, K, N, G):
     x, bias = torch.randn(M, K, generator=g, device="cuda").half(), torch.randn(N, generator=g, device="cuda").half()
     want = x.double() @ ops.awq_dequantize(qw, sc, qz).double() + bias.double()
     assert rel_fro(ops.awq_gemm(x, ops.AwqPacked(qw, sc, qz), bias), want) < 5e-4      # the fp16 rounding of the result
+
+
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,K", [(16, 16), (40, 1040), (4864, 896), (520, 2048), (520, 2064), (16384, 2048)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_quantized_by_the_gemm(M, N, K, dt):
+    """The layers' results are those of the quantizer and the GEMM one after the other: int8 bit for bit (a zero row and
+    an infinite one among them), fp8 up to the order of the fp32 sums."""
+    from llmqrt_b200 import ops
+    from llmqrt_b200.linear import FP8DynamicLinear, SqW8A8BBF16OBF16PerChannel
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    lin = torch.nn.Linear(K, N, device="cuda")
+    x = torch.randn(M, K, generator=g, device="cuda").to(dt)
+    if M > 2:
+        x[1] = 0
+        x[2, K // 2] = float("inf")
+    sq = SqW8A8BBF16OBF16PerChannel.from_linear(lin, 8, 0, init_only=False, dtype=dt)
+    q, _, s = ops.quantize_int8(x, True)
+    want = ops.int8_linear_per_channel(q, sq.qweight, sq.bias, s, sq.weight_scale, dt, True)
+    assert torch.equal(sq(x).view(torch.int16), want.view(torch.int16)) or torch.equal(sq(x).isnan(), want.isnan()) and \
+        torch.equal(sq(x)[~want.isnan()], want[~want.isnan()])
+    f8 = FP8DynamicLinear.from_linear(lin, init_only=False, dtype=torch.bfloat16, per_tensor=False)
+    q, s = ops.quantize_fp8(x, True)
+    want = ops.fp8_linear_rowwise(q, f8.weight.to(torch.float8_e4m3fn), f8.bias.data, s, f8.weight_scale.data, True).to(dt)
+    y, ok = f8(x), ~want.isnan()
+    assert torch.equal(y.isnan(), want.isnan())
+    assert rel_fro(y[ok & want.isfinite()], want[ok & want.isfinite()].double()) < 2 ** -9     # (a bf16 rounding falling the other way)
