@@ -132,7 +132,7 @@ struct DecodeAppend {
   int table_rows;
   int twice;                         // 1: the new row is also written one row earlier, and its angle is that row's
   int len_add;                       // length of sequence b: (seqlens ? seqlens[b] : 0) + len_add
-  int merge_in_cluster;              // (host) the splits of a short sequence may be merged by a cluster
+  int merge_in_cluster;              // (host) a step: seqlens may be null, the splits of a short sequence may be merged by a cluster
   int cache_rows;                    // > 0: the new row is written wherever it lies inside a cache of that many rows,
                                      // also beyond the bound of this call; 0: only within the bound
 };
@@ -698,7 +698,7 @@ static int attn_decode_entry(const void* q, int64_t q_batch_stride, const void* 
   LLMQRT_REQUIRE(q_batch_stride >= Hq * d && q_batch_stride % 8 == 0, "attn_decode: q_batch_stride must be a multiple of 8 and at least Hq * d");
   LLMQRT_REQUIRE(!out_q || (out_scale && Hq * d <= 8192), "attn_decode: quantized output needs out_scale and Hq * d <= 8192");
   if (B == 0) return LLMQRT_OK;
-  LLMQRT_REQUIRE(q && k_cache && v_cache && (seqlens || ap.len_add > 0) && out, "attn_decode: null pointer");
+  LLMQRT_REQUIRE(q && k_cache && v_cache && (seqlens || ap.merge_in_cluster) && out, "attn_decode: null pointer");
   LLMQRT_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) |
                    reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(out_q) & 7) == 0, "attn_decode: pointers must be 16-byte aligned (out_q: 8)");
@@ -750,8 +750,8 @@ int llmqrt_attn_decode_step(const void* q, int64_t q_batch_stride, const void* k
                             llmqrt_stream_t stream) {
   LLMQRT_REQUIRE((k_new == nullptr) == (v_new == nullptr), "attn_decode_step: k_new and v_new go together");
   LLMQRT_REQUIRE((cos_table == nullptr) == (sin_table == nullptr), "attn_decode_step: cos and sin tables go together");
-  LLMQRT_REQUIRE(len_add >= 0 && cache_rows >= 0 && cache_rows <= 0x7fffffffll && max_seqlen <= cache_rows, "attn_decode_step: bad lengths");
-  LLMQRT_REQUIRE((twice == 0 || twice == 1) && (!(twice || cos_table) || (k_new && !seqlens && len_add <= max_seqlen)),
+  LLMQRT_REQUIRE(cache_rows >= 0 && cache_rows <= 0x7fffffffll && max_seqlen <= cache_rows, "attn_decode_step: bad lengths");
+  LLMQRT_REQUIRE((twice == 0 || twice == 1) && (!(twice || cos_table) || (k_new && !seqlens && len_add > 0 && len_add <= max_seqlen)),
                  "attn_decode_step: rotation and the doubled row need k_new and one length within max_seqlen");
   LLMQRT_REQUIRE(!k_new || (kv_batch_stride >= Hkv * d && kv_batch_stride % 8 == 0 &&
                             ((reinterpret_cast<uintptr_t>(k_new) | reinterpret_cast<uintptr_t>(v_new)) & 15) == 0),

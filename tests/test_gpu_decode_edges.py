@@ -54,6 +54,14 @@ def test_decode_step(lens, cap, bound, Hq, Hkv, d, dt, append):
         assert rel_fro(out2, out.double()) < (1e-3 if dt == torch.float16 else 8e-3)
 
 
+def test_decode_step_without_keys():
+    """A length of zero, as a number or as a tensor, gives zeros."""
+    from llmqrt_b200.attention import flash_attn_with_kvcache
+    q, kc = torch.randn(2, 1, 4, 64, device="cuda").half(), torch.randn(2, 40, 2, 64, device="cuda").half()
+    for lens in (0, torch.zeros(2, dtype=torch.int32, device="cuda")):
+        assert not flash_attn_with_kvcache(q, kc, kc.clone(), cache_seqlens=lens).any()
+
+
 @pytest.mark.parametrize("pos,cap", [(0, 2), (0, 1), (63, 65), (64, 65), (63, 64), (127, 200), (511, 1000), (700, 708), (4094, 4200)])
 @pytest.mark.parametrize("B,Hq,Hkv,d", [(1, 12, 2, 128), (3, 14, 2, 64)])
 @pytest.mark.parametrize("twice", [True, False])
