@@ -134,12 +134,12 @@ int launch_dequantize_t(const uint32_t* wq_t, const uint32_t* sz_t, int64_t K, i
 // over the WHOLE reduction dimension: its warps take the 128-value chunks of K in turn and their sums meet in shared
 // memory, so there are no partials in global memory, no arrival counter and no last block that adds the slices up.
 // Activations (a few rows) come straight from L2, no staging and no barrier before the first weights; the weights of
-// kRowsAhead chunks of a warp are in flight together, and 64 registers a thread keep two 512-thread blocks on an SM.
+// one or two chunks of a warp are in flight together, and 64 registers a thread keep two 512-thread blocks on an SM.
 // Latency-bound: a 17920 x 1536 layer (14 MB) at one token is 2 us of HBM time.  Weights from HBM, against 128-row
 // blocks with the slices of K in separate blocks: 17920 x 1536 at one token 8.0 us (11.1), 1536 x 8960 7.5 (12.1),
-// 2048 x 1536 2.6 (6.0), 3584 x 18944 20.0 (22.5); 16 tokens 16.4 (14.7), 12.4 (19.4), 3.8 (10.6), 33.7 us (35.3).
+// 2048 x 1536 2.6 (6.0), 3584 x 18944 20.0 (22.5); at 16 tokens 17920 x 1536 13.9 (14.7), 1536 x 8960 11.1 (19.4),
+// 4608 x 3584 8.1 (17.3), 37888 x 3584 46.6 (51.9).
 constexpr int kChunkK = 128;           // k-values per warp step: 4 lanes x 32 per weight row
-constexpr int kRowsAhead = 2;
 //
 // What follows the GEMM in a decoder block may be done on its sums (each step rounded to fp16 as the separate kernels
 // round it): TAIL_RESIDUAL adds a row of the residual stream, TAIL_SILU makes the 16 rows of a block eight gate and
@@ -157,6 +157,8 @@ awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* 
   const int KW = K / 8, KG = K / G;
   const int second = TAIL == TAIL_SILU ? N / 2 : 8;    // (N / 2 is a multiple of eight: whole blocks)
   const int rows[2] = {min(n0 + g, N - 1), min(n0 + g + second, N - 1)};
+  // (16 tokens: one chunk ahead, so that 64 registers nearly do -- 17920 x 1536 13.9 us, 16.4 with two)
+  constexpr int kRowsAhead = MB == 2 ? 1 : 2;
   float acc[MB][4];
 #pragma unroll
   for (int mb = 0; mb < MB; ++mb)
