@@ -70,6 +70,12 @@ __device__ __forceinline__ void pdl_wait_then_trigger() {
   pdl_wait();
   pdl_trigger();
 }
+// Cluster barrier in two halves.  A CTA's shared memory may be reached by its peers once it is known to have started:
+// a kernel that stores to a peer arrives when it starts and waits just before the store, by when the others have
+// long arrived.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 bool pdl_enabled();   // capi.cu: on unless the environment variable LLMQRT_PDL is "0"
 
 template <typename... KArgs, typename... Args>

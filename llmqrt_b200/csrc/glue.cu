@@ -233,8 +233,9 @@ __global__ void __launch_bounds__(1024)
 silu_mul_regs_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ y, int8_t* __restrict__ q,
                      float* __restrict__ scale_f32, int64_t I, int64_t slice) {
   __shared__ float slot_amax[8];                       // slot r: the maximum found by the cluster's CTA r
-  pdl_wait_then_trigger();
   const int cl = gridDim.x, rank = blockIdx.x;
+  if (q && cl > 1) cluster_arrive_relaxed();
+  pdl_wait_then_trigger();
   const int64_t m = blockIdx.y, c0 = (int64_t)rank * slice;
   float amax = 0.f;
   const T* gr = gate_up + m * ld + c0;
@@ -260,14 +261,17 @@ silu_mul_regs_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ 
     if (cl > 1) {
       // every CTA stores its maximum into its slot in EVERY CTA of the cluster, then ONE cluster barrier
       // (release / acquire) and each CTA reads its own copy: nobody reads remote memory afterwards, so
-      // there is no second barrier before leaving
+      // there is no further barrier before leaving.  (The wait belongs to the arrival at the kernel's start: the
+      // peers have started, so their shared memory may be written.)
+      cluster_wait();
       if (threadIdx.x < cl) {
         uint32_t remote;
         const uint32_t local = (uint32_t)__cvta_generic_to_shared(&slot_amax[rank]);
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"((uint32_t)threadIdx.x));
         asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(amax) : "memory");
       }
-      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+      cluster_arrive();
+      cluster_wait();
       amax = 0.f;
       for (int c = 0; c < cl; ++c) amax = fmaxf(amax, slot_amax[c]);
     }
@@ -621,6 +625,7 @@ __global__ void __launch_bounds__(256)
 argmax_rows_kernel(const T* __restrict__ x, int64_t ld, int64_t N, int64_t slice, int vec, int64_t base,
                    T* __restrict__ val, int64_t* __restrict__ idx) {
   __shared__ unsigned long long red[8], slot[8];
+  cluster_arrive_relaxed();
   pdl_wait_then_trigger();
   const int cl = gridDim.x, rank = blockIdx.x;
   const int64_t m = blockIdx.y;
@@ -656,6 +661,7 @@ argmax_rows_kernel(const T* __restrict__ x, int64_t ld, int64_t N, int64_t slice
   for (int o = 16; o > 0; o >>= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
   __syncthreads();
+  cluster_wait();                                      // the first CTA has started: its shared memory may be written
   if (threadIdx.x == 0) {
     for (int w = 1; w < 8; ++w) c = max(c, red[w]);
     uint32_t remote;
@@ -663,7 +669,8 @@ argmax_rows_kernel(const T* __restrict__ x, int64_t ld, int64_t N, int64_t slice
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(0u));
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(c) : "memory");
   }
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
   if (rank == 0 && threadIdx.x == 0) {
     c = 0;
     for (int r = 0; r < cl; ++r) c = max(c, slot[r]);
