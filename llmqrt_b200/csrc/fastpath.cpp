@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <atomic>
 
@@ -32,15 +33,18 @@ Tensor tensor_arg(PyObject* o, const char* what) {
   TORCH_CHECK_TYPE(THPVariable_Check(o), "llmqrt_b200: ", what, " must be a tensor, not ", Py_TYPE(o)->tp_name);
   return THPVariable_Unpack(o);
 }
+// int(o) and float(o): whatever converts to a number is one.
 int64_t int_arg(PyObject* o) {
-  const long long v = PyLong_AsLongLong(o);
+  THPObjectPtr n(PyNumber_Long(o));
+  if (!n) throw python_error();
+  const long long v = PyLong_AsLongLong(n.get());
   if (v == -1 && PyErr_Occurred()) throw python_error();
   return v;
 }
 double float_arg(PyObject* o) {
-  const double v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) throw python_error();
-  return v;
+  THPObjectPtr f(PyNumber_Float(o));
+  if (!f) throw python_error();
+  return PyFloat_AS_DOUBLE(f.get());
 }
 bool bool_arg(PyObject* o) {
   const int v = PyObject_IsTrue(o);
