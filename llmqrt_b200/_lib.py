@@ -114,12 +114,14 @@ if _missing:
 
 
 def _load_fast():
-    """The native host path (csrc/fastpath.cpp), built beside the library it calls."""
+    """The native host path (csrc/fastpath.cpp), built beside the library it calls.  Its file name says what it was built
+    from: where that is not the present source, C ABI, interpreter and torch, it is built anew."""
     import importlib.machinery
     import importlib.util
-    path = os.path.join(_PKG, "lib", "_fast.so")
+
+    from . import build as _build
+    path = _build.fast_path()
     if not os.path.exists(path):
-        from . import build as _build
         _build.build()
     loader = importlib.machinery.ExtensionFileLoader("_fast", path)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fast", loader))

@@ -6,13 +6,15 @@
 
 Every .cu under llmqrt_b200/csrc is compiled with nvcc to an object file and the objects are
 linked into llmqrt_b200/lib/libllmqrt_b200.so.  nvcc cross-compiles, so no GPU is needed.
-csrc/fastpath.cpp becomes the Python extension llmqrt_b200/lib/_fast.so (g++, ATen), which calls that library.
+csrc/fastpath.cpp becomes the Python extension llmqrt_b200/lib/_fast.<tag>.so (g++, ATen), which calls that library; the
+tag names what the file was made from and for (see fast_tag), so a stale one is never taken for the present one.
 """
 from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
 import glob
+import hashlib
 import os
 import shutil
 import subprocess
@@ -24,7 +26,6 @@ LIBDIR = os.path.join(PKG, "lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libllmqrt_b200.so")
 FAST_SRC = os.path.join(CSRC, "fastpath.cpp")
-FAST = os.path.join(LIBDIR, "_fast.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 NVCC_FLAGS = [
@@ -48,6 +49,21 @@ def _stale(target: str, deps: list[str]) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def fast_tag() -> str:
+    """What the host path's binary depends on: its source, the C ABI it calls, the interpreter and ATen."""
+    import torch
+    h = hashlib.sha256()
+    for path in (FAST_SRC, os.path.join(INCLUDE, "llmqrt_b200.h")):
+        with open(path, "rb") as f:
+            h.update(f.read() + b"\0")
+    h.update(repr((sys.implementation.cache_tag, torch.__version__, torch._C._GLIBCXX_USE_CXX11_ABI)).encode())
+    return h.hexdigest()[:12]
+
+
+def fast_path() -> str:
+    return os.path.join(LIBDIR, "_fast.%s.so" % fast_tag())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -84,7 +100,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n" + p.stdout + p.stderr)
-    if force or _stale(FAST, [FAST_SRC, LIB, os.path.join(INCLUDE, "llmqrt_b200.h")]):
+    if force or not os.path.exists(fast_path()):
         _build_fast()
     return LIB
 
@@ -95,7 +111,8 @@ def _build_fast() -> None:
     import torch
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
-    tmp = FAST + ".tmp%d" % os.getpid()
+    target = fast_path()
+    tmp = target + ".tmp%d" % os.getpid()
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
            "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(tdir, "include"),
            "-I" + os.path.join(tdir, "include", "torch", "csrc", "api", "include"), "-I" + os.path.join(cuda, "include"),
@@ -104,7 +121,10 @@ def _build_fast() -> None:
     p = subprocess.run(cmd, capture_output=True, text=True)
     if p.returncode != 0:
         raise RuntimeError("building the host path failed:\n" + p.stdout + p.stderr)
-    os.replace(tmp, FAST)
+    os.replace(tmp, target)
+    for old in glob.glob(os.path.join(LIBDIR, "_fast*.so")):
+        if old != target:
+            os.remove(old)
 
 
 if __name__ == "__main__":
