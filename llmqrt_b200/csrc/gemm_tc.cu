@@ -429,6 +429,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  // split mode: the second half of this barrier is in the exchange, before anything is stored into a peer
+  if (BN <= 128 && S > 1) cluster_arrive();
   // Everything above touched only shared and tensor memory; from here on global memory is read.
   // The producer thread waits later: it first requests weight tiles, which the preceding kernel of
   // the stream does not write.
@@ -764,6 +766,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
     }
     // A CTA whose waits ran out tells every CTA of the cluster before the barrier, and then ALL of
     // them skip the exchange: nobody copies into, or arrives on a barrier of, a CTA that may have left.
+    cluster_wait();                                    // (arrived at the start: every CTA of the cluster runs and has cleared its flag)
     if (!own_healthy && threadIdx.x == 64) {
       for (int o = 0; o < S; ++o) {
         uint32_t remote;

@@ -10,7 +10,7 @@ import re
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-SOURCES = [p for p in sorted(glob.glob(os.path.join(ROOT, "llmqrt_b200", "csrc", "*.cu"))) if not p.endswith("gemm_tc.cu")]
+SOURCES = sorted(glob.glob(os.path.join(ROOT, "llmqrt_b200", "csrc", "*.cu")))
 REMOTE = re.compile(r"(?:st|ld|red|atom)[a-z.]*\.shared::cluster|map_shared_rank\(|mbar_arrive_remote\(|bulk_copy_to_cta\(|"
                     r"cluster_addr\(")
 BARRIER = re.compile(r"barrier\.cluster\.wait|cluster_sync_all\(\)|cluster_wait\(\)|\.sync\(\)")
