@@ -458,9 +458,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           if (lane == 0) tc::mbar_arrive(tc::smem_u32(c == 2 ? &bar_p_ready[w] : &bar_p_rest[w]));
         }
       }
-      float s0, s1;
-      f2_split(f2_add(f2_add(ps[0], ps[1]), f2_add(ps[2], ps[3])), s0, s1);
-      l_run += s0 + s1;
+      // (halves of a pair first, then neighbouring pairs: an order that is part of the result's bits)
+      float sum[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float s0, s1;
+        f2_split(ps[i], s0, s1);
+        sum[i] = s0 + s1;
+      }
+      l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     }
 
     if (ok && n > 0) {

@@ -28,3 +28,20 @@ def test_prefill_halves(S, causal, dt, d, growth):
     want = torch.einsum("bhst,bthd->bshd", s.softmax(-1), v.double().repeat_interleave(2, 2))
     # P and the result are rounded to 16 bits: 2^-11 (fp16) or 2^-8 (bf16) each at most
     assert rel_fro(out, want) < (1e-3 if dt == torch.float16 else 8e-3)
+
+
+def test_prefill_row_sum_order():
+    """The eight partial sums of a row's P are added as neighbours, then as neighbouring pairs.  Two keys of weight 1
+    share the first one; two of weight 0.8 * 2^-23, each below half a unit of the sum and together above it, lie in the
+    third and the fourth.  The result is made a tie of fp16 but for them: added as a pair they tip it, as 64 bits do."""
+    from llmqrt_b200.attention import flash_attn_func
+    S, d = 128, 64
+    q, k, v = (torch.zeros(1, S, 1, d, device="cuda") for _ in range(3))
+    q[..., 0] = 16.0
+    k[..., 0] = -1000.0                                      # e^-2000: weight 0
+    k[:, [0, 8], :, 0] = 0.0
+    k[:, [2, 3], :, 0] = -8.0859375                          # 2^(-8.0859 * 16 / 8 * log2(e)) = 0.795 * 2^-23
+    v[:, 0], v[:, 8] = 1 + 2 ** -10, 1 + 2 ** -9
+    out = flash_attn_func(*(t.half() for t in (q, k, v)), causal=False)
+    p = (q[0, :, 0].double() @ k[0, :, 0].double().t() * d ** -0.5).softmax(-1)
+    assert torch.equal(out[0, :, 0], (p @ v[0, :, 0].double()).half())
