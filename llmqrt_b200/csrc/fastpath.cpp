@@ -20,6 +20,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "../../include/llmqrt_b200.h"
@@ -442,6 +443,25 @@ Tensor token_strided(const Tensor& x) {
   return ok ? x : x.contiguous();
 }
 
+// Key and value caches of at least B sequences, [B, rows, Hkv, d] with heads and d contiguous and one set of strides.
+// Returns the rows that both have.  The kernels index them by what the caller says, so nothing is launched before this
+// holds; the checks of shapes come before those of devices.
+int64_t check_caches(const Tensor& kc, const Tensor& vc, int64_t B, int64_t d, const char* what) {
+  TORCH_CHECK(kc.dim() == 4 && vc.dim() == 4 && kc.size(3) == d && vc.size(3) == d && vc.size(2) == kc.size(2) &&
+              kc.stride(3) == 1 && kc.stride(2) == d && vc.strides() == kc.strides(),
+              what, ": caches must be [B, S, Hkv, d] with heads and d contiguous");
+  TORCH_CHECK(kc.size(0) >= B && vc.size(0) >= B, what, ": the caches hold ", std::min(kc.size(0), vc.size(0)),
+              " sequences, the call has ", B);
+  return std::min(kc.size(1), vc.size(1));
+}
+// Lengths of B sequences, back to back.
+Tensor check_lens(const Tensor& lens, int64_t B, const char* what) {
+  if (!lens.defined()) return lens;
+  TORCH_CHECK_TYPE(lens.scalar_type() == at::kInt, what, ": sequence lengths must be int32");
+  TORCH_CHECK(lens.numel() >= B, what, ": ", lens.numel(), " sequence lengths for ", B, " sequences");
+  return lens.contiguous();
+}
+
 // (q, k, v, causal, softcap) -> out
 FAST_FN(attn_prefill) {
   FAST_BEGIN(5)
@@ -449,6 +469,8 @@ FAST_FN(attn_prefill) {
   const bool causal = bool_arg(a[3]);
   const float softcap = (float)float_arg(a[4]);
   GilRelease gil;
+  TORCH_CHECK_TYPE(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
+                   "flash_attn_func: q, k and v must share one dtype");
   Call c(same_device({&q, &k, &v}));
   TORCH_CHECK(q.dim() == 4 && k.dim() == 4 && k.size(1) == q.size(1) && v.sizes() == k.sizes() && k.size(0) == q.size(0) &&
               k.size(3) == q.size(3), "flash_attn_func: q, k, v must share batch, sequence length and head_dim");
@@ -472,17 +494,21 @@ FAST_FN(attn_prefill) {
 FAST_FN(kv_append) {
   FAST_BEGIN(6)
   const Tensor kc = tensor_arg(a[0], "k_cache"), vc = tensor_arg(a[1], "v_cache"), k0 = tensor_arg(a[2], "k");
-  const Tensor v0 = tensor_arg(a[3], "v"), lens = tensor_arg(a[4], "cache_seqlens");
+  const Tensor v0 = tensor_arg(a[3], "v"), lens0 = tensor_arg(a[4], "cache_seqlens");
   const int64_t start = int_arg(a[5]);
   GilRelease gil;
+  TORCH_CHECK(k0.dim() == 4 && v0.sizes() == k0.sizes(), "kv_append: k and v must be [B, S, Hkv, d]");
+  TORCH_CHECK_TYPE(k0.scalar_type() == kc.scalar_type() && v0.scalar_type() == kc.scalar_type() &&
+                   vc.scalar_type() == kc.scalar_type(), "kv_append: k, v and the caches must share one dtype");
+  const int64_t B = k0.size(0), S = k0.size(1), Hkv = k0.size(2), d = k0.size(3);
+  const int64_t cache_rows = check_caches(kc, vc, B, d, "kv_append");
+  TORCH_CHECK(kc.size(2) >= Hkv, "kv_append: the caches have ", kc.size(2), " heads, k has ", Hkv);
+  const Tensor lens = check_lens(lens0, B, "kv_append");
   Call c(same_device({&kc, &vc, &k0, &v0, &lens}));
   const Tensor k = k0.contiguous(), v = v0.contiguous();
-  const int64_t B = k.size(0), S = k.size(1), Hkv = k.size(2), d = k.size(3);
-  TORCH_CHECK(kc.stride(3) == 1 && kc.stride(2) == d && vc.strides() == kc.strides(),
-              "kv_append: caches must be [B, S, Hkv, d] with heads and d contiguous");
   check(llmqrt_kv_append(mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), ptr(k), ptr(v),
                          static_cast<const int32_t*>(ptr(lens)), (int32_t)start, dtype_code(kc.scalar_type()), B, S, Hkv, d,
-                         kc.size(1), c.stream));
+                         cache_rows, c.stream));
   gil.done();
   Py_RETURN_NONE;
   FAST_END
@@ -501,21 +527,21 @@ int64_t rows_stride(const Tensor& t, int64_t B, int64_t H, int64_t d, const char
 FAST_FN(attn_decode) {
   FAST_BEGIN(11)
   Tensor q = tensor_arg(a[0], "q");
-  const Tensor kc = tensor_arg(a[1], "k_cache"), vc = tensor_arg(a[2], "v_cache"), lens = tensor_arg(a[3], "seqlens");
-  const int64_t max_seqlen = int_arg(a[4]);
+  const Tensor kc = tensor_arg(a[1], "k_cache"), vc = tensor_arg(a[2], "v_cache"), lens0 = tensor_arg(a[3], "seqlens");
+  const int64_t max_seqlen0 = int_arg(a[4]);
   const float softcap = (float)float_arg(a[5]);
   const bool quantize = bool_arg(a[6]);
   const Tensor kn = tensor_arg(a[7], "k_new"), vn = tensor_arg(a[8], "v_new");
   const Tensor cos = tensor_arg(a[9], "cos"), sin = tensor_arg(a[10], "sin");
   GilRelease gil;
+  TORCH_CHECK(q.dim() == 3, "attn_decode: q must be [B, Hq, d] and the caches [B, S, Hkv, d]");
+  const int64_t B = q.size(0), Hq = q.size(1), d = q.size(2);
+  const int64_t max_seqlen = std::min(max_seqlen0, check_caches(kc, vc, B, d, "attn_decode")), Hkv = kc.size(2);
+  TORCH_CHECK_TYPE(lens0.defined(), "attn_decode: seqlens must be int32");
+  const Tensor lens = check_lens(lens0, B, "attn_decode");
   Call c(same_device({&q, &kc, &vc, &lens, &kn, &vn, &cos, &sin}));
-  TORCH_CHECK(q.dim() == 3 && kc.dim() == 4, "attn_decode: q must be [B, Hq, d] and the caches [B, S, Hkv, d]");
-  const int64_t B = q.size(0), Hq = q.size(1), d = q.size(2), Hkv = kc.size(2);
-  TORCH_CHECK(kc.stride(3) == 1 && kc.stride(2) == d && vc.strides() == kc.strides(),
-              "attn_decode: caches must be [B, S, Hkv, d] with heads and d contiguous");
   TORCH_CHECK_TYPE(kc.scalar_type() == q.scalar_type() && vc.scalar_type() == q.scalar_type(),
                    "attn_decode: q and the caches must share one dtype");
-  TORCH_CHECK_TYPE(lens.scalar_type() == at::kInt, "attn_decode: seqlens must be int32");
   if (B > 0 && (q.stride(2) != 1 || q.stride(1) != d || (B > 1 && (q.stride(0) < Hq * d || q.stride(0) % 8)) ||
                 reinterpret_cast<uintptr_t>(q.data_ptr()) % 16))
     q = q.contiguous();
@@ -551,20 +577,20 @@ FAST_FN(attn_decode) {
 FAST_FN(attn_decode_step) {
   FAST_BEGIN(12)
   const Tensor q4 = tensor_arg(a[0], "q"), kc = tensor_arg(a[1], "k_cache"), vc = tensor_arg(a[2], "v_cache");
-  const Tensor k4 = tensor_arg(a[3], "k"), v4 = tensor_arg(a[4], "v"), lens = tensor_arg(a[5], "cache_seqlens");
-  const int64_t len_add = int_arg(a[6]), max_seqlen = int_arg(a[7]);
+  const Tensor k4 = tensor_arg(a[3], "k"), v4 = tensor_arg(a[4], "v"), lens0 = tensor_arg(a[5], "cache_seqlens");
+  const int64_t len_add = int_arg(a[6]), max_seqlen0 = int_arg(a[7]);
   const float softcap = (float)float_arg(a[8]);
   const Tensor cos = tensor_arg(a[9], "cos"), sin = tensor_arg(a[10], "sin");
   const bool twice = bool_arg(a[11]);
   GilRelease gil;
+  TORCH_CHECK(q4.dim() == 4 && q4.size(1) == 1, "attn_decode: q must be [B, 1, Hq, d] and the caches [B, S, Hkv, d]");
+  const int64_t B = q4.size(0), Hq = q4.size(2), d = q4.size(3);
+  const int64_t cache_rows = check_caches(kc, vc, B, d, "attn_decode"), Hkv = kc.size(2);
+  const int64_t max_seqlen = std::min(max_seqlen0, cache_rows);
+  const Tensor lens = check_lens(lens0, B, "attn_decode");
   Call c(same_device({&q4, &kc, &vc, &k4, &v4, &lens, &cos, &sin}));
-  TORCH_CHECK(q4.dim() == 4 && kc.dim() == 4 && vc.dim() == 4, "attn_decode: q must be [B, 1, Hq, d] and the caches [B, S, Hkv, d]");
-  const int64_t B = q4.size(0), Hq = q4.size(2), d = q4.size(3), Hkv = kc.size(2);
-  TORCH_CHECK(kc.stride(3) == 1 && kc.stride(2) == d && vc.strides() == kc.strides(),
-              "attn_decode: caches must be [B, S, Hkv, d] with heads and d contiguous");
   TORCH_CHECK_TYPE(kc.scalar_type() == q4.scalar_type() && vc.scalar_type() == q4.scalar_type(),
                    "attn_decode: q and the caches must share one dtype");
-  TORCH_CHECK_TYPE(!lens.defined() || lens.scalar_type() == at::kInt, "attn_decode: seqlens must be int32");
   auto usable = [&](const Tensor& t, int64_t H) {
     return t.stride(3) == 1 && t.stride(2) == d && (B <= 1 || (t.stride(0) >= H * d && t.stride(0) % 8 == 0)) &&
            reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
@@ -591,7 +617,7 @@ FAST_FN(attn_decode_step) {
   Tensor out = empty(q4, q4.sizes(), q4.scalar_type());
   check(llmqrt_attn_decode_step(ptr(q), B > 1 ? q.stride(0) : Hq * d, ptr(k), ptr(v), k.defined() && B > 1 ? k.stride(0) : Hkv * d,
                                 static_cast<const float*>(ptr(cos)), static_cast<const float*>(ptr(sin)),
-                                cos.defined() ? cos.size(0) : 0, twice ? 1 : 0, mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), kc.size(1),
+                                cos.defined() ? cos.size(0) : 0, twice ? 1 : 0, mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), cache_rows,
                                 static_cast<const int32_t*>(ptr(lens)), (int32_t)len_add, mptr(out),
                                 dtype_code(q4.scalar_type()), B, Hq, Hkv, d, max_seqlen, softcap, c.workspace(), c.stream));
   gil.done();
