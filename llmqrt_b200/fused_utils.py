@@ -22,6 +22,7 @@ from __future__ import annotations
 import torch
 
 from .linear import FP8DynamicLinear, SqW8A8BBF16OBF16PerChannel, WQLinear_GEMM
+from .linear.linear_base import forward_is
 
 
 def _cat_bias(layers):
@@ -121,7 +122,7 @@ class FusedGateUpMLP(torch.nn.Module):
 
     def add_to(self, residual, x):
         """residual + forward(x)."""
-        if torch.is_grad_enabled() and residual.requires_grad:
+        if torch.is_grad_enabled() and residual.requires_grad or not forward_is(self, FusedGateUpMLP, _MLP_FORWARD):
             return residual + self.forward(x)
         with torch.no_grad():
             h, down = self._hidden(x), self.down_proj
@@ -129,3 +130,6 @@ class FusedGateUpMLP(torch.nn.Module):
                     and residual.device == h.device and residual.shape == (*h.shape[:-1], down.out_features):
                 return down.add_to(residual, h)
             return residual + down(h)
+
+
+_MLP_FORWARD = FusedGateUpMLP.forward

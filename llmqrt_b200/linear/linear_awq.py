@@ -12,7 +12,7 @@ import torch
 
 from .. import ops
 from .._lib import fast
-from .linear_base import LinearBase, tensor_key
+from .linear_base import LinearBase, calls_plainly, tensor_key
 
 AWQ_PACK_ORDER = [0, 2, 4, 6, 1, 3, 5, 7]
 
@@ -93,11 +93,11 @@ class WQLinear_GEMM(LinearBase):
         return fast.awq_linear(x.detach().to(torch.float16), p.wq_t, p.sz_t, self.bias, p.K, p.N, p.G).to(input_dtype)
 
     def takes_tail(self, x, multiple=8) -> bool:
-        """Whether `silu_halves` / `add_to` apply: a few fp16 tokens, and no hook that would see the plain output."""
+        """Whether `silu_halves` / `add_to` apply: a few fp16 tokens, and nobody who would see the plain output."""
         return (x.dtype == torch.float16 and x.is_cuda and 0 < x.numel() <= 16 * self.in_features
                 and x.shape[-1] == self.in_features and self.in_features % 32 == 0 and self.group_size % 32 == 0
                 and self.out_features % multiple == 0 and x.device == self.qweight.device
-                and not (self._forward_hooks or self._forward_pre_hooks) and type(self) is WQLinear_GEMM)
+                and calls_plainly(self, WQLinear_GEMM, _FORWARD))
 
     def silu_halves(self, x):
         """silu(y[..., :N/2]) * y[..., N/2:] of y = self(x), one kernel (see takes_tail, multiple 16)."""
@@ -112,3 +112,6 @@ class WQLinear_GEMM(LinearBase):
     def extra_repr(self) -> str:
         return "in_features={}, out_features={}, bias={}, w_bit={}, group_size={}".format(
             self.in_features, self.out_features, self.bias is not None, self.w_bit, self.group_size)
+
+
+_FORWARD = WQLinear_GEMM.forward

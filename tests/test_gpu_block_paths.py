@@ -1,0 +1,129 @@
+"""A few-token 4-bit decoder block runs its additions and SiLU inside the GEMMs.  Whoever watches, replaces or
+differentiates one of its modules must see the calls that the plain composition makes, and the same numbers."""
+import contextlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+H, HQ, HKV, D, I, G = 128, 2, 1, 64, 256, 32
+
+
+def _layer(n, k, g):
+    from llmqrt_b200.linear import WQLinear_GEMM
+    layer = WQLinear_GEMM(4, G, k, n, False, "cuda")
+    layer.qweight.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+    layer.qzeros.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
+    layer.scales.uniform_(0.001, 0.01, generator=g)
+    return layer
+
+
+def _block(rows=16):
+    from llmqrt_b200.fused_utils import FusedGateUpMLP
+    from llmqrt_b200.nonlinear import LlamaLikeBlock, RMSNorm
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mlp = FusedGateUpMLP(_layer(I, H, g), _layer(I, H, g), _layer(H, I, g))
+    norms = [RMSNorm((1 + 0.1 * torch.randn(H, generator=g, device="cuda")).half()) for _ in range(2)]
+    return LlamaLikeBlock(H, HQ, HKV, _layer((HQ + 2 * HKV) * D, H, g), None, None, None, _layer(H, HQ * D, g), mlp, *norms,
+                          dev="cuda", max_seq_len=rows)
+
+
+def _plain(block, x):
+    """The block as a composition of calls, each one its module's own."""
+    h = x + block.attn(block.norm_1(x))[0]
+    return h + block.mlp.forward(block.norm_2(h))
+
+
+def _run(block, f, x):
+    block.attn.start_pos = 3
+    return f(block, x)
+
+
+@contextlib.contextmanager
+def _watch(block, name, how, seen):
+    """Puts a witness on the module `name`; it adds 1 to what the module gives, so passing it by also shows."""
+    from torch.nn.modules import module as M
+    target = block.get_submodule(name)
+    cls, forward = type(target), type(target).forward
+
+    def hook(module, *args):
+        if module is target:
+            seen.append(name)
+            return args[-1] + 1
+
+    def replaced(*args):
+        seen.append(name)
+        return forward(*(args if args[0] is target else (target, *args))) + 1
+
+    if how == "hook":
+        handle = target.register_forward_hook(hook)
+    elif how == "pre-hook":
+        handle = target.register_forward_pre_hook(lambda m, a: (seen.append(name), (a[0] + 1,))[1])
+    elif how == "global":
+        handle = M.register_module_forward_hook(hook)
+    elif how == "instance":
+        target.forward = replaced
+    else:
+        cls.forward = lambda self, *a: replaced(self, *a) if self is target else forward(self, *a)
+    try:
+        yield
+    finally:
+        if how in ("hook", "pre-hook", "global"):
+            handle.remove()
+        elif how == "instance":
+            del target.forward
+        else:
+            cls.forward = forward
+
+
+@pytest.mark.parametrize("how", ["hook", "pre-hook", "global", "instance", "class"])
+@pytest.mark.parametrize("name", ["mlp.gate_up", "mlp.down_proj", "norm_2", "mlp"])
+def test_witnesses_see_their_calls(name, how):
+    if name == "mlp" and how in ("hook", "pre-hook", "global"):
+        pytest.skip("the block takes the MLP's forward, not its call")
+    block, x = _block(), torch.randn(1, 1, H, device="cuda").half()
+    want = _run(block, _plain, x)
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want)          # the fused form rounds as the plain one
+    seen = []
+    with _watch(block, name, how, seen):
+        got = _run(block, lambda b, t: b(t), x)
+        assert seen == [name]
+        assert torch.equal(got, _run(block, _plain, x)) and not torch.equal(got, want)
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want)
+
+
+def test_gradients_reach_the_residual():
+    """The layers have no backward; the residual stream around them has one."""
+    block, g = _block(), torch.Generator(device="cuda").manual_seed(5)
+    h, y = (torch.randn(1, 1, H, generator=g, device="cuda").half() for _ in range(2))
+    want = h + block.mlp.forward(y)
+    h.requires_grad_()
+    out = block.mlp.add_to(h, y)
+    assert torch.equal(out, want)
+    out.sum().backward()
+    assert torch.equal(h.grad, torch.ones_like(h))
+    a, b = h.detach(), y.clone().requires_grad_()
+    s, n = block.norm_2.add(a, b)
+    assert s.requires_grad and torch.equal(s, a + y) and torch.equal(n, block.norm_2(a + y))
+    s.sum().backward()
+    assert torch.equal(b.grad, torch.ones_like(b))
+
+
+def test_full_cache():
+    """A token beyond the cache's last row: attended over the whole cache, neither rotated nor written."""
+    rows = 16
+    block = _block(rows)
+    a, g = block.attn, torch.Generator(device="cuda").manual_seed(7)
+    a.cache.k.normal_(generator=g)
+    a.cache.v.normal_(generator=g)
+    kept = a.cache.k.clone(), a.cache.v.clone()
+    x = torch.randn(1, 1, H, generator=g, device="cuda").half()
+    q = a.qkv_proj(x).view(HQ + 2 * HKV, D)[:HQ].double()
+    for pos in (rows, rows + 5):
+        a.start_pos = pos
+        _, weight, _ = a(x)
+        p = (q @ kept[0][0, :, 0].double().t() * D ** -0.5).softmax(-1)
+        want = (p @ kept[1][0, :, 0].double()).reshape(1, 1, HQ * D)
+        assert float((weight.double() - want).norm() / want.norm()) < 1e-3     # P and the result in fp16: 2^-11 each
+        assert torch.equal(a.cache.k, kept[0]) and torch.equal(a.cache.v, kept[1]) and a.start_pos == pos + 1
