@@ -117,6 +117,21 @@ def test_rmsnorm_small_blocks(H, dt):
     assert torch.equal(y2, y)
 
 
+@pytest.mark.parametrize("H", [8, 264, 1016, 1032, 2056, 3584, 4104, 8192])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_rmsnorm_bits_do_not_depend_on_the_batch(H, dt):
+    """Many rows take small blocks with several units per thread, few rows one unit per thread: one order of the sum."""
+    from llmqrt_b200 import glue
+    x, r = (torch.randn(600, H, generator=_g(8 + i), device="cuda").to(dt) for i in range(2))
+    w = (1 + 0.1 * torch.randn(H, generator=_g(10), device="cuda")).to(dt)
+    many = glue.rmsnorm(x, w, 1e-6, residual=r, quantize=True)
+    for i in range(0, 600, 200):
+        few = glue.rmsnorm(x[i:i + 200], w, 1e-6, residual=r[i:i + 200], quantize=True)
+        for a, b in zip(many, few):
+            a = a[i:i + 200]
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16)) if a.dtype == dt else torch.equal(a, b)
+
+
 @pytest.mark.parametrize("M,N", [(1, 1), (3, 7), (2, 4096), (64, 8200), (5, 9001), (64, 152064), (300, 1024)])
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
 def test_argmax_rows(M, N, dt):
