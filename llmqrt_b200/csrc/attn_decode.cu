@@ -25,7 +25,12 @@ namespace {
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kClusterMergeMaxLen = 4096;   // longest sequence whose splits a cluster merges (512 keys per block)
+// Greatest bound (with a fixed cache its capacity) whose splits a cluster merges.  The blocks share out the sequence's own
+// length, so a short one in a large cache is split as far as a full one.  One sequence of 60 / 500 / 4000 keys in 4096
+// rows, 12 / 2 heads of 128: 5.0 / 5.1 / 9.3 us, with the merge kernel 7.6 / 9.3 / 22.6 (shares of the bound, as they were,
+// left the 500 keys to one block: 9.5); 16 sequences, 14 / 2 heads of 64: 5.3 / 5.3 / 9.8 against 7.2 / 10.8 / 15.5.  In 8192
+// rows the shortest of many would lose (16 x 60 keys 5.6 against 5.1).
+constexpr int kClusterMergeMaxLen = 4096;
 constexpr int kRing = 3;            // cp.async stages per warp (2 measured slower: too few bytes in flight)
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void* src) {
@@ -165,6 +170,12 @@ attn_decode_kernel(const uint16_t* __restrict__ q, int64_t q_batch_stride, const
   // nothing is appended, so neither the cache nor a neighbour's partial slots are touched.
   const int L_raw = (seqlens ? seqlens[b] : 0) + ap.len_add;
   const int L = min(L_raw, max_len);
+  // The blocks of a merging cluster share this sequence's own length out, in whole steps of the block's warps: the bound
+  // (with a fixed cache its capacity) may be many times as long.
+  if (merge_cluster > 1) {
+    constexpr int kStep = 16 * kWarps;
+    chunk = max(kStep, ((L + merge_cluster - 1) / merge_cluster + kStep - 1) / kStep * kStep);
+  }
   const int key_begin = split * chunk;
   if (ap.cache_rows > 0 && split == 0 && L_raw > max_len && L_raw <= ap.cache_rows) {
     // the new row lies beyond what this call attends to: no block covers it, the first one writes it

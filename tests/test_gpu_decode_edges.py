@@ -1,5 +1,5 @@
 """Edges of the decode-sized kernels: splits merged by a cluster, the row appended by the attention kernel, and the
-4-bit GEMM of at most eight tokens."""
+4-bit GEMM of a few tokens with and without the next step on its sums."""
 import pytest
 import torch
 
@@ -135,3 +135,45 @@ def test_awq_expansion_bits(K, N, G):
     qw, qz, sc = oa.random_layer(K, N, G, seed=K)
     packed = ops.AwqPacked(qw.cuda(), sc.cuda(), qz.cuda())
     assert torch.equal(ops.awq_dequantize_t(packed).cpu(), oa.dequantize(qw, qz, sc, G).t())
+
+
+@pytest.mark.parametrize("lens,cap", [([1], 4096), ([63], 4096), ([64], 2048), ([65], 4096), ([500], 4096), ([511], 4096),
+                                      ([512], 4096), ([513, 2, 4000], 4096), ([1025, 64], 2048), ([3000], 3072)])
+@pytest.mark.parametrize("Hq,Hkv,d", [(12, 2, 128), (14, 2, 64)])
+@pytest.mark.parametrize("append", [True, False])
+def test_short_sequences_in_a_large_cache(lens, cap, Hq, Hkv, d, append):
+    """A cluster's blocks share out the sequence's own length, whatever the cache could hold."""
+    test_decode_step(lens, cap, None, Hq, Hkv, d, torch.float16, append)
+
+
+@pytest.mark.parametrize("pos,cap", [(0, 2), (0, 1), (63, 65), (64, 66), (127, 200), (700, 2048), (4094, 4200)])
+@pytest.mark.parametrize("B,Hq,Hkv,d,dt", [(1, 12, 2, 128, torch.float16), (3, 14, 2, 64, torch.bfloat16)])
+@pytest.mark.parametrize("twice", [True, False])
+def test_decode_rotary_step_against_64_bits(pos, cap, B, Hq, Hkv, d, dt, twice):
+    from llmqrt_b200 import glue
+    from llmqrt_b200.attention import decode_rotary_step
+    if pos + 1 + twice > cap:
+        pytest.skip("the second row does not fit")
+    g = torch.Generator(device="cuda").manual_seed(pos + cap)
+    kc, vc = (torch.randn(B, cap, Hkv, d, generator=g, device="cuda").to(dt) for _ in range(2))
+    row = torch.randn(B, 1, Hq + 2 * Hkv, d, generator=g, device="cuda").to(dt)
+    q, k, v = row[:, :, :Hq], row[:, :, Hq:Hq + Hkv], row[:, :, Hq + Hkv:]
+    cos, sin = glue.rope_tables(d, cap, 1e6, "cuda")
+    ang = pos * 1e6 ** (-torch.arange(0, d, 2, dtype=torch.float64, device="cuda") / d)
+
+    def rotate(x):
+        a, b = x[:, 0].double().chunk(2, -1)
+        return torch.cat([a * ang.cos() - b * ang.sin(), a * ang.sin() + b * ang.cos()], -1)
+
+    want_k, want_v = kc.double(), vc.double()
+    for r in range(pos, pos + 1 + twice):
+        want_k[:, r], want_v[:, r] = rotate(k), v[:, 0].double()
+    n, rq = pos + 1 + twice, rotate(q)
+    want = torch.stack([_attend(rq[b], want_k[b, :n], want_v[b, :n]) for b in range(B)])
+    out = decode_rotary_step(q, k, v, kc, vc, cos, sin, pos, twice)
+    eps = 2 ** -11 if dt == torch.float16 else 2 ** -8
+    assert torch.equal(vc.double(), want_v)
+    # the angle in fp32 (position times 2^-24, twice) and one rounding of the rotated key
+    assert rel_fro(kc, want_k) < eps + 4 * pos * 2 ** -24
+    # q, k, P and the result rounded once each; scores of d products of unit variance pass on sqrt(2) of q's and k's
+    assert rel_fro(out[:, 0], want) < 4 * eps + 8 * pos * 2 ** -24
