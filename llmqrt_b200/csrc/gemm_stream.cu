@@ -220,7 +220,8 @@ constexpr int kRowsAhead = 2;
 // Activations that the kernel quantizes itself (per token, bit for bit as the stand-alone quantizer): T the 16-bit
 // type, void for activations that arrive quantized.  Every block reads the rows once for their scales and once as
 // fragments, which is cheap while a few blocks share a few rows, and saves a launch and its hand-over: a pass over a
-// 4864 x 896 layer of 16 tokens takes 9.4 us instead of 10.9.
+// 4864 x 896 layer of 16 tokens takes 9.4 us instead of 10.9.  (The fp8 form for 9 to 16 tokens spills 68 bytes a thread:
+// 64 registers keep two 512-thread blocks on an SM.)
 template <typename T> struct DynScale {                // of one token
   float s;
   RowScale c;
@@ -412,11 +413,16 @@ w8a8_wide_kernel(const uint8_t* __restrict__ A, int64_t lda, const uint8_t* __re
   }
 }
 
+// Warps of a block: the chunks of K in as few rounds as twelve warps need.
+int wide_warps(int64_t K) {
+  const int64_t chunks = ceil_div(K, (int64_t)kChunk);
+  return (int)ceil_div(chunks, ceil_div(chunks, (int64_t)kWideWarps));
+}
+
 template <int KIND>
 int launch_wide(const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int M, int N, int K, const Epilogue& epi,
                 cudaStream_t st, bool static_w) {
-  const int blocks = (int)ceil_div(N, kWideRows), chunks = (int)ceil_div(K, kChunk);
-  const int rounds = (int)ceil_div(chunks, kWideWarps), warps = (int)ceil_div(chunks, rounds);
+  const int blocks = (int)ceil_div(N, kWideRows), chunks = (int)ceil_div(K, kChunk), warps = wide_warps(K);
   const size_t smem = (size_t)warps * 32 * kWidePitch * 4;
   auto kern = w8a8_wide_kernel<KIND>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kWideWarps * 32 * kWidePitch * 4)) return rc;
@@ -457,6 +463,20 @@ int w8a8_gemm_dynamic(int kind, int x_dtype, const void* x, int64_t ldx, const u
   using F8 = std::integral_constant<int, KIND_F8_E4M3>;
   if (kind == KIND_I8) return x_dtype == LLMQRT_F16 ? go(I8(), __half()) : go(I8(), __nv_bfloat16());
   return x_dtype == LLMQRT_F16 ? go(F8(), __half()) : go(F8(), __nv_bfloat16());
+}
+
+// Blocks that are all resident at once, over a reduction short enough for the tcgen05 kernel's fixed cost to outweigh
+// the activations that every block fetches.  Quantizer and GEMM of 32 tokens, weights from HBM, us (tcgen05):
+//   int8, a block per SM:   2048 x 1536 5.8 (8.1), 4736 x 3584 9.6 (11.9), 1536 x 4096 9.3 (9.5); 1536 x 4608 9.9 (9.7)
+//   int8, two blocks per SM, as 118 registers allow for at most eight warps: 4864 x 896 6.5 (8.5), 9472 x 1024 6.8 (9.6);
+//     with nine warps 4864 x 1152 9.8 (9.0), beyond two blocks 12288 x 896 11.7 (8.3)
+//   fp8, whose loop is slower (168 registers: one block per SM): 4736 x 1536 7.8 (9.5), 896 x 2048 7.5 (8.0);
+//     896 x 3072 9.5 (8.9), 1536 x 3584 10.7 (9.3), 4864 x 896 11.0 (8.7)
+// At 17 tokens the lines lie at the same places.
+bool w8a8_wide_fits(int kind, int64_t N, int64_t K) {
+  const int64_t blocks = ceil_div(N, (int64_t)kWideRows), sms = sm_count();
+  if (kind != KIND_I8) return blocks <= sms && K <= 2048;
+  return (blocks <= sms && K <= 4096) || (blocks <= 2 * sms && wide_warps(K) <= 8);
 }
 
 int w8a8_gemm_wide(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N, int64_t K,

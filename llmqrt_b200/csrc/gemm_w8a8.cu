@@ -36,10 +36,7 @@ int run(int kind, const void* a, int64_t lda, const void* w, int64_t ldw, int64_
   if (stream)
     return w8a8_gemm_stream(kind, reinterpret_cast<const uint8_t*>(a), lda, reinterpret_cast<const uint8_t*>(w), ldw,
                             M, N, K, epi, workspace, st, (flags & LLMQRT_GEMM_STATIC_WEIGHT) != 0);
-  // 17 to 32 tokens and blocks of 32 rows that fit the device at once, over a short reduction: the kernel without the
-  // tcgen05 kernel's fixed cost.  Quantizer and GEMM of 32 tokens: 2048 x 1536 5.7 us (7.9), 4864 x 896 6.6 (8.6), 4608
-  // x 3584 10.2 (11.1); beyond that the activations of every block outweigh the weights: 1536 x 8960 16.1 (11.9).
-  if (path == 0 && M <= 32 && N <= 32 * (int64_t)sm_count() && K <= 3584)
+  if (path == 0 && M <= 32 && w8a8_wide_fits(kind, N, K))
     return w8a8_gemm_wide(kind, reinterpret_cast<const uint8_t*>(a), lda, reinterpret_cast<const uint8_t*>(w), ldw, M, N, K, epi, st,
                           (flags & LLMQRT_GEMM_STATIC_WEIGHT) != 0);
   return gemm_tc(kind, a, lda, w, ldw, M, N, K, epi, workspace, st, (flags & LLMQRT_GEMM_STATIC_WEIGHT) != 0);

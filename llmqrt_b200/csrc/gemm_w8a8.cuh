@@ -18,7 +18,8 @@ enum GemmKind : int {
 bool w8a8_dynamic_fits(int64_t M, int64_t N, int64_t K);
 int w8a8_gemm_dynamic(int kind, int x_dtype, const void* x, int64_t ldx, const uint8_t* W, int64_t ldw, int64_t M, int64_t N,
                       int64_t K, const Epilogue& epi, cudaStream_t st);
-// 17 to 32 tokens of a small layer (gemm_stream.cu).
+// 17 to 32 tokens of a small layer (gemm_stream.cu): whether the sizes suit it, and the call.
+bool w8a8_wide_fits(int kind, int64_t N, int64_t K);
 int w8a8_gemm_wide(int kind, const uint8_t* A, int64_t lda, const uint8_t* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
                    const Epilogue& epi, cudaStream_t st, bool static_w);
 // Register-operand streaming kernels (gemm_stream.cu): any M, tuned for M <= 16.

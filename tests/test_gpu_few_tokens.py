@@ -28,6 +28,25 @@ def test_few_tokens(M, N, K):
     assert rel_fro(y, (x8.double() @ w8.double().t()) * s[:, None] * ws) < 2 ** -8      # bf16 result
 
 
+@pytest.mark.parametrize("M", [17, 24, 32])
+@pytest.mark.parametrize("N,K", [(4608, 3584), (2048, 1536), (4736, 4096), (4729, 3568), (1001, 2048), (9472, 1024), (9465, 896),
+                                 (4864, 512), (4737, 1152), (9473, 896), (896, 2064), (1536, 4112)])
+def test_wide_blocks(M, N, K):
+    """The 32-row blocks at their largest (twelve warps, several rounds of chunks, two blocks to an SM, ragged N and K) and
+    the first sizes beyond: int8 exact, fp8 up to the rounding of its result."""
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    want = a.double() @ w.double().t()
+    assert torch.equal(ops.int8_gemm_s32(a, w, True).double(), want)
+    s, ws = torch.rand(M, generator=g, device="cuda"), torch.rand(N, generator=g, device="cuda")
+    x8 = torch.randn(M, K, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    w8 = torch.randn(N, K, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    y = ops.fp8_linear_rowwise(x8, w8, None, s.view(M, 1), ws.view(1, N), True)
+    assert rel_fro(y, (x8.double() @ w8.double().t()) * s[:, None] * ws) < 2 ** -8      # bf16 result
+
+
 @pytest.mark.parametrize("M", [129, 160, 255, 257, 333, 512, 640, 1025, 1100])
 @pytest.mark.parametrize("N,K", [(40, 1040), (136, 64), (896, 4864), (1000, 1536), (1001, 512), (1536, 8960), (4864, 896)])
 def test_chunk_schedules(M, N, K):
