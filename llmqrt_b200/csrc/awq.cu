@@ -157,7 +157,8 @@ awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* 
   const int KW = K / 8, KG = K / G;
   const int second = TAIL == TAIL_SILU ? N / 2 : 8;    // (N / 2 is a multiple of eight: whole blocks)
   const int rows[2] = {min(n0 + g, N - 1), min(n0 + g + second, N - 1)};
-  // (16 tokens: one chunk ahead, so that 64 registers nearly do -- 17920 x 1536 13.9 us, 16.4 with two)
+  // (16 tokens: one chunk ahead, so that 64 registers nearly do -- 8 to 16 bytes are spilled; 17920 x 1536 13.9 us, 16.4
+  // with two)
   constexpr int kRowsAhead = MB == 2 ? 1 : 2;
   float acc[MB][4];
 #pragma unroll
@@ -227,7 +228,7 @@ awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* 
       const int m = i >> 3, r = i & 7, n = n0 + r;
       const float gate = round_to<__half>(epilogue_value(epi, total(m * 16 + r), m, n, 1.f));
       const float up = round_to<__half>(epilogue_value(epi, total(m * 16 + 8 + r), m, n + second, 1.f));
-      reinterpret_cast<__half*>(epi.out)[m * epi.ldo + n] = from_f32<__half>(round_to<__half>(silu_f32(gate)) * up);
+      reinterpret_cast<__half*>(epi.out)[m * epi.ldo + n] = from_f32<__half>(round_to<__half>(silu_pair<__half>(make_float2(gate, gate)).x) * up);
     }
   } else {
     for (int i = tid; i < M * 16; i += blockDim.x) {

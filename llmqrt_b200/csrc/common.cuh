@@ -10,6 +10,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <type_traits>
 
 #include "../../include/llmqrt_b200.h"
 
@@ -212,13 +213,72 @@ template <typename T> __device__ __forceinline__ float absmax8(const uint4& v, f
   }
   return m;
 }
-// x / (1 + e^-x), for a result that is then rounded to 16 bits: the special-function unit's exponential and
-// reciprocal (each within 2 ulp of fp32) instead of the library's, an eighth of the instructions.
-__device__ __forceinline__ float silu_f32(float x) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return x * r;
+// Two fp32 operations per instruction (packed pairs).
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_split(F2 p, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+// silu of two values of type T, x / (1 + e^-x) in fp32: rounded to T, the bits of that expression with the library's
+// exponential and a true division, for every one of T's 65536 values.  The divisor is carried as (1 + e^-x) / 4, whose
+// reciprocal is a normal number while e^-x is finite.
+// bf16: the special-function unit's exponential and reciprocal are exact enough for its eight bits.
+// fp16: they would round two gates the other way.  The reciprocal (within an ulp) gives a quotient q that one step on
+// its remainder rounds correctly, without a division's checks of range; an infinity of either side is carried as the
+// greatest number (min.NaN keeps a NaN), and with d the divisor, r = -1 / d and x4 = -x / 4 a negative zero keeps its sign.
+// 4096 rows of 18944: 97 us in fp16 (79 with the special-function unit alone, which bf16 keeps), 157 us with the plain
+// expression in the staged kernel.
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float a) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+template <typename T> __device__ __forceinline__ float2 silu_pair(float2 x) {
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    auto one = [](float v) {
+      float e;
+      asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * -1.4426950408889634f));
+      return (v * 0.25f) * rcp_approx(__fmaf_rn(e, 0.25f, 0.25f));
+    };
+    return make_float2(one(x.x), one(x.y));
+  }
+  constexpr float kMax = 3.402823466e38f;
+  const F2 quarter = f2(0.25f, 0.25f);
+  float da, db;
+  f2_split(f2_fma(f2(expf(-x.x), expf(-x.y)), quarter, quarter), da, db);
+  da = min_nan(da, kMax);
+  db = min_nan(db, kMax);
+  const F2 d = f2(da, db), r = f2(rcp_approx(-da), rcp_approx(-db));
+  const F2 x4 = f2_mul(f2(min_nan(x.x, kMax), min_nan(x.y, kMax)), f2(-0.25f, -0.25f));
+  const F2 q = f2_mul(x4, r);
+  float2 y;
+  f2_split(f2_fma(f2_fma(q, d, x4), r, q), y.x, y.y);
+  return y;
 }
 // The int8 quantizers' scale of a row: T(T(max(absmax, 1e-5)) * (1 / 127)).
 template <typename T> __device__ __forceinline__ float int8_scale(float amax) {

@@ -227,7 +227,7 @@ __device__ __forceinline__ uint4 silu_mul8(const uint4& g, const uint4& up, floa
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     const float2 gv = unpack_pair<T>(gw[p]), uv = unpack_pair<T>(uw[p]);
-    const float2 act = unpack_pair<T>(pack_pair<T>(silu_f32(gv.x), silu_f32(gv.y)));       // silu in T
+    const float2 s = silu_pair<T>(gv), act = unpack_pair<T>(pack_pair<T>(s.x, s.y));                 // silu in T
     h[p] = pack_pair<T>(act.x * uv.x, act.y * uv.y);                                              // * up, in T
     const float2 hv = unpack_pair<T>(h[p]);
     amax = fmaxf(amax, fmaxf(fabsf(hv.x), fabsf(hv.y)));

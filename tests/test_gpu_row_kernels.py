@@ -61,6 +61,32 @@ def test_silu_one_block_per_row(I, dt):
     assert torch.isinf(s[9]) and not q[9].any()
 
 
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_silu_of_every_gate(dt):
+    """All 65536 gates: every variant gives the bits of the staged one, which divides by 1 + e^-gate, and those are within
+    a rounding of 64 bits as long as e^-gate is finite in fp32 (beyond, the result is a zero)."""
+    from llmqrt_b200 import glue
+    gates = torch.arange(-2 ** 15, 2 ** 15, device="cuda", dtype=torch.int32).to(torch.int16).view(dt).reshape(16, 4096)
+    rows = torch.cat([gates, torch.ones_like(gates)], 1)
+    staged = torch.zeros(16, 8192 + 8, dtype=dt, device="cuda")              # rows off a 16-byte boundary
+    staged[:, 1:8193] = rows
+    want = glue.silu_mul(staged[:, 1:8193])[0]
+    many = glue.silu_mul(rows.repeat(20, 1))[0]                               # one block per row
+    for got in (glue.silu_mul(rows)[0], many[:16], many[-16:]):
+        assert torch.equal(got.isnan(), want.isnan())
+        ok = ~want.isnan()
+        assert torch.equal(got[ok].view(torch.int16), want[ok].view(torch.int16))
+    g = gates.double()
+    assert torch.equal(want.isnan(), g.isnan() | (g == -float("inf")))
+    exact, y = g * torch.sigmoid(g), want.double()
+    ok = g.isfinite() & (g > -88.7)                                          # e^88.7 is the last below the largest fp32
+    half = torch.finfo(dt).eps / 2
+    tiny = torch.finfo(dt).smallest_normal * torch.finfo(dt).eps              # spacing of the subnormals
+    # one rounding to 16 bits after a relative error of a few 2^-24
+    assert bool(((y - exact).abs() <= half * 1.01 * exact.abs() + tiny * 0.51)[ok].all())
+    assert bool((y[(g < -90) & g.isfinite()] == 0).all()) and bool((y[g == float("inf")] == float("inf")).all())
+
+
 @pytest.mark.parametrize("M,K", [(1, 8), (3, 1032), (3, 18944), (2, 65536), (2, 65544), (300, 1016), (300, 1024), (300, 2056),
                                  (300, 4104), (296, 8200), (1200, 896)])
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
