@@ -361,10 +361,6 @@ int launch_silu_rows(const void* gate_up, int64_t ld, void* y, int8_t* q, float*
   return check_launch("silu_mul");
 }
 
-// Rows from which one block per row is the faster split of SiLU (two blocks to an SM): 300 rows of 4864 / 8960 /
-// 18944 elements take 13.7 / 12.3 / 18.4 us against 16.1 / 16.4 / 24.6 us in clusters; fewer leave SMs idle.
-constexpr int64_t kSiluRowsMinM = 296;
-
 // RMSNorm of one row held in registers, eight elements per thread (rows of up to 8192 elements, one
 // block per row): `h` are the row's values already rounded to T (x, or x + residual), `on` says
 // whether this thread owns a unit.  Two block reductions, no staging; optional quantized store.
@@ -934,8 +930,9 @@ int llmqrt_silu_mul(const void* gate_up, int64_t ld, void* y, int8_t* q, float* 
   cudaStream_t st = (cudaStream_t)stream;
   const bool vec = I % 8 == 0 && ld % 8 == 0 && aligned16(gate_up) && aligned16(y) &&
                    (reinterpret_cast<uintptr_t>(q) & 7) == 0;
-  // Enough rows to fill the chip twice over with one block each, and rows that fit a block's registers.
-  if (vec && M >= kSiluRowsMinM && M <= 0x7fffffffll && I <= 8 * 8 * 512)
+  // Enough rows for two blocks of one row on every SM, and rows that fit a block's registers.  (300 rows of 4864 / 8960 /
+  // 18944 elements took 13.7 / 12.3 / 18.4 us, 16.1 / 16.4 / 24.6 in clusters; fewer leave SMs idle.)
+  if (vec && M >= 2 * sm_count() && M <= 0x7fffffffll && I <= 8 * 8 * 512)
     return dtype == LLMQRT_F16 ? launch_silu_rows<__half>(gate_up, ld, y, q, scale_f32, M, I, st)
                                : launch_silu_rows<__nv_bfloat16>(gate_up, ld, y, q, scale_f32, M, I, st);
   // Register-resident variant: the smallest cluster whose slices fit one block (8 elements per
