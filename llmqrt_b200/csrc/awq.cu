@@ -258,6 +258,22 @@ int launch_rows(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32
   return check_launch("awq_gemm_rows");
 }
 
+// 17 to 32 tokens: every block fetches all activations, so its time goes with blocks x tokens on an SM.  It stands against
+// the tcgen05 kernel, whose weight tiles of 128 rows go to clusters of three up to about 44 tiles and of two beyond.
+// us at 17 / 24 / 32 tokens (tcgen05):
+//   up to 65 blocks x tokens:  4736 x 4096 13.0 / 15.0 / 16.8 (21.0); 5120 x 4096 17.3 / 20.5 (21.0), beyond: 23.6 (21.1)
+//   up to 83, in twos:         6144 x 4096 17.9 / 20.9 / 24.0 (27.5); 8192 x 8960 42.7 / 48.2 (48.6), beyond: 56.1 (48.8);
+//                              9472 x 4096 27.2 (27.8), beyond: 31.4 / 34.8 (27.9)
+//   two small blocks to an SM: 9472 x 896 8.3 / 9.5 / 10.8 (13.3)
+// The worst of it are long reductions whose clusters happen to fill the device: 3072 x 14336 41.3 (38.7), 3584 x 18944
+// 52.5 (50.5), both at 32 tokens.
+bool rows_suit(int64_t M, int64_t N, int64_t K) {
+  const int64_t sms = sm_count();
+  if (N > 64 * sms) return false;
+  const int64_t most = 3 * ceil_div(N, (int64_t)128) <= sms - 16 ? 65 : 83;
+  return K <= 1024 || ceil_div(N, (int64_t)16) * M <= most * sms;
+}
+
 int check_layer(int64_t K, int64_t N, int64_t G) {
   LLMQRT_REQUIRE(K > 0 && N > 0 && G > 0, "awq: bad shape K=%lld N=%lld G=%lld", (long long)K, (long long)N, (long long)G);
   LLMQRT_REQUIRE(N % 8 == 0, "awq: N=%lld must be a multiple of 8", (long long)N);
@@ -346,10 +362,7 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   }
   if (M <= 0) return LLMQRT_OK;
   e.out = out;
-  // At most 16 tokens, and up to 32 where the layer is narrow enough for the activations, which every block of 16
-  // rows fetches, not to outweigh the weights: 32 tokens 1536 x 8960 15.0 us (tcgen05 17.3), 4608 x 3584 15.4
-  // (19.3), 3584 x 18944 52 (50), 17920 x 1536 25.8 (19.2).
-  if (M <= 16 || (M <= 32 && N <= 64 * (int64_t)sm_count())) {
+  if (M <= 16 || (M <= 32 && rows_suit(M, N, K))) {
     auto go = M <= 8 ? launch_rows<1> : M <= 16 ? launch_rows<2> : launch_rows<4>;
     return go(xp, ldx, wq_t, sz_t, (int)M, (int)N, (int)K, (int)group_size, e, st, nullptr, 0);
   }

@@ -77,6 +77,14 @@ def test_awq_schedules(M, K, N, G):
     assert rel_fro(ops.awq_gemm(x, ops.AwqPacked(qw, sc, qz), bias), want) < 5e-4      # the fp16 rounding of the result
 
 
+@pytest.mark.parametrize("M", [17, 24, 25, 32])
+@pytest.mark.parametrize("K,N,G", [(1152, 4736, 128), (1152, 5120, 128), (1152, 6144, 128), (1152, 9472, 128), (1152, 9480, 128),
+                                   (1024, 9472, 64), (1056, 7168, 32)])
+def test_awq_rows_or_tiles(M, K, N, G):
+    """Both sides of the rule for 17 to 32 tokens of a 4-bit layer."""
+    test_awq_schedules(M, K, N, G)
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17])
 @pytest.mark.parametrize("N,K", [(16, 16), (40, 1040), (4864, 896), (520, 2048), (520, 2064), (16384, 2048)])
 @pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
