@@ -5,9 +5,11 @@
 // and stream look-ups through context managers, two ctypes calls of a dozen arguments, four or five output
 // tensors) took the host fifty.  Here it is a METH_FASTCALL function that checks the tensors, allocates the
 // results through ATen and calls the C ABI: one crossing of the language border for one call.  A pass over a
-// 4864 x 896 layer went from 53 to 11 us (int8, 16 tokens), a 28-layer 4-bit model's step from 9.4 to 4.2 ms.
+// 4864 x 896 layer went from 53 to 11 us (int8, 16 tokens; 9.5 since its GEMM quantizes), a 28-layer 4-bit model's step
+// from 9.4 to 4.2 ms (2.7 with fewer launches).
 //
-// The checks are those of the Python wrappers (ops.py, glue.py, attention.py) and raise the same exceptions.
+// The checks are those of the Python wrappers before it (ops.py, glue.py, attention.py), with the same exceptions; the
+// attention calls also check caches and lengths against the query's batch.
 // Nothing is kept between calls but the devices' workspaces, which the package owns for the life of the
 // process.
 #include <Python.h>

@@ -299,10 +299,10 @@ silu_mul_regs_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ 
 
 // SiLU(gate) * up for prefill-sized M: one block per row, U units of eight elements per thread, the packed
 // results kept in registers from the loads to the quantized store.
-// HBM-bound (8192 rows of 2 x 18944: 932 MB, 140 us at 6.65 TB/s) only if the arithmetic is short: the
-// staged form below spends over 60 instructions and five special-function operations on an element and
-// took 385 us; here it is about 30 and three (e^x, reciprocal, float -> int), and all of a thread's loads are
-// in flight at once.
+// 8192 rows of 2 x 18944 (932 MB, 142 us at the copy rate) take 168 us in bf16 and 181 in fp16: the schedulers are the
+// bound (an instruction in 73 % of their cycles, DRAM at half its rate), with three special-function operations an element
+// (e^x, reciprocal, float -> int).  All of a thread's loads are in flight at once.  The staged form above takes over
+// 300 us.  Rows beyond 20480 elements keep eight units a thread, one block an SM: 4096 rows of 20488 153 us, staged 170.
 template <typename T, int U>
 __global__ void __launch_bounds__(512, U <= 5 ? 2 : 1)
 silu_mul_rows_kernel(const T* __restrict__ gate_up, int64_t ld, T* __restrict__ y, int8_t* __restrict__ q,
@@ -399,9 +399,10 @@ __device__ __forceinline__ void rmsnorm_regs_finish(bool on, float (&f)[8], int6
 }
 
 // The same for many rows: one block of at most 128 threads per row, U units of eight elements per thread.
-// HBM-bound (8192 rows of 3584 with residual and int8 output: 205 MB, 31 us at 6.65 TB/s).  With one unit per
-// thread a row's two reductions each stall a whole 448-thread block, four blocks to an SM: 56 us.  Four
-// units per thread put fifteen rows on an SM and make the reductions a quarter as wide: 38 us.
+// 8192 rows of 3584 with residual and int8 output are 205 MB, 31 us at the copy rate; bound by issue (an instruction in
+// 83 % of the schedulers' cycles).  With one unit per thread a row's two reductions each stall a whole 448-thread block,
+// four blocks to an SM: 56 us (fp16).  Four units per thread put ten to fifteen rows on an SM and make the reductions a
+// quarter as wide: 38 us (bf16: 42).
 template <typename T, int U>
 __global__ void __launch_bounds__(128)
 rmsnorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ residual, T* __restrict__ x_out,

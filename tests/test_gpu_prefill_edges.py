@@ -1,4 +1,4 @@
-"""Prompt attention at the edges of its 64-key halves and 128-row tiles, with maxima that keep moving."""
+"""Prompt attention at the edges of its 128-key and 128-row tiles, with maxima that keep moving."""
 import pytest
 import torch
 
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
                                          (torch.bfloat16, 128, -40)])
 def test_prefill_halves(S, causal, dt, d, growth):
     """growth: the score rises (falls) by that many powers of e over every 64 keys, so a row's reference maximum moves
-    in every half and the accumulator is rescaled while a product may be on its way (or never again)."""
+    in every tile and the accumulator is rescaled while a product may be on its way (or never again)."""
     from llmqrt_b200.attention import flash_attn_func
     g = torch.Generator(device="cuda").manual_seed(S)
     q, k, v = (torch.randn(2, S, h, d, generator=g, device="cuda") for h in (4, 2, 2))
