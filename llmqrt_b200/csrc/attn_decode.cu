@@ -15,7 +15,10 @@
 // unnormalised partial (max, sum, O) that a small combine kernel reduces; the combine kernel can also
 // emit the per-token int8 quantization of the result, which is what an int8 output projection reads.
 #include <cstdlib>
+#include <map>
+#include <mutex>
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 
@@ -583,10 +586,44 @@ bool quant_fused_enabled() {
   return on;
 }
 
+// How many clusters of `cluster` blocks of the attention kernel can be resident at once (cached per device).
+template <bool BF16, int D>
+int max_active_clusters(int cluster, int smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> cache;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = cache.find({dev, cluster});
+  if (it != cache.end()) return it->second;
+  auto kern = attn_decode_kernel<BF16, D>;
+  int n = 0;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) == LLMQRT_OK) {
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)cluster, 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+  }
+  cache[{dev, cluster}] = n;
+  return n;
+}
+
 template <bool BF16, int D>
 int launch_decode(const void* q, int64_t qbs, const void* kc, const void* vc, int64_t bs, int64_t rs,
                   const int32_t* seqlens, void* out, int8_t* out_q, float* out_scale, int B, int Hq, int Hkv,
                   int max_seqlen, float softcap, void* workspace, cudaStream_t st, const DecodeAppend& ap) {
+  constexpr int smem = kWarps * kRing * 2 * 16 * D * 2;           // per-warp rings; also holds the 16 KiB merge tile
   // Keys per block: the smallest power of two for which all blocks are resident at once (two fit an
   // SM), i.e. as many blocks as one wave takes and no second wave -- a block costs about 3 us beyond
   // its keys (first loads, merge of its warps), so waves of short blocks lose to one wave of long
@@ -615,8 +652,11 @@ int launch_decode(const void* q, int64_t qbs, const void* kc, const void* vc, in
   // 12 / 2 heads of 128: 6.0 us in one kernel, against 4.5 + 4.6 us in 64-key splits with the merge kernel.
   int merge_cluster = 1;
   if (max_splits > 1 && ap.merge_in_cluster && !out_q && !forced_chunk && max_seqlen <= kClusterMergeMaxLen) {
+    // (Resident is the device's answer: a cluster lies within one group of SMs, and the groups' sizes are not multiples of
+    // eight.  17 sequences of 2 KV heads are 272 blocks of 128-wide heads, two to an SM, but 34 clusters are not all
+    // resident: 500 keys take 10.5 us in two waves of clusters, 8.8 with the merge kernel; 16 sequences 6.7 against 8.6.)
     const int splits = max_splits < 8 ? max_splits : 8;
-    if ((int64_t)B * Hkv * splits <= 2 * (int64_t)sm_count() - 16) {
+    if ((int64_t)B * Hkv * splits <= 2 * (int64_t)sm_count() - 16 && (int64_t)B * Hkv <= max_active_clusters<BF16, D>(splits, smem)) {
       chunk = (int)ceil_div(ceil_div(max_seqlen, splits), 16 * kWarps) * 16 * kWarps;
       max_splits = (int)ceil_div(max_seqlen, chunk);
       merge_cluster = max_splits;
@@ -634,7 +674,6 @@ int launch_decode(const void* q, int64_t qbs, const void* kc, const void* vc, in
     part_ml = part_o + (size_t)B * Hq * max_splits * D;
   }
   const float scale = 1.0f / sqrtf((float)D);
-  constexpr int smem = kWarps * kRing * 2 * 16 * D * 2;           // per-warp rings; also holds the 16 KiB merge tile
   static_assert(smem >= kWarps * 8 * D * 4 + 8 * D * 2 + 8 * 4 + 8 * D * 4 + 64, "ring too small for the merge tile and the scratch behind it");
   static_assert(kWarps + 1 <= 8, "scratch layout");
   auto kern = attn_decode_kernel<BF16, D>;

@@ -177,3 +177,10 @@ def test_decode_rotary_step_against_64_bits(pos, cap, B, Hq, Hkv, d, dt, twice):
     assert rel_fro(kc, want_k) < eps + 4 * pos * 2 ** -24
     # q, k, P and the result rounded once each; scores of d products of unit variance pass on sqrt(2) of q's and k's
     assert rel_fro(out[:, 0], want) < 4 * eps + 8 * pos * 2 ** -24
+
+
+@pytest.mark.parametrize("B", [16, 17, 18, 33, 35])
+@pytest.mark.parametrize("Hq,Hkv,d", [(12, 2, 128), (14, 2, 64), (8, 1, 128)])
+def test_as_many_clusters_as_fit_and_more(B, Hq, Hkv, d):
+    """The largest batches that clusters merge, and the first ones left to the merge kernel."""
+    test_decode_step([300 + 10 * b % 200 for b in range(B)], 512, None, Hq, Hkv, d, torch.float16, True)
