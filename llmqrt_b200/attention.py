@@ -87,7 +87,7 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
         raise RuntimeError("flash_attn_with_kvcache: cache_seqlens is required")
     if k is not None and v is None:
         raise RuntimeError("flash_attn_with_kvcache: k and v must be given together")
-    cap = min(k_cache.shape[1], v_cache.shape[1])
+    cap = k_cache.shape[1]                                 # (the native call also goes by the shorter of the two caches)
     bound = min(cap, max_seqlen_k) if max_seqlen_k is not None else cap
     if rotary:
         Hkv = k_cache.shape[2]
