@@ -32,7 +32,11 @@
 // fp32 multiply-adds or additions per instruction, maxima of three), its warps wait for S on their own, and
 // P V starts on the first three quarters of P while the last quarter is still being computed; blocks are
 // ordered heaviest first over all heads.  4 x 2048 causal tokens, 28 / 4 heads of 128: 194 -> 180 us; with each product's
-// MMAs issued back to back and the tiles waited for ahead of P, 170 us a pass.
+// MMAs issued back to back and the tiles waited for ahead of P, 167 us a pass.  The row's maximum is found in the shadow of
+// the first half's exponentials, which are done again where the reference had to move, and the output leaves through shared
+// memory: 151 us (16 x 512 tokens: 89 -> 77; 1 x 4096, not causal: 276 -> 262).  At 4 x 2048 the board's 1000 W bound it then
+// (1.65 to 1.8 GHz), so that every instruction saved counts twice; with a quarter of the exponentials as polynomials on the
+// multiply-add pipe it was 1 % slower.
 //
 // Every wait on an mbarrier is bounded; when one runs out the block raises a flag, every role
 // leaves its loop, outstanding copies are drained, tensor memory is freed and a status word is set.
@@ -218,7 +222,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   // Register budget per warpgroup (8 x 216 + 4 x 72 registers per lane fit the SM's file): each role
   // branch starts by shrinking or growing its warpgroup's share.
   if (warp >= 8) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
   if (warp == 8) {
     // ------------------------------- TMA producer -------------------------------
     if (lane == 0) {
@@ -337,7 +341,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   }
   } else {
     // ------------------------------- softmax groups ------------------------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
     const int w = warp >> 2;                           // query tile of this group
     const int quad = warp & 3;                         // tensor-memory lane quadrant of this warp
     const int r = quad * 32 + lane;                    // row of the tile handled by this thread
@@ -350,6 +354,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     const bool capped = prm.softcap != 0.f;
     float m_ref = -INFINITY, l_run = 0.f;              // reference maximum of the exponentials, running sum
     bool ok = true;
+    // whether any row of this warp misses keys of the tile that starts at key0 (the same answer in every lane)
+    auto tile_masked = [&](int key0) {
+      return capped || S - key0 < kRows || (prm.causal && row - lane - key0 + 1 < kRows);
+    };
 
     for (int j = 0; j < n; ++j) {
       // (a warp leaves by itself when its wait runs out: tensor-memory accesses and arrivals are per warp, and
@@ -372,56 +380,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       float mxs[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) mxs[i] = -INFINITY;
-      if (capped || need_mask) {                        // soft cap and mask applied in place (diagonal / last tile)
+      auto max_of = [&](int c) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int i = 0; i < 32; i += 2)
+          mxs[(i >> 1) & 7] = max3(mxs[(i >> 1) & 7], __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
+      };
+      auto row_max = [&]() {
+        return fmaxf(max3(max3(mxs[0], mxs[1], mxs[2]), mxs[3], mxs[4]), max3(mxs[5], mxs[6], mxs[7]));
+      };
+      // P = exp2(s * sl - m * sl) of 32 keys, their part of the row sum, packed 16-bit pairs into the first half of S
+      const F2 sl2 = f2(sl, sl);
+      F2 nm2, ps[4];
+      auto start = [&]() {
+        const float neg_ms = m_ref == -INFINITY ? 0.f : -m_ref * sl;
+        nm2 = f2(neg_ms, neg_ms);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float x = __uint_as_float(v[c][i]);
-            if (capped) x = prm.softcap * tanhf(x * prm.scale / prm.softcap) / prm.scale;
-            if (need_mask && c * 32 + i >= limit) x = -INFINITY;
-            v[c][i] = __float_as_uint(x);
-            mxs[i & 7] = fmaxf(mxs[i & 7], x);
-          }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; i += 2)
-            mxs[(i >> 1) & 7] = max3(mxs[(i >> 1) & 7], __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
-      }
-      const float mx = fmaxf(max3(max3(mxs[0], mxs[1], mxs[2]), mxs[3], mxs[4]), max3(mxs[5], mxs[6], mxs[7]));
-      // Move the reference only when the maximum has outgrown it by more than 2^8 (always on the first
-      // tile).  tcgen05.ld / st are warp-wide, so the decision is taken per warp; a lane of a moving warp
-      // moves to its own exact maximum.
-      const bool grow = (mx - m_ref) * sl > 8.f;       // m_ref = -inf: true unless the row sees no key at all
-      if (__any_sync(0xffffffffu, grow)) {
-        const float m_new = fmaxf(m_ref, mx);
-        const float m_safe = m_new == -INFINITY ? 0.f : m_new;
-        const float corr = m_new == m_ref ? 1.f : fast_exp2((m_ref - m_safe) * sl);     // m_ref = -inf: 0
-        m_ref = m_new;
-        l_run *= corr;
-        if (j > 0) {                                    // O holds the tiles before this one: scale its row
-#pragma unroll 1
-          for (int c = 0; c < D / 16; ++c) {            // (a rare path: short, rolled, few registers)
-            uint32_t ov[16];
-            tmem_ld_32x16(t_o + (uint32_t)(c * 16), ov);
-            tc::tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-            tmem_st_32x16(t_o + (uint32_t)(c * 16), ov);
-          }
-        }
-      }
-      const float neg_ms = m_ref == -INFINITY ? 0.f : -m_ref * sl;
-
-      // P = exp2(s * sl - m * sl), row sum, packed 16-bit pairs into the first half of S
-      const F2 sl2 = f2(sl, sl), nm2 = f2(neg_ms, neg_ms);
-      F2 ps[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ps[i] = f2(0.f, 0.f);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
+        for (int i = 0; i < 4; ++i) ps[i] = f2(0.f, 0.f);
+      };
+      auto exp_of = [&](int c) {
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
@@ -433,12 +409,73 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           pk[i / 2] = pack2<BF16>(p0, p1);
         }
         tmem_st_32x16(t_s + (uint32_t)(c * 16), pk);
-        if (c >= 2) {                                   // three quarters written: P V may start; then the rest
-          tmem_st_wait();
-          tc::fence_before_sync();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(tc::smem_u32(c == 2 ? &bar_p_ready[w] : &bar_p_rest[w]));
+      };
+
+      float mx;
+      bool again = true;
+      if (j == 0 || tile_masked(key0)) {                // the reference is unknown, or the soft cap and the mask come first
+        if (capped || need_mask) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              float x = __uint_as_float(v[c][i]);
+              if (capped) x = prm.softcap * tanhf(x * prm.scale / prm.softcap) / prm.scale;
+              if (need_mask && c * 32 + i >= limit) x = -INFINITY;
+              v[c][i] = __float_as_uint(x);
+            }
         }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) max_of(c);
+        mx = row_max();
+      } else {
+        // The first half of P with the reference as it stands, the row's maximum beside it: the maxima run in the shadow
+        // of the exponentials, and hardly a tile after the first few moves the reference and has to do its half again.
+        start();
+        max_of(0);
+        max_of(1);
+        exp_of(0);
+        max_of(2);
+        max_of(3);
+        exp_of(1);
+        mx = row_max();
+        again = __any_sync(0xffffffffu, (mx - m_ref) * sl > 8.f);
+      }
+      if (again) {
+        // Move the reference only when the maximum has outgrown it by more than 2^8 (always on the first
+        // tile).  tcgen05.ld / st are warp-wide, so the decision is taken per warp; a lane of a moving warp
+        // moves to its own exact maximum.
+        const bool grow = (mx - m_ref) * sl > 8.f;     // m_ref = -inf: true unless the row sees no key at all
+        if (__any_sync(0xffffffffu, grow)) {
+          const float m_new = fmaxf(m_ref, mx);
+          const float m_safe = m_new == -INFINITY ? 0.f : m_new;
+          const float corr = m_new == m_ref ? 1.f : fast_exp2((m_ref - m_safe) * sl);   // m_ref = -inf: 0
+          m_ref = m_new;
+          l_run *= corr;
+          if (j > 0) {                                  // O holds the tiles before this one: scale its row
+#pragma unroll 1
+            for (int c = 0; c < D / 16; ++c) {          // (a rare path: short, rolled, few registers)
+              uint32_t ov[16];
+              tmem_ld_32x16(t_o + (uint32_t)(c * 16), ov);
+              tc::tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+              tmem_st_32x16(t_o + (uint32_t)(c * 16), ov);
+            }
+          }
+        }
+        start();
+        exp_of(0);
+        exp_of(1);
+      }
+#pragma unroll
+      for (int c = 2; c < 4; ++c) {
+        exp_of(c);
+        // three quarters written: P V may start; then the rest
+        tmem_st_wait();
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(tc::smem_u32(c == 2 ? &bar_p_ready[w] : &bar_p_rest[w]));
       }
       // (halves of a pair first, then neighbouring pairs: an order that is part of the result's bits)
       float sum[4];
@@ -455,21 +492,32 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       if (tc::mbar_wait_warp(tc::smem_u32(&bar_o_full[w]), 0u, abort)) {
         tc::fence_after_sync();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        uint4* dst = reinterpret_cast<uint4*>(prm.out + ((long long)b * S + row) * prm.out_ts + (long long)hq * D);
+        // The warp's 32 rows pass through its part of Q_w, whose last product has retired: a lane that wrote its own row
+        // straight to global memory would touch 32 lines with every store (3600 cycles a block, 2300 this way).
+        uint8_t* sO = sQ + w * kTile + quad * 32 * (D * 2);
+        constexpr int kUnits = D / 8;                   // 16-byte units of a row; unit u of row r lies at u ^ (r & 7)
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t ov[32];
           tc::tmem_ld_32x32(t_o + (uint32_t)(c * 32), ov);
           tc::tmem_ld_wait();
-          if (row < S) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              dst[c * 4 + i] = make_uint4(
-                  pack2<BF16>(__uint_as_float(ov[8 * i]) * inv, __uint_as_float(ov[8 * i + 1]) * inv),
-                  pack2<BF16>(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv),
-                  pack2<BF16>(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv),
-                  pack2<BF16>(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv));
-          }
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(sO + lane * (D * 2) + (((c * 4 + i) ^ (lane & 7)) << 4)) = make_uint4(
+                pack2<BF16>(__uint_as_float(ov[8 * i]) * inv, __uint_as_float(ov[8 * i + 1]) * inv),
+                pack2<BF16>(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv),
+                pack2<BF16>(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv),
+                pack2<BF16>(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv));
+        }
+        __syncwarp();
+        const int u = lane % kUnits, row0 = row - lane;
+        uint16_t* dst = prm.out + ((long long)b * S + row0) * prm.out_ts + (long long)hq * D + u * 8;
+#pragma unroll
+        for (int it = 0; it < kUnits; ++it) {
+          const int rr = it * (32 / kUnits) + lane / kUnits;
+          if (row0 + rr < S)
+            *reinterpret_cast<uint4*>(dst + rr * prm.out_ts) =
+                *reinterpret_cast<const uint4*>(sO + rr * (D * 2) + ((u ^ (rr & 7)) << 4));
         }
       }
     }

@@ -45,3 +45,29 @@ def test_prefill_row_sum_order():
     out = flash_attn_func(*(t.half() for t in (q, k, v)), causal=False)
     p = (q[0, :, 0].double() @ k[0, :, 0].double().t() * d ** -0.5).softmax(-1)
     assert torch.equal(out[0, :, 0], (p @ v[0, :, 0].double()).half())
+
+
+@pytest.mark.parametrize("S,key", [(257, 128), (300, 250), (513, 383), (640, 511)])
+@pytest.mark.parametrize("d,dt", [(64, torch.bfloat16), (128, torch.float16)])
+def test_prefill_one_row_leaps(S, key, d, dt):
+    """The first half of a tile's P is computed with the reference as it stands.  Here the score of ONE key outgrows it by
+    far more than 2^8, for one row of a warp only, in either half of a tile after the first: the half is done again, the
+    row's earlier sum and output are scaled down, and the warp's other rows keep their reference.  A row that meets a NaN
+    is NaN and no other."""
+    from llmqrt_b200.attention import flash_attn_func
+    g = torch.Generator(device="cuda").manual_seed(S + key)
+    q, k, v = (torch.randn(1, S, 2, d, generator=g, device="cuda") for _ in range(3))
+    leap, nan = S - 40, S - 3
+    q[..., 0], k[..., 0] = 0.0, 0.0
+    q[:, leap, :, 0], k[:, key, :, 0] = 40.0, 40.0
+    q[:, nan, 0, 1] = float("nan")
+    q, k, v = (t.to(dt) for t in (q, k, v))
+    out = flash_attn_func(q, k, v, causal=True)
+    s = torch.einsum("bshd,bthd->bhst", q.double(), k.double()) * d ** -0.5
+    s.masked_fill_(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.einsum("bhst,bthd->bshd", s.softmax(-1), v.double())
+    assert out[0, nan, 0].isnan().all() and int(out.isnan().sum()) == d
+    keep = [i for i in range(S) if i != nan]
+    # as above: P and the result rounded to 16 bits
+    assert rel_fro(out[:, keep], want[:, keep]) < (1e-3 if dt == torch.float16 else 8e-3)
+    assert rel_fro(out[:, leap], want[:, leap]) < (1e-3 if dt == torch.float16 else 8e-3)
