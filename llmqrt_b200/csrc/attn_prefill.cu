@@ -81,15 +81,6 @@ __device__ __forceinline__ uint64_t smem_desc_mn_major_sw128(uint32_t smem_addr,
   return ((uint64_t)hi << 32) | lo;
 }
 
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand is read from tensor memory (packed 16-bit pairs).
-__device__ __forceinline__ void mma_ts_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-
 // 32 lanes x 16 consecutive 32-bit columns, registers -> tensor memory.
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -106,8 +97,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -300,7 +289,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         if (tc::elect_one()) {
 #pragma unroll
           for (int t = t_begin; t < t_end; ++t)
-            mma_ts_f16(d_tmem, a_tmem + (uint32_t)(t * 8), db + (uint64_t)(t * (16 * 128 >> 4)), prm.idesc_pv,
+            tc::mma_ts_f16(d_tmem, a_tmem + (uint32_t)(t * 8), db + (uint64_t)(t * (16 * 128 >> 4)), prm.idesc_pv,
                        (j > 0 || t > 0) ? 1u : 0u);
         }
         __syncwarp();
@@ -472,7 +461,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       for (int c = 2; c < 4; ++c) {
         exp_of(c);
         // three quarters written: P V may start; then the rest
-        tmem_st_wait();
+        tc::tmem_st_wait();
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(tc::smem_u32(c == 2 ? &bar_p_ready[w] : &bar_p_rest[w]));

@@ -258,20 +258,18 @@ int launch_rows(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32
   return check_launch("awq_gemm_rows");
 }
 
-// 17 to 32 tokens: every block fetches all activations, so its time goes with blocks x tokens on an SM.  It stands against
-// the tcgen05 kernel, whose weight tiles of 128 rows go to clusters of three up to about 44 tiles and of two beyond.
-// us at 17 / 24 / 32 tokens (tcgen05):
-//   up to 65 blocks x tokens:  4736 x 4096 13.0 / 15.0 / 16.8 (21.0); 5120 x 4096 17.3 / 20.5 (21.0), beyond: 23.6 (21.1)
-//   up to 83, in twos:         6144 x 4096 17.9 / 20.9 / 24.0 (27.5); 8192 x 8960 42.7 / 48.2 (48.6), beyond: 56.1 (48.8);
-//                              9472 x 4096 27.2 (27.8), beyond: 31.4 / 34.8 (27.9)
-//   two small blocks to an SM: 9472 x 896 8.3 / 9.5 / 10.8 (13.3)
-// The worst of it are long reductions whose clusters happen to fill the device: 3072 x 14336 41.3 (38.7), 3584 x 18944
-// 52.5 (50.5), both at 32 tokens.
+// 9 to 32 tokens: every block fetches all activations, so the time of this file's kernel goes with the blocks on an SM x
+// tokens x K, while the tcgen05 kernel takes the same time for any of them.  us at 9 / 16 / 17 / 24 / 32 tokens (tcgen05):
+//   1536 x 1536 3.3 / 3.3 / 3.9 / 4.6 / 5.0 (8.8)      4608 x 3584 7.0 / 8.3 / 12.0 / 13.7 / 15.4 (13.8)
+//   17920 x 1536 10.8 / 14.0 / 19 / 22 / 26 (13)       3584 x 18944 27 / 30 / 38 / 43 / 52 (29)
+//   37888 x 3584 38 / 45 / 58 / 69 / 84 (38)           9728 x 896 5.8 / 6.9 / 9.4 / 10.8 / 12.7 (9.0)
+// The estimates are fitted to N = 896 .. 37888, K = 896 .. 18944; the kernel they choose is more than 4 % slower than the
+// other in 10 of 245 measured cases (6144 x 3584 at 24 tokens: 19.0 against 16.4).
 bool rows_suit(int64_t M, int64_t N, int64_t K) {
-  const int64_t sms = sm_count();
-  if (N > 64 * sms) return false;
-  const int64_t most = 3 * ceil_div(N, (int64_t)128) <= sms - 16 ? 65 : 83;
-  return K <= 1024 || ceil_div(N, (int64_t)16) * M <= most * sms;
+  const double blocks = (double)ceil_div(ceil_div(N, (int64_t)16), (int64_t)sm_count()), k = 1e-3 * (double)K;
+  const double us = M <= 16 ? 1.7 + blocks * (0.27 + k * (0.367 + 0.0315 * (double)M))
+                            : 1.75 + blocks * (0.84 + k * (0.485 + 0.0298 * (double)M));
+  return us < awq_tc_us(M, N, K, nullptr);
 }
 
 int check_layer(int64_t K, int64_t N, int64_t G) {
@@ -337,14 +335,15 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   e.ldo = ldo;
   const __half* xp = reinterpret_cast<const __half*>(x);
   cudaStream_t st = (cudaStream_t)stream;
-  // More than 128 tokens: the weights are expanded panel by panel into the workspace (same rounding:
-  // fp16((v - z) * s)) and each panel is multiplied by the dense kernel, whose tensor core is not held up by the
-  // dequantizing warps' traffic in the same shared memory.  256 / 512 tokens: 17920 x 1536 25 / 34 us (fused 31 / 51),
-  // 4608 x 3584 28 / 29 (30 / 49), 3584 x 18944 88 / 127 (101 / 197).  A layer of more than one panel travels to HBM
-  // and back as fp16, which only pays from about 640 tokens on: 37888 x 3584 at 256 / 512 / 768 tokens 132 / 174 / 219
-  // us against 93 / 166 / 238.  (Panels of 64 MB, which would stay in L2, are worse: 113 us for 3584 x 18944 at 256.)
-  const bool one_panel = N * K * 2 <= (int64_t)LLMQRT_WS_PARTIAL_BYTES;
-  if (M > 128 && (one_panel || M >= 640) && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0) {
+  // More than 128 tokens: the weights may be expanded panel by panel into the workspace (same rounding:
+  // fp16((v - z) * s)) and each panel multiplied by the dense kernel, which reads an expanded tile again for every 256
+  // tokens; the kernel that dequantizes its own tiles makes each of them again for every 256 tokens.  Expanded against fused
+  // us at 256 / 512 / 1024 tokens: 17920 x 1536 26 / 34 / 56 (25 / 46 / 87), 4608 x 3584 28 / 30 / 31 (22 / 33 / 36), 3584 x 18944
+  // 86 / 117 / 135 (57 / 104 / 123), 37888 x 3584 139 / 187 / 268 (71 / 167 / 265), 9728 x 896 15 / 19 / 25 (21 / 37 / 54).  The
+  // estimates choose; a twelfth in favour of the expansion is what they are off by.  (Panels of 64 MB, which would stay in L2, are
+  // worse: 113 us for 3584 x 18944 at 256.)  Above 1024 tokens it is always expanded.
+  if (M > 128 && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0 &&
+      (M > 1024 || 0.92 * awq_expanded_us(M, N, K) < awq_tc_us(M, N, K, nullptr))) {
     const int64_t cap_rows = (int64_t)(LLMQRT_WS_PARTIAL_BYTES / (size_t)(K * 2)) / 256 * 256;
     if (cap_rows >= 256) {
       __half* deq = reinterpret_cast<__half*>(ws_partials(workspace));
@@ -362,12 +361,12 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   }
   if (M <= 0) return LLMQRT_OK;
   e.out = out;
-  if (M <= 16 || (M <= 32 && rows_suit(M, N, K))) {
+  if (M <= 8 || (M <= 32 && rows_suit(M, N, K))) {
     auto go = M <= 8 ? launch_rows<1> : M <= 16 ? launch_rows<2> : launch_rows<4>;
     return go(xp, ldx, wq_t, sz_t, (int)M, (int)N, (int)K, (int)group_size, e, st, nullptr, 0);
   }
   // ONE kernel: the tcgen05 GEMM runs with extra warps that turn the packed 4-bit tiles into fp16 operand tiles in
-  // shared memory (same rounding), so the dequantized weights never exist in global memory.
+  // tensor memory (same rounding), so the dequantized weights never exist in global memory.
   const AwqOperand op = {wq_t, sz_t, group_size};
   return gemm_tc(KIND_F16, x, ldx, nullptr, 0, M, N, K, e, workspace, st, false, &op);
 }

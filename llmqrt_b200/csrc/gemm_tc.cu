@@ -47,8 +47,9 @@ namespace llmqrt {
 namespace {
 
 constexpr int kThreads = 192;
-constexpr int kAwqWarps = 8;                  // warps that dequantize the 4-bit weight tiles (two per scheduler)
-constexpr int kThreadsAwq = kThreads + kAwqWarps * 32;
+constexpr int kAwqGroups = 4;                 // groups of four warps that dequantize the 4-bit weight tiles in turn
+constexpr int kAwqWarps = 4 * kAwqGroups;
+constexpr int kThreadsAwq = kThreads + kAwqWarps * 32 + 32;      // (+ the warp that fetches the packed tiles)
 constexpr int kBM = 128;           // rows of P per tile (UMMA M)
 constexpr int kRowBytes = 128;     // bytes of K per stage row (one swizzle span)
 constexpr int kSmemBudget = 226 * 1024;   // of the 227 KiB a block may use
@@ -65,12 +66,13 @@ struct TcParams {
   uint32_t idesc;
   unsigned* status;                // set to 1 if a bounded wait ran out
   Epilogue epi;
-  // AWQ mode: the weight operand is not fetched by TMA but produced in shared memory by four extra
+  // AWQ mode: the weight operand is not fetched by TMA but produced in tensor memory by sixteen extra
   // warps from the packed 4-bit layer (wq_t [N, K/8] words of eight K-consecutive values, sz_t
   // [N, K/G] half2 {scale, -(1024 + zero)}, see awq.cu)
   const uint32_t* awq_w;
   const uint32_t* awq_sz;
-  int awq_kw, awq_kg, awq_g;       // K / 8, K / G, G
+  int awq_kw, awq_kg, awq_gw;      // K / 8, K / G, G / 8
+  int awq_gshift;                  // log2(G / 8), or -1 if that is no whole number
   // Row-parallel output under tensor parallelism: instead of going to `out`, the 16-bit results are
   // stored as the tagged words of the NEXT all-reduce call into the peers' buffers (peer_comm.cuh);
   // the row kernel that consumes the sum then only gathers.
@@ -89,24 +91,24 @@ template <int BN> constexpr int num_stages() {
   return s > 8 ? 8 : s;
 }
 template <int BN> constexpr int smem_bytes() { return num_stages<BN>() * stage_bytes<BN>() + kEpiStageBytes + 1024; }
-// AWQ mode (always with the weights as the 128-lane operand): every stage also holds the PACKED 4-bit
-// weight tile (32 bytes = 64 values of K per row, 128 rows) that TMA delivers and the dequantizing warps
-// expand into the stage's fp16 weight tile.  The output is 16-bit and transposed through a 32 x 128
-// staging tile, so the staging area is half the general one -- which buys the 256-token tile a fourth
-// pipeline stage.
+// AWQ mode (always with the weights as the 128-lane operand): packed 4-bit weight tiles (32 bytes = 64 values of K per row,
+// 128 rows) and activation tiles arrive by TMA in a ring each, and the dequantizing warps turn the packed tiles into fp16
+// operand tiles in TENSOR MEMORY, 32 columns a stage beside the accumulators.  Through shared memory the fp16
+// tile is written and read again, 32 KiB per K block beside 12 KiB of everything else, and its bandwidth bounds the kernel:
+// 100 x 37888 x 3584 took 56 us with 16 dequantizing warps (78 with eight that expanded one tile together), 49 this way.
+// The output is 16-bit and transposed through a 32 x 128 staging tile, so the staging area is half the general one.
 constexpr int kPackedRowBytes = 32;
 constexpr int kPackedBytes = kBM * kPackedRowBytes;
 constexpr int kEpiStageBytesAwq = 9 * 1024;            // kChunk rows x (128 x 2 B + 16 B pad)
-template <int BN> constexpr int num_stages_awq() {
-  constexpr int budget = BN > 128 ? kSmemBudget : 200 * 1024;
-  int s = (budget - 1024 - kEpiStageBytesAwq) / (stage_bytes<BN>() + kPackedBytes);
-  return s > 8 ? 8 : s;
-}
-template <int BN> constexpr int smem_bytes_awq() {
-  return num_stages_awq<BN>() * (stage_bytes<BN>() + kPackedBytes) + kEpiStageBytesAwq + 1024;
-}
+constexpr int kAwqPk = 12;                              // packed tiles: 48 KiB of weights under way to every SM
+constexpr int kAwqWtCols = 32;                          // tensor-memory columns of an fp16 weight tile
+template <int BN> constexpr int awq_act_stages() { return BN > 128 ? 5 : 8; }      // activation and fp16 weight tiles
+template <int BN> constexpr int awq_ring_bytes() { return awq_act_stages<BN>() * BN * kRowBytes + kAwqPk * kPackedBytes; }
+template <int BN> constexpr int smem_bytes_awq() { return awq_ring_bytes<BN>() + kEpiStageBytesAwq + 1024; }
 template <int BN, bool AWQ> constexpr int smem_bytes_of() { return AWQ ? smem_bytes_awq<BN>() : smem_bytes<BN>(); }
 template <int BN> constexpr uint32_t tmem_cols() { return 2 * BN < 32 ? 32 : 2 * BN; }
+// AWQ: one accumulator of 256 columns, or two narrower ones, and the weight tiles behind them
+template <int BN, bool AWQ> constexpr int acc_buffers() { return AWQ && BN > 128 ? 1 : 2; }
 
 template <typename AccT> __device__ __forceinline__ AccT acc_from_bits(uint32_t b);
 template <> __device__ __forceinline__ int acc_from_bits<int>(uint32_t b) { return (int)b; }
@@ -370,21 +372,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
                const __grid_constant__ CUtensorMap tm_w, TcParams prm) {
   static_assert(!AWQ || KIND == tc::MMA_F16, "the 4-bit weights dequantize to fp16");
   using AccT = typename std::conditional<KIND == tc::MMA_I8, int, float>::type;
-  constexpr int kStages = AWQ ? num_stages_awq<BN>() : num_stages<BN>();
+  constexpr int kStages = num_stages<BN>();
   constexpr int kStageBytes = stage_bytes<BN>();
-  constexpr int kPkBytes = kPackedBytes;
-  constexpr uint32_t kTmemCols = tmem_cols<BN>();
-  constexpr int kBurst = kStages >= 8 ? 4 : (kStages >= 4 ? 2 : 1);  static_assert(BN > 128 || kStages * kStageBytes >= (2 * BN + 64) * kBM * 4, "ring too small for the reduce buffers");
+  constexpr int kRingBytes = AWQ ? awq_ring_bytes<BN>() : kStages * kStageBytes;
+  constexpr int kAct = awq_act_stages<BN>(), kPk = kAwqPk;      // AWQ: the two rings
+  constexpr int kAccBufs = acc_buffers<BN, AWQ>();
+  constexpr uint32_t kTmemCols = AWQ ? 512 : tmem_cols<BN>();
+  static_assert(!AWQ || kAccBufs * BN + awq_act_stages<BN>() * kAwqWtCols <= 512, "tensor memory has 512 columns");
+  constexpr int kBurst = kStages >= 8 ? 4 : (kStages >= 4 ? 2 : 1);  static_assert(BN > 128 || kRingBytes >= (2 * BN + 64) * kBM * 4, "ring too small for the reduce buffers");
   static_assert(kStages >= 3, "pipeline too shallow");
 
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment is what the 128-byte swizzle pattern and the descriptors assume.
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* stage = tiles + kStages * kStageBytes;      // epilogue staging tile
-  uint8_t* packed = stage + (AWQ ? kEpiStageBytesAwq : kEpiStageBytes);   // AWQ: [kStages][kPkBytes] packed weight tiles
-  __shared__ __align__(8) uint64_t bar_full[kStages];
-  __shared__ __align__(8) uint64_t bar_empty[kStages];
-  __shared__ __align__(8) uint64_t bar_pk[AWQ ? kStages : 1];   // AWQ: packed weight tile of the stage has landed
+  uint8_t* stage = tiles + kRingBytes;                 // epilogue staging tile
+  uint8_t* packed = tiles + kAct * BN * kRowBytes;     // AWQ: [kPk] packed weight tiles behind the [kAct] activation tiles
+  constexpr int kFull = AWQ ? kAct : kStages;
+  __shared__ __align__(8) uint64_t bar_full[kFull];
+  __shared__ __align__(8) uint64_t bar_empty[kFull];
+  __shared__ __align__(8) uint64_t bar_pk_full[AWQ ? kPk : 1];
+  __shared__ __align__(8) uint64_t bar_pk_empty[AWQ ? kPk : 1];
   __shared__ __align__(8) uint64_t bar_acc_full[2];
   __shared__ __align__(8) uint64_t bar_acc_empty[2];
   __shared__ __align__(8) uint64_t bar_reduce;         // split mode: counts the bytes of the incoming slices
@@ -406,10 +413,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
   if (threadIdx.x == 0) {
     abort_flag = 0;
     cluster_abort = 0;
-    for (int s = 0; s < kStages; ++s) {
-      tc::mbar_init(tc::smem_u32(&bar_full[s]), AWQ ? 1 + kAwqWarps : 1);   // AWQ: + one arrival per dequantizing warp
+    for (int s = 0; s < kFull; ++s) {
+      tc::mbar_init(tc::smem_u32(&bar_full[s]), AWQ ? 1 + 4 : 1);      // AWQ: + the four warps that made the weight tile
       tc::mbar_init(tc::smem_u32(&bar_empty[s]), 1);
-      if (AWQ) tc::mbar_init(tc::smem_u32(&bar_pk[s]), 1);
+    }
+    if constexpr (AWQ) {
+      for (int s = 0; s < kPk; ++s) {
+        tc::mbar_init(tc::smem_u32(&bar_pk_full[s]), 1);
+        tc::mbar_init(tc::smem_u32(&bar_pk_empty[s]), 4);
+      }
     }
     for (int b = 0; b < 2; ++b) {
       tc::mbar_init(tc::smem_u32(&bar_acc_full[b]), 1);
@@ -456,7 +468,49 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
   const int kb_count = (int)((int64_t)(my_split + 1) * prm.k_blocks / S) - kb_begin;
   EpiConsts ec_split = {};           // split mode: set by the epilogue warps before they wait for the MMAs
 
-  if (warp == 0) {
+  // AWQ: one ring's share of the TMA loads -- the activation tiles (warp 0) or the packed weight tiles (the last warp)
+  auto awq_load = [&](bool act) {
+    const int ring = act ? kAct : kPk;
+    const uint32_t full0 = tc::smem_u32(act ? &bar_full[0] : &bar_pk_full[0]);
+    const uint32_t empty0 = tc::smem_u32(act ? &bar_empty[0] : &bar_pk_empty[0]);
+    const uint32_t base = tc::smem_u32(act ? tiles : packed), bytes = act ? (uint32_t)(BN * kRowBytes) : (uint32_t)kPackedBytes;
+    int stage_i = 0, issued = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
+      const int tq = tile % prm.tiles_q, tp = tile / prm.tiles_q;
+      int kr = (tp * 5 + tq * 3) % kb_count;           // (see the general producer)
+      for (int it = 0; it < kb_count; ++it) {
+        tc::mbar_wait_or_flag(empty0 + (uint32_t)stage_i * 8u, phase ^ 1u, abort_u32);
+        if ((it & 3) == 0 && *abort) { ok = false; break; }
+        const uint32_t full = full0 + (uint32_t)stage_i * 8u;
+        tc::mbar_arrive_expect_tx(full, bytes);
+        if (act) tc::tma_load_2d(base + (uint32_t)stage_i * bytes, &tm_q, full, (kb_begin + kr) * (kRowBytes / 2), tq * BN);
+        else tc::tma_load_2d(base + (uint32_t)stage_i * bytes, &tm_w, full, (kb_begin + kr) * 8, tp * kBM);
+        ++issued;
+        if (++kr == kb_count) kr = 0;
+        if (++stage_i == ring) { stage_i = 0; phase ^= 1u; }
+      }
+    }
+    // after a failure: no copy may be in flight when the block exits
+    if (*abort) {
+      const uint64_t t0 = tc::global_timer_ns();
+      for (int i = 0; i < min(issued, ring); ++i) {
+        if (--stage_i < 0) { stage_i = ring - 1; phase ^= 1u; }
+        while (!tc::mbar_try_wait(full0 + (uint32_t)stage_i * 8u, phase) && tc::global_timer_ns() - t0 < tc::kWaitLimitNs) {}
+      }
+    }
+  };
+
+  if (AWQ && warp == 0) {
+    if (lane == 0) {
+      pdl_wait();
+      pdl_trigger();
+      awq_load(true);
+    }
+  } else if (AWQ && warp == 6 + kAwqWarps) {
+    if (lane == 0) awq_load(false);
+  } else if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
     if (lane == 0) {
       int stage_i = 0;
@@ -474,10 +528,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       // preceding kernel has just produced (a weight quantized on the fly, an AWQ layer dequantized
       // for a large M) must be waited for like the activations.
       const bool early_w = prm.early_w != 0;
-      // AWQ: only the activation tile arrives by TMA (the weight tile is written by the dequantizing warps)
-      const bool tma_p = !(AWQ && prm.swap != 0), tma_q = !(AWQ && prm.swap == 0);
-      const uint32_t tx_bytes = AWQ ? (uint32_t)((prm.swap ? BN : kBM) * kRowBytes) : (uint32_t)kStageBytes;
-      const uint32_t pk_bytes = (uint32_t)kPackedBytes;
+      const uint32_t tx_bytes = (uint32_t)kStageBytes;
       if (!early_w) {
         pdl_wait();
         pdl_trigger();
@@ -494,13 +545,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
           const uint32_t full = tc::smem_u32(&bar_full[g]);
           uint8_t* sp = tiles + g * kStageBytes;
           if (phase_w) tc::mbar_arrive_expect_tx(full, tx_bytes);
-          if (AWQ && phase_w) {                        // packed 4-bit tile: words 8 kb .. 8 kb + 7 of the tile's weight rows
-            const uint32_t pk = tc::smem_u32(&bar_pk[g]);
-            tc::mbar_arrive_expect_tx(pk, pk_bytes);
-            tc::tma_load_2d(tc::smem_u32(packed + g * kPkBytes), &tm_w, pk, (kb_begin + kr) * 8, tp * kBM);
-          }
-          if (load_p) { if (tma_p) tc::tma_load_2d(tc::smem_u32(sp), &tm_p, full, x, tp * kBM); }
-          else if (tma_q) tc::tma_load_2d(tc::smem_u32(sp + kBM * kRowBytes), &tm_q, full, x, tq * BN);
+          if (load_p) tc::tma_load_2d(tc::smem_u32(sp), &tm_p, full, x, tp * kBM);
+          else tc::tma_load_2d(tc::smem_u32(sp + kBM * kRowBytes), &tm_q, full, x, tq * BN);
         }
         if (phase_w && early_w) {
           // (Prefetching further weight tiles into L2 here was measured to slow the kernel down: the
@@ -537,13 +583,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
             uint8_t* sp = tiles + stage_i * kStageBytes;
             tc::mbar_arrive_expect_tx(full, tx_bytes);
             const int x = kb * kXPerBlock;
-            if (AWQ) {
-              const uint32_t pk = tc::smem_u32(&bar_pk[stage_i]);
-              tc::mbar_arrive_expect_tx(pk, pk_bytes);
-              tc::tma_load_2d(tc::smem_u32(packed + stage_i * kPkBytes), &tm_w, pk, kb * 8, tp * kBM);
-            }
-            if (tma_p) tc::tma_load_2d(tc::smem_u32(sp), &tm_p, full, x, tp * kBM);
-            if (tma_q) tc::tma_load_2d(tc::smem_u32(sp + kBM * kRowBytes), &tm_q, full, x, tq * BN);
+            tc::tma_load_2d(tc::smem_u32(sp), &tm_p, full, x, tp * kBM);
+            tc::tma_load_2d(tc::smem_u32(sp + kBM * kRowBytes), &tm_q, full, x, tq * BN);
             ++issued;
             if (++stage_i == kStages) { stage_i = 0; phase ^= 1u; }
           }
@@ -559,8 +600,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
           const uint64_t t0 = tc::global_timer_ns();
           while (!tc::mbar_try_wait(tc::smem_u32(&bar_full[s]), ph) &&
                  tc::global_timer_ns() - t0 < tc::kWaitLimitNs) {}
-          if (AWQ)
-            while (!tc::mbar_try_wait(tc::smem_u32(&bar_pk[s]), ph) && tc::global_timer_ns() - t0 < tc::kWaitLimitNs) {}
         }
       }
     }
@@ -582,104 +621,117 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         // the barrier orders them before MMAs issued after the wait; the flag is checked per tile.
         tc::mbar_wait_or_flag(tc::smem_u32(&bar_full[stage_i]), phase, abort_u32);
         __syncwarp();
-        const uint32_t sp = tc::smem_u32(tiles + stage_i * kStageBytes);
+        if constexpr (AWQ) tc::fence_after_sync();     // (the weight tile was stored to tensor memory by other threads)
+        const uint32_t sp = tc::smem_u32(tiles + stage_i * (AWQ ? BN * kRowBytes : kStageBytes));
         const uint64_t dp = tc::smem_desc_k_major_sw128(sp);
-        const uint64_t dq = tc::smem_desc_k_major_sw128(sp + kBM * kRowBytes);
+        const uint64_t dq = tc::smem_desc_k_major_sw128(AWQ ? sp : sp + kBM * kRowBytes);
+        const uint32_t a_tmem = tmem_base + (uint32_t)(kAccBufs * BN + stage_i * kAwqWtCols);
         if (tc::elect_one()) {
 #pragma unroll
           for (int j = 0; j < kRowBytes / 32; ++j) {
             // 32 bytes of K per instruction (32 8-bit or 16 16-bit elements): +2 in the >>4 address field.
-            tc::mma_ss<KIND>(d_tmem, dp + (uint64_t)(2 * j), dq + (uint64_t)(2 * j), prm.idesc,
-                             (it > 0 || j > 0) ? 1u : 0u);
+            const uint32_t more = (it > 0 || j > 0) ? 1u : 0u;
+            if constexpr (AWQ) tc::mma_ts_f16(d_tmem, a_tmem + (uint32_t)(8 * j), dq + (uint64_t)(2 * j), prm.idesc, more);
+            else tc::mma_ss<KIND>(d_tmem, dp + (uint64_t)(2 * j), dq + (uint64_t)(2 * j), prm.idesc, more);
           }
           tc::mma_commit(tc::smem_u32(&bar_empty[stage_i]));    // frees the stage once the MMAs retire
         }
         __syncwarp();
-        if (++stage_i == kStages) { stage_i = 0; phase ^= 1u; }
+        if (++stage_i == kFull) { stage_i = 0; phase ^= 1u; }
       }
       if (*abort) break;
       if (tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_acc_full[buf]));        // accumulator complete
       acc_phase[buf] ^= 1u;
-      buf ^= 1;
+      if (kAccBufs > 1) buf ^= 1;
     }
   } else if (AWQ && warp >= 6) {
     // ------------------------------- AWQ weight producer -------------------------
-    // 256 threads expand the packed 4-bit tile of every stage (delivered by TMA: 32 bytes = 64 values
-    // of K per weight row, 128 rows) into the stage's fp16 weight tile: a thread owns half a row --
-    // four packed words (eight values of K each) -> four 16-byte chunks of fp16, stored at the
-    // 128-byte-swizzle positions a TMA load of fp16 weights would have used, then made visible to the
-    // tensor core (async proxy) before the warp's arrival.  Two warps share a
-    // scheduler so that one's arithmetic hides the other's latencies.  The {scale, zero} pair of the
-    // row's quantization group is the only thing read from global memory here, kDepth blocks ahead.
+    // A packed 4-bit tile (32 bytes = 64 values of K per weight row, 128 rows) becomes an fp16 operand tile in tensor
+    // memory: a thread owns a row = lane, and pair p of its 64 values goes to column p.  The warps form kAwqGroups groups
+    // of 128 rows that take the tiles in turn: expanding one is a chain of latencies (barriers, load, arithmetic, store,
+    // arrival), so several have to be under way.  The
+    // {scale, zero} pairs of a row's quantization groups are the only thing read from global memory here, kDepth of the
+    // group's tiles ahead.
     constexpr int kDepth = 4;
-    const int t = (int)threadIdx.x - 6 * 32;
-    const int rr = t & (kBM - 1);                      // my row of the 128-row weight tile
-    const int j0 = 4 * (t >> 7);                       // my four of the row's eight words
-    // prefetch cursor of the scale / zero pairs: walks the (tile, K block) sequence kDepth blocks ahead
-    int pf_tile = first_tile, pf_it = 0, pf_rot = 0;
-    const uint32_t* pf_z = nullptr;                    // my row's scale-zero pairs in the cursor's tile
-    auto pf_enter_tile = [&]() {
-      pf_z = nullptr;
-      if (pf_tile >= num_tiles) return;
+    const int rr = (warp & 3) * 32 + lane;             // my row of a 128-row weight tile (a warp's quadrant of the lanes)
+    const int grp = (warp - 6) >> 2;
+    const uint32_t t_w = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(kAccBufs * BN);
+    const int my_tiles = first_tile < num_tiles ? (num_tiles - first_tile + tile_step - 1) / tile_step : 0;
+    const int total = my_tiles * kb_count;             // K blocks this CTA consumes, in ring order
+    // prefetch cursor of the scale / zero pairs: walks the group's share of the (tile, K block) sequence kDepth steps ahead
+    int pf_tile = first_tile, pf_it = grp, pf_rot = 0;
+    const uint32_t* pf_z = nullptr;                    // my row's pairs in the cursor's tile
+    auto pf_settle = [&]() {
+      while (pf_it >= kb_count) {
+        pf_it -= kb_count;
+        pf_tile += tile_step;
+      }
       const int tq = pf_tile % prm.tiles_q, tp = pf_tile / prm.tiles_q;
       pf_rot = (tp * 5 + tq * 3) % kb_count;           // the TMA producer's K rotation
       const int n = tp * kBM + rr;
-      if (n < prm.N) pf_z = prm.awq_sz + (int64_t)n * prm.awq_kg;
+      pf_z = pf_tile < num_tiles && n < prm.N ? prm.awq_sz + (int64_t)n * prm.awq_kg : nullptr;
     };
-    uint32_t szv[kDepth];                              // {scale, -(1024 + zero)} of my 32 values (groups of >= 32 values)
-    auto fetch = [&](uint32_t& z) {
-      z = 0u;                                          // scale 0: rows outside the matrix and values beyond K dequantize to 0
+    uint32_t szv[kDepth][2];                           // {scale, -(1024 + zero)} of the row's two halves of 32 values
+    auto fetch = [&](uint32_t (&z)[2]) {
+      int kr = pf_it + pf_rot;
+      if (kr >= kb_count) kr -= kb_count;
+      const int wi = (kb_begin + kr) * 8;              // first word of this K block
+      z[0] = z[1] = 0u;                                // scale 0: rows outside the matrix and values beyond K dequantize to 0
       if (pf_z != nullptr) {
-        int kr = pf_it + pf_rot;
-        if (kr >= kb_count) kr -= kb_count;
-        const int wi = (kb_begin + kr) * 8 + j0;       // my first word of this K block
-        if (wi < prm.awq_kw) z = __ldg(pf_z + (wi * 8) / prm.awq_g);
+        // (K is a multiple of the group, so a half of the block that begins inside the matrix ends inside it)
+        if (prm.awq_gshift >= 0) {
+          if (wi < prm.awq_kw) z[0] = __ldg(pf_z + (wi >> prm.awq_gshift));
+          if (wi + 4 < prm.awq_kw) z[1] = prm.awq_gw >= 8 ? z[0] : __ldg(pf_z + ((wi + 4) >> prm.awq_gshift));
+        } else {
+          if (wi < prm.awq_kw) z[0] = __ldg(pf_z + wi / prm.awq_gw);
+          if (wi + 4 < prm.awq_kw) z[1] = __ldg(pf_z + (wi + 4) / prm.awq_gw);
+        }
       }
-      if (++pf_it == kb_count) {                       // advance the cursor
-        pf_it = 0;
-        pf_tile += tile_step;
-        pf_enter_tile();
-      }
+      pf_it += kAwqGroups;
+      if (pf_it >= kb_count) pf_settle();
     };
-    pf_enter_tile();
+    pf_settle();
 #pragma unroll
     for (int d = 0; d < kDepth; ++d) fetch(szv[d]);
-    const int my_tiles = first_tile < num_tiles ? (num_tiles - first_tile + tile_step - 1) / tile_step : 0;
-    const int total = my_tiles * kb_count;             // K blocks this CTA consumes, in ring order
-    int stage_i = 0;
-    uint32_t phase = 0;
+    static_assert(kAwqGroups <= kFull && kAwqGroups <= kPk, "or a parity could stand for two turns of a ring");
+    int ps = grp, ws = grp;                            // my packed tile, the stage whose weight tile it becomes
+    uint32_t p_phase = 0, w_phase = 0;
     bool ok = true;
-    for (int q0 = 0; q0 < total && ok; q0 += kDepth) {
+    for (int q0 = grp; q0 < total && ok; q0 += kDepth * kAwqGroups) {
 #pragma unroll
       for (int d = 0; d < kDepth; ++d) {
-        if (q0 + d >= total || !ok) continue;
-        // the packed tile has landed; the TMA thread requested it only after the stage's previous
-        // contents had been consumed, so the fp16 tile may be overwritten as well
-        tc::mbar_wait_or_flag(tc::smem_u32(&bar_pk[stage_i]), phase, abort_u32);
-        if (*abort) { ok = false; continue; }
-        {
-          const uint4 a = *reinterpret_cast<const uint4*>(packed + stage_i * kPkBytes + rr * kPackedRowBytes + j0 * 4);
-          uint4* dst = reinterpret_cast<uint4*>(tiles + stage_i * kStageBytes + rr * kRowBytes);
-          const uint32_t words[4] = {a.x, a.y, a.z, a.w};
-          const __half2 sz = *reinterpret_cast<const __half2*>(&szv[d]);
+        if (q0 + d * kAwqGroups >= total || !ok) continue;
+        tc::mbar_wait_or_flag(tc::smem_u32(&bar_pk_full[ps]), p_phase, abort_u32);
+        if (d == 0 && *abort) { ok = false; continue; }
+        const uint4* src = reinterpret_cast<const uint4*>(packed + ps * kPackedBytes + rr * kPackedRowBytes);
+        const uint4 a0 = src[0], a1 = src[1];
+        const uint32_t words[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        uint32_t o[32];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const __half2 sz = *reinterpret_cast<const __half2*>(&szv[d][j >> 2]);
           const __half2 negz = __half2half2(__high2half(sz)), sc = __half2half2(__low2half(sz));
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t o[4];
-#pragma unroll
-            for (int p4 = 0; p4 < 4; ++p4) {
-              uint32_t h = ((words[j] >> (4 * p4)) & 0x000F000Fu) | 0x64006400u;         // {1024 + v[2p], 1024 + v[2p+1]}
-              const __half2 v2 = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&h), negz), sc);
-              o[p4] = *reinterpret_cast<const uint32_t*>(&v2);
-            }
-            dst[(j0 + j) ^ (rr & 7)] = make_uint4(o[0], o[1], o[2], o[3]);
+          for (int p4 = 0; p4 < 4; ++p4) {
+            uint32_t h = ((words[j] >> (4 * p4)) & 0x000F000Fu) | 0x64006400u;           // {1024 + v[2p], 1024 + v[2p+1]}
+            const __half2 v2 = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&h), negz), sc);
+            o[4 * j + p4] = *reinterpret_cast<const uint32_t*>(&v2);
           }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // generic writes -> tensor-core reads
+        tc::mbar_wait_or_flag(tc::smem_u32(&bar_empty[ws]), w_phase ^ 1u, abort_u32);
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(tc::smem_u32(&bar_full[stage_i]));
-        if (++stage_i == kStages) { stage_i = 0; phase ^= 1u; }
-        fetch(szv[d]);                                 // refill the slot for kDepth blocks ahead
+        tc::fence_after_sync();
+        tc::tmem_st_32x32(t_w + (uint32_t)(ws * kAwqWtCols), o);
+        tc::tmem_st_wait();
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          tc::mbar_arrive(tc::smem_u32(&bar_full[ws]));
+          tc::mbar_arrive(tc::smem_u32(&bar_pk_empty[ps]));
+        }
+        if ((ps += kAwqGroups) >= kPk) { ps -= kPk; p_phase ^= 1u; }
+        if ((ws += kAwqGroups) >= kFull) { ws -= kFull; w_phase ^= 1u; }
+        fetch(szv[d]);                                 // refill the slot for kDepth steps ahead
       }
     }
   } else {
@@ -730,7 +782,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       // accumulator buffer may be overwritten by the next-but-one tile
       tc::fence_before_sync();
       tc::mbar_arrive(tc::smem_u32(&bar_acc_empty[buf]));
-      buf ^= 1;
+      if (kAccBufs > 1) buf ^= 1;
     }
   }
 
@@ -1292,6 +1344,24 @@ int max_active_clusters(int cluster) {
   return n;
 }
 
+// The cluster size (any from 1 to 8: 36 tiles fit as clusters of three, not of four) with the smallest estimated time: waves
+// of co-resident clusters x (K blocks per CTA + a fixed per-CTA cost of about eight K blocks for pipeline fill,
+// reduce-scatter and epilogue).
+int pick_splits(int64_t tiles, int k_blocks, int most, int (*active)(int), int* waves) {
+  const float fixed = 8.f;
+  int splits = 1, w = (int)ceil_div(tiles, (int64_t)sm_count());
+  float best = (float)w * ((float)k_blocks + fixed);
+  for (int s = 2; s <= 8 && tiles < sm_count(); ++s) {
+    if (k_blocks < 2 * s || most < s) continue;
+    const int n = active(s);
+    if (n <= 0) continue;
+    const float t = (float)ceil_div(tiles, (int64_t)n) * ((float)k_blocks / s + fixed);
+    if (t < best) { best = t; splits = s; w = (int)ceil_div(tiles, (int64_t)n); }
+  }
+  if (waves) *waves = w;
+  return splits;
+}
+
 template <int KIND, int BN, bool AWQ = false, bool PUSH = false>
 int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& tm_w, TcParams prm, cudaStream_t st) {
   auto kern = gemm_tc_kernel<KIND, BN, AWQ, PUSH>;
@@ -1300,19 +1370,8 @@ int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& 
   const int tiles = prm.tiles_p * prm.tiles_q;
   int splits = 1;
   if (BN <= 128 && tiles < sms) {
-    // Pick the cluster size (1, 2, 4, 8) with the smallest estimated time: waves of co-resident
-    // clusters x (K blocks per CTA + a fixed per-CTA cost of about eight K blocks for pipeline fill,
-    // reduce-scatter and epilogue).
-    const float fixed = 8.f;
-    float best = (float)ceil_div(tiles, sms) * ((float)prm.k_blocks + fixed);
     if (prm.tiles_q > 1 && !AWQ) panel_us(tiles, prm.k_blocks, &splits, max_active_clusters<KIND, BN, AWQ, PUSH>);
-    else for (int s = 2; s <= 8; ++s) {                     // (any size: 36 tiles fit as clusters of three, not of four)
-      if (prm.k_blocks < 2 * s || BN / 8 < s) continue;
-      const int active = max_active_clusters<KIND, BN, AWQ, PUSH>(s);
-      if (active <= 0) continue;
-      const float t = (float)ceil_div(tiles, active) * ((float)prm.k_blocks / s + fixed);
-      if (t < best) { best = t; splits = s; }
-    }
+    else splits = pick_splits(tiles, prm.k_blocks, BN / 8, max_active_clusters<KIND, BN, AWQ, PUSH>, nullptr);
   }
   prm.splits = splits;
   const int grid = splits > 1 ? tiles * splits : (tiles < sms ? tiles : sms);
@@ -1395,6 +1454,14 @@ int launch_bn(int bn, const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CU
   }
 }
 
+// Estimated microseconds of the kernel that dequantizes its weights, fitted to times over N = 896 .. 37888, K = 896 .. 18944:
+// up to 64 tokens, and above 128 with the tokens in panels of 128 or (*panels = false) in tiles of 256.
+double awq_split_us(int64_t tiles, int k_blocks, int most, int (*active)(int), double base, double kb, double tile, double exchange) {
+  int waves;
+  const int s = pick_splits(tiles, k_blocks, most, active, &waves);
+  return base + waves * (kb * k_blocks / s + tile + (s > 1 ? exchange : 0.));
+}
+
 // The two-CTA kernel is used unless the environment variable LLMQRT_GEMM_PAIR is "0".
 bool pair_enabled() {
   static const bool on = [] {
@@ -1405,6 +1472,25 @@ bool pair_enabled() {
 }
 
 }  // namespace
+
+double awq_tc_us(int64_t M, int64_t N, int64_t K, bool* panels) {
+  const int kb = (int)ceil_div(K, (int64_t)64);
+  const int64_t tiles = ceil_div(N, (int64_t)kBM);
+  if (M <= 128)
+    return awq_split_us(tiles, kb, 8, max_active_clusters<tc::MMA_F16, 64, true>, 2.4, 0.324, 2.2, 3.8);
+  const double p = awq_split_us(tiles * ceil_div(M, (int64_t)128), kb, 16, max_active_clusters<tc::MMA_F16, 128, true>,
+                                5.7, 0.28, 4.3, 3.7);
+  const double t = (double)ceil_div(tiles * ceil_div(M, (int64_t)256), (int64_t)sm_count()) * (0.327 * kb + 14.2);
+  if (panels) *panels = p < t;
+  return p < t ? p : t;
+}
+
+double awq_expanded_us(int64_t M, int64_t N, int64_t K) {
+  const int kb = (int)ceil_div(K, (int64_t)64);
+  double g = pair_us(ceil_div(M, (int64_t)256) * ceil_div(N, (int64_t)kPairBN), kb);
+  const double p = panel_us(ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM), kb, nullptr);
+  return 2.1 + 0.906 * (p < g ? p : g) + 0.518e-6 * (double)(N * K);
+}
 
 int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
             const Epilogue& epi, void* workspace, cudaStream_t st, bool static_w, const AwqOperand* awq,
@@ -1439,8 +1525,7 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
     if (pair_ok) {
       panels = panel_us(panel_tiles, k_blocks, nullptr) < pair_us(ceil_div(M, (int64_t)256) * ceil_div(N, (int64_t)256), k_blocks);
     } else if (awq) {
-      const int64_t tiles = ceil_div(M, (int64_t)kBM) * ceil_div(N, (int64_t)(N <= 128 ? 128 : 256));
-      panels = tiles * 4 <= sm_count();
+      awq_tc_us(M, N, K, &panels);
     } else {
       panels = true;
     }
@@ -1513,7 +1598,8 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
     prm.awq_sz = awq->sz_t;
     prm.awq_kw = (int)(K / 8);
     prm.awq_kg = (int)(K / awq->G);
-    prm.awq_g = (int)awq->G;
+    prm.awq_gw = (int)(awq->G / 8);
+    prm.awq_gshift = (prm.awq_gw & (prm.awq_gw - 1)) == 0 ? __builtin_ctz((unsigned)prm.awq_gw) : -1;
     // packed words as a 2-D uint32 matrix [N, K / 8]; box = the 8 words of a K block x the tile's weight rows
     CUtensorMap tm_w;
     if (int rc = make_packed_map(&tm_w, awq->wq_t, N, K / 8, kBM)) return rc;

@@ -110,3 +110,22 @@ def test_quantized_by_the_gemm(M, N, K, dt):
     y, ok = f8(x), ~want.isnan()
     assert torch.equal(y.isnan(), want.isnan())
     assert rel_fro(y[ok & want.isfinite()], want[ok & want.isfinite()].double()) < 2 ** -9     # (a bf16 rounding falling the other way)
+
+
+@pytest.mark.parametrize("M", [9, 16, 64, 65, 128, 257, 1025])
+@pytest.mark.parametrize("K,N,G", [(32, 8, 32), (160, 136, 32), (1056, 264, 96), (8960, 1536, 128), (704, 17920, 64)])
+def test_awq_tensor_memory_tiles(M, K, N, G):
+    """The kernel that dequantizes into tensor memory, at the edges of its tiles: one K block and rings that go round many
+    times, half a block, groups that are no power of two, clusters of every size, single tiles and several to a block, rows
+    and tokens beyond the matrix; and the kernels that take over from it below and above."""
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    qz = torch.randint(-2 ** 31, 2 ** 31 - 1, (K // G, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    sc = torch.rand(K // G, N, generator=g, device="cuda").mul_(0.02).half()
+    x, bias = torch.randn(M, K, generator=g, device="cuda").half(), torch.randn(N, generator=g, device="cuda").half()
+    want = x.double() @ ops.awq_dequantize(qw, sc, qz).double() + bias.double()
+    packed = ops.AwqPacked(qw, sc, qz)
+    y = ops.awq_gemm(x, packed, bias)
+    assert rel_fro(y, want) < 5e-4                          # the fp16 rounding of the result
+    assert torch.equal(y, ops.awq_gemm(x, packed, bias))    # one order of the sums
