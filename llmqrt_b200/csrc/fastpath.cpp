@@ -6,7 +6,7 @@
 // tensors) took the host fifty.  Here it is a METH_FASTCALL function that checks the tensors, allocates the
 // results through ATen and calls the C ABI: one crossing of the language border for one call.  A pass over a
 // 4864 x 896 layer went from 53 to 11 us (int8, 16 tokens; 9.5 since its GEMM quantizes), a 28-layer 4-bit model's step
-// from 9.4 to 4.2 ms (2.7 with fewer launches).
+// from 9.4 to 4.2 ms (2.7 with fewer launches, 1.0 with a block's step as one call).
 //
 // The checks are those of the Python wrappers before it (ops.py, glue.py, attention.py), with the same exceptions; the
 // attention calls also check caches and lengths against the query's batch.
@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <optional>
 
 #include "../../include/llmqrt_b200.h"
 
@@ -627,24 +628,332 @@ FAST_FN(attn_decode_step) {
   FAST_END
 }
 
+// Identity and in-place version of a tensor, appended to a key.
+using Key = c10::SmallVector<int64_t, 32>;
+void key_of(const Tensor& t, Key& k) {
+  if (!t.defined()) return;
+  k.push_back((int64_t)reinterpret_cast<intptr_t>(t.data_ptr()));
+  k.push_back(t._version());
+  k.push_back((int64_t)t.scalar_type());
+  k.push_back((int64_t)t.device().type() * 256 + t.device().index());
+  k.push_back(t.dim());
+  for (int64_t s : t.sizes()) k.push_back(s);
+}
+
 // (tensor or None, ...) -> identity and in-place version of the tensors, as one tuple of integers.
 FAST_FN(tensor_key) {
   HANDLE_TH_ERRORS
-  c10::SmallVector<int64_t, 32> k;
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    const Tensor t = tensor_arg(a[i], "buffer");
-    if (!t.defined()) continue;
-    k.push_back((int64_t)reinterpret_cast<intptr_t>(t.data_ptr()));
-    k.push_back(t._version());
-    k.push_back((int64_t)t.scalar_type());
-    k.push_back((int64_t)t.device().type() * 256 + t.device().index());
-    k.push_back(t.dim());
-    for (int64_t s : t.sizes()) k.push_back(s);
-  }
+  Key k;
+  for (Py_ssize_t i = 0; i < n; ++i) key_of(tensor_arg(a[i], "buffer"), k);
   PyObject* tup = PyTuple_New((Py_ssize_t)k.size());
   if (!tup) throw python_error();
   for (size_t i = 0; i < k.size(); ++i) PyTuple_SET_ITEM(tup, i, PyLong_FromLongLong(k[i]));
   return tup;
+  FAST_END
+}
+
+// ---- a 4-bit decoder block's step ------------------------------------------------------------------
+
+// A block of a few tokens is seven kernels of 2 to 9 us; as eight calls of Python modules it took the host 90 us.  The call
+// below does the whole step or, wherever anything about the block is not as these classes made it, nothing: it returns
+// None, having changed nothing, and the caller goes on with the modules, whose behaviour (and errors) this one has.
+
+PyObject* g_plain = nullptr;                           // ((class, attribute, the function it was defined with), ...)
+PyObject* g_hooks = nullptr;                           // the dictionaries of hooks on all modules
+PyTypeObject *g_norm = nullptr, *g_attn = nullptr, *g_mlp = nullptr, *g_linear = nullptr;
+
+// (RMSNorm, QuantAttentionFused, FusedGateUpMLP, WQLinear_GEMM, plain, hooks)
+FAST_FN(set_block_classes) {
+  FAST_BEGIN(6)
+  for (int i = 0; i < 6; ++i) Py_INCREF(a[i]);         // (for the life of the process)
+  g_norm = reinterpret_cast<PyTypeObject*>(a[0]);
+  g_attn = reinterpret_cast<PyTypeObject*>(a[1]);
+  g_mlp = reinterpret_cast<PyTypeObject*>(a[2]);
+  g_linear = reinterpret_cast<PyTypeObject*>(a[3]);
+  g_plain = a[4];
+  g_hooks = a[5];
+  Py_RETURN_NONE;
+  FAST_END
+}
+
+struct NotPlain {};                                    // whatever the step does not cover
+
+PyObject* name_of(const char* text) {
+  PyObject* s = PyUnicode_InternFromString(text);
+  if (!s) throw python_error();
+  return s;
+}
+#define NAME(text) ([]() { static PyObject* const s = name_of(text); return s; }())
+
+// Reads an object's own attributes: straight from its dictionary, a module's registered tensors and children included.
+class Fields {
+ public:
+  explicit Fields(PyObject* o) : owner_(PyObject_GenericGetDict(o, nullptr)), dict_(owner_.get()) {
+    if (dict_) return;
+    PyErr_Clear();                                     // (an object without a dictionary)
+    throw NotPlain();
+  }
+  PyObject* find(PyObject* name) const {               // borrowed; null if there is none
+    PyObject* v = PyDict_GetItemWithError(dict_, name);
+    if (!v && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+  PyObject* get(PyObject* name) const {
+    PyObject* v = find(name);
+    if (!v) throw NotPlain();
+    return v;
+  }
+  PyObject* in(PyObject* group, PyObject* name) const {   // of _modules, _buffers or _parameters
+    PyObject* d = find(group);
+    if (!d || !PyDict_Check(d)) return nullptr;
+    PyObject* v = PyDict_GetItemWithError(d, name);
+    if (!v && PyErr_Occurred()) throw python_error();
+    return v;
+  }
+  PyObject* child(PyObject* name) const {
+    PyObject* v = in(NAME("_modules"), name);
+    if (!v || find(name)) throw NotPlain();
+    return v;
+  }
+  Tensor tensor(PyObject* name) const {                // attribute, buffer or parameter; undefined if it is None
+    PyObject* v = find(name);
+    if (!v) v = in(NAME("_buffers"), name);
+    if (!v) v = in(NAME("_parameters"), name);
+    if (!v) throw NotPlain();
+    if (v == Py_None) return Tensor();
+    if (!THPVariable_Check(v)) throw NotPlain();
+    return THPVariable_Unpack(v);
+  }
+  bool none(PyObject* name) const {
+    PyObject* v = find(name);
+    if (!v) v = in(NAME("_modules"), name);
+    return v == Py_None;
+  }
+  int64_t integer(PyObject* name) const {
+    PyObject* v = get(name);
+    if (!PyLong_CheckExact(v)) throw NotPlain();
+    const long long i = PyLong_AsLongLong(v);
+    if (i == -1 && PyErr_Occurred()) { PyErr_Clear(); throw NotPlain(); }
+    return i;
+  }
+  double number(PyObject* name) const {
+    PyObject* v = get(name);
+    if (PyFloat_CheckExact(v)) return PyFloat_AS_DOUBLE(v);
+    if (!PyLong_CheckExact(v)) throw NotPlain();
+    return PyLong_AsDouble(v);
+  }
+  bool empty(PyObject* name) const {
+    PyObject* v = get(name);
+    return PyDict_Check(v) && PyDict_GET_SIZE(v) == 0;
+  }
+  PyObject* dict() const { return dict_; }
+
+ private:
+  THPObjectPtr owner_;
+  PyObject* dict_;
+};
+
+// obj.name, through the class where the instance has none.
+bool flag(PyObject* obj, PyObject* name) {
+  THPObjectPtr v(PyObject_GetAttr(obj, name));
+  if (!v) throw python_error();
+  return bool_arg(v.get());
+}
+
+// A module whose call is its class's forward and nothing else.
+Fields plain_module(PyObject* m, PyTypeObject* cls, bool called = true) {
+  if (Py_TYPE(m) != cls) throw NotPlain();
+  Fields f(m);
+  if (f.find(NAME("forward"))) throw NotPlain();
+  if (called) {
+    PyObject* compiled = f.find(NAME("_compiled_call_impl"));
+    if (!f.empty(NAME("_forward_hooks")) || !f.empty(NAME("_forward_pre_hooks")) || !f.empty(NAME("_backward_hooks")) ||
+        !f.empty(NAME("_backward_pre_hooks")) || (compiled && compiled != Py_None))
+      throw NotPlain();
+  }
+  return f;
+}
+
+// One WQLinear_GEMM whose packed weights are those of its buffers as they are now.
+struct PlainLinear {
+  PlainLinear(PyObject* m, c10::Device dev) {
+    const Fields f = plain_module(m, g_linear);
+    PyObject* packed = f.get(NAME("_packed"));
+    PyObject* key = f.get(NAME("_packed_key"));
+    if (packed == Py_None || !PyTuple_CheckExact(key)) throw NotPlain();
+    Key now;
+    const Tensor qw = f.tensor(NAME("qweight"));
+    if (!qw.defined() || qw.device() != dev) throw NotPlain();
+    key_of(qw, now);
+    key_of(f.tensor(NAME("qzeros")), now);
+    key_of(f.tensor(NAME("scales")), now);
+    if ((size_t)PyTuple_GET_SIZE(key) != now.size()) throw NotPlain();
+    for (size_t i = 0; i < now.size(); ++i)
+      if (PyLong_AsLongLong(PyTuple_GET_ITEM(key, i)) != now[i]) throw NotPlain();
+    wq = tensor_of(packed, NAME("wq_t"));
+    sz = tensor_of(packed, NAME("sz_t"));
+    K = int_of(packed, NAME("K"));
+    N = int_of(packed, NAME("N"));
+    G = int_of(packed, NAME("G"));
+    bias = f.tensor(NAME("bias"));
+    if (bias.defined() && (bias.device() != dev || bias.scalar_type() != at::kHalf || bias.numel() != N || !bias.is_contiguous()))
+      throw NotPlain();
+    if (f.integer(NAME("in_features")) != K || f.integer(NAME("out_features")) != N || K % 32 || G % 32 || N % 8) throw NotPlain();
+  }
+  void run(const void* x, void* out, int64_t M, Call& c) const {
+    check(llmqrt_awq_gemm(x, K, words(wq), words(sz), ptr(bias), out, N, M, N, K, G, c.workspace(), c.stream));
+  }
+  void run_tail(const void* x, const void* residual, void* out, int64_t M, Call& c) const {
+    check(llmqrt_awq_gemm_tail(x, K, words(wq), words(sz), ptr(bias), residual, residual ? N : 0, out, residual ? N : N / 2, M, N,
+                               K, G, c.stream));
+  }
+  Tensor wq, sz, bias;
+  int64_t K, N, G;
+
+ private:
+  static const uint32_t* words(const Tensor& t) { return static_cast<const uint32_t*>(ptr(t)); }
+  static Tensor tensor_of(PyObject* o, PyObject* name) {
+    THPObjectPtr v(PyObject_GetAttr(o, name));
+    if (!v) throw python_error();
+    return tensor_arg(v.get(), "packed weights");
+  }
+  static int64_t int_of(PyObject* o, PyObject* name) {
+    THPObjectPtr v(PyObject_GetAttr(o, name));
+    if (!v) throw python_error();
+    return int_arg(v.get());
+  }
+};
+
+struct PlainNorm {
+  PlainNorm(PyObject* m, c10::Device dev, int64_t hidden) {
+    const Fields f = plain_module(m, g_norm);
+    w = f.tensor(NAME("weight"));
+    eps = (float)f.number(NAME("variance_epsilon"));
+    if (!w.defined() || w.device() != dev || w.scalar_type() != at::kHalf || w.numel() != hidden || !w.is_contiguous()) throw NotPlain();
+  }
+  void run(const void* x, const void* residual, void* h, void* y, int64_t M, Call& c) const {
+    check(llmqrt_rmsnorm(x, residual, h, ptr(w), eps, y, nullptr, nullptr, LLMQRT_F16, M, w.numel(), c.stream));
+  }
+  Tensor w;
+  float eps;
+};
+
+Tensor plain_cache(PyObject* o, PyObject* name, const Tensor& x) {
+  const Tensor t = Fields(o).tensor(name);
+  if (!t.defined() || t.dim() != 4 || t.scalar_type() != at::kHalf || t.device() != x.device() || t.stride(3) != 1 ||
+      t.stride(2) != t.size(3) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16)
+    throw NotPlain();
+  return t;
+}
+
+// Everything the step reads, gathered before anything is launched.
+struct BlockStep {
+  BlockStep(PyObject* block, const Tensor& x)
+      : me(block), attn_o(me.child(NAME("attn"))), mlp(plain_module(me.child(NAME("mlp")), g_mlp, false)),
+        attn(plain_module(attn_o, g_attn, false)), dev(x.device()), B(x.size(0)), hidden(x.size(2)),
+        norm1(me.child(NAME("norm_1")), dev, hidden), norm2(me.child(NAME("norm_2")), dev, hidden),
+        qkv(attn.child(NAME("qkv_proj")), dev), o(attn.child(NAME("o_proj")), dev), gate_up(mlp.child(NAME("gate_up")), dev),
+        down(mlp.child(NAME("down_proj")), dev) {
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(g_plain); ++i) {
+      PyObject* p = PyTuple_GET_ITEM(g_plain, i);
+      THPObjectPtr now(PyObject_GetAttr(PyTuple_GET_ITEM(p, 0), PyTuple_GET_ITEM(p, 1)));
+      if (!now) throw python_error();
+      if (now.get() != PyTuple_GET_ITEM(p, 2)) throw NotPlain();
+    }
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(g_hooks); ++i)
+      if (PyObject_Size(PyTuple_GET_ITEM(g_hooks, i)) != 0) throw NotPlain();
+    if (!attn.none(NAME("q_proj")) || !attn.none(NAME("q_norm")) || !attn.none(NAME("k_norm"))) throw NotPlain();
+    Hq = attn.integer(NAME("n_heads"));
+    Hkv = attn.integer(NAME("n_kv_heads"));
+    if (!Hkv) Hkv = Hq;
+    d = attn.integer(NAME("head_dim"));
+    pos = attn.integer(NAME("start_pos"));
+    softcap = (float)attn.number(NAME("attn_logit_softcapping"));
+    PyObject* cache = attn.get(NAME("cache"));
+    kc = plain_cache(cache, NAME("k"), x);
+    vc = plain_cache(cache, NAME("v"), x);
+    const Fields rope(attn.child(NAME("rope")));
+    cos = rope.tensor(NAME("cos"));
+    sin = rope.tensor(NAME("sin"));
+    if (attn.integer(NAME("cache_batch_size")) != B || kc.size(0) < B || vc.sizes() != kc.sizes() || vc.strides() != kc.strides() ||
+        kc.size(2) != Hkv || kc.size(3) != d || (d != 64 && d != 128) || Hq <= 0 || Hkv <= 0 || Hq % Hkv || pos < 0 || pos >= kc.size(1))
+      throw NotPlain();
+    for (const Tensor* t : {&cos, &sin})
+      if (!t->defined() || t->device() != dev || t->scalar_type() != at::kFloat || t->dim() != 2 || t->size(1) != d / 2 ||
+          !t->is_contiguous() || t->size(0) <= pos)
+        throw NotPlain();
+    if (cos.sizes() != sin.sizes() || qkv.K != hidden || qkv.N != (Hq + 2 * Hkv) * d || o.K != Hq * d || o.N != hidden ||
+        gate_up.K != hidden || gate_up.N % 16 || down.K != gate_up.N / 2 || down.N != hidden)
+      throw NotPlain();
+    twice = flag(attn_o, NAME("REFERENCE_DOUBLE_APPEND")) && pos + 1 < kc.size(1);
+    rewind = flag(attn_o, NAME("is_hf_transformers"));
+  }
+
+  Tensor run(const Tensor& x0) {
+    Call c(dev);
+    const Tensor x = x0.contiguous();
+    const int64_t M = B, sizes[] = {hidden, qkv.N, o.K, hidden, hidden, hidden, down.K};
+    int64_t at[8] = {0};                               // the intermediate results, each on a boundary of 256 bytes
+    for (int i = 0; i < 7; ++i) at[i + 1] = at[i] + (M * sizes[i] * 2 + 255) / 256 * 256;
+    const Tensor scratch = empty(x, {at[7]}, at::kByte);
+    Tensor out = empty(x, {B, 1, hidden}, at::kHalf);
+    uint8_t* base = static_cast<uint8_t*>(scratch.data_ptr());
+    auto* y1 = base + at[0]; auto* p = base + at[1]; auto* w = base + at[2]; auto* ao = base + at[3];
+    auto* h = base + at[4]; auto* y2 = base + at[5]; auto* g = base + at[6];
+    norm1.run(ptr(x), nullptr, nullptr, y1, M, c);
+    qkv.run(y1, p, M, c);
+    const int64_t len = pos + (twice ? 2 : 1);
+    check(llmqrt_attn_decode_step(p, B > 1 ? qkv.N : Hq * d, p + Hq * d * 2, p + (Hq + Hkv) * d * 2, B > 1 ? qkv.N : Hkv * d,
+                                  static_cast<const float*>(ptr(cos)), static_cast<const float*>(ptr(sin)), cos.size(0), twice ? 1 : 0,
+                                  mptr(kc), mptr(vc), kc.stride(0), kc.stride(1), kc.size(1), nullptr, (int32_t)len, w, LLMQRT_F16, B,
+                                  Hq, Hkv, d, std::min(len, kc.size(1)), softcap, c.workspace(), c.stream));
+    o.run(w, ao, M, c);
+    norm2.run(ptr(x), ao, h, y2, M, c);
+    gate_up.run_tail(y2, nullptr, g, M, c);
+    down.run_tail(g, h, mptr(out), M, c);
+    return out;
+  }
+  void advance() {
+    THPObjectPtr next(PyLong_FromLongLong(rewind ? 0 : pos + 1));
+    if (!next || PyDict_SetItem(attn.dict(), NAME("start_pos"), next.get()) < 0) throw python_error();
+  }
+
+  Fields me;
+  PyObject* attn_o;
+  Fields mlp, attn;
+  c10::Device dev;
+  int64_t B, hidden;
+  PlainNorm norm1, norm2;
+  PlainLinear qkv, o, gate_up, down;
+  int64_t Hq, Hkv, d, pos;
+  float softcap;
+  Tensor kc, vc, cos, sin;
+  bool twice, rewind;
+};
+
+// (block, hidden_states [B, 1, hidden]) -> the block's output and its start_pos moved on, or None.
+FAST_FN(awq_block_step) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_TYPE(n == 2, "llmqrt_b200: expected 2 arguments, got ", (int64_t)n);
+  if (!g_plain || !THPVariable_CheckExact(a[1])) Py_RETURN_NONE;
+  const Tensor x = THPVariable_Unpack(a[1]);
+  if (!x.is_cuda() || x.scalar_type() != at::kHalf || x.dim() != 3 || x.size(1) != 1 || x.size(0) < 1 || x.size(0) > 16 ||
+      (at::GradMode::is_enabled() && x.requires_grad()))
+    Py_RETURN_NONE;
+  at::NoGradGuard no_grad;
+  std::optional<BlockStep> step;
+  try {
+    step.emplace(a[0], x);
+  } catch (const NotPlain&) {
+    Py_RETURN_NONE;
+  }
+  Tensor out;
+  {
+    GilRelease gil;
+    out = step->run(x);
+  }
+  step->advance();
+  return wrap(out);
   FAST_END
 }
 
@@ -660,6 +969,7 @@ FAST_FN(set_workspace_maker) {
 PyMethodDef methods[] = {FAST_DEF(sq_per_channel), FAST_DEF(sq_per_tensor), FAST_DEF(fp8_per_token), FAST_DEF(fp8_per_tensor),
                          FAST_DEF(awq_linear), FAST_DEF(awq_tail), FAST_DEF(rmsnorm), FAST_DEF(silu_mul), FAST_DEF(rope_kv_write),
                          FAST_DEF(attn_prefill), FAST_DEF(kv_append), FAST_DEF(attn_decode), FAST_DEF(attn_decode_step), FAST_DEF(tensor_key),
+                         FAST_DEF(set_block_classes), FAST_DEF(awq_block_step),
                          FAST_DEF(set_workspace_maker), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast", "Native host path of llmqrt_b200.", -1, methods,
                       nullptr, nullptr, nullptr, nullptr};

@@ -7,7 +7,10 @@ from typing import List
 import torch
 import torch.nn as nn
 
+from .._lib import fast
 from ..fused_utils import FusedGateUpMLP
+from ..linear import WQLinear_GEMM
+from ..linear import linear_base
 from .attn import QuantAttentionFused
 from .norm import RMSNorm
 
@@ -30,6 +33,9 @@ class LlamaLikeBlock(nn.Module):
         self.device = dev
 
     def forward(self, hidden_states):
+        out = fast.awq_block_step(self, hidden_states)       # a few 4-bit tokens: the whole step, one native call
+        if out is not None:
+            return out
         attn_output, _, _ = self.attn.forward(hidden_states=self.norm_1(hidden_states))
         hidden_states = hidden_states.to(attn_output.device)
         if type(self.norm_2) is RMSNorm:
@@ -79,3 +85,13 @@ class LlamaLikeModel(nn.Module):
         for layer in self.blocks:
             h = layer(h.to(layer.device))
         return self.norm(h)
+
+
+# What has to be as it was defined for the native step to stand for the modules' own code.
+fast.set_block_classes(
+    RMSNorm, QuantAttentionFused, FusedGateUpMLP, WQLinear_GEMM,
+    tuple((cls, name, getattr(cls, name)) for cls, names in
+          ((RMSNorm, ("forward", "add")), (QuantAttentionFused, ("forward",)), (FusedGateUpMLP, ("forward", "add_to", "_hidden")),
+           (WQLinear_GEMM, ("forward", "packed", "takes_tail", "silu_halves", "add_to"))) for name in names),
+    (linear_base._global_forward_hooks, linear_base._global_forward_pre_hooks, linear_base._global_backward_hooks,
+     linear_base._global_backward_pre_hooks))

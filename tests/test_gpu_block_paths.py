@@ -127,3 +127,78 @@ def test_full_cache():
         want = (p @ kept[1][0, :, 0].double()).reshape(1, 1, HQ * D)
         assert float((weight.double() - want).norm() / want.norm()) < 1e-3     # P and the result in fp16: 2^-11 each
         assert torch.equal(a.cache.k, kept[0]) and torch.equal(a.cache.v, kept[1]) and a.start_pos == pos + 1
+
+
+@pytest.mark.parametrize("B", [1, 2, 16])
+def test_step_in_one_call(B):
+    """The block's native step against the composition of its modules: outputs, caches and positions, over several steps, up
+    to the cache's last row, with weights changed in place and replaced on the way."""
+    from llmqrt_b200._lib import fast
+    rows, g = 12, torch.Generator(device="cuda").manual_seed(B)
+    blocks = [_block(rows) for _ in range(2)]
+    for block in blocks:
+        block.attn.cache.increase_batch_size(B)
+        block.attn.cache_batch_size = B
+        block.attn.start_pos = 7
+    for step in range(7):
+        x = torch.randn(B, 1, H, generator=g, device="cuda").half()
+        if step == 1:
+            for block in blocks:
+                block.attn.o_proj.qweight.add_(1)
+        if step == 2:
+            for block in blocks:
+                block.mlp.down_proj.scales = block.mlp.down_proj.scales * 0.5
+        if step == 3:
+            for block in blocks:
+                block.attn.REFERENCE_DOUBLE_APPEND = False
+        want = _plain(blocks[0], x)
+        native = fast.awq_block_step(blocks[1], x)
+        # (a layer whose buffers changed is packed again by its own code, a full cache is that code's as well)
+        assert (native is None) == (step in (0, 1, 2) or 7 + step >= rows)
+        got = native if native is not None else blocks[1](x)
+        assert torch.equal(got, want)
+        for name in ("k", "v"):
+            assert torch.equal(getattr(blocks[0].attn.cache, name), getattr(blocks[1].attn.cache, name))
+        assert blocks[0].attn.start_pos == blocks[1].attn.start_pos == 8 + step
+
+
+@pytest.mark.parametrize("how", ["hook", "pre-hook", "global", "instance", "class"])
+@pytest.mark.parametrize("name", ["norm_1", "attn", "attn.qkv_proj", "attn.o_proj"])
+def test_witnesses_of_the_attention_see_their_calls(name, how):
+    if name == "attn" and (how in ("hook", "pre-hook", "global") or how == "class"):
+        pytest.skip("the block takes the attention's forward, not its call; its result is a triple")
+    block, x = _block(), torch.randn(1, 1, H, device="cuda").half()
+    want = _run(block, lambda b, t: b(t), x)
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want)
+    seen = []
+    if name == "attn":
+        forward = type(block.attn).forward
+        block.attn.forward = lambda *a, **k: (seen.append(name), forward(block.attn, *a, **k))[1]
+        assert torch.equal(_run(block, lambda b, t: b(t), x), want) and seen == [name]
+        return
+    with _watch(block, name, how, seen):
+        got = _run(block, lambda b, t: b(t), x)
+        assert seen == [name]
+        assert torch.equal(got, _run(block, _plain, x)) and not torch.equal(got, want)
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want)
+
+
+def test_step_declines_what_it_does_not_cover():
+    from llmqrt_b200._lib import fast
+    block, x = _block(), torch.randn(1, 1, H, device="cuda").half()
+    block.attn.start_pos = 3
+    block(x)
+    takes = lambda t: fast.awq_block_step(block, t) is not None
+    assert takes(x)
+    pos = block.attn.start_pos
+    assert not takes(x.bfloat16()) and not takes(x.expand(1, 2, H)) and not takes(x.expand(2, 1, H)) and not takes(x[0])
+    assert not takes(x.cpu()) and not takes(x.clone().requires_grad_()) and fast.awq_block_step(torch.nn.Linear(2, 2), x) is None
+    block.attn.cache.k = block.attn.cache.k.bfloat16()
+    assert not takes(x)
+    block.attn.cache.k = block.attn.cache.k.half()
+    block.norm_2.weight = block.norm_2.weight.float()
+    assert not takes(x)
+    block.norm_2.weight = block.norm_2.weight.half()
+    block.attn.q_norm = torch.nn.Identity()
+    assert not takes(x)
+    assert block.attn.start_pos == pos
