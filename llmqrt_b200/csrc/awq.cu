@@ -75,15 +75,6 @@ awq_repack_scales_kernel(const __half* __restrict__ scales, const uint32_t* __re
 }
 
 // ---- streaming layout -> W^T[N, K] fp16 -----------------------------------------------------------
-__device__ __forceinline__ void dequant_word(uint32_t w, __half2 negz, __half2 s, uint32_t (&out)[4]) {
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    uint32_t h = ((w >> (4 * p)) & 0x000F000Fu) | 0x64006400u;
-    __half2 v = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&h), negz), s);
-    out[p] = *reinterpret_cast<uint32_t*>(&v);
-  }
-}
-
 // A thread expands kDequantWords words a block's width apart: loads of 128 and stores of 512 contiguous bytes
 // per warp, several of each in flight, 32-bit index arithmetic.  With one word per thread and
 // 64-bit divisions the expansion of 17920 x 1536 (14 MB read, 55 MB written) took 21.5 us; so it takes 13.8.
@@ -107,9 +98,8 @@ awq_dequantize_t_kernel(const uint32_t* __restrict__ wq_t, const uint32_t* __res
   for (int k = 0; k < kDequantWords; ++k) {
     const uint32_t idx = i0 + 256u * k;
     if (idx < total) {
-      const __half2 sz = *reinterpret_cast<const __half2*>(&szv[k]);
       uint32_t o[4];
-      dequant_word(w[k], __half2half2(__high2half(sz)), __half2half2(__low2half(sz)), o);
+      dequant_word(w[k], AwqGroup(szv[k]), o);
       *reinterpret_cast<uint4*>(out + (size_t)idx * 8) = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
@@ -135,10 +125,12 @@ int launch_dequantize_t(const uint32_t* wq_t, const uint32_t* sz_t, int64_t K, i
 // memory, so there are no partials in global memory, no arrival counter and no last block that adds the slices up.
 // Activations (a few rows) come straight from L2, no staging and no barrier before the first weights; the weights of
 // one or two chunks of a warp are in flight together, and 64 registers a thread keep two 512-thread blocks on an SM.
-// Latency-bound: a 17920 x 1536 layer (14 MB) at one token is 2 us of HBM time.  Weights from HBM, against 128-row
-// blocks with the slices of K in separate blocks: 17920 x 1536 at one token 8.0 us (11.1), 1536 x 8960 7.5 (12.1),
-// 2048 x 1536 2.6 (6.0), 3584 x 18944 20.0 (22.5); at 16 tokens 17920 x 1536 13.9 (14.7), 1536 x 8960 11.1 (19.4),
-// 4608 x 3584 8.1 (17.3), 37888 x 3584 46.6 (51.9).
+// Bound by latency where a layer is small, by the instructions of the dequantization where it is large: 37888 x 3584 at one
+// token (11 us of HBM time) issued 39 instructions a packed word, a third of them the division by the group size, in 28.7 us;
+// with a shift in its place and two of a word's four pairs sharing one it takes 26.  us from HBM at 1 / 8 / 16 tokens, before
+// in brackets: 17920 x 1536 7.7 / 8.0 / 11.3 (8.2 / 9.8 / 14.0), 1536 x 8960 7.1 / 7.3 / 10.2 (7.6 / 7.8 / 11.1), 8192 x 4096
+// 9.2 / 10.1 / 14.9 (11.7 / 12.5 / 17.2), 2048 x 1536 2.4 / 2.5 / 3.1 (2.5 / 2.7 / 3.2), 3584 x 18944 18.5 / 18.7 / 27.5
+// (19.8 / 20.6 / 30).  (Chunks fetched in a ring instead of in twos do not fit 64 registers: 17920 x 1536 9.5 us.)
 constexpr int kChunkK = 128;           // k-values per warp step: 4 lanes x 32 per weight row
 //
 // What follows the GEMM in a decoder block may be done on its sums (each step rounded to fp16 as the separate kernels
@@ -148,7 +140,7 @@ enum RowsTail { TAIL_NONE, TAIL_RESIDUAL, TAIL_SILU };
 template <int MB, int TAIL>
 __global__ void __launch_bounds__(512, MB <= 2 ? 2 : 1)
 awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* __restrict__ wq_t,
-                     const uint32_t* __restrict__ sz_t, int M, int N, int K, int G, int chunks, Epilogue epi,
+                     const uint32_t* __restrict__ sz_t, int M, int N, int K, int G, int gshift, int chunks, Epilogue epi,
                      const __half* __restrict__ residual, int64_t ldr) {
   extern __shared__ __align__(16) float red[];         // [warp][token][16 rows]
   pdl_wait_then_trigger();
@@ -156,7 +148,15 @@ awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* 
   const int warps = blockDim.x >> 5, n0 = blockIdx.x * (TAIL == TAIL_SILU ? 8 : 16);
   const int KW = K / 8, KG = K / G;
   const int second = TAIL == TAIL_SILU ? N / 2 : 8;    // (N / 2 is a multiple of eight: whole blocks)
-  const int rows[2] = {min(n0 + g, N - 1), min(n0 + g + second, N - 1)};
+  // This lane's 32 values of a chunk, which lie in one group: of weight rows g and g + 8, and of tokens mb * 8 + g.
+  const uint32_t *wp[2], *zp[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int64_t row = min(n0 + g + (r ? second : 0), N - 1);
+    wp[r] = wq_t + row * KW + 4 * t;
+    zp[r] = sz_t + row * KG;
+  }
+  const __half* xp = X + (int64_t)g * ldx + 32 * t;
   // (16 tokens: one chunk ahead, so that 64 registers nearly do -- 8 to 16 bytes are spilled; 17920 x 1536 13.9 us, 16.4
   // with two)
   constexpr int kRowsAhead = MB == 2 ? 1 : 2;
@@ -170,40 +170,38 @@ awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* 
     uint32_t sz[kRowsAhead][2];
 #pragma unroll
     for (int i = 0; i < kRowsAhead; ++i) {
-      const int kk = (c0 + i * warps) * kChunkK + 32 * t;      // this lane's 32 values of the chunk: one group
-      const bool valid = kk < K;
+      const int c = c0 + i * warps, kk = c * kChunkK + 32 * t;
+      const int gi = gshift >= 0 ? kk >> gshift : kk / G;
+      const bool valid = kk < K;                               // (K is a multiple of 32)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         w[i][r] = make_uint4(0u, 0u, 0u, 0u);
         sz[i][r] = 0u;                                         // scale 0: contributes nothing
         if (valid) {
-          w[i][r] = ldg_stream_16B(wq_t + (int64_t)rows[r] * KW + kk / 8);
-          sz[i][r] = __ldg(sz_t + (int64_t)rows[r] * KG + kk / G);
+          w[i][r] = ldg_stream_16B(wp[r] + c * (kChunkK / 8));
+          sz[i][r] = __ldg(zp[r] + gi);
         }
       }
     }
 #pragma unroll
     for (int i = 0; i < kRowsAhead; ++i) {
-      if (c0 + i * warps >= chunks) break;
-      const int kk = (c0 + i * warps) * kChunkK + 32 * t;
-      uint4 x[MB][4];                                          // tokens mb * 8 + g
+      const int c = c0 + i * warps;
+      if (c >= chunks) break;
+      uint4 x[MB][4];
 #pragma unroll
       for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
         for (int wi = 0; wi < 4; ++wi) {
-          x[mb][wi] = make_uint4(0u, 0u, 0u, 0u);
-          if (kk < K && mb * 8 + g < M)
-            x[mb][wi] = *reinterpret_cast<const uint4*>(X + (int64_t)(mb * 8 + g) * ldx + kk + 8 * wi);
+          if (c * kChunkK + 32 * t < K && mb * 8 + g < M) x[mb][wi] = *reinterpret_cast<const uint4*>(xp + mb * 8 * ldx + c * kChunkK + 8 * wi);
+          else x[mb][wi] = make_uint4(0u, 0u, 0u, 0u);
         }
       const uint32_t wr[2][4] = {{w[i][0].x, w[i][0].y, w[i][0].z, w[i][0].w}, {w[i][1].x, w[i][1].y, w[i][1].z, w[i][1].w}};
+      const AwqGroup grp[2] = {AwqGroup(sz[i][0]), AwqGroup(sz[i][1])};
 #pragma unroll
       for (int wi = 0; wi < 4; ++wi) {
         uint32_t a[2][4];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const __half2 s2 = *reinterpret_cast<const __half2*>(&sz[i][r]);
-          dequant_word(wr[r][wi], __half2half2(__high2half(s2)), __half2half2(__low2half(s2)), a[r]);
-        }
+        for (int r = 0; r < 2; ++r) dequant_word(wr[r][wi], grp[r], a[r]);
 #pragma unroll
         for (int mb = 0; mb < MB; ++mb) {
           mma_16816<false>(acc[mb], a[0][0], a[1][0], a[0][1], a[1][1], x[mb][wi].x, x[mb][wi].y);
@@ -248,27 +246,31 @@ template <int MB, int TAIL = TAIL_NONE>
 int launch_rows(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32_t* sz_t, int M, int N, int K, int G,
                 const Epilogue& epi, cudaStream_t st, const __half* residual, int64_t ldr) {
   const int blocks = (int)ceil_div(N, 16), chunks = (int)ceil_div(K, kChunkK);
-  // warps per block: about 40 per SM in all, at least four, at most one per chunk
-  int warps = (int)ceil_div(40 * sm_count(), blocks);
-  warps = warps < 4 ? 4 : warps > 16 ? 16 : warps;
+  // Warps per block: as many as leave all blocks resident at once (64 registers a thread make 32 warps an SM, 128 make
+  // 16), two to sixteen, at most one per chunk of K.  About 40 an SM in all, as it was, took a second wave for a few blocks:
+  // 17920 x 1536 at one token 8.7 us with six warps, 7.6 with four; 9728 x 896 5.4 (7), 4.1 (6); 8192 x 4096 10.7 (12), 8.7 (8).
+  const int resident = MB <= 2 ? 32 : 16;
+  int warps = resident / (int)ceil_div(blocks, sm_count());
+  warps = warps < 2 ? 2 : warps > 16 ? 16 : warps;
   if (warps > chunks) warps = chunks;
+  const int gshift = (G & (G - 1)) == 0 ? __builtin_ctz((unsigned)G) : -1;
   if (int rc = launch_chained(awq_gemm_rows_kernel<MB, TAIL>, dim3((unsigned)blocks), dim3((unsigned)(32 * warps)), (size_t)warps * MB * 512, st, 1,
-                              X, ldx, wq_t, sz_t, M, N, K, G, chunks, epi, residual, ldr))
+                              X, ldx, wq_t, sz_t, M, N, K, G, gshift, chunks, epi, residual, ldr))
     return rc;
   return check_launch("awq_gemm_rows");
 }
 
 // 9 to 32 tokens: every block fetches all activations, so the time of this file's kernel goes with the blocks on an SM x
 // tokens x K, while the tcgen05 kernel takes the same time for any of them.  us at 9 / 16 / 17 / 24 / 32 tokens (tcgen05):
-//   1536 x 1536 3.3 / 3.3 / 3.9 / 4.6 / 5.0 (8.8)      4608 x 3584 7.0 / 8.3 / 12.0 / 13.7 / 15.4 (13.8)
-//   17920 x 1536 10.8 / 14.0 / 19 / 22 / 26 (13)       3584 x 18944 27 / 30 / 38 / 43 / 52 (29)
-//   37888 x 3584 38 / 45 / 58 / 69 / 84 (38)           9728 x 896 5.8 / 6.9 / 9.4 / 10.8 / 12.7 (9.0)
-// The estimates are fitted to N = 896 .. 37888, K = 896 .. 18944; the kernel they choose is more than 4 % slower than the
-// other in 10 of 245 measured cases (6144 x 3584 at 24 tokens: 19.0 against 16.4).
+//   1536 x 1536 2.7 / 3.1 / 3.9 / 4.3 / 4.9 (8.8)      4608 x 3584 6.4 / 8.0 / 9.4 / 11.1 / 12.9 (13.8)
+//   17920 x 1536 8.9 / 11.3 / 15 / 17 / 20 (12.2)      5120 x 4096 10.0 / 12.3 / 15 / 18 / 21 (13.9)
+//   27648 x 2560 22 / 31 / 37 / 44 / 54 (28)           37888 x 3584 33 / 41 / 50 / 60 / 75 (37)
+// The estimates are fitted to N = 896 .. 37888, K = 896 .. 13824; the kernel they choose is more than 4 % slower than the
+// other in 21 of 516 measured cases, mostly by 10 to 15 % (12 tokens of 17920 rows, 17 to 24 of 12288).
 bool rows_suit(int64_t M, int64_t N, int64_t K) {
   const double blocks = (double)ceil_div(ceil_div(N, (int64_t)16), (int64_t)sm_count()), k = 1e-3 * (double)K;
-  const double us = M <= 16 ? 1.7 + blocks * (0.27 + k * (0.367 + 0.0315 * (double)M))
-                            : 1.75 + blocks * (0.84 + k * (0.485 + 0.0298 * (double)M));
+  const double us = M <= 16 ? 2.1 + blocks * (0.07 + k * (0.358 + 0.0240 * (double)M))
+                            : 2.3 + blocks * (0.24 + k * (0.316 + 0.0323 * (double)M));
   return us < awq_tc_us(M, N, K, nullptr);
 }
 

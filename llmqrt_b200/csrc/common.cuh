@@ -239,6 +239,31 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
   return r;
 }
 
+// One quantization group of a repacked 4-bit layer: {scale, -(1024 + zero)} of its word, spread over pairs.
+struct AwqGroup {
+  __half2 s, negz, negz64;
+  __device__ __forceinline__ explicit AwqGroup(uint32_t word) {
+    const __half2 v = *reinterpret_cast<const __half2*>(&word);
+    s = __half2half2(__low2half(v));
+    negz = __half2half2(__high2half(v));
+    negz64 = __hadd2(negz, __float2half2_rn(960.f));          // -(64 + zero)
+  }
+};
+// Eight 4-bit values (pair p in nibbles p and p + 4) -> four pairs fp16((v - zero) * scale).  A nibble v in the mantissa of
+// 1024 is 1024 + v, or 1024 + 16 v one nibble higher, and both differences come out exactly, the second by a multiply-add
+// with 1/16: two pairs share a shift.
+__device__ __forceinline__ void dequant_word(uint32_t w, const AwqGroup& g, uint32_t (&out)[4]) {
+  const __half2 sixteenth = __float2half2_rn(0.0625f);
+#pragma unroll
+  for (int p = 0; p < 4; p += 2) {
+    const uint32_t wp = w >> (4 * p), lo = (wp & 0x000F000Fu) | 0x64006400u, hi = (wp & 0x00F000F0u) | 0x64006400u;
+    const __half2 a = __hmul2(__hadd2(*reinterpret_cast<const __half2*>(&lo), g.negz), g.s);
+    const __half2 b = __hmul2(__hfma2(*reinterpret_cast<const __half2*>(&hi), sixteenth, g.negz64), g.s);
+    out[p] = *reinterpret_cast<const uint32_t*>(&a);
+    out[p + 1] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+}
+
 // silu of two values of type T, x / (1 + e^-x) in fp32: rounded to T, the bits of that expression with the library's
 // exponential and a true division, for every one of T's 65536 values.  The divisor is carried as (1 + e^-x) / 4, whose
 // reciprocal is a normal number while e^-x is finite.

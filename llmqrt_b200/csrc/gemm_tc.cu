@@ -708,14 +708,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         const uint32_t words[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
         uint32_t o[32];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const __half2 sz = *reinterpret_cast<const __half2*>(&szv[d][j >> 2]);
-          const __half2 negz = __half2half2(__high2half(sz)), sc = __half2half2(__low2half(sz));
+        for (int half = 0; half < 2; ++half) {
+          const AwqGroup grp_sz(szv[d][half]);
 #pragma unroll
-          for (int p4 = 0; p4 < 4; ++p4) {
-            uint32_t h = ((words[j] >> (4 * p4)) & 0x000F000Fu) | 0x64006400u;           // {1024 + v[2p], 1024 + v[2p+1]}
-            const __half2 v2 = __hmul2(__hadd2(*reinterpret_cast<__half2*>(&h), negz), sc);
-            o[4 * j + p4] = *reinterpret_cast<const uint32_t*>(&v2);
+          for (int j = 4 * half; j < 4 * half + 4; ++j) {
+            uint32_t pairs[4];
+            dequant_word(words[j], grp_sz, pairs);
+#pragma unroll
+            for (int p4 = 0; p4 < 4; ++p4) o[4 * j + p4] = pairs[p4];
           }
         }
         tc::mbar_wait_or_flag(tc::smem_u32(&bar_empty[ws]), w_phase ^ 1u, abort_u32);
@@ -1455,7 +1455,7 @@ int launch_bn(int bn, const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CU
 }
 
 // Estimated microseconds of the kernel that dequantizes its weights, fitted to times over N = 896 .. 37888, K = 896 .. 18944:
-// up to 64 tokens, and above 128 with the tokens in panels of 128 or (*panels = false) in tiles of 256.
+// up to 32 tokens, and above 128 with the tokens in panels of 128 or (*panels = false) in tiles of 256.
 double awq_split_us(int64_t tiles, int k_blocks, int most, int (*active)(int), double base, double kb, double tile, double exchange) {
   int waves;
   const int s = pick_splits(tiles, k_blocks, most, active, &waves);
@@ -1477,7 +1477,7 @@ double awq_tc_us(int64_t M, int64_t N, int64_t K, bool* panels) {
   const int kb = (int)ceil_div(K, (int64_t)64);
   const int64_t tiles = ceil_div(N, (int64_t)kBM);
   if (M <= 128)
-    return awq_split_us(tiles, kb, 8, max_active_clusters<tc::MMA_F16, 64, true>, 2.4, 0.324, 2.2, 3.8);
+    return awq_split_us(tiles, kb, 8, max_active_clusters<tc::MMA_F16, 64, true>, 1.2, 0.294, 2.4, 4.3);
   const double p = awq_split_us(tiles * ceil_div(M, (int64_t)128), kb, 16, max_active_clusters<tc::MMA_F16, 128, true>,
                                 5.7, 0.28, 4.3, 3.7);
   const double t = (double)ceil_div(tiles * ceil_div(M, (int64_t)256), (int64_t)sm_count()) * (0.327 * kb + 14.2);
@@ -1538,9 +1538,11 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   prm.early_w = static_w ? 1 : 0;
   prm.swap = (M <= 128 || panels) ? 1 : 0;
   int bn;
-  // (4-bit weights: 64 columns also for few tokens, so that the reduction may be split in eight instead of four)
-  if (prm.swap) bn = M <= 32 && !awq ? 32 : (M <= 64 ? 64 : 128);
+  if (prm.swap) bn = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   else bn = N <= 128 ? 128 : 256;
+  // 4-bit weights: a reduction that is better split in more than four has 64 columns also for few tokens.  (Otherwise not: with
+  // three quarters of a 64-column box beyond the tokens, 16 tokens of 37888 x 3584 took 38 or 56 us, by where x lay; 37 in 32.)
+  if (awq && M <= 32 && pick_splits(ceil_div(N, (int64_t)kBM), k_blocks, 8, max_active_clusters<tc::MMA_F16, 64, true>, nullptr) > 4) bn = 64;
   if (awq && !prm.swap) {
     // AWQ with many tokens: the weights stay the 128-lane operand and the tokens come in tiles of 256.
     // A dequantized weight tile (the expensive operand: it is produced by arithmetic, not by a copy)
