@@ -76,7 +76,6 @@ struct TcParams {
   // Row-parallel output under tensor parallelism: instead of going to `out`, the 16-bit results are
   // stored as the tagged words of the NEXT all-reduce call into the peers' buffers (peer_comm.cuh);
   // the row kernel that consumes the sum then only gathers.
-  int store32;                     // two-CTA kernel: output rows are 32-byte aligned, 256-bit stores may be used
   int comm_on, comm_threads, comm_two_step;
   CommDev comm;
 };
@@ -914,26 +913,40 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
 // Each CTA's tensor memory receives its 128 accumulator rows (2 x 256 columns, double buffered).
 //   producer (warp 0, both CTAs): TMA loads whose bytes are counted on the LEADER's `full` barrier
 //   MMA issuer (warp 1, leader only): 4 MMAs per stage, commits fan out to both CTAs' barriers
-//   epilogue (warps 2-9, both CTAs): TMEM -> registers -> scales / bias -> global memory, 64 or 128
-//     contiguous bytes per thread and step straight from registers (a staged TMA store was measured
-//     three times slower with one staging tile: its completion latency of a few microseconds
-//     serialises the chunks, and shared memory has no room for a deeper staging ring next to six stages)
+//   epilogue (warps 2-9, both CTAs): TMEM -> registers -> scales / bias -> a staging tile of the warp's own, 32 rows of
+//     128 bytes, which leaves by a TMA store (rows and columns beyond the matrix are clipped).  A thread that writes its
+//     own row straight from registers makes the warp touch 32 lines with every store: 5130 cycles a tile, against 3584
+//     of its seven K blocks at K = 896 (4096 x 4864 x 896 in int8 25.4 us, 23.2 this way).  (With one staging tile
+//     for all warps the completion of a store serialises the tiles.)
 constexpr int kPairBN = 256;
 constexpr int kPairHalfB = kPairBN / 2;
 constexpr int kPairStageBytes = (kBM + kPairHalfB) * kRowBytes;         // 32 KiB
 constexpr int kPairStages = 6;
-constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 1024;
+constexpr int kPairOutBytes = 32 * 128;                                // staging tile of an epilogue warp
+struct PairShared {                                                    // (one struct: static arrays and a margin for its alignment do not fit)
+  uint8_t tiles[kPairStages * kPairStageBytes];
+  uint8_t out[8 * kPairOutBytes];
+  float q_scale[kPairBN], q_bias[kPairBN];
+  uint64_t bar_full[kPairStages];      // used in the leader only
+  uint64_t bar_empty[kPairStages];
+  uint64_t bar_acc_full[2];
+  uint64_t bar_acc_empty[2];           // used in the leader only: one arrival per CTA
+  uint32_t tmem_base_slot;
+  int abort_flag;
+};
+constexpr int kPairSmemBytes = sizeof(PairShared);
+static_assert(kPairSmemBytes <= 227 * 1024, "a block has 227 KiB of shared memory");
 constexpr uint32_t kPairTmemCols = 2 * kPairBN;
 constexpr int kPairThreads = 64 + 256;                                 // producer warp, MMA warp, eight epilogue warps
 __device__ __forceinline__ void pair_epi_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// 32 bytes from registers to global memory in one instruction (the address must be 32-byte aligned): half
-// the store instructions, and every lane writes a whole 32-byte sector.
-__device__ __forceinline__ void st_global_256(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
-                                              uint32_t f, uint32_t g, uint32_t h) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e),
-               "r"(f), "r"(g), "r"(h) : "memory");
+// A 2-D tile from shared memory to global memory; the issuing thread's stores are counted in bulk groups.
+__device__ __forceinline__ void tma_store_2d(const void* tensor_map, uint32_t src_smem, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n\t"
+               "cp.async.bulk.commit_group;" ::"l"(tensor_map), "r"(src_smem), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_stores_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Tile order: the weight tiles are walked in groups of kPairGroup; inside a group the token tile
 // changes fastest.  The clusters that run at the same time then share a few weight tiles and a few
@@ -951,18 +964,17 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_p, int tile
 
 template <int KIND>
 __global__ void __launch_bounds__(kPairThreads, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, TcParams prm) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
+                    const __grid_constant__ CUtensorMap tm_out, TcParams prm) {
   using AccT = typename std::conditional<KIND == tc::MMA_I8, int, float>::type;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t bar_full[kPairStages];      // used in the leader only
-  __shared__ __align__(8) uint64_t bar_empty[kPairStages];
-  __shared__ __align__(8) uint64_t bar_acc_full[2];
-  __shared__ __align__(8) uint64_t bar_acc_empty[2];           // used in the leader only: one arrival per CTA
-  __shared__ __align__(16) float q_scale[kPairBN];
-  __shared__ __align__(16) float q_bias[kPairBN];
-  __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag;
+  extern __shared__ __align__(1024) uint8_t smem_pair[];       // (the swizzle and the descriptors assume 1024-byte alignment)
+  PairShared& sh = *reinterpret_cast<PairShared*>(smem_pair);
+  uint8_t* tiles = sh.tiles;
+  auto& bar_full = sh.bar_full; auto& bar_empty = sh.bar_empty;
+  auto& bar_acc_full = sh.bar_acc_full; auto& bar_acc_empty = sh.bar_acc_empty;
+  auto& q_scale = sh.q_scale; auto& q_bias = sh.q_bias;
+  auto& tmem_base_slot = sh.tmem_base_slot;
+  int& abort_flag = sh.abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort = &abort_flag;
@@ -983,6 +995,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     tc::mbar_fence_init();
     tc::tma_prefetch_descriptor(&tm_a);
     tc::tma_prefetch_descriptor(&tm_w);
+    tc::tma_prefetch_descriptor(&tm_out);
   }
   if (warp == 1) {
     tc::tmem_alloc_pair(tc::smem_u32(&tmem_base_slot), kPairTmemCols);
@@ -1024,29 +1037,33 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader) {                                      // (the whole warp: see the single-CTA kernel)
       int stage_i = 0;
       uint32_t phase = 0;
       uint32_t acc_phase[2] = {0, 0};
       int buf = 0;
       for (int tile = first_tile; tile < num_tiles; tile += tile_step) {
-        if (!tc::mbar_wait(tc::smem_u32(&bar_acc_empty[buf]), acc_phase[buf] ^ 1u, abort)) break;
+        if (!tc::mbar_wait_warp(tc::smem_u32(&bar_acc_empty[buf]), acc_phase[buf] ^ 1u, abort)) break;
         tc::fence_after_sync();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kPairBN);
         for (int it = 0; it < kb_count; ++it) {
           tc::mbar_wait_or_flag(tc::smem_u32(&bar_full[stage_i]), phase, abort_u32);
+          __syncwarp();
           const uint32_t sp = tc::smem_u32(tiles + stage_i * kPairStageBytes);
           const uint64_t da = tc::smem_desc_k_major_sw128(sp);
           const uint64_t db = tc::smem_desc_k_major_sw128(sp + kBM * kRowBytes);
+          if (tc::elect_one()) {
 #pragma unroll
-          for (int j = 0; j < kRowBytes / 32; ++j)
-            tc::mma_ss_pair<KIND>(d_tmem, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), prm.idesc,
-                                  (it > 0 || j > 0) ? 1u : 0u);
-          tc::mma_commit_pair(tc::smem_u32(&bar_empty[stage_i]));      // frees the stage in both CTAs
+            for (int j = 0; j < kRowBytes / 32; ++j)
+              tc::mma_ss_pair<KIND>(d_tmem, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), prm.idesc,
+                                    (it > 0 || j > 0) ? 1u : 0u);
+            tc::mma_commit_pair(tc::smem_u32(&bar_empty[stage_i]));    // frees the stage in both CTAs
+          }
+          __syncwarp();
           if (++stage_i == kPairStages) { stage_i = 0; phase ^= 1u; }
         }
         if (*abort) break;
-        tc::mma_commit_pair(tc::smem_u32(&bar_acc_full[buf]));          // accumulators complete in both CTAs
+        if (tc::elect_one()) tc::mma_commit_pair(tc::smem_u32(&bar_acc_full[buf]));          // accumulators complete in both CTAs
         acc_phase[buf] ^= 1u;
         buf ^= 1;
       }
@@ -1066,7 +1083,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     const bool bf16 = e.out_dtype == LLMQRT_BF16;
     const bool has_bias = e.bias != nullptr;
     const bool col_first = e.mode == EPI_COL_ROW;                       // (acc * col_scale) * row_scale
-    const int es = wide ? 4 : 2;
+    uint8_t* out_tile = sh.out + (warp - 2) * kPairOutBytes;
     const float alpha = e.alpha_dev ? *e.alpha_dev : e.alpha;
     const float bmul = tensor ? e.beta : 1.f;
     const uint32_t acc_empty0 = tc::cluster_addr(tc::smem_u32(&bar_acc_empty[0]), 0u);
@@ -1095,11 +1112,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       acc_phase[buf] ^= 1u;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * kPairBN + half * 128);
       const int ncols = min(128, prm.N - tq * kPairBN - half * 128);    // my columns inside the matrix (may be <= 0)
-      uint8_t* orow = reinterpret_cast<uint8_t*>(e.out) + ((int64_t)row * e.ldo + (int64_t)tq * kPairBN + half * 128) * es;
-      // 32 accumulator columns per step; the load of the next step is issued before this step's
-      // arithmetic and stores so that its latency is hidden.  A thread owns 32 consecutive outputs of
-      // one row (64 or 128 contiguous bytes) and writes them straight from registers: fire-and-forget
-      // stores, nothing to wait for, the accumulator buffer is free as soon as the last load is back.
+      // 32 accumulator columns per step; the load of the next step is issued before this step's arithmetic so that its
+      // latency is hidden.  The staging tile holds one step of 32-bit or two of 16-bit outputs, 16-byte unit u of row r at
+      // u ^ (r & 7); the accumulator buffer is free as soon as the last load is back.
+      const int row0 = row - lane, x0 = tq * kPairBN + half * 128;
       uint32_t r[2][32];
       if (ncols > 0) tc::tmem_ld_32x32(taddr, r[0]);
 #pragma unroll 1
@@ -1167,38 +1183,25 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
               }
             }
           }
-          if (row_ok) {
-            if (wide) {                                // v[0..32): 32-bit outputs
-              if (c + 32 <= ncols && prm.store32) {
+          const bool first = wide || h == 0, last = wide || h == 1 || c + 32 >= ncols;
+          if (first) {                                   // the store before has read the tile
+            if (lane == 0) tma_stores_read();
+            __syncwarp();
+          }
+          uint8_t* dst = out_tile + lane * 128;
+          if (wide) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  st_global_256(orow + c * 4 + 32 * k, v[8 * k], v[8 * k + 1], v[8 * k + 2], v[8 * k + 3], v[8 * k + 4],
-                                v[8 * k + 5], v[8 * k + 6], v[8 * k + 7]);
-              } else if (c + 32 <= ncols) {
+            for (int k = 0; k < 8; ++k)
+              *reinterpret_cast<uint4*>(dst + ((k ^ (lane & 7)) << 4)) = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          } else {
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                  reinterpret_cast<uint4*>(orow + c * 4)[k] = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-              } else {
-#pragma unroll
-                for (int jj = 0; jj < 32; ++jj)
-                  if (c + jj < ncols) reinterpret_cast<uint32_t*>(orow + c * 4)[jj] = v[jj];
-              }
-            } else {                                   // v[0..16): pairs of 16-bit outputs
-              if (c + 32 <= ncols && prm.store32) {
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                  st_global_256(orow + c * 2 + 32 * k, v[8 * k], v[8 * k + 1], v[8 * k + 2], v[8 * k + 3], v[8 * k + 4],
-                                v[8 * k + 5], v[8 * k + 6], v[8 * k + 7]);
-              } else if (c + 32 <= ncols) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  reinterpret_cast<uint4*>(orow + c * 2)[k] = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-              } else {
-#pragma unroll
-                for (int jj = 0; jj < 32; ++jj)
-                  if (c + jj < ncols) reinterpret_cast<uint16_t*>(orow + c * 2)[jj] = (uint16_t)(v[jj >> 1] >> (16 * (jj & 1)));
-              }
-            }
+            for (int k = 0; k < 4; ++k)
+              *reinterpret_cast<uint4*>(dst + (((4 * h + k) ^ (lane & 7)) << 4)) = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          }
+          if (last) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // generic writes -> TMA reads
+            __syncwarp();
+            if (lane == 0 && row0 < prm.M) tma_store_2d(&tm_out, tc::smem_u32(out_tile), x0 + (wide ? c : c0), row0);
           }
         }
       }
@@ -1208,6 +1211,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       if (issuer) tc::mbar_arrive_cluster(acc_empty0 + (uint32_t)buf * 8u);
       buf ^= 1;
     }
+    if (lane == 0) tma_stores_done();
   }
 
   // ------------------------------- teardown ---------------------------------------
@@ -1258,6 +1262,21 @@ int make_operand_map(CUtensorMap* map, const void* base, int elt_bytes, int64_t 
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return set_error(LLMQRT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return LLMQRT_OK;
+}
+
+// 2-D output [rows, cols] with `ld` elements between rows; box = 128 bytes x 32 rows, the two-CTA kernel's staging tile.
+int make_output_map(CUtensorMap* map, void* base, int elt_bytes, int64_t rows, int64_t cols, int64_t ld) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return set_error(LLMQRT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld * elt_bytes)};
+  cuuint32_t box[2] = {(cuuint32_t)(128 / elt_bytes), 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, elt_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, base, dims, strides, box,
+                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(LLMQRT_ERR_CUDA, "cuTensorMapEncodeTiled (output) failed with code %d", (int)r);
   return LLMQRT_OK;
 }
 
@@ -1415,7 +1434,7 @@ int pair_max_clusters() {
 }
 
 template <int KIND>
-int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const TcParams& prm, cudaStream_t st) {
+int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const CUtensorMap& tm_out, const TcParams& prm, cudaStream_t st) {
   auto kern = gemm_tc_pair_kernel<KIND>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kPairSmemBytes)) return rc;
   int clusters = pair_max_clusters<KIND>();
@@ -1439,7 +1458,7 @@ int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const TcParams
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 2;
   }
-  LLMQRT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm_a, tm_w, prm));
+  LLMQRT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm_a, tm_w, tm_out, prm));
   return check_launch("gemm_tc_pair");
 }
 
@@ -1579,13 +1598,13 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
     prm.tiles_p = (int)ceil_div(M, (int64_t)(2 * kBM));
     prm.tiles_q = (int)ceil_div(N, (int64_t)kPairBN);
     prm.idesc = tc::instr_desc(c_fmt, fmt_act, fmt_w, 2 * kBM, kPairBN);
-    prm.store32 = ((reinterpret_cast<uintptr_t>(epi.out) & 31) == 0 && (epi.ldo * es) % 32 == 0) ? 1 : 0;
-    CUtensorMap tm_a, tm_w;
+    CUtensorMap tm_a, tm_w, tm_out;
     if (int rc = make_operand_map(&tm_a, A, elt, M, K, lda, kBM)) return rc;
     if (int rc = make_operand_map(&tm_w, W, elt, N, K, ldw, kPairHalfB)) return rc;
-    if (mk == tc::MMA_I8) return launch_pair<tc::MMA_I8>(tm_a, tm_w, prm, st);
-    if (mk == tc::MMA_F8) return launch_pair<tc::MMA_F8>(tm_a, tm_w, prm, st);
-    return launch_pair<tc::MMA_F16>(tm_a, tm_w, prm, st);
+    if (int rc = make_output_map(&tm_out, epi.out, es, M, N, epi.ldo)) return rc;
+    if (mk == tc::MMA_I8) return launch_pair<tc::MMA_I8>(tm_a, tm_w, tm_out, prm, st);
+    if (mk == tc::MMA_F8) return launch_pair<tc::MMA_F8>(tm_a, tm_w, tm_out, prm, st);
+    return launch_pair<tc::MMA_F16>(tm_a, tm_w, tm_out, prm, st);
   }
   prm.idesc = tc::instr_desc(c_fmt, prm.swap ? fmt_w : fmt_act, prm.swap ? fmt_act : fmt_w, kBM, (uint32_t)bn);
 

@@ -328,3 +328,30 @@ def test_gemm_rejects_bad_arguments(ops):
         ops.int8_gemm_s32(a, w)
     with pytest.raises(RuntimeError, match="CUDA"):
         ops.int8_gemm_s32(a.cpu(), w.cpu())
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 136, 64), (257, 264, 896), (300, 1000, 3584), (544, 72 + 256, 128), (1056, 2056, 528)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_two_cta_stores_are_clipped(ops, M, N, K, wide):
+    """The two-CTA kernel's tiles of 32 rows x 128 bytes at the matrix' edges, in 16 and 32 bits: results to the last row and
+    column, and not a byte beyond them (rows of a wider buffer, more rows behind)."""
+    from llmqrt_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    acc = (a.double() @ w.double().t())
+    ld = N + 24
+    dev = a.device
+    if wide:
+        buf = torch.full((M + 40, ld), 12345678, dtype=torch.int32, device="cuda")
+        L.call("llmqrt_w8a8_int8_gemm_s32", L.ptr(a), K, L.ptr(w), K, L.ptr(buf), ld, M, N, K, L.ptr(L.workspace(dev)), L.stream(dev), 0)
+        want = acc.to(torch.int32)
+    else:
+        xs = torch.rand(M, generator=g, device="cuda") + 0.5
+        ws = (torch.rand(N, generator=g, device="cuda") + 0.5) * 1e-3
+        buf = torch.full((M + 40, ld), 77.0, dtype=torch.bfloat16, device="cuda")
+        L.call("llmqrt_w8a8_int8_linear_per_channel", L.ptr(a), K, L.ptr(w), K, None, L.BF16, L.ptr(xs), L.ptr(ws), L.ptr(buf),
+               L.BF16, ld, M, N, K, L.ptr(L.workspace(dev)), L.stream(dev), 0)
+        want = ((acc.float() * ws) * xs[:, None]).bfloat16()          # float(acc) is exact here or rounded once, as in the kernel
+    assert torch.equal(buf[:M, :N], want)
+    assert bool((buf[:M, N:] == buf[-1, -1]).all()) and bool((buf[M:] == (12345678 if wide else 77.0)).all())
