@@ -355,3 +355,18 @@ def test_two_cta_stores_are_clipped(ops, M, N, K, wide):
         want = ((acc.float() * ws) * xs[:, None]).bfloat16()          # float(acc) is exact here or rounded once, as in the kernel
     assert torch.equal(buf[:M, :N], want)
     assert bool((buf[:M, N:] == buf[-1, -1]).all()) and bool((buf[M:] == (12345678 if wide else 77.0)).all())
+
+
+@pytest.mark.parametrize("M,K", [(1, 8), (64, 4864), (333, 3584), (592, 2048), (593, 2048), (1184, 2048), (1187, 4104), (4096, 8960)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_per_tensor_quantizers_of_every_size(ops, M, K, dt):
+    """One, two, four and more units of eight per thread, and grids that end in the middle of a pass, against the torch ops."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn(M, K, generator=g, device="cuda").to(dt)
+    x.view(-1)[-1] = 9.5                                     # the maximum lies in the last unit
+    s = x.abs().amax().clamp(min=1e-5).div(127)
+    q, _, scale = ops.quantize_int8(x, per_token=False)
+    assert torch.equal(q, (x / s).round().clamp(-128, 127).to(torch.int8)) and float(scale) == float(s)
+    s = x.abs().amax().clamp(min=1e-12).div(448)
+    q, scale = ops.quantize_fp8(x, per_token=False)[:2]
+    assert torch.equal(q.view(torch.uint8), (x / s).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8))
