@@ -340,8 +340,8 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   // More than 128 tokens: the weights may be expanded panel by panel into the workspace (same rounding:
   // fp16((v - z) * s)) and each panel multiplied by the dense kernel, which reads an expanded tile again for every 256
   // tokens; the kernel that dequantizes its own tiles makes each of them again for every 256 tokens.  Expanded against fused
-  // us at 256 / 512 / 1024 tokens: 17920 x 1536 26 / 34 / 56 (25 / 46 / 87), 4608 x 3584 28 / 30 / 31 (22 / 33 / 36), 3584 x 18944
-  // 86 / 117 / 135 (57 / 104 / 123), 37888 x 3584 139 / 187 / 268 (71 / 167 / 265), 9728 x 896 15 / 19 / 25 (21 / 37 / 54).  The
+  // us at 256 / 512 / 1024 tokens: 17920 x 1536 26 / 34 / 53 (25 / 46 / 86), 4608 x 3584 22 / 23 / 32 (22 / 27 / 36), 3584 x 18944
+  // 88 / 90 / 132 (58 / 96 / 119), 37888 x 3584 129 / 169 / 255 (68 / 132 / 269), 9728 x 896 15 / 19 / 24 (21 / 32 / 51).  The
   // estimates choose; a twelfth in favour of the expansion is what they are off by.  (Panels of 64 MB, which would stay in L2, are
   // worse: 113 us for 3584 x 18944 at 256.)  Above 1024 tokens it is always expanded.
   if (M > 128 && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0 &&

@@ -919,24 +919,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
 //     of its seven K blocks at K = 896 (4096 x 4864 x 896 in int8 25.4 us, 23.2 this way).  (With one staging tile
 //     for all warps the completion of a store serialises the tiles.)
 constexpr int kPairBN = 256;
-constexpr int kPairHalfB = kPairBN / 2;
-constexpr int kPairStageBytes = (kBM + kPairHalfB) * kRowBytes;         // 32 KiB
-constexpr int kPairStages = 6;
+constexpr int kPairNarrowBN = 128;      // where tiles of 256 columns leave most SMs idle: see pair_us
+template <int BN> constexpr int pair_stage_bytes() { return (kBM + BN / 2) * kRowBytes; }      // 32 or 24 KiB
+template <int BN> constexpr int pair_stages() { return BN == kPairBN ? 6 : 8; }
 constexpr int kPairOutBytes = 32 * 128;                                // staging tile of an epilogue warp
+template <int BN>
 struct PairShared {                                                    // (one struct: static arrays and a margin for its alignment do not fit)
-  uint8_t tiles[kPairStages * kPairStageBytes];
+  uint8_t tiles[pair_stages<BN>() * pair_stage_bytes<BN>()];
   uint8_t out[8 * kPairOutBytes];
-  float q_scale[kPairBN], q_bias[kPairBN];
-  uint64_t bar_full[kPairStages];      // used in the leader only
-  uint64_t bar_empty[kPairStages];
+  float q_scale[BN], q_bias[BN];
+  uint64_t bar_full[pair_stages<BN>()];      // used in the leader only
+  uint64_t bar_empty[pair_stages<BN>()];
   uint64_t bar_acc_full[2];
   uint64_t bar_acc_empty[2];           // used in the leader only: one arrival per CTA
   uint32_t tmem_base_slot;
   int abort_flag;
 };
-constexpr int kPairSmemBytes = sizeof(PairShared);
-static_assert(kPairSmemBytes <= 227 * 1024, "a block has 227 KiB of shared memory");
-constexpr uint32_t kPairTmemCols = 2 * kPairBN;
+template <int BN> constexpr int pair_smem_bytes() {
+  static_assert(sizeof(PairShared<BN>) <= 227 * 1024, "a block has 227 KiB of shared memory");
+  return (int)sizeof(PairShared<BN>);
+}
 constexpr int kPairThreads = 64 + 256;                                 // producer warp, MMA warp, eight epilogue warps
 __device__ __forceinline__ void pair_epi_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
@@ -962,13 +964,14 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int tiles_p, int tile
   tq = group * kPairGroup + within - tp * gw;
 }
 
-template <int KIND>
+template <int KIND, int BN>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                     const __grid_constant__ CUtensorMap tm_out, TcParams prm) {
   using AccT = typename std::conditional<KIND == tc::MMA_I8, int, float>::type;
   extern __shared__ __align__(1024) uint8_t smem_pair[];       // (the swizzle and the descriptors assume 1024-byte alignment)
-  PairShared& sh = *reinterpret_cast<PairShared*>(smem_pair);
+  constexpr int kPairStages = pair_stages<BN>(), kPairStageBytes = pair_stage_bytes<BN>(), kHalf = BN / 2;
+  PairShared<BN>& sh = *reinterpret_cast<PairShared<BN>*>(smem_pair);
   uint8_t* tiles = sh.tiles;
   auto& bar_full = sh.bar_full; auto& bar_empty = sh.bar_empty;
   auto& bar_acc_full = sh.bar_acc_full; auto& bar_acc_empty = sh.bar_acc_empty;
@@ -998,7 +1001,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     tc::tma_prefetch_descriptor(&tm_out);
   }
   if (warp == 1) {
-    tc::tmem_alloc_pair(tc::smem_u32(&tmem_base_slot), kPairTmemCols);
+    tc::tmem_alloc_pair(tc::smem_u32(&tmem_base_slot), 2 * BN);
     tc::tmem_relinquish_pair();
   }
   tc::fence_before_sync();
@@ -1023,7 +1026,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
         int tp, tq;
         pair_tile_coords(tile, prm.tiles_p, prm.tiles_q, tp, tq);
-        const int row_a = tp * 2 * kBM + (int)rank * kBM, row_w = tq * kPairBN + (int)rank * kPairHalfB;
+        const int row_a = tp * 2 * kBM + (int)rank * kBM, row_w = tq * BN + (int)rank * kHalf;
         for (int it = 0; it < kb_count; ++it) {
           tc::mbar_wait_or_flag(tc::smem_u32(&bar_empty[stage_i]), phase ^ 1u, abort_u32);
           if (leader) tc::mbar_arrive_expect_tx(tc::smem_u32(&bar_full[stage_i]), 2u * kPairStageBytes);
@@ -1045,7 +1048,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       for (int tile = first_tile; tile < num_tiles; tile += tile_step) {
         if (!tc::mbar_wait_warp(tc::smem_u32(&bar_acc_empty[buf]), acc_phase[buf] ^ 1u, abort)) break;
         tc::fence_after_sync();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kPairBN);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
         for (int it = 0; it < kb_count; ++it) {
           tc::mbar_wait_or_flag(tc::smem_u32(&bar_full[stage_i]), phase, abort_u32);
           __syncwarp();
@@ -1069,11 +1072,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       }
     }
   } else {
-    // Eight warps: two per tensor-memory lane quadrant, each taking one half (128) of the tile's columns.
+    // Eight warps: two per tensor-memory lane quadrant, each taking one half of the tile's columns.
     // One warp per scheduler does not hide its own latencies, and the epilogue of a 128 x 256 tile must
     // finish within the main loop of the next (K = 3584: 11 us) or the tensor pipe waits for it.
     const int quad = warp & 3, et = quad * 32 + lane;
-    const int half = (warp - 2) >> 2;                                   // which 128 columns
+    const int half = (warp - 2) >> 2;                                   // which half of the columns
     const int te = (int)threadIdx.x - 64;                               // 0 .. 255
     const bool issuer = threadIdx.x == 64;
     const Epilogue& e = prm.epi;
@@ -1096,26 +1099,28 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       const bool row_ok = row < prm.M;
       pair_epi_barrier();                              // previous tile no longer reads q_scale / q_bias
       {
-        const int j = tq * kPairBN + te;               // one column's scale and bias per thread
+        const int j = tq * BN + te;               // one column's scale and bias per thread
         float sc = 1.f, bi = 0.f;
-        if (j < prm.N) {
+        if (te < BN && j < prm.N) {
           if (scaled) sc = e.col_scale[j];
           if (has_bias && !raw) bi = __fmul_rn(bmul, load_as_f32(e.bias, j, e.bias_dtype));
         }
-        q_scale[te] = sc;
-        q_bias[te] = bi;
+        if (te < BN) {
+          q_scale[te] = sc;
+          q_bias[te] = bi;
+        }
       }
       const float rs = (scaled && row_ok) ? e.row_scale[row] : 1.f;
       const bool failed = !tc::mbar_wait(tc::smem_u32(&bar_acc_full[buf]), acc_phase[buf], abort);
       if (tc::named_barrier_or(2, 256, failed)) break;
       tc::fence_after_sync();
       acc_phase[buf] ^= 1u;
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * kPairBN + half * 128);
-      const int ncols = min(128, prm.N - tq * kPairBN - half * 128);    // my columns inside the matrix (may be <= 0)
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN + half * kHalf);
+      const int ncols = min(kHalf, prm.N - tq * BN - half * kHalf);    // my columns inside the matrix (may be <= 0)
       // 32 accumulator columns per step; the load of the next step is issued before this step's arithmetic so that its
       // latency is hidden.  The staging tile holds one step of 32-bit or two of 16-bit outputs, 16-byte unit u of row r at
       // u ^ (r & 7); the accumulator buffer is free as soon as the last load is back.
-      const int row0 = row - lane, x0 = tq * kPairBN + half * 128;
+      const int row0 = row - lane, x0 = tq * BN + half * kHalf;
       uint32_t r[2][32];
       if (ncols > 0) tc::tmem_ld_32x32(taddr, r[0]);
 #pragma unroll 1
@@ -1129,8 +1134,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           uint32_t (&v)[32] = r[h];
           // the operator's arithmetic, its run-time choices made once per 32 columns
           if (!raw) {
-            const float4* qs4 = reinterpret_cast<const float4*>(q_scale + half * 128 + c);
-            const float4* qb4 = reinterpret_cast<const float4*>(q_bias + half * 128 + c);
+            const float4* qs4 = reinterpret_cast<const float4*>(q_scale + half * kHalf + c);
+            const float4* qb4 = reinterpret_cast<const float4*>(q_bias + half * kHalf + c);
             float f[32];
 #pragma unroll
             for (int jj = 0; jj < 32; ++jj) f[jj] = (float)acc_from_bits<AccT>(v[jj]);
@@ -1225,7 +1230,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   cluster_sync_all();                                  // nobody leaves while its peer may still signal it
   if (warp == 1) {
     tc::fence_after_sync();
-    tc::tmem_dealloc_pair(tmem_base, kPairTmemCols);
+    tc::tmem_dealloc_pair(tmem_base, 2 * BN);
   }
   if (threadIdx.x == 0 && abort_flag && prm.status) *prm.status = 1u;
 }
@@ -1316,13 +1321,19 @@ cudaLaunchConfig_t make_config(int grid, int cluster, cudaStream_t st, cudaLaunc
   return cfg;
 }
 
-// Estimated microseconds of the two schedules for more than 128 tokens, fitted to times measured over N = 896 .. 37888,
-// K = 896 .. 18944 and M = 160 .. 1024 (within 10 %): both are bound by what one SM can fetch from L2 (about
-// 105 GB/s), 32 KiB per K block of 128 bytes and CTA -- for a 128 x 128 tile in panels, for half of a 256 x 256
-// tile in pairs.  panel_us also picks the cluster size of the split (1 .. 8) where `splits` asks for it; `active`
-// says how many clusters of a size fit the device (without it: one CTA per SM).
-double pair_us(int64_t tiles, int k_blocks) {
-  return 2.2 + (double)ceil_div(tiles, sm_count() / 2) * (0.297 * k_blocks + 3.5);
+// Estimated microseconds of the schedules for more than 128 tokens, fitted to times measured over N = 896 .. 37888,
+// K = 896 .. 18944 and M = 160 .. 4096 (within 10 % but for the smallest): all are bound by what one SM can fetch from L2
+// (about 105 GB/s), per K block of 128 bytes 32 KiB a CTA for a 128 x 128 tile in panels and for half of a 256 x 256 tile in
+// pairs, 24 KiB for half of a 256 x 128 tile.  The narrow pair's tiles cost more traffic and fill twice as many SMs: 333 x
+// 3584 x 3584 14.3 us in 28 wide pairs, 10.3 in 56 narrow ones (panels 15.1); 1024 x 1536 x 8960 25.9 and 17.5 (27.7); 512 x
+// 896 x 896 7.8 and 6.1; but 4096 x 4608 x 3584 42.9 and 51.0.  panel_us also picks the cluster size of the split (1 .. 8) where
+// `splits` asks for it; `active` says how many clusters of a size fit the device (without it: one CTA per SM).
+double pair_us(int64_t M, int64_t N, int k_blocks, bool* narrow) {
+  const int64_t rows = ceil_div(M, (int64_t)(2 * kBM)), clusters = sm_count() / 2;
+  const double wide_us = 4.57 + (double)ceil_div(rows * ceil_div(N, (int64_t)kPairBN), clusters) * (0.286 * k_blocks + 1.59);
+  const double narrow_us = 3.56 + (double)ceil_div(rows * ceil_div(N, (int64_t)kPairNarrowBN), clusters) * (0.160 * k_blocks + 1.59);
+  if (narrow) *narrow = 1.03 * narrow_us < wide_us;
+  return 1.03 * narrow_us < wide_us ? narrow_us : wide_us;
 }
 double panel_us(int64_t tiles, int k_blocks, int* splits, int (*active)(int) = nullptr) {
   double best = 5.2 + (double)ceil_div(tiles, sm_count()) * (0.306 * k_blocks + 1.7);
@@ -1401,7 +1412,7 @@ int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& 
 }
 
 // Clusters of two CTAs of the pair kernel that can be resident at once (cached per device).
-template <int KIND>
+template <int KIND, int BN>
 int pair_max_clusters() {
   static std::mutex mu;
   static std::map<int, int> cache;
@@ -1410,14 +1421,14 @@ int pair_max_clusters() {
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(dev);
   if (it != cache.end()) return it->second;
-  auto kern = gemm_tc_pair_kernel<KIND>;
+  auto kern = gemm_tc_pair_kernel<KIND, BN>;
   int n = 0;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kPairSmemBytes) == LLMQRT_OK) {
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), pair_smem_bytes<BN>()) == LLMQRT_OK) {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2, 1, 1);
     cfg.blockDim = dim3(kPairThreads, 1, 1);
-    cfg.dynamicSmemBytes = kPairSmemBytes;
+    cfg.dynamicSmemBytes = pair_smem_bytes<BN>();
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
@@ -1433,11 +1444,11 @@ int pair_max_clusters() {
   return n;
 }
 
-template <int KIND>
+template <int KIND, int BN>
 int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const CUtensorMap& tm_out, const TcParams& prm, cudaStream_t st) {
-  auto kern = gemm_tc_pair_kernel<KIND>;
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kPairSmemBytes)) return rc;
-  int clusters = pair_max_clusters<KIND>();
+  auto kern = gemm_tc_pair_kernel<KIND, BN>;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), pair_smem_bytes<BN>())) return rc;
+  int clusters = pair_max_clusters<KIND, BN>();
   if (clusters <= 0) return set_error(LLMQRT_ERR_CUDA, "tcgen05 pair gemm: no cluster of two CTAs fits on this device");
   const int tiles = prm.tiles_p * prm.tiles_q;
   if (clusters > tiles) clusters = tiles;
@@ -1445,7 +1456,7 @@ int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const CUtensor
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
   cfg.blockDim = dim3(kPairThreads, 1, 1);
-  cfg.dynamicSmemBytes = kPairSmemBytes;
+  cfg.dynamicSmemBytes = pair_smem_bytes<BN>();
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
@@ -1460,6 +1471,12 @@ int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const CUtensor
   }
   LLMQRT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm_a, tm_w, tm_out, prm));
   return check_launch("gemm_tc_pair");
+}
+
+template <int KIND>
+int launch_pair_bn(bool narrow, const CUtensorMap& tm_a, const CUtensorMap& tm_w, const CUtensorMap& tm_out, const TcParams& prm,
+                   cudaStream_t st) {
+  return narrow ? launch_pair<KIND, kPairNarrowBN>(tm_a, tm_w, tm_out, prm, st) : launch_pair<KIND, kPairBN>(tm_a, tm_w, tm_out, prm, st);
 }
 
 template <int KIND, bool AWQ = false>
@@ -1506,9 +1523,8 @@ double awq_tc_us(int64_t M, int64_t N, int64_t K, bool* panels) {
 
 double awq_expanded_us(int64_t M, int64_t N, int64_t K) {
   const int kb = (int)ceil_div(K, (int64_t)64);
-  double g = pair_us(ceil_div(M, (int64_t)256) * ceil_div(N, (int64_t)kPairBN), kb);
-  const double p = panel_us(ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM), kb, nullptr);
-  return 2.1 + 0.906 * (p < g ? p : g) + 0.518e-6 * (double)(N * K);
+  const double g = pair_us(M, N, kb, nullptr), p = 1.03 * panel_us(ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM), kb, nullptr);
+  return 1.0 + (p < g ? p : g) + 0.518e-6 * (double)(N * K);
 }
 
 int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
@@ -1530,19 +1546,20 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
 
   // More than 128 tokens: the two-CTA kernel wherever its vector stores may be used (16-byte aligned output rows),
   // unless the small-M schedule -- weights as the 128-lane operand, tokens in panels of 128 as the column operand,
-  // cluster split-K -- is estimated to be faster, as it is where few 256 x 256 tiles meet a long reduction
-  // (M = 160, N = 896, K = 4864: 11.7 us in panels, 16.4 us in pairs; M = 160, N = K = 3584: 15.1 against 14.0).
+  // cluster split-K -- is estimated to be faster, as it is where few tiles meet a long reduction
+  // (M = 160: N = 896, K = 8960 12.8 us in panels, 15.0 in narrow pairs; N = K = 3584 15.1 against 9.9).
   // The 128 x 256 tiles of a lone CTA feed 48 KiB per K block through one SM's share of L2 (28 us at
   // M = 160 .. 640, N = K = 3584): they are left to the outputs that neither can serve.
   const int es = (epi.mode == EPI_RAW || epi.out_dtype == LLMQRT_F32) ? 4 : 2;
   const bool out_ok = (reinterpret_cast<uintptr_t>(epi.out) & 15) == 0 && (epi.ldo * es) % 16 == 0;
   const int k_blocks = (int)ceil_div(K * elt, kRowBytes);
   const bool pair_ok = !awq && !push && M > 128 && N > 128 && out_ok && pair_enabled();
-  bool panels = false;
+  bool panels = false, narrow = false;
+  const double pairs_us = pair_ok ? pair_us(M, N, k_blocks, &narrow) : 0.;
   if (M > 128 && M <= 1024) {
     const int64_t panel_tiles = ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM);
     if (pair_ok) {
-      panels = panel_us(panel_tiles, k_blocks, nullptr) < pair_us(ceil_div(M, (int64_t)256) * ceil_div(N, (int64_t)256), k_blocks);
+      panels = 1.03 * panel_us(panel_tiles, k_blocks, nullptr) < pairs_us;
     } else if (awq) {
       awq_tc_us(M, N, K, &panels);
     } else {
@@ -1596,15 +1613,16 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
 
   if (pair_ok && !panels) {
     prm.tiles_p = (int)ceil_div(M, (int64_t)(2 * kBM));
-    prm.tiles_q = (int)ceil_div(N, (int64_t)kPairBN);
-    prm.idesc = tc::instr_desc(c_fmt, fmt_act, fmt_w, 2 * kBM, kPairBN);
+    const int pair_bn = narrow ? kPairNarrowBN : kPairBN;
+    prm.tiles_q = (int)ceil_div(N, (int64_t)pair_bn);
+    prm.idesc = tc::instr_desc(c_fmt, fmt_act, fmt_w, 2 * kBM, (uint32_t)pair_bn);
     CUtensorMap tm_a, tm_w, tm_out;
     if (int rc = make_operand_map(&tm_a, A, elt, M, K, lda, kBM)) return rc;
-    if (int rc = make_operand_map(&tm_w, W, elt, N, K, ldw, kPairHalfB)) return rc;
+    if (int rc = make_operand_map(&tm_w, W, elt, N, K, ldw, pair_bn / 2)) return rc;
     if (int rc = make_output_map(&tm_out, epi.out, es, M, N, epi.ldo)) return rc;
-    if (mk == tc::MMA_I8) return launch_pair<tc::MMA_I8>(tm_a, tm_w, tm_out, prm, st);
-    if (mk == tc::MMA_F8) return launch_pair<tc::MMA_F8>(tm_a, tm_w, tm_out, prm, st);
-    return launch_pair<tc::MMA_F16>(tm_a, tm_w, tm_out, prm, st);
+    if (mk == tc::MMA_I8) return launch_pair_bn<tc::MMA_I8>(narrow, tm_a, tm_w, tm_out, prm, st);
+    if (mk == tc::MMA_F8) return launch_pair_bn<tc::MMA_F8>(narrow, tm_a, tm_w, tm_out, prm, st);
+    return launch_pair_bn<tc::MMA_F16>(narrow, tm_a, tm_w, tm_out, prm, st);
   }
   prm.idesc = tc::instr_desc(c_fmt, prm.swap ? fmt_w : fmt_act, prm.swap ? fmt_act : fmt_w, kBM, (uint32_t)bn);
 
