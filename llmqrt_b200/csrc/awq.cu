@@ -260,18 +260,15 @@ int launch_rows(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32
   return check_launch("awq_gemm_rows");
 }
 
-// 9 to 32 tokens: every block fetches all activations, so the time of this file's kernel goes with the blocks on an SM x
-// tokens x K, while the tcgen05 kernel takes the same time for any of them.  us at 9 / 16 / 17 / 24 / 32 tokens (tcgen05):
-//   1536 x 1536 2.7 / 3.1 / 3.9 / 4.3 / 4.9 (8.8)      4608 x 3584 6.4 / 8.0 / 9.4 / 11.1 / 12.9 (13.8)
-//   17920 x 1536 8.9 / 11.3 / 15 / 17 / 20 (12.2)      5120 x 4096 10.0 / 12.3 / 15 / 18 / 21 (13.9)
-//   27648 x 2560 22 / 31 / 37 / 44 / 54 (28)           37888 x 3584 33 / 41 / 50 / 60 / 75 (37)
-// The estimates are fitted to N = 896 .. 37888, K = 896 .. 13824; the kernel they choose is more than 4 % slower than the
-// other in 21 of 516 measured cases, mostly by 10 to 15 % (12 tokens of 17920 rows, 17 to 24 of 12288).
+// 17 to 32 tokens: every block fetches all activations, so the time of this file's kernel goes with the blocks on an SM x
+// tokens x K, while the tcgen05 kernel takes the same time for any of them.  us at 17 / 24 / 32 tokens (tcgen05):
+//   1536 x 1536 3.9 / 4.3 / 4.9 (8.8)      4608 x 3584 9.4 / 11.1 / 12.9 (13.8)      5120 x 4096 15 / 18 / 21 (13.9)
+//   17920 x 1536 15 / 17 / 20 (12.2)       27648 x 2560 37 / 44 / 54 (28)            37888 x 3584 50 / 60 / 75 (37)
+// The estimates are fitted to N = 896 .. 37888, K = 896 .. 13824; the kernel they choose is up to 15 % slower than the other
+// around 17 to 24 tokens of 12288 rows.
 bool rows_suit(int64_t M, int64_t N, int64_t K) {
   const double blocks = (double)ceil_div(ceil_div(N, (int64_t)16), (int64_t)sm_count()), k = 1e-3 * (double)K;
-  const double us = M <= 16 ? 2.1 + blocks * (0.07 + k * (0.358 + 0.0240 * (double)M))
-                            : 2.3 + blocks * (0.24 + k * (0.316 + 0.0323 * (double)M));
-  return us < awq_tc_us(M, N, K, nullptr);
+  return 2.3 + blocks * (0.24 + k * (0.316 + 0.0323 * (double)M)) < awq_tc_us(M, N, K, nullptr);
 }
 
 int check_layer(int64_t K, int64_t N, int64_t G) {
@@ -363,7 +360,10 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   }
   if (M <= 0) return LLMQRT_OK;
   e.out = out;
-  if (M <= 8 || (M <= 32 && rows_suit(M, N, K))) {
+  // Up to 16 tokens every layer is this file's kernel, as in llmqrt_awq_gemm_tail: the sums of both are added in one order, so
+  // a tail rounds as the separate steps do.  (On tcgen05 only 13 to 16 tokens of the largest layers
+  // are faster: 16 of 37888 x 3584 38 us against 43, but of 17920 x 1536 12.3 against 11.5, of 3584 x 18944 38 against 35.)
+  if (M <= 16 || (M <= 32 && rows_suit(M, N, K))) {
     auto go = M <= 8 ? launch_rows<1> : M <= 16 ? launch_rows<2> : launch_rows<4>;
     return go(xp, ldx, wq_t, sz_t, (int)M, (int)N, (int)K, (int)group_size, e, st, nullptr, 0);
   }

@@ -10,9 +10,9 @@ pytestmark = pytest.mark.gpu
 H, HQ, HKV, D, I, G = 128, 2, 1, 64, 256, 32
 
 
-def _layer(n, k, g):
+def _layer(n, k, g, group=G):
     from llmqrt_b200.linear import WQLinear_GEMM
-    layer = WQLinear_GEMM(4, G, k, n, False, "cuda")
+    layer = WQLinear_GEMM(4, group, k, n, False, "cuda")
     layer.qweight.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
     layer.qzeros.random_(-2 ** 31, 2 ** 31 - 1, generator=g)
     layer.scales.uniform_(0.001, 0.01, generator=g)
@@ -160,6 +160,31 @@ def test_step_in_one_call(B):
         for name in ("k", "v"):
             assert torch.equal(getattr(blocks[0].attn.cache, name), getattr(blocks[1].attn.cache, name))
         assert blocks[0].attn.start_pos == blocks[1].attn.start_pos == 8 + step
+
+
+@pytest.mark.parametrize("B", [9, 12, 16])
+@pytest.mark.parametrize("H,I", [(1536, 8960), (3584, 18944)])
+def test_step_of_a_large_block(B, H, I):
+    """The native step against every layer's plain call and the separate additions and SiLU, where the layers are large."""
+    from llmqrt_b200 import glue
+    from llmqrt_b200._lib import fast
+    from llmqrt_b200.fused_utils import FusedGateUpMLP
+    from llmqrt_b200.nonlinear import LlamaLikeBlock, RMSNorm
+    g = torch.Generator(device="cuda").manual_seed(B)
+    mlp = FusedGateUpMLP(_layer(I, H, g, 128), _layer(I, H, g, 128), _layer(H, I, g, 128))
+    norms = [RMSNorm((1 + 0.1 * torch.randn(H, generator=g, device="cuda")).half()) for _ in range(2)]
+    block = LlamaLikeBlock(H, 2, 1, _layer(4 * 64, H, g, 128), None, None, None, _layer(H, 2 * 64, g, 128), mlp, *norms,
+                           dev="cuda", max_seq_len=16, head_dim=64)
+    for layer in (block.attn.qkv_proj, block.attn.o_proj, mlp.gate_up, mlp.down_proj):
+        layer.packed()
+    block.attn.cache.increase_batch_size(B)
+    block.attn.cache_batch_size = B
+    x = torch.randn(B, 1, H, generator=g, device="cuda").half()
+    h = _run(block, lambda b, t: t + b.attn(b.norm_1(t))[0], x)
+    want = h + mlp.down_proj(glue.silu_mul(mlp.gate_up(block.norm_2(h)))[0])
+    got = _run(block, fast.awq_block_step, x)
+    assert got is not None and torch.equal(got, want)
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want)
 
 
 @pytest.mark.parametrize("how", ["hook", "pre-hook", "global", "instance", "class"])

@@ -108,6 +108,13 @@ def test_awq_tail(M, K, N, G):
     assert not layer.takes_tail(torch.zeros(17, K, dtype=torch.float16, device="cuda"))
 
 
+@pytest.mark.parametrize("M", [9, 12, 13, 16])
+@pytest.mark.parametrize("K,N,G", [(3584, 37888, 128), (18944, 3584, 128), (1536, 17920, 64)])
+def test_awq_tail_of_large_layers(M, K, N, G):
+    """The sizes at which a plain call might prefer another kernel than its tail has."""
+    test_awq_tail(M, K, N, G)
+
+
 @pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 16, 17, 32, 33, 64])
 @pytest.mark.parametrize("K,N,G", [(32, 8, 32), (96, 24, 32), (128, 16, 128), (1536, 2056, 128), (2080, 40, 32),
                                    (8960, 1536, 128), (4096, 17920, 64)])
