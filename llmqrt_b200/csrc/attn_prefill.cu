@@ -429,6 +429,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         exp_of(1);
         mx = row_max();
         again = __any_sync(0xffffffffu, (mx - m_ref) * sl > 8.f);
+        if (again) tc::tmem_st_wait();                  // two stores to one column are not ordered by themselves
       }
       if (again) {
         // Move the reference only when the maximum has outgrown it by more than 2^8 (always on the first
