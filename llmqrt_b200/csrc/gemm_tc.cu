@@ -466,6 +466,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
   const int kb_begin = (int)((int64_t)my_split * prm.k_blocks / S);
   const int kb_count = (int)((int64_t)(my_split + 1) * prm.k_blocks / S) - kb_begin;
   EpiConsts ec_split = {};           // split mode: set by the epilogue warps before they wait for the MMAs
+  bool mmas_done = false;            // split mode: the epilogue warps' common answer
 
   // AWQ: one ring's share of the TMA loads -- the activation tiles (warp 0) or the packed weight tiles (the last warp)
   auto awq_load = [&](bool act) {
@@ -638,7 +639,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         __syncwarp();
         if (++stage_i == kFull) { stage_i = 0; phase ^= 1u; }
       }
-      if (*abort) break;
+      if (tc::warp_aborted(abort)) break;
       if (tc::elect_one()) tc::mma_commit(tc::smem_u32(&bar_acc_full[buf]));        // accumulator complete
       acc_phase[buf] ^= 1u;
       if (kAccBufs > 1) buf ^= 1;
@@ -701,7 +702,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       for (int d = 0; d < kDepth; ++d) {
         if (q0 + d * kAwqGroups >= total || !ok) continue;
         tc::mbar_wait_or_flag(tc::smem_u32(&bar_pk_full[ps]), p_phase, abort_u32);
-        if (d == 0 && *abort) { ok = false; continue; }
+        if (d == 0 && tc::warp_aborted(abort)) { ok = false; continue; }
         const uint4* src = reinterpret_cast<const uint4*>(packed + ps * kPackedBytes + rr * kPackedRowBytes);
         const uint4 a0 = src[0], a1 = src[1];
         const uint32_t words[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
@@ -760,7 +761,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       if (tc::named_barrier_or(2, 128, failed)) break;
       tc::fence_after_sync();
       acc_phase[buf] ^= 1u;
-      if (S > 1) break;                                // split mode: the reduce-scatter below takes over
+      if (S > 1) {                                     // split mode: the reduce-scatter below takes over
+        mmas_done = true;
+        break;
+      }
 
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
 #pragma unroll 1
@@ -799,9 +803,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
     const uint32_t slice_bytes = (uint32_t)cpo * kBM * 4;              // what every CTA sends to this one
     const int cpo_max = ((BN / 8 + S - 1) / S) * 8;
     uint32_t* send = reinterpret_cast<uint32_t*>(tiles + S * cpo_max * kBM * 4);
-    const bool own_healthy = abort_flag == 0;          // own MMAs finished (epilogue warps waited for them)
     const int quad = warp & 3, et = quad * 32 + lane;
     const bool epi_warp = warp >= 2 && warp < 6;       // (AWQ mode has more warps behind them)
+    const bool own_healthy = mmas_done || !epi_warp;   // (the others learn of a failure from cluster_abort)
     const int tq = first_tile % prm.tiles_q, tp = first_tile / prm.tiles_q;
     const EpiConsts& ec = ec_split;                    // q_scale / q_bias cover only the columns this CTA owns
     if (epi_warp && own_healthy) {
@@ -1065,7 +1069,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           __syncwarp();
           if (++stage_i == kPairStages) { stage_i = 0; phase ^= 1u; }
         }
-        if (*abort) break;
+        if (tc::warp_aborted(abort)) break;
         if (tc::elect_one()) tc::mma_commit_pair(tc::smem_u32(&bar_acc_full[buf]));          // accumulators complete in both CTAs
         acc_phase[buf] ^= 1u;
         buf ^= 1;

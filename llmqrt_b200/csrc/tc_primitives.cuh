@@ -102,6 +102,10 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort));
 }
 
+// The abort flag as one answer for the whole warp.  Lanes that looked for themselves could see it raised at different moments
+// and part, ahead of instructions that every lane of the warp has to reach.
+__device__ __forceinline__ bool warp_aborted(const volatile int* abort) { return __any_sync(0xffffffffu, *abort != 0); }
+
 // Named barrier over `nthreads` threads that also ORs a predicate across them (uniform result).
 __device__ __forceinline__ bool named_barrier_or(int id, int nthreads, bool pred) {
   uint32_t r;
