@@ -268,7 +268,7 @@ int launch_rows(const __half* X, int64_t ldx, const uint32_t* wq_t, const uint32
 // around 17 to 24 tokens of 12288 rows.
 bool rows_suit(int64_t M, int64_t N, int64_t K) {
   const double blocks = (double)ceil_div(ceil_div(N, (int64_t)16), (int64_t)sm_count()), k = 1e-3 * (double)K;
-  return 2.3 + blocks * (0.24 + k * (0.316 + 0.0323 * (double)M)) < awq_tc_us(M, N, K, nullptr);
+  return !awq_tc_faster(M, N, K, 2.3 + blocks * (0.24 + k * (0.316 + 0.0323 * (double)M)));
 }
 
 int check_layer(int64_t K, int64_t N, int64_t G) {
@@ -342,7 +342,7 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   // estimates choose; a twelfth in favour of the expansion is what they are off by.  (Panels of 64 MB, which would stay in L2, are
   // worse: 113 us for 3584 x 18944 at 256.)  Above 1024 tokens it is always expanded.
   if (M > 128 && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0 &&
-      (M > 1024 || 0.92 * awq_expanded_us(M, N, K) < awq_tc_us(M, N, K, nullptr))) {
+      (M > 1024 || !awq_tc_faster(M, N, K, 0.92 * awq_expanded_us(M, N, K)))) {
     const int64_t cap_rows = (int64_t)(LLMQRT_WS_PARTIAL_BYTES / (size_t)(K * 2)) / 256 * 256;
     if (cap_rows >= 256) {
       __half* deq = reinterpret_cast<__half*>(ws_partials(workspace));

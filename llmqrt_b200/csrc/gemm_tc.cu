@@ -39,7 +39,7 @@
 #include "peer_comm.cuh"
 #include "tc_primitives.cuh"
 
-#include <map>
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -52,6 +52,8 @@ constexpr int kAwqWarps = 4 * kAwqGroups;
 constexpr int kThreadsAwq = kThreads + kAwqWarps * 32 + 32;      // (+ the warp that fetches the packed tiles)
 constexpr int kBM = 128;           // rows of P per tile (UMMA M)
 constexpr int kRowBytes = 128;     // bytes of K per stage row (one swizzle span)
+constexpr int kMaxCluster = 8;     // CTAs that may share a reduction
+constexpr int kMaxDevices = 64;
 constexpr int kSmemBudget = 226 * 1024;   // of the 227 KiB a block may use
 constexpr int kChunk = 32;         // accumulator columns handled per epilogue step
 constexpr int kEpiStageBytes = 18 * 1024;  // staging tile for one chunk (worst case 128 x 32 x 4 B + padding)
@@ -1339,11 +1341,12 @@ double pair_us(int64_t M, int64_t N, int k_blocks, bool* narrow) {
   if (narrow) *narrow = 1.03 * narrow_us < wide_us;
   return 1.03 * narrow_us < wide_us ? narrow_us : wide_us;
 }
-double panel_us(int64_t tiles, int k_blocks, int* splits, int (*active)(int) = nullptr) {
-  double best = 5.2 + (double)ceil_div(tiles, sm_count()) * (0.306 * k_blocks + 1.7);
+double panel_us(int64_t tiles, int k_blocks, int* splits, const int* active = nullptr) {
+  const int sms = sm_count();
+  double best = 5.2 + (double)ceil_div(tiles, sms) * (0.306 * k_blocks + 1.7);
   if (splits) *splits = 1;
-  for (int s = 2; s <= 8 && k_blocks >= 2 * s && tiles < sm_count(); ++s) {
-    const int n = active ? active(s) : sm_count() / s;
+  for (int s = 2; s <= kMaxCluster && k_blocks >= 2 * s && tiles < sms; ++s) {
+    const int n = active ? active[s] : sms / s;
     if (n <= 0) continue;
     const double t = 5.2 + (double)ceil_div(tiles, n) * (0.306 * k_blocks / s + 5.2);
     if (t < best) {
@@ -1354,40 +1357,41 @@ double panel_us(int64_t tiles, int k_blocks, int* splits, int (*active)(int) = n
   return best;
 }
 
-// How many clusters of `cluster` CTAs of this kernel can be resident at once (cached per device).
+// How many clusters of [1 .. kMaxCluster] CTAs of this kernel can be resident at once, asked once per device.  (Small calls are
+// bound by the host: with a lock, a look-up and a question for the current device to every size the estimates try, a 4-bit
+// layer of 130 tokens took the host 10.7 us, now 8.6; of 20 tokens 7.0, now 6.0.)
 template <int KIND, int BN, bool AWQ = false, bool PUSH = false>
-int max_active_clusters(int cluster) {
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, int> cache;
+const int* active_clusters() {
+  static std::once_flag once[kMaxDevices];
+  static int known[kMaxDevices][kMaxCluster + 1];
+  static const int none[kMaxCluster + 1] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find({dev, cluster});
-  if (it != cache.end()) return it->second;
-  auto kern = gemm_tc_kernel<KIND, BN, AWQ, PUSH>;
-  int n = 0;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes_of<BN, AWQ>()) == LLMQRT_OK) {
-    cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = make_config<KIND, BN, AWQ>(cluster, cluster, nullptr, attr);
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return none;
+  std::call_once(once[dev], [dev] {
+    auto kern = gemm_tc_kernel<KIND, BN, AWQ, PUSH>;
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes_of<BN, AWQ>()) != LLMQRT_OK) return;
+    for (int cluster = 1; cluster <= kMaxCluster; ++cluster) {
+      cudaLaunchAttribute attr[2];
+      cudaLaunchConfig_t cfg = make_config<KIND, BN, AWQ>(cluster, cluster, nullptr, attr);
+      if (cudaOccupancyMaxActiveClusters(&known[dev][cluster], kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        known[dev][cluster] = 0;
+      }
     }
-  }
-  cache[{dev, cluster}] = n;
-  return n;
+  });
+  return known[dev];
 }
 
 // The cluster size (any from 1 to 8: 36 tiles fit as clusters of three, not of four) with the smallest estimated time: waves
 // of co-resident clusters x (K blocks per CTA + a fixed per-CTA cost of about eight K blocks for pipeline fill,
 // reduce-scatter and epilogue).
-int pick_splits(int64_t tiles, int k_blocks, int most, int (*active)(int), int* waves) {
+int pick_splits(int64_t tiles, int k_blocks, int most, const int* active, int* waves) {
   const float fixed = 8.f;
-  int splits = 1, w = (int)ceil_div(tiles, (int64_t)sm_count());
+  const int64_t sms = sm_count();
+  int splits = 1, w = (int)ceil_div(tiles, sms);
   float best = (float)w * ((float)k_blocks + fixed);
-  for (int s = 2; s <= 8 && tiles < sm_count(); ++s) {
-    if (k_blocks < 2 * s || most < s) continue;
-    const int n = active(s);
+  for (int s = 2; s <= kMaxCluster && k_blocks >= 2 * s && most >= s && tiles < sms; ++s) {
+    const int n = active[s];
     if (n <= 0) continue;
     const float t = (float)ceil_div(tiles, (int64_t)n) * ((float)k_blocks / s + fixed);
     if (t < best) { best = t; splits = s; w = (int)ceil_div(tiles, (int64_t)n); }
@@ -1404,8 +1408,8 @@ int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& 
   const int tiles = prm.tiles_p * prm.tiles_q;
   int splits = 1;
   if (BN <= 128 && tiles < sms) {
-    if (prm.tiles_q > 1 && !AWQ) panel_us(tiles, prm.k_blocks, &splits, max_active_clusters<KIND, BN, AWQ, PUSH>);
-    else splits = pick_splits(tiles, prm.k_blocks, BN / 8, max_active_clusters<KIND, BN, AWQ, PUSH>, nullptr);
+    if (prm.tiles_q > 1 && !AWQ) panel_us(tiles, prm.k_blocks, &splits, active_clusters<KIND, BN, AWQ, PUSH>());
+    else splits = pick_splits(tiles, prm.k_blocks, BN / 8, active_clusters<KIND, BN, AWQ, PUSH>(), nullptr);
   }
   prm.splits = splits;
   const int grid = splits > 1 ? tiles * splits : (tiles < sms ? tiles : sms);
@@ -1415,19 +1419,16 @@ int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& 
   return check_launch("gemm_tc");
 }
 
-// Clusters of two CTAs of the pair kernel that can be resident at once (cached per device).
+// Clusters of two CTAs of the pair kernel that can be resident at once (asked once per device).
 template <int KIND, int BN>
 int pair_max_clusters() {
-  static std::mutex mu;
-  static std::map<int, int> cache;
+  static std::once_flag once[kMaxDevices];
+  static int known[kMaxDevices];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(dev);
-  if (it != cache.end()) return it->second;
-  auto kern = gemm_tc_pair_kernel<KIND, BN>;
-  int n = 0;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), pair_smem_bytes<BN>()) == LLMQRT_OK) {
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kMaxDevices) return 0;
+  std::call_once(once[dev], [dev] {
+    auto kern = gemm_tc_pair_kernel<KIND, BN>;
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), pair_smem_bytes<BN>()) != LLMQRT_OK) return;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2, 1, 1);
@@ -1439,13 +1440,12 @@ int pair_max_clusters() {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&known[dev], kern, &cfg) != cudaSuccess) {
       cudaGetLastError();
-      n = 0;
+      known[dev] = 0;
     }
-  }
-  cache[dev] = n;
-  return n;
+  });
+  return known[dev];
 }
 
 template <int KIND, int BN>
@@ -1495,11 +1495,21 @@ int launch_bn(int bn, const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CU
 }
 
 // Estimated microseconds of the kernel that dequantizes its weights, fitted to times over N = 896 .. 37888, K = 896 .. 18944:
-// up to 32 tokens, and above 128 with the tokens in panels of 128 or (*panels = false) in tiles of 256.
-double awq_split_us(int64_t tiles, int k_blocks, int most, int (*active)(int), double base, double kb, double tile, double exchange) {
-  int waves;
-  const int s = pick_splits(tiles, k_blocks, most, active, &waves);
-  return base + waves * (kb * k_blocks / s + tile + (s > 1 ? exchange : 0.));
+// up to 32 tokens, and above 128 with the tokens in panels of 128 or in tiles of 256.
+struct AwqFit {
+  double base, kb, tile, exchange;                     // a launch; a K block; a tile; a split reduction's exchange
+  double us(int64_t tiles, int k_blocks, int most, const int* active) const {
+    int waves;
+    const int s = pick_splits(tiles, k_blocks, most, active, &waves);
+    return base + waves * (kb * k_blocks / s + tile + (s > 1 ? exchange : 0.));
+  }
+  double least(int k_blocks) const {                   // of any number of tiles
+    return base + tile + std::min(kb * k_blocks, kb * k_blocks / kMaxCluster + exchange);
+  }
+};
+constexpr AwqFit kAwqFew = {1.2, 0.294, 2.4, 4.3}, kAwqPanels = {5.7, 0.28, 4.3, 3.7};
+double awq_tile_us(int64_t tiles, int k_blocks) {
+  return (double)ceil_div(tiles, (int64_t)sm_count()) * (0.327 * k_blocks + 14.2);
 }
 
 // The two-CTA kernel is used unless the environment variable LLMQRT_GEMM_PAIR is "0".
@@ -1516,13 +1526,17 @@ bool pair_enabled() {
 double awq_tc_us(int64_t M, int64_t N, int64_t K, bool* panels) {
   const int kb = (int)ceil_div(K, (int64_t)64);
   const int64_t tiles = ceil_div(N, (int64_t)kBM);
-  if (M <= 128)
-    return awq_split_us(tiles, kb, 8, max_active_clusters<tc::MMA_F16, 64, true>, 1.2, 0.294, 2.4, 4.3);
-  const double p = awq_split_us(tiles * ceil_div(M, (int64_t)128), kb, 16, max_active_clusters<tc::MMA_F16, 128, true>,
-                                5.7, 0.28, 4.3, 3.7);
-  const double t = (double)ceil_div(tiles * ceil_div(M, (int64_t)256), (int64_t)sm_count()) * (0.327 * kb + 14.2);
+  if (M <= 128) return kAwqFew.us(tiles, kb, 8, active_clusters<tc::MMA_F16, 64, true>());
+  const double p = kAwqPanels.us(tiles * ceil_div(M, (int64_t)128), kb, 16, active_clusters<tc::MMA_F16, 128, true>());
+  const double t = awq_tile_us(tiles * ceil_div(M, (int64_t)256), kb);
   if (panels) *panels = p < t;
   return p < t ? p : t;
+}
+
+bool awq_tc_faster(int64_t M, int64_t N, int64_t K, double than) {
+  const int kb = (int)ceil_div(K, (int64_t)64);
+  const double least = M <= 128 ? kAwqFew.least(kb) : std::min(kAwqPanels.least(kb), awq_tile_us(1, kb));
+  return least < than && awq_tc_us(M, N, K, nullptr) < than;
 }
 
 double awq_expanded_us(int64_t M, int64_t N, int64_t K) {
@@ -1582,7 +1596,7 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   else bn = N <= 128 ? 128 : 256;
   // 4-bit weights: a reduction that is better split in more than four has 64 columns also for few tokens.  (Otherwise not: with
   // three quarters of a 64-column box beyond the tokens, 16 tokens of 37888 x 3584 took 38 or 56 us, by where x lay; 37 in 32.)
-  if (awq && M <= 32 && pick_splits(ceil_div(N, (int64_t)kBM), k_blocks, 8, max_active_clusters<tc::MMA_F16, 64, true>, nullptr) > 4) bn = 64;
+  if (awq && M <= 32 && pick_splits(ceil_div(N, (int64_t)kBM), k_blocks, 8, active_clusters<tc::MMA_F16, 64, true>(), nullptr) > 4) bn = 64;
   if (awq && !prm.swap) {
     // AWQ with many tokens: the weights stay the 128-lane operand and the tokens come in tiles of 256.
     // A dequantized weight tile (the expensive operand: it is produced by arithmetic, not by a copy)

@@ -42,6 +42,7 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
 // Estimated microseconds of a 4-bit layer: dequantized by that kernel (panels, if wanted: whether tokens beyond 128 go in
 // panels of 128 rather than tiles of 256), or expanded first and multiplied by the dense one.
 double awq_tc_us(int64_t M, int64_t N, int64_t K, bool* panels);
+bool awq_tc_faster(int64_t M, int64_t N, int64_t K, double than);    // (a small layer is decided without the whole estimate)
 double awq_expanded_us(int64_t M, int64_t N, int64_t K);
 // push != nullptr (decode-sized M only): the results do not go to epi.out but, as the tagged words of
 // the next all-reduce call, into the peers' buffers; llmqrt_comm_allreduce_rmsnorm with a null

@@ -116,3 +116,18 @@ def test_prompt_attention_of_mixed_types_is_refused():
         attention.flash_attn_func(x, x.bfloat16(), x)
     with pytest.raises(TypeError, match="one dtype"):
         attention.flash_attn_func(x, x, x.bfloat16())
+
+
+@pytest.mark.parametrize("name", ["gemm_tc.cu", "awq.cu"])
+def test_schedules_ask_the_device_once(name):
+    """Small calls are bound by the host: an estimate that asks the runtime for the device (or takes a lock) for every size
+    it tries shows in them.  Read off the source: no loop's header does, and no loop calls what does."""
+    import os
+    import re
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = re.sub(r"//[^\n]*", "", open(os.path.join(root, "llmqrt_b200", "csrc", name)).read())
+    host = src[src.rindex("__global__"):]
+    for loop in re.finditer(r"\b(?:for|while) \((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)", host):
+        body = host[loop.end():].split("\n  }\n")[0] if host[loop.end():].lstrip().startswith("{") else ""
+        assert "sm_count()" not in loop.group(0), loop.group(0)
+        assert not re.search(r"\bactive(?:_clusters)?(?:<[^;]*>)?\(", body), loop.group(0)
