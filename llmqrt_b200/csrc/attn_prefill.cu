@@ -128,7 +128,13 @@ template <int D> constexpr int v_stages() { return D == 128 ? 2 : 4; }
 template <int D> constexpr int tile_bytes() { return (D / 64) * kSubBytes; }
 template <int D> constexpr int smem_bytes() { return (2 + k_stages<D>() + v_stages<D>()) * tile_bytes<D>() + 1024; }
 
-template <bool BF16, int D>
+// SHORT: sequences of at most kShortRows tokens.  They are one tile, and a launch is mostly the latency of code that runs once:
+// their rows, few of a warp's 32, are written straight from registers, and the half that reckons ahead is left out.  us, this
+// form / the general one: 9 x 18 tokens, 28 heads of 128 11.2 / 12.3; 8 of 14 heads of 64 at 32 5.8 / 6.1, 40 5.92 / 6.08, 48 5.92 /
+// 6.06, 64 6.14 / 6.06; 4 of 28 heads of 128 at 32 6.60 / 6.89, 40 6.79 / 6.86, 48 6.95 / 6.85.  (Both in one kernel, the general
+// one loses 0.1 us.)
+constexpr int kShortRows = 40;
+template <bool BF16, int D, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, PrefillParams prm) {
@@ -402,7 +408,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
       float mx;
       bool again = true;
-      if (j == 0 || tile_masked(key0)) {                // the reference is unknown, or the soft cap and the mask come first
+      if (SHORT || j == 0 || tile_masked(key0)) {       // the reference is unknown, or the soft cap and the mask come first
         if (capped || need_mask) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
@@ -482,32 +488,39 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       if (tc::mbar_wait_warp(tc::smem_u32(&bar_o_full[w]), 0u, abort)) {
         tc::fence_after_sync();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+        auto unit = [&](const uint32_t (&o)[32], int i) {  // eight of a row's values
+          return make_uint4(pack2<BF16>(__uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv),
+                            pack2<BF16>(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv),
+                            pack2<BF16>(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv),
+                            pack2<BF16>(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv));
+        };
         // The warp's 32 rows pass through its part of Q_w, whose last product has retired: a lane that wrote its own row
         // straight to global memory would touch 32 lines with every store (3600 cycles a block, 2300 this way).
         uint8_t* sO = sQ + w * kTile + quad * 32 * (D * 2);
         constexpr int kUnits = D / 8;                   // 16-byte units of a row; unit u of row r lies at u ^ (r & 7)
+        uint4* own = reinterpret_cast<uint4*>(prm.out + ((long long)b * S + row) * prm.out_ts + (long long)hq * D);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t ov[32];
           tc::tmem_ld_32x32(t_o + (uint32_t)(c * 32), ov);
           tc::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(sO + lane * (D * 2) + (((c * 4 + i) ^ (lane & 7)) << 4)) = make_uint4(
-                pack2<BF16>(__uint_as_float(ov[8 * i]) * inv, __uint_as_float(ov[8 * i + 1]) * inv),
-                pack2<BF16>(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv),
-                pack2<BF16>(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv),
-                pack2<BF16>(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv));
+          for (int i = 0; i < 4; ++i) {
+            if (!SHORT) *reinterpret_cast<uint4*>(sO + lane * (D * 2) + (((c * 4 + i) ^ (lane & 7)) << 4)) = unit(ov, i);
+            else if (row < S) own[c * 4 + i] = unit(ov, i);
+          }
         }
-        __syncwarp();
-        const int u = lane % kUnits, row0 = row - lane;
-        uint16_t* dst = prm.out + ((long long)b * S + row0) * prm.out_ts + (long long)hq * D + u * 8;
+        if constexpr (!SHORT) {
+          __syncwarp();
+          const int u = lane % kUnits, row0 = row - lane;
+          uint16_t* dst = prm.out + ((long long)b * S + row0) * prm.out_ts + (long long)hq * D + u * 8;
 #pragma unroll
-        for (int it = 0; it < kUnits; ++it) {
-          const int rr = it * (32 / kUnits) + lane / kUnits;
-          if (row0 + rr < S)
-            *reinterpret_cast<uint4*>(dst + rr * prm.out_ts) =
-                *reinterpret_cast<const uint4*>(sO + rr * (D * 2) + ((u ^ (rr & 7)) << 4));
+          for (int it = 0; it < kUnits; ++it) {
+            const int rr = it * (32 / kUnits) + lane / kUnits;
+            if (row0 + rr < S)
+              *reinterpret_cast<uint4*>(dst + rr * prm.out_ts) =
+                  *reinterpret_cast<const uint4*>(sO + rr * (D * 2) + ((u ^ (rr & 7)) << 4));
+          }
         }
       }
     }
@@ -558,10 +571,10 @@ int make_token_map(CUtensorMap* map, const void* base, int64_t B, int64_t S, int
   return LLMQRT_OK;
 }
 
-template <bool BF16, int D>
+template <bool BF16, int D, bool SHORT>
 int launch_prefill(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, PrefillParams prm, int64_t B,
                    cudaStream_t st) {
-  auto kern = attn_prefill_tc_kernel<BF16, D>;
+  auto kern = attn_prefill_tc_kernel<BF16, D, SHORT>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes<D>())) return rc;
   const uint32_t fmt = BF16 ? 1u : 0u;
   prm.idesc_s = tc::instr_desc(1, fmt, fmt, kRows, kRows);
@@ -605,7 +618,11 @@ extern "C" int llmqrt_attn_prefill(const void* q, int64_t q_token_stride, const 
   prm.out_ts = out_token_stride;
   prm.status = nullptr;
   const bool bf = dtype == LLMQRT_BF16;
-  if (d == 128) return bf ? launch_prefill<true, 128>(tq, tk, tv, prm, B, st) : launch_prefill<false, 128>(tq, tk, tv, prm, B, st);
-  return bf ? launch_prefill<true, 64>(tq, tk, tv, prm, B, st) : launch_prefill<false, 64>(tq, tk, tv, prm, B, st);
+  auto go = [&](auto shrt) {
+    constexpr bool kS = decltype(shrt)::value;
+    if (d == 128) return bf ? launch_prefill<true, 128, kS>(tq, tk, tv, prm, B, st) : launch_prefill<false, 128, kS>(tq, tk, tv, prm, B, st);
+    return bf ? launch_prefill<true, 64, kS>(tq, tk, tv, prm, B, st) : launch_prefill<false, 64, kS>(tq, tk, tv, prm, B, st);
+  };
+  return S <= kShortRows ? go(std::true_type()) : go(std::false_type());
 }
 

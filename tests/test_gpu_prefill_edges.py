@@ -71,3 +71,24 @@ def test_prefill_one_row_leaps(S, key, d, dt):
     # as above: P and the result rounded to 16 bits
     assert rel_fro(out[:, keep], want[:, keep]) < (1e-3 if dt == torch.float16 else 8e-3)
     assert rel_fro(out[:, leap], want[:, leap]) < (1e-3 if dt == torch.float16 else 8e-3)
+
+
+@pytest.mark.parametrize("S", [1, 17, 31, 32, 33, 40, 41])
+@pytest.mark.parametrize("d,dt", [(64, torch.bfloat16), (128, torch.float16)])
+@pytest.mark.parametrize("softcap", [0.0, 5.0])
+def test_prefill_short_sequences(S, d, dt, softcap):
+    """The form for short sequences and the general one, up to both sides of the line between them: a causal prompt's rows have
+    the bits of the same rows of a longer one (keys that a row does not see count as zeros)."""
+    from llmqrt_b200.attention import flash_attn_func
+    g = torch.Generator(device="cuda").manual_seed(S + d)
+    q, k, v = (torch.randn(3, 100, h, d, generator=g, device="cuda").to(dt) for h in (4, 2, 2))
+    whole = flash_attn_func(q, k, v, causal=True, softcap=softcap)
+    out = flash_attn_func(*(t[:, :S].contiguous() for t in (q, k, v)), causal=True, softcap=softcap)
+    assert torch.equal(out, whole[:, :S])
+    kk, vv = (t[:, :S].double().repeat_interleave(2, 2) for t in (k, v))
+    s = torch.einsum("bshd,bthd->bhst", q[:, :S].double(), kk) * d ** -0.5
+    if softcap:
+        s = softcap * (s / softcap).tanh()
+    want = torch.einsum("bhst,bthd->bshd", s.softmax(-1), vv)
+    out = flash_attn_func(*(t[:, :S].contiguous() for t in (q, k, v)), causal=False, softcap=softcap)
+    assert rel_fro(out, want) < (1e-3 if dt == torch.float16 else 8e-3)      # P and the result rounded to 16 bits
