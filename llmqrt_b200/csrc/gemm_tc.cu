@@ -431,7 +431,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
     tc::mbar_init(tc::smem_u32(&bar_reduce), 1);
     tc::mbar_init(tc::smem_u32(&bar_release), (uint32_t)S);
     tc::mbar_fence_init();
-    tc::tma_prefetch_descriptor(&tm_p);
+    tc::tma_prefetch_descriptor(AWQ ? &tm_w : &tm_p);
     tc::tma_prefetch_descriptor(&tm_q);
   }
   if (warp == 1) {
@@ -668,10 +668,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         pf_it -= kb_count;
         pf_tile += tile_step;
       }
+      pf_z = nullptr;
+      if (pf_tile >= num_tiles) return;                // (a split reduction of a few K blocks is soon past its only tile)
       const int tq = pf_tile % prm.tiles_q, tp = pf_tile / prm.tiles_q;
       pf_rot = (tp * 5 + tq * 3) % kb_count;           // the TMA producer's K rotation
       const int n = tp * kBM + rr;
-      pf_z = pf_tile < num_tiles && n < prm.N ? prm.awq_sz + (int64_t)n * prm.awq_kg : nullptr;
+      if (n < prm.N) pf_z = prm.awq_sz + (int64_t)n * prm.awq_kg;
     };
     uint32_t szv[kDepth][2];                           // {scale, -(1024 + zero)} of the row's two halves of 32 values
     auto fetch = [&](uint32_t (&z)[2]) {
