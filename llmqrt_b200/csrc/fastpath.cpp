@@ -660,18 +660,19 @@ FAST_FN(tensor_key) {
 
 PyObject* g_plain = nullptr;                           // ((class, attribute, the function it was defined with), ...)
 PyObject* g_hooks = nullptr;                           // the dictionaries of hooks on all modules
-PyTypeObject *g_norm = nullptr, *g_attn = nullptr, *g_mlp = nullptr, *g_linear = nullptr;
+PyTypeObject *g_norm = nullptr, *g_attn = nullptr, *g_mlp = nullptr, *g_linear = nullptr, *g_cache = nullptr;
 
-// (RMSNorm, QuantAttentionFused, FusedGateUpMLP, WQLinear_GEMM, plain, hooks)
+// (RMSNorm, QuantAttentionFused, FusedGateUpMLP, WQLinear_GEMM, WindowedCache, plain, hooks)
 FAST_FN(set_block_classes) {
-  FAST_BEGIN(6)
-  for (int i = 0; i < 6; ++i) Py_INCREF(a[i]);         // (for the life of the process)
+  FAST_BEGIN(7)
+  for (int i = 0; i < 7; ++i) Py_INCREF(a[i]);         // (for the life of the process)
   g_norm = reinterpret_cast<PyTypeObject*>(a[0]);
   g_attn = reinterpret_cast<PyTypeObject*>(a[1]);
   g_mlp = reinterpret_cast<PyTypeObject*>(a[2]);
   g_linear = reinterpret_cast<PyTypeObject*>(a[3]);
-  g_plain = a[4];
-  g_hooks = a[5];
+  g_cache = reinterpret_cast<PyTypeObject*>(a[4]);
+  g_plain = a[5];
+  g_hooks = a[6];
   Py_RETURN_NONE;
   FAST_END
 }
@@ -760,11 +761,20 @@ bool flag(PyObject* obj, PyObject* name) {
   return bool_arg(v.get());
 }
 
+// An object of exactly this class that has none of the class's functions replaced on itself.
+Fields plain_object(PyObject* o, PyTypeObject* cls) {
+  if (Py_TYPE(o) != cls) throw NotPlain();
+  Fields f(o);
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(g_plain); ++i) {
+    PyObject* p = PyTuple_GET_ITEM(g_plain, i);
+    if (PyTuple_GET_ITEM(p, 0) == reinterpret_cast<PyObject*>(cls) && f.find(PyTuple_GET_ITEM(p, 1))) throw NotPlain();
+  }
+  return f;
+}
+
 // A module whose call is its class's forward and nothing else.
 Fields plain_module(PyObject* m, PyTypeObject* cls, bool called = true) {
-  if (Py_TYPE(m) != cls) throw NotPlain();
-  Fields f(m);
-  if (f.find(NAME("forward"))) throw NotPlain();
+  Fields f = plain_object(m, cls);
   if (called) {
     PyObject* compiled = f.find(NAME("_compiled_call_impl"));
     if (!f.empty(NAME("_forward_hooks")) || !f.empty(NAME("_forward_pre_hooks")) || !f.empty(NAME("_backward_hooks")) ||
@@ -838,8 +848,8 @@ struct PlainNorm {
   float eps;
 };
 
-Tensor plain_cache(PyObject* o, PyObject* name, const Tensor& x) {
-  const Tensor t = Fields(o).tensor(name);
+Tensor plain_cache(const Fields& cache, PyObject* name, const Tensor& x) {
+  const Tensor t = cache.tensor(name);
   if (!t.defined() || t.dim() != 4 || t.scalar_type() != at::kHalf || t.device() != x.device() || t.stride(3) != 1 ||
       t.stride(2) != t.size(3) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16)
     throw NotPlain();
@@ -869,7 +879,7 @@ struct BlockStep {
     d = attn.integer(NAME("head_dim"));
     pos = attn.integer(NAME("start_pos"));
     softcap = (float)attn.number(NAME("attn_logit_softcapping"));
-    PyObject* cache = attn.get(NAME("cache"));
+    const Fields cache = plain_object(attn.get(NAME("cache")), g_cache);
     kc = plain_cache(cache, NAME("k"), x);
     vc = plain_cache(cache, NAME("v"), x);
     const Fields rope(attn.child(NAME("rope")));

@@ -12,6 +12,7 @@ from ..fused_utils import FusedGateUpMLP
 from ..linear import WQLinear_GEMM
 from ..linear import linear_base
 from .attn import QuantAttentionFused
+from .cache import WindowedCache
 from .norm import RMSNorm
 
 
@@ -87,11 +88,13 @@ class LlamaLikeModel(nn.Module):
         return self.norm(h)
 
 
-# What has to be as it was defined for the native step to stand for the modules' own code.
+# What has to be as it was defined for the native step to stand for the modules' own code, on the classes and on each object.
 fast.set_block_classes(
-    RMSNorm, QuantAttentionFused, FusedGateUpMLP, WQLinear_GEMM,
+    RMSNorm, QuantAttentionFused, FusedGateUpMLP, WQLinear_GEMM, WindowedCache,
     tuple((cls, name, getattr(cls, name)) for cls, names in
-          ((RMSNorm, ("forward", "add")), (QuantAttentionFused, ("forward",)), (FusedGateUpMLP, ("forward", "add_to", "_hidden")),
-           (WQLinear_GEMM, ("forward", "packed", "takes_tail", "silu_halves", "add_to"))) for name in names),
+          ((RMSNorm, ("__call__", "forward", "add")), (QuantAttentionFused, ("forward",)),
+           (FusedGateUpMLP, ("forward", "add_to", "_hidden")),
+           (WQLinear_GEMM, ("__call__", "forward", "packed", "takes_tail", "silu_halves", "add_to")), (WindowedCache, ("to",)))
+          for name in names),
     (linear_base._global_forward_hooks, linear_base._global_forward_pre_hooks, linear_base._global_backward_hooks,
      linear_base._global_backward_pre_hooks))

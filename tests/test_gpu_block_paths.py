@@ -227,3 +227,49 @@ def test_step_declines_what_it_does_not_cover():
     block.attn.q_norm = torch.nn.Identity()
     assert not takes(x)
     assert block.attn.start_pos == pos
+
+
+@pytest.mark.parametrize("on", ["instance", "class"])
+@pytest.mark.parametrize("owner,name", [
+    ("norm_2", "add"), ("mlp", "add_to"), ("mlp", "_hidden"), ("mlp.gate_up", "packed"), ("mlp.gate_up", "takes_tail"),
+    ("mlp.gate_up", "silu_halves"), ("mlp.down_proj", "add_to"), ("attn.o_proj", "packed"), ("norm_1", "__call__"),
+    ("attn.qkv_proj", "__call__"), ("attn.cache", "to")])
+def test_replaced_functions_are_called(owner, name, on):
+    """The native step stands for functions beside `forward` as well: whoever replaces one sees it called."""
+    import operator
+    block, x = _block(), torch.randn(1, 1, H, device="cuda").half()
+    want = _run(block, lambda b, t: b(t), x)
+    target, seen = operator.attrgetter(owner)(block), []
+    cls, own = type(target), name in vars(type(target))
+    function = getattr(cls, name)
+    if on == "instance" and name == "__call__":
+        pytest.skip("a call looks up its class")
+    if on == "instance":
+        setattr(target, name, lambda *a: (seen.append(name), function(target, *a))[1])
+    else:
+        setattr(cls, name, lambda self, *a: (seen.append(name) if self is target else None, function(self, *a))[1])
+    try:
+        assert torch.equal(_run(block, lambda b, t: b(t), x), want) and seen
+    finally:
+        if on == "instance":
+            delattr(target, name)
+        elif own:
+            setattr(cls, name, function)
+        else:
+            delattr(cls, name)
+    seen.clear()
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want) and not seen
+
+
+def test_a_cache_of_another_class_is_asked():
+    """A cache that converts itself on its own terms (as one that lives elsewhere would) does so before every step."""
+    block, x, seen = _block(), torch.randn(1, 1, H, device="cuda").half(), []
+    want = _run(block, lambda b, t: b(t), x)
+
+    class Cache(type(block.attn.cache)):
+        def to(self, like):
+            seen.append(like.shape)
+            super().to(like)
+
+    block.attn.cache.__class__ = Cache
+    assert torch.equal(_run(block, lambda b, t: b(t), x), want) and seen
