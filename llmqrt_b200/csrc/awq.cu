@@ -339,10 +339,10 @@ int llmqrt_awq_gemm(const void* x, int64_t ldx, const uint32_t* wq_t, const uint
   // tokens; the kernel that dequantizes its own tiles makes each of them again for every 256 tokens.  Expanded against fused
   // us at 256 / 512 / 1024 tokens: 17920 x 1536 26 / 34 / 53 (25 / 46 / 86), 4608 x 3584 22 / 23 / 32 (22 / 27 / 36), 3584 x 18944
   // 88 / 90 / 132 (58 / 96 / 119), 37888 x 3584 129 / 169 / 255 (68 / 132 / 269), 9728 x 896 15 / 19 / 24 (21 / 32 / 51).  The
-  // estimates choose; a twelfth in favour of the expansion is what they are off by.  (Panels of 64 MB, which would stay in L2, are
+  // estimates choose; a twentieth in favour of the expansion is what they are off by.  (Panels of 64 MB, which would stay in L2, are
   // worse: 113 us for 3584 x 18944 at 256.)  Above 1024 tokens it is always expanded.
   if (M > 128 && workspace && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % 8 == 0 &&
-      (M > 1024 || !awq_tc_faster(M, N, K, 0.92 * awq_expanded_us(M, N, K)))) {
+      (M > 1024 || !awq_tc_faster(M, N, K, 0.95 * awq_expanded_us(M, N, K)))) {
     const int64_t cap_rows = (int64_t)(LLMQRT_WS_PARTIAL_BYTES / (size_t)(K * 2)) / 256 * 256;
     if (cap_rows >= 256) {
       __half* deq = reinterpret_cast<__half*>(ws_partials(workspace));

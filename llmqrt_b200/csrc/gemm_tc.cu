@@ -927,7 +927,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
 //     of its seven K blocks at K = 896 (4096 x 4864 x 896 in int8 25.4 us, 23.2 this way).  (With one staging tile
 //     for all warps the completion of a store serialises the tiles.)
 constexpr int kPairBN = 256;
-constexpr int kPairNarrowBN = 128;      // where tiles of 256 columns leave most SMs idle: see pair_us
+constexpr int kPairNarrowBN = 128;      // where tiles of 256 columns leave most SMs idle: see dense_us
 template <int BN> constexpr int pair_stage_bytes() { return (kBM + BN / 2) * kRowBytes; }      // 32 or 24 KiB
 template <int BN> constexpr int pair_stages() { return BN == kPairBN ? 6 : 8; }
 constexpr int kPairOutBytes = 32 * 128;                                // staging tile of an epilogue warp
@@ -1329,34 +1329,51 @@ cudaLaunchConfig_t make_config(int grid, int cluster, cudaStream_t st, cudaLaunc
   return cfg;
 }
 
-// Estimated microseconds of the schedules for more than 128 tokens, fitted to times measured over N = 896 .. 37888,
-// K = 896 .. 18944 and M = 160 .. 4096 (within 10 % but for the smallest): all are bound by what one SM can fetch from L2
-// (about 105 GB/s), per K block of 128 bytes 32 KiB a CTA for a 128 x 128 tile in panels and for half of a 256 x 256 tile in
-// pairs, 24 KiB for half of a 256 x 128 tile.  The narrow pair's tiles cost more traffic and fill twice as many SMs: 333 x
-// 3584 x 3584 14.3 us in 28 wide pairs, 10.3 in 56 narrow ones (panels 15.1); 1024 x 1536 x 8960 25.9 and 17.5 (27.7); 512 x
-// 896 x 896 7.8 and 6.1; but 4096 x 4608 x 3584 42.9 and 51.0.  panel_us also picks the cluster size of the split (1 .. 8) where
-// `splits` asks for it; `active` says how many clusters of a size fit the device (without it: one CTA per SM).
-double pair_us(int64_t M, int64_t N, int k_blocks, bool* narrow) {
-  const int64_t rows = ceil_div(M, (int64_t)(2 * kBM)), clusters = sm_count() / 2;
-  const double wide_us = 4.57 + (double)ceil_div(rows * ceil_div(N, (int64_t)kPairBN), clusters) * (0.286 * k_blocks + 1.59);
-  const double narrow_us = 3.56 + (double)ceil_div(rows * ceil_div(N, (int64_t)kPairNarrowBN), clusters) * (0.160 * k_blocks + 1.59);
-  if (narrow) *narrow = 1.03 * narrow_us < wide_us;
-  return 1.03 * narrow_us < wide_us ? narrow_us : wide_us;
-}
-double panel_us(int64_t tiles, int k_blocks, int* splits, const int* active = nullptr) {
+// In how many CTAs a cluster of the panels' kernel shares a reduction (1 .. 8); `active` says how many clusters of a size fit
+// the device (without it: one CTA per SM).
+int panel_splits(int64_t tiles, int k_blocks, const int* active = nullptr) {
   const int sms = sm_count();
   double best = 5.2 + (double)ceil_div(tiles, sms) * (0.306 * k_blocks + 1.7);
-  if (splits) *splits = 1;
+  int splits = 1;
   for (int s = 2; s <= kMaxCluster && k_blocks >= 2 * s && tiles < sms; ++s) {
     const int n = active ? active[s] : sms / s;
     if (n <= 0) continue;
     const double t = 5.2 + (double)ceil_div(tiles, n) * (0.306 * k_blocks / s + 5.2);
-    if (t < best) {
-      best = t;
-      if (splits) *splits = s;
-    }
+    if (t < best) { best = t; splits = s; }
   }
-  return best;
+  return splits;
+}
+
+// Estimated microseconds of the three schedules for more than 128 tokens: tiles of 256 x 256 or 256 x 128 on pairs of CTAs, and
+// panels of 128 tokens with a split reduction.  All are bound by what an SM fetches from L2 for a K block of 128 bytes: 32 KiB
+// for half of a wide tile, 24 for half of a narrow one, 32 for a panel's.  A row of a box that does not begin on a line takes
+// two (operands whose row pitch is no multiple of 128 bytes), and a fifth sector where it does not begin on a sector either
+// (of 32): 271 x 336 x 5392 takes 16.5 us in narrow tiles, 11.8 in panels.  A schedule that fills few SMs has more of L2 to
+// itself: `fill`.  Fitted to 860 sizes, M = 129 .. 4096, N = 136 .. 37888, K = 256 .. 18944, three types, each timed in all
+// three: the median error is 3 %, the choice 0.2 % off the best on average.
+// us, wide / narrow / panels: 333 x 3584 x 3584 14.3 / 10.3 / 15.1, 161 x 152 x 5760 17 / 10.9 / 9.8, 219 x 2016 x 5840 22.9 / 17.8 /
+// 15.8, 1600 x 5856 x 9824 75.7 / 83.5, 154 x 18944 x 3584 (in fp8) 18.1 / 18.3 / 25.9.
+enum DenseSchedule { DENSE_WIDE, DENSE_NARROW, DENSE_PANELS };
+double dense_us(int64_t M, int64_t N, int k_blocks, int64_t pitch, DenseSchedule* which) {
+  static const double extra[3][3] = {{0., 0., 0.}, {0.004, 0.025, 0.027}, {0.097, 0.122, 0.103}};
+  const double* x = extra[pitch % 128 == 0 ? 0 : pitch % 32 == 0 ? 1 : 2];
+  const int64_t rows = ceil_div(M, (int64_t)(2 * kBM)), sms = sm_count(), clusters = sms / 2;
+  const int64_t wide = rows * ceil_div(N, (int64_t)kPairBN), narrow = rows * ceil_div(N, (int64_t)kPairNarrowBN);
+  const double wfill = std::min(1., (double)wide / clusters), nfill = std::min(1., (double)narrow / clusters);
+  const double w = 4.25 + 1.65 * wfill + (double)ceil_div(wide, clusters) * (0.94 + k_blocks * (0.284 + 0.02 * wfill + x[0]));
+  const double n = 2.9 + 1.12 * nfill + (double)ceil_div(narrow, clusters) * (1.45 + k_blocks * (0.162 + x[1]));
+  DenseSchedule best = 1.03 * n < w ? DENSE_NARROW : DENSE_WIDE;
+  double us = best == DENSE_NARROW ? n : w;
+  if (M <= 1024) {
+    const int64_t tiles = ceil_div(M, (int64_t)kBM) * ceil_div(N, (int64_t)kBM);
+    const int s = panel_splits(tiles, k_blocks);
+    const double fill = std::min(1., (double)tiles * s / sms), kb = (double)k_blocks / s;
+    const double p = 3.15 + 1.7 * fill + (double)ceil_div(tiles, sms / s) *
+                     (3. + kb * (0.32 - 0.056 * fill + x[2]) + (s > 1 ? 1. + 3.2 * fill : 0.));
+    if (1.02 * p < us) { best = DENSE_PANELS; us = p; }
+  }
+  if (which) *which = best;
+  return us;
 }
 
 // How many clusters of [1 .. kMaxCluster] CTAs of this kernel can be resident at once, asked once per device.  (Small calls are
@@ -1410,7 +1427,7 @@ int launch(const CUtensorMap& tm_p, const CUtensorMap& tm_q, const CUtensorMap& 
   const int tiles = prm.tiles_p * prm.tiles_q;
   int splits = 1;
   if (BN <= 128 && tiles < sms) {
-    if (prm.tiles_q > 1 && !AWQ) panel_us(tiles, prm.k_blocks, &splits, active_clusters<KIND, BN, AWQ, PUSH>());
+    if (prm.tiles_q > 1 && !AWQ) splits = panel_splits(tiles, prm.k_blocks, active_clusters<KIND, BN, AWQ, PUSH>());
     else splits = pick_splits(tiles, prm.k_blocks, BN / 8, active_clusters<KIND, BN, AWQ, PUSH>(), nullptr);
   }
   prm.splits = splits;
@@ -1542,9 +1559,7 @@ bool awq_tc_faster(int64_t M, int64_t N, int64_t K, double than) {
 }
 
 double awq_expanded_us(int64_t M, int64_t N, int64_t K) {
-  const int kb = (int)ceil_div(K, (int64_t)64);
-  const double g = pair_us(M, N, kb, nullptr), p = 1.03 * panel_us(ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM), kb, nullptr);
-  return 1.0 + (p < g ? p : g) + 0.518e-6 * (double)(N * K);
+  return 1.0 + dense_us(M, N, (int)ceil_div(K, (int64_t)64), 2 * K, nullptr) + 0.518e-6 * (double)(N * K);
 }
 
 int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, int64_t M, int64_t N, int64_t K,
@@ -1564,10 +1579,9 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   LLMQRT_REQUIRE((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0,
                  "tcgen05 gemm: operands must be 16-byte aligned");
 
-  // More than 128 tokens: the two-CTA kernel wherever its vector stores may be used (16-byte aligned output rows),
+  // More than 128 tokens: the two-CTA kernel wherever its output tiles may leave by TMA (16-byte aligned output rows),
   // unless the small-M schedule -- weights as the 128-lane operand, tokens in panels of 128 as the column operand,
-  // cluster split-K -- is estimated to be faster, as it is where few tiles meet a long reduction
-  // (M = 160: N = 896, K = 8960 12.8 us in panels, 15.0 in narrow pairs; N = K = 3584 15.1 against 9.9).
+  // cluster split-K -- is estimated to be faster, as it is where few tiles meet a long reduction (see dense_us).
   // The 128 x 256 tiles of a lone CTA feed 48 KiB per K block through one SM's share of L2 (28 us at
   // M = 160 .. 640, N = K = 3584): they are left to the outputs that neither can serve.
   const int es = (epi.mode == EPI_RAW || epi.out_dtype == LLMQRT_F32) ? 4 : 2;
@@ -1575,16 +1589,14 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   const int k_blocks = (int)ceil_div(K * elt, kRowBytes);
   const bool pair_ok = !awq && !push && M > 128 && N > 128 && out_ok && pair_enabled();
   bool panels = false, narrow = false;
-  const double pairs_us = pair_ok ? pair_us(M, N, k_blocks, &narrow) : 0.;
-  if (M > 128 && M <= 1024) {
-    const int64_t panel_tiles = ceil_div(M, (int64_t)128) * ceil_div(N, (int64_t)kBM);
-    if (pair_ok) {
-      panels = 1.03 * panel_us(panel_tiles, k_blocks, nullptr) < pairs_us;
-    } else if (awq) {
-      awq_tc_us(M, N, K, &panels);
-    } else {
-      panels = true;
-    }
+  if (pair_ok) {
+    DenseSchedule which;
+    dense_us(M, N, k_blocks, (lda | ldw) * elt, &which);
+    panels = which == DENSE_PANELS;
+    narrow = which == DENSE_NARROW;
+  } else if (M > 128 && M <= 1024) {
+    if (awq) awq_tc_us(M, N, K, &panels);
+    else panels = true;
   }
 
   TcParams prm{};

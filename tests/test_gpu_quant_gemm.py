@@ -370,3 +370,14 @@ def test_per_tensor_quantizers_of_every_size(ops, M, K, dt):
     s = x.abs().amax().clamp(min=1e-12).div(448)
     q, scale = ops.quantize_fp8(x, per_token=False)[:2]
     assert torch.equal(q.view(torch.uint8), (x / s).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8))
+
+
+@pytest.mark.parametrize("M,N,K", [(161, 152, 5760), (271, 336, 5392), (219, 2016, 5840), (153, 424, 3792), (333, 1000, 2064),
+                                   (260, 264, 272), (1025, 1304, 1040), (1600, 2056, 656)])
+def test_schedules_by_row_pitch(ops, M, N, K):
+    """More than 128 tokens, rows that begin on a line, on a sector or on neither, few tiles with a long reduction and many with
+    a short one: whichever schedule is chosen, the sums are exact."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    assert torch.equal(ops.int8_gemm_s32(a, w), (a.double() @ w.double().t()).to(torch.int32))
