@@ -381,3 +381,36 @@ def test_schedules_by_row_pitch(ops, M, N, K):
     a = torch.randint(-128, 128, (M, K), generator=g, device="cuda", dtype=torch.int8)
     w = torch.randint(-128, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
     assert torch.equal(ops.int8_gemm_s32(a, w), (a.double() @ w.double().t()).to(torch.int32))
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 160, 64), (257, 288, 896), (300, 1056, 3584), (333, 3584, 1040), (200, 9728, 128),
+                                   (1300, 2464, 240)])
+@pytest.mark.parametrize("kind", ["s32", "f16", "f8"])
+def test_two_cta_rows_from_registers(ops, M, N, K, kind):
+    """The two-CTA kernel's other way out, rows of whole sectors written by the epilogue's threads, with one tile a cluster and
+    with more: results to the last row and column, and not a byte beyond them."""
+    from llmqrt_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randint(-8, 8, (M, K), generator=g, device="cuda", dtype=torch.int8)
+    w = torch.randint(-8, 8, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    acc = a.double() @ w.double().t()                       # whole numbers below 2^24: exact in every type's sums
+    xs = torch.rand(M, generator=g, device="cuda") + 0.5
+    ws = (torch.rand(N, generator=g, device="cuda") + 0.5) * 1e-3
+    ld, dev = N + 32, a.device
+    dt = {"s32": torch.int32, "f16": torch.float16, "f8": torch.bfloat16}[kind]
+    buf = torch.full((M + 40, ld), 77, dtype=dt, device="cuda")
+    ws_ptr, stream = L.ptr(L.workspace(dev)), L.stream(dev)
+    if kind == "s32":
+        L.call("llmqrt_w8a8_int8_gemm_s32", L.ptr(a), K, L.ptr(w), K, L.ptr(buf), ld, M, N, K, ws_ptr, stream, 0)
+        want = acc.to(torch.int32)
+    elif kind == "f16":
+        L.call("llmqrt_w8a8_int8_linear_per_channel", L.ptr(a), K, L.ptr(w), K, None, L.F16, L.ptr(xs), L.ptr(ws), L.ptr(buf),
+               L.F16, ld, M, N, K, ws_ptr, stream, 0)
+        want = ((acc.float() * ws) * xs[:, None]).half()
+    else:
+        a8, w8 = a.to(torch.float8_e4m3fn), w.to(torch.float8_e4m3fn)      # (-8 .. 8 are e4m3 numbers)
+        L.call("llmqrt_f8f8bf16_rowwise", L.ptr(a8), L.dtype_code(a8.dtype), K, L.ptr(w8), K, None, L.BF16, L.ptr(xs), L.ptr(ws),
+               L.ptr(buf), ld, M, N, K, ws_ptr, stream, 0)
+        want = ((acc.float() * xs[:, None]) * ws).bfloat16()
+    assert torch.equal(buf[:M, :N], want)
+    assert bool((buf[:M, N:] == 77).all()) and bool((buf[M:] == 77).all())
