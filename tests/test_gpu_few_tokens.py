@@ -129,3 +129,26 @@ def test_awq_tensor_memory_tiles(M, K, N, G):
     y = ops.awq_gemm(x, packed, bias)
     assert rel_fro(y, want) < 5e-4                          # the fp16 rounding of the result
     assert torch.equal(y, ops.awq_gemm(x, packed, bias))    # one order of the sums
+
+
+@pytest.mark.parametrize("M,K,N,G,scratch", [
+    (160, 1536, 17920, 128, True), (256, 1536, 17920, 64, True), (512, 3584, 37888, 128, True), (1000, 18944, 3584, 128, True),
+    (1100, 1056, 264, 96, False), (1030, 160, 4104, 32, False), (1537, 32, 2056, 32, False)])
+def test_awq_token_tiles(M, K, N, G, scratch):
+    """The tiles of 256 tokens of the kernel that dequantizes into tensor memory (one accumulator, a ring of five): layers well
+    inside their range, and, as a call without scratch cannot expand its weights, small odd ones with several token tiles,
+    with more tiles than SMs, and with a single K block."""
+    from llmqrt_b200 import _lib as L
+    from llmqrt_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    qz = torch.randint(-2 ** 31, 2 ** 31 - 1, (K // G, N // 8), generator=g, device="cuda", dtype=torch.int32)
+    sc = torch.rand(K // G, N, generator=g, device="cuda").mul_(0.02).half()
+    x, bias = torch.randn(M, K, generator=g, device="cuda").half(), torch.randn(N, generator=g, device="cuda").half()
+    want = x.double() @ ops.awq_dequantize(qw, sc, qz).double() + bias.double()
+    p, y = ops.AwqPacked(qw, sc, qz), torch.full((M + 1, N), 7.0, dtype=torch.float16, device="cuda")
+    for _ in range(2):
+        L.call("llmqrt_awq_gemm", L.ptr(x), K, L.ptr(p.wq_t), L.ptr(p.sz_t), L.ptr(bias), L.ptr(y), N, M, N, K, G,
+               L.ptr(L.workspace(x.device)) if scratch else None, L.stream(x.device))
+        assert rel_fro(y[:M], want) < 5e-4                  # the fp16 rounding of the result
+        assert bool((y[M] == 7.0).all())
