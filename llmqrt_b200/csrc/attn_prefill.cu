@@ -34,7 +34,7 @@
 // ordered heaviest first over all heads.  4 x 2048 causal tokens, 28 / 4 heads of 128: 194 -> 180 us; with each product's
 // MMAs issued back to back and the tiles waited for ahead of P, 167 us a pass.  The row's maximum is found in the shadow of
 // the first half's exponentials, which are done again where the reference had to move, and the output leaves through shared
-// memory: 151 us (16 x 512 tokens: 89 -> 77; 1 x 4096, not causal: 276 -> 262).  At 4 x 2048 the board's 1000 W bound it then
+// memory: 155 to 157 us (in a graph 154 -> 139; so also 16 x 512 tokens 87 -> 75, 1 x 4096 tokens, not causal, 262 -> 247).  At 4 x 2048 the board's 1000 W bound it then
 // (1.65 to 1.8 GHz), so that every instruction saved counts twice; with a quarter of the exponentials as polynomials on the
 // multiply-add pipe it was 1 % slower.
 //
@@ -214,7 +214,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
 
-  // Register budget per warpgroup (8 x 216 + 4 x 72 registers per lane fit the SM's file): each role
+  // Register budget per warpgroup (8 x 200 + 4 x 104 registers a lane are the 12 x 168 of the launch): each role
   // branch starts by shrinking or growing its warpgroup's share.
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");

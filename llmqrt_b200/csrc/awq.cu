@@ -13,8 +13,9 @@
 // subtraction is exact and the product is rounded once, like the reference's kernels.
 //
 // The GEMM has three forms: a weight-streaming kernel of warp-level MMAs for few tokens (below), the TMA + tcgen05
-// GEMM with the weight operand dequantized tile by tile into shared memory by extra warps (gemm_tc.cu) up to 128
-// tokens, and above that the expansion of the weights, panel by panel, ahead of the dense tcgen05 GEMM.
+// GEMM with the weight operand dequantized tile by tile into tensor memory by extra warps (gemm_tc.cu), and, above 128
+// tokens where that is estimated to be faster and always above 1024, the expansion of the weights, panel by panel, ahead of
+// the dense tcgen05 GEMM.
 #include "gemm_w8a8.cuh"
 
 namespace llmqrt {
@@ -127,10 +128,10 @@ int launch_dequantize_t(const uint32_t* wq_t, const uint32_t* sz_t, int64_t K, i
 // one or two chunks of a warp are in flight together, and 64 registers a thread keep two 512-thread blocks on an SM.
 // Bound by latency where a layer is small, by the instructions of the dequantization where it is large: 37888 x 3584 at one
 // token (11 us of HBM time) issued 39 instructions a packed word, a third of them the division by the group size, in 28.7 us;
-// with a shift in its place and two of a word's four pairs sharing one it takes 26.  us from HBM at 1 / 8 / 16 tokens, before
-// in brackets: 17920 x 1536 7.7 / 8.0 / 11.3 (8.2 / 9.8 / 14.0), 1536 x 8960 7.1 / 7.3 / 10.2 (7.6 / 7.8 / 11.1), 8192 x 4096
-// 9.2 / 10.1 / 14.9 (11.7 / 12.5 / 17.2), 2048 x 1536 2.4 / 2.5 / 3.1 (2.5 / 2.7 / 3.2), 3584 x 18944 18.5 / 18.7 / 27.5
-// (19.8 / 20.6 / 30).  (Chunks fetched in a ring instead of in twos do not fit 64 registers: 17920 x 1536 9.5 us.)
+// with a shift in its place and two of a word's four pairs sharing one it takes 26.  us a kernel in a graph, weights from HBM, at
+// 1 / 8 / 16 tokens, before in brackets: 17920 x 1536 7.6 / 8.0 / 11.5 (8.1 / 9.9 / 14.1), 1536 x 8960 7.1 / 7.3 / 10.5 (8.2 / 8.3 /
+// 11.8), 8192 x 4096 9.2 / 10.1 / 14.9 (11.8 / 12.6 / 17.2), 2048 x 1536 2.7 / 2.8 / 3.4 (2.8 / 2.9 / 3.5), 37888 x 3584 25.9 / 26.2 /
+// 43 (29.5 / 30.6 / 45.5).  A call on its own is bound by the host and takes 8.2 us for the first, then as before.  (Chunks fetched in a ring instead of in twos do not fit 64 registers: 17920 x 1536 9.5 us.)
 constexpr int kChunkK = 128;           // k-values per warp step: 4 lanes x 32 per weight row
 //
 // What follows the GEMM in a decoder block may be done on its sums (each step rounded to fp16 as the separate kernels
@@ -157,8 +158,8 @@ awq_gemm_rows_kernel(const __half* __restrict__ X, int64_t ldx, const uint32_t* 
     zp[r] = sz_t + row * KG;
   }
   const __half* xp = X + (int64_t)g * ldx + 32 * t;
-  // (16 tokens: one chunk ahead, so that 64 registers nearly do -- 8 to 16 bytes are spilled; 17920 x 1536 13.9 us, 16.4
-  // with two)
+  // (16 tokens: one chunk ahead, so that 64 registers nearly do -- 8 to 16 bytes are spilled; two were a sixth slower at
+  // 17920 x 1536)
   constexpr int kRowsAhead = MB == 2 ? 1 : 2;
   float acc[MB][4];
 #pragma unroll

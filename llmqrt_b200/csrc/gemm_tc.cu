@@ -71,7 +71,6 @@ struct TcParams {
   // AWQ mode: the weight operand is not fetched by TMA but produced in tensor memory by sixteen extra
   // warps from the packed 4-bit layer (wq_t [N, K/8] words of eight K-consecutive values, sz_t
   // [N, K/G] half2 {scale, -(1024 + zero)}, see awq.cu)
-  const uint32_t* awq_w;
   const uint32_t* awq_sz;
   int awq_kw, awq_kg, awq_gw;      // K / 8, K / G, G / 8
   int awq_gshift;                  // log2(G / 8), or -1 if that is no whole number
@@ -378,7 +377,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
   constexpr int kRingBytes = AWQ ? awq_ring_bytes<BN>() : kStages * kStageBytes;
   constexpr int kAct = awq_act_stages<BN>(), kPk = kAwqPk;      // AWQ: the two rings
   constexpr int kAccBufs = acc_buffers<BN, AWQ>();
-  constexpr uint32_t kTmemCols = AWQ ? 512 : tmem_cols<BN>();
+  constexpr uint32_t kTmemCols = AWQ ? 512 : tmem_cols<BN>();   // (AWQ: its registers leave no other block that allocates any on the SM)
   static_assert(!AWQ || kAccBufs * BN + awq_act_stages<BN>() * kAwqWtCols <= 512, "tensor memory has 512 columns");
   constexpr int kBurst = kStages >= 8 ? 4 : (kStages >= 4 ? 2 : 1);  static_assert(BN > 128 || kRingBytes >= (2 * BN + 64) * kBM * 4, "ring too small for the reduce buffers");
   static_assert(kStages >= 3, "pipeline too shallow");
@@ -913,8 +912,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
 
 
 // ---- two-CTA kernel for prefill-sized problems -------------------------------------------------
-// Tokens are the 128-lane operand.  The two CTAs of a cluster compute one 256 x 256 output tile with
-// tcgen05.mma.cta_group::2 (M = 256, N = 256): each CTA stages ITS 128 token rows and ITS 128 of the
+// Tokens are the 128-lane operand.  The two CTAs of a cluster compute one 256 x 256 (or 256 x 128) output tile with
+// tcgen05.mma.cta_group::2 (M = 256, N = 256; the figures are for that width): each CTA stages ITS 128 token rows and ITS 128 of the
 // tile's 256 weight rows, 32 KiB per K block of 128 bytes instead of the 48 KiB a lone CTA needs for a
 // 128 x 256 tile, and each MMA reads 8 KiB instead of 12 KiB of a CTA's shared memory per 128 x 256 x 32
 // multiply -- the shared-memory operand feed, not the tensor pipe, is what bounds the single-CTA form.
@@ -924,8 +923,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
 //   epilogue (warps 2-9, both CTAs): TMEM -> registers -> scales / bias -> a staging tile of the warp's own, 32 rows of
 //     128 bytes, which leaves by a TMA store (rows and columns beyond the matrix are clipped).  A thread that writes its
 //     own row straight from registers makes the warp touch 32 lines with every store: 5130 cycles a tile, against 3584
-//     of its seven K blocks at K = 896 (4096 x 4864 x 896 in int8 25.4 us, 23.2 this way).  (With one staging tile
-//     for all warps the completion of a store serialises the tiles.)
+//     of its seven K blocks at K = 896 (4096 x 4864 x 896 in int8 24.6 us, 22.6 this way).  (With one staging tile
+//     for all warps the completion of a store serialises the tiles.)  Where nothing covers a store it is the faster way
+//     all the same: DIRECT, see launch_pair_bn.
 constexpr int kPairBN = 256;
 constexpr int kPairNarrowBN = 128;      // where tiles of 256 columns leave most SMs idle: see dense_us
 template <int BN> constexpr int pair_stage_bytes() { return (kBM + BN / 2) * kRowBytes; }      // 32 or 24 KiB
@@ -1025,7 +1025,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   pdl_wait();
   pdl_trigger();
 
-  const int num_tiles = prm.tiles_p * prm.tiles_q;     // in units of 256 x 256
+  const int num_tiles = prm.tiles_p * prm.tiles_q;     // in units of 256 x BN
   const int first_tile = (int)(blockIdx.x >> 1), tile_step = (int)(gridDim.x >> 1);
   const int kb_count = prm.k_blocks;
 
@@ -1594,7 +1594,7 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
             const Epilogue& epi, void* workspace, cudaStream_t st, bool static_w, const AwqOperand* awq,
             const CommPush* push) {
   const int elt = (kind == KIND_F16 || kind == KIND_BF16) ? 2 : 1;
-  if (awq) {                                           // W is produced in shared memory from the packed layer
+  if (awq) {                                           // W is produced in tensor memory from the packed layer
     LLMQRT_REQUIRE(kind == KIND_F16 && awq->wq_t && awq->sz_t && awq->G > 0 && K % 32 == 0 && K % awq->G == 0 &&
                    awq->G % 32 == 0 && (reinterpret_cast<uintptr_t>(awq->wq_t) & 15) == 0,
                    "tcgen05 awq gemm: fp16 activations, K and group size multiples of 32, 16-byte aligned packed weights");
@@ -1698,7 +1698,6 @@ int gemm_tc(int kind, const void* A, int64_t lda, const void* W, int64_t ldw, in
   if (int rc = make_operand_map(&tm_q, q_base, elt, prm.rows_q, K, prm.swap ? lda : ldw, bn)) return rc;
 
   if (awq) {
-    prm.awq_w = awq->wq_t;
     prm.awq_sz = awq->sz_t;
     prm.awq_kw = (int)(K / 8);
     prm.awq_kg = (int)(K / awq->G);

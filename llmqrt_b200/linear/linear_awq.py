@@ -3,8 +3,9 @@
 Name, constructor arguments, buffer names / shapes / dtypes and `from_linear` follow
 runtime/nn_models/modules/linear/linear_awq.py:78-267, so AWQ checkpoints load unchanged.  On the
 first forward after the buffers change, the layer is repacked once into the K-major streaming layout
-the CUDA kernels read; decode-sized inputs then stream the 4-bit weights directly, larger inputs
-dequantize once and use the tcgen05 fp16 GEMM.
+the CUDA kernels read.  Few tokens then stream the 4-bit weights through warp-level MMAs, more of them
+take the tcgen05 GEMM that dequantizes its own tiles, and prompts expand the layer panel by panel ahead of
+the dense tcgen05 GEMM.
 """
 from __future__ import annotations
 

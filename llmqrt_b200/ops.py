@@ -210,6 +210,6 @@ def awq_dequantize_t(packed: AwqPacked) -> torch.Tensor:
 
 def awq_gemm(x: torch.Tensor, packed: AwqPacked, bias=None) -> torch.Tensor:
     """C[M, N] fp16 = x[M, K] fp16 @ dequant(W) (+ bias): a weight-streaming mma.sync kernel up to 16 tokens (32 for narrow
-    layers), the tcgen05 GEMM with in-kernel dequantization up to 128, above that the weights expanded into the
-    workspace and multiplied by the dense kernel."""
+    layers), the tcgen05 GEMM with in-kernel dequantization up to 128, above that it or (always above 1024) the weights
+    expanded into the workspace and multiplied by the dense kernel, by estimate."""
     return L.fast.awq_linear(_rows(x), packed.wq_t, packed.sz_t, bias, packed.K, packed.N, packed.G)
